@@ -169,9 +169,28 @@ int pairs_error_flag(void* ws, size_t ws_bytes, uint64_t m, unsigned int* flag, 
 // d_out_* in partition order, d_offsets (2^radix_bits + 1, optional) the
 // partition starts; rows are row_base + input index
 size_t partition_ws_bytes(uint64_t m, uint32_t radix_bits, int sm_count);
+// The way back from a partitioned relation to probe order, left by a
+// partition pass that is given one (it then writes no row ids): every key's
+// offset inside its tile, and per tile and partition where the run went.
+struct partition_inverse {
+    uint16_t* offsets;  // m, in relation order
+    uint32_t* delta;    // tiles x fanout
+    uint16_t* start;    // tiles x fanout
+};
+// room for one of m probes inside ws; false when ws is too small for it
+bool carve_partition_inverse(void* ws, size_t ws_bytes, uint64_t m, uint32_t radix_bits, int sm_count,
+                             partition_inverse* out);
+// d_out[row] = value of the probe of that row, for values in relation order:
+// entry d of the relation has its value at d_values[value_index(d)]
+constexpr uint32_t kValueTile = 2048;
+__host__ __device__ inline uint64_t value_index(uint32_t d) {
+    return (uint64_t)(d / kValueTile) * (2 * kValueTile) + d % kValueTile;
+}
+int gather_values(const uint32_t* d_values, uint64_t m, uint32_t radix_bits, const partition_inverse& iv,
+                  uint32_t* d_out, cudaStream_t s);
 int range_partition_impl(const uint64_t* d_keys, uint64_t m, uint64_t min_key, uint32_t shift, uint32_t radix_bits,
                          uint64_t row_base, uint64_t* d_out_keys, uint32_t* d_out_rows, uint64_t* d_offsets, void* ws,
-                         size_t ws_bytes, cudaStream_t s);
+                         size_t ws_bytes, cudaStream_t s, const partition_inverse* inverse = nullptr);
 // fanout for an index of n keys (about 2^21 keys a partition, 2^5..2^12)
 uint32_t default_radix_bits(uint64_t n);
 // smallest shift that maps [min_key, max_key] onto 2^radix_bits partitions

@@ -131,6 +131,20 @@ __device__ __forceinline__ void block_exclusive_scan(const uint32_t* in, uint32_
         }
 }
 
+// Where tile t of the relation's runs went: the j-th key of the tile in
+// partition order lies at relation index delta[p] + j (modulo 2^32: m is below
+// it), p being the partition whose run [start[p], start[p + 1]) holds j.
+// Tiles are numbered block by block, every block's share rounded up to whole
+// tiles.
+__device__ __forceinline__ uint64_t tile_number(uint64_t t0, uint64_t b0, uint64_t chunk, uint32_t tile) {
+    return blockIdx.x * ((chunk + tile - 1) / tile) + (t0 - b0) / tile;
+}
+__device__ __forceinline__ void leave_run(const partition_inverse& iv, uint64_t tile, uint32_t fanout, uint32_t p,
+                                          uint64_t delta, uint32_t start) {
+    iv.delta[tile * fanout + p] = (uint32_t)delta;
+    iv.start[tile * fanout + p] = (uint16_t)start;
+}
+
 // Scatter block b's chunk.  The flat (partition, block) order of the scanned
 // histogram makes the start of cell c the inclusive sum of cell c - 1, so the
 // keys are read once.  Each tile of kScatterTile keys is first grouped by
@@ -141,11 +155,16 @@ __device__ __forceinline__ void block_exclusive_scan(const uint32_t* in, uint32_
 // the block and tile order; inside a tile it is not fixed.
 // kScatterPerSM resident blocks (the register cap; about 52 KB of shared
 // memory per 512-thread block for fanouts up to 2^8)
+//
+// kInverse: instead of row ids the relation gets each key's offset inside its
+// tile (16 bits), and the tile leaves where its runs went (iv): what
+// k_part_gather needs to bring results back to probe order.
+template <bool kInverse>
 __global__ void __launch_bounds__(kScatterBlock, kScatterPerSM) k_part_scatter(const uint64_t* __restrict__ keys, uint64_t m,
                                                              uint64_t chunk, uint64_t min_key, uint32_t shift,
                                                              uint32_t fanout, const uint64_t* __restrict__ incl,
                                                              uint64_t row_base, uint64_t* __restrict__ out_keys,
-                                                             uint32_t* __restrict__ out_rows) {
+                                                             uint32_t* __restrict__ out_rows, partition_inverse iv) {
     extern __shared__ unsigned long long s_mem[];
     uint64_t* s_keys = reinterpret_cast<uint64_t*>(s_mem);                       // kScatterTile
     unsigned long long* s_dst = s_mem + kScatterTile;                            // fanout: next output slot
@@ -186,17 +205,21 @@ __global__ void __launch_bounds__(kScatterBlock, kScatterPerSM) k_part_scatter(c
             if (j < tn) {
                 const uint32_t q = s_start[slot[k] >> 13] + (slot[k] & ((1u << 13) - 1));
                 s_keys[q] = key[k];
-                s_rows[q] = (uint32_t)(row_base + t0 + j);
+                s_rows[q] = kInverse ? j : (uint32_t)(row_base + t0 + j);
             }
         }
         // output index of the tile's j-th sorted key = s_delta[p] + j
-        for (uint32_t p = threadIdx.x; p < fanout; p += blockDim.x) s_delta[p] = s_dst[p] - s_start[p];
+        for (uint32_t p = threadIdx.x; p < fanout; p += blockDim.x) {
+            s_delta[p] = s_dst[p] - s_start[p];
+            if constexpr (kInverse) leave_run(iv, tile_number(t0, b0, chunk, kScatterTile), fanout, p, s_delta[p], s_start[p]);
+        }
         __syncthreads();
         for (uint32_t j = threadIdx.x; j < tn; j += kScatterBlock) {
             const uint64_t k = s_keys[j];
             const uint64_t d = s_delta[part_of(k, min_key, shift, fanout)] + j;
             __stcg(reinterpret_cast<unsigned long long*>(out_keys) + d, (unsigned long long)k);
-            __stcg(out_rows + d, s_rows[j]);
+            if constexpr (kInverse) iv.offsets[d] = (uint16_t)s_rows[j];
+            else __stcg(out_rows + d, s_rows[j]);
         }
         __syncthreads();
         for (uint32_t p = threadIdx.x; p < fanout; p += blockDim.x) s_dst[p] += s_cnt[p];
@@ -221,12 +244,6 @@ size_t scatter_smem_bytes(uint32_t fanout) {
 #define GJ_WIDE_RADIX_BITS 8
 #endif
 constexpr uint32_t kWideRadixBits = GJ_WIDE_RADIX_BITS;
-// the sorted tile keeps each key's partition beside its offset (one 32-bit
-// word), so the write pass reads it instead of recomputing it from the key
-// (1); GJ_SCATTER_META=0 recomputes it
-#ifndef GJ_SCATTER_META
-#define GJ_SCATTER_META 1
-#endif
 // block size, resident blocks per SM and the register prefetch of the next
 // tile (one 1024-thread block with the prefetch measured fastest: 10.63 ms
 // per partitioned step of 2^29 probes, against 11.71 for two 1024-thread
@@ -247,22 +264,19 @@ constexpr int kWidePerSM = GJ_WIDE_PER_SM;
 constexpr int kWideItems = 8;
 constexpr uint32_t kWideTile = kWideBlock * kWideItems;
 
+template <bool kInverse>
 __global__ void __launch_bounds__(kWideBlock, kWidePerSM) k_part_scatter_wide(const uint64_t* __restrict__ keys, uint64_t m,
                                                                      uint64_t chunk, uint64_t min_key, uint32_t shift,
                                                                      uint32_t fanout, const uint64_t* __restrict__ incl,
                                                                      uint64_t row_base, uint64_t* __restrict__ out_keys,
-                                                                     uint32_t* __restrict__ out_rows) {
+                                                                     uint32_t* __restrict__ out_rows, partition_inverse iv) {
     extern __shared__ unsigned long long s_mem[];
     uint64_t* s_keys = reinterpret_cast<uint64_t*>(s_mem);             // kWideTile
     unsigned long long* s_dst = s_mem + kWideTile;                     // fanout: next output slot
     uint32_t* s_cnt = reinterpret_cast<uint32_t*>(s_dst + fanout);     // fanout
     uint32_t* s_start = s_cnt + fanout;                                // fanout
     unsigned long long* s_delta = reinterpret_cast<unsigned long long*>(s_start + fanout);  // fanout
-#if GJ_SCATTER_META
     uint32_t* s_meta = reinterpret_cast<uint32_t*>(s_delta + fanout);  // kWideTile: partition << 16 | offset
-#else
-    uint16_t* s_off = reinterpret_cast<uint16_t*>(s_delta + fanout);   // kWideTile
-#endif
     for (uint32_t p = threadIdx.x; p < fanout; p += kWideBlock) {
         const uint64_t cell = (uint64_t)p * gridDim.x + blockIdx.x;
         s_dst[p] = cell == 0 ? 0ull : incl[cell - 1];
@@ -316,29 +330,23 @@ __global__ void __launch_bounds__(kWideBlock, kWidePerSM) k_part_scatter_wide(co
             if (j < tn) {
                 const uint32_t q = s_start[slot[k] >> 13] + (slot[k] & ((1u << 13) - 1));
                 s_keys[q] = key[k];
-#if GJ_SCATTER_META
                 s_meta[q] = ((slot[k] >> 13) << 16) | j;
-#else
-                s_off[q] = (uint16_t)j;
-#endif
             }
         }
         // output index of the tile's j-th sorted key = s_delta[p] + j
-        for (uint32_t p = threadIdx.x; p < fanout; p += kWideBlock) s_delta[p] = s_dst[p] - s_start[p];
+        for (uint32_t p = threadIdx.x; p < fanout; p += kWideBlock) {
+            s_delta[p] = s_dst[p] - s_start[p];
+            if constexpr (kInverse) leave_run(iv, tile_number(t0, b0, chunk, kWideTile), fanout, p, s_delta[p], s_start[p]);
+        }
         __syncthreads();
         for (uint32_t j = threadIdx.x; j < tn; j += kWideBlock) {
             const uint64_t k = s_keys[j];
-#if GJ_SCATTER_META
             // the partition and the tile offset were stored with the key
             const uint32_t meta = s_meta[j];
             const uint64_t d = s_delta[meta >> 16] + j;
             __stcg(reinterpret_cast<unsigned long long*>(out_keys) + d, (unsigned long long)k);
-            __stcg(out_rows + d, (uint32_t)(row_base + t0 + (meta & 0xFFFFu)));
-#else
-            const uint64_t d = s_delta[part_of(k, min_key, shift, fanout)] + j;
-            __stcg(reinterpret_cast<unsigned long long*>(out_keys) + d, (unsigned long long)k);
-            __stcg(out_rows + d, (uint32_t)(row_base + t0 + s_off[j]));
-#endif
+            if constexpr (kInverse) iv.offsets[d] = (uint16_t)meta;
+            else __stcg(out_rows + d, (uint32_t)(row_base + t0 + (meta & 0xFFFFu)));
         }
         __syncthreads();
         for (uint32_t p = threadIdx.x; p < fanout; p += kWideBlock) {
@@ -350,14 +358,79 @@ __global__ void __launch_bounds__(kWideBlock, kWidePerSM) k_part_scatter_wide(co
 }
 
 size_t scatter_wide_smem_bytes(uint32_t fanout) {
-    return (size_t)kWideTile * (sizeof(uint64_t) + (GJ_SCATTER_META ? sizeof(uint32_t) : sizeof(uint16_t))) +
+    return (size_t)kWideTile * (sizeof(uint64_t) + sizeof(uint32_t)) +
            (size_t)fanout * (8 + 4 + 4 + 8);
+}
+
+// The scatter backwards for values of the relation: out[row] = the value of
+// the probe that came from row.  A tile's values are read where the scatter
+// put its keys -- one run per partition, consecutive addresses -- placed in
+// probe order in shared memory and written with consecutive threads on
+// consecutive rows, so every sector is whole both ways.  Storing through row
+// ids instead (out[rows[i]] = value) writes each output sector in as many
+// pieces as it has rows, at as many different times: 2^29 positions over 2 GB
+// that way took 16 of the probe pass's 23 ms.
+// Bound by HBM: 2 + 4 bytes read and 4 written per probe.  One block per
+// tile, not persistent: two or more blocks per SM overlap one's loads with
+// the other's writes.
+// values is dense per kValueTile relation entries, at a stride of twice that
+// (each tile's values lie in the first half of the room its keys took).
+template <int kB, int kPerSM>
+__global__ void __launch_bounds__(kB, kPerSM) k_part_gather(const uint32_t* __restrict__ values, uint64_t m, uint64_t chunk,
+                                                     uint32_t fanout, uint32_t tiles_per_chunk, partition_inverse iv,
+                                                     uint32_t* __restrict__ out) {
+    constexpr uint32_t kTile = kB * 8;
+    extern __shared__ unsigned long long s_mem[];
+    uint32_t* s_out = reinterpret_cast<uint32_t*>(s_mem);              // kTile
+    uint32_t* s_delta = s_out + kTile;                                 // fanout
+    uint16_t* s_start = reinterpret_cast<uint16_t*>(s_delta + fanout); // fanout + 2
+    uint16_t* s_part = s_start + fanout + 2;                           // kTile: partition of sorted place j
+    const uint64_t b0 = blockIdx.x / tiles_per_chunk * chunk, b1 = min(m, b0 + chunk);
+    const uint64_t t0 = b0 + (uint64_t)(blockIdx.x % tiles_per_chunk) * kTile;
+    if (t0 >= b1) return;
+    const uint32_t tn = b1 - t0 < kTile ? (uint32_t)(b1 - t0) : kTile;
+    const uint64_t cell = (uint64_t)blockIdx.x * fanout;
+    for (uint32_t p = threadIdx.x; p < fanout; p += kB) {
+        s_delta[p] = __ldcs(iv.delta + cell + p);
+        s_start[p] = __ldcs(iv.start + cell + p);
+    }
+    if (threadIdx.x == 0) s_start[fanout] = (uint16_t)tn;
+    __syncthreads();
+    for (uint32_t p = threadIdx.x >> 5; p < fanout; p += kB / 32)
+        for (uint32_t j = s_start[p] + (threadIdx.x & 31); j < s_start[p + 1]; j += 32) s_part[j] = (uint16_t)p;
+    __syncthreads();
+    uint32_t v[8];
+    uint16_t o[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+        const uint32_t j = k * kB + threadIdx.x;
+        if (j < tn) {
+            const uint32_t d = s_delta[s_part[j]] + j;
+            v[k] = __ldcs(values + value_index(d));
+            o[k] = __ldcs(iv.offsets + d);
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < 8; ++k)
+        if (k * kB + threadIdx.x < tn) s_out[o[k]] = v[k];
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+        const uint32_t j = k * kB + threadIdx.x;
+        if (j < tn) __stcs(out + t0 + j, s_out[j]);
+    }
+}
+
+size_t gather_smem_bytes(uint32_t tile, uint32_t fanout) {
+    return (size_t)tile * (4 + 2) + (size_t)fanout * 4 + ((size_t)fanout + 2) * 2;
 }
 
 struct partition_plan {
     uint32_t fanout, nblocks;
     uint64_t chunk;
     bool wide;
+    uint32_t tile() const { return wide ? kWideTile : kScatterTile; }
+    uint32_t tiles_per_chunk() const { return (uint32_t)((chunk + tile() - 1) / tile()); }
 };
 
 partition_plan plan_partition(uint64_t m, uint32_t radix_bits, int sm_count) {
@@ -384,7 +457,7 @@ size_t partition_ws_bytes(uint64_t m, uint32_t radix_bits, int sm_count) {
 
 int range_partition_impl(const uint64_t* d_keys, uint64_t m, uint64_t min_key, uint32_t shift, uint32_t radix_bits,
                          uint64_t row_base, uint64_t* d_out_keys, uint32_t* d_out_rows, uint64_t* d_offsets, void* ws,
-                         size_t ws_bytes, cudaStream_t s) {
+                         size_t ws_bytes, cudaStream_t s, const partition_inverse* inverse) {
     device_info di;
     GJ_TRY(current_device_info(&di));
     const partition_plan pl = plan_partition(m ? m : 1, radix_bits, di.sm_count);
@@ -402,15 +475,6 @@ int range_partition_impl(const uint64_t* d_keys, uint64_t m, uint64_t min_key, u
         return GJ_OK;
     }
     const size_t smem_hist = (size_t)pl.fanout * hist_copies(pl.fanout) * sizeof(uint32_t);
-    const size_t smem_scatter = pl.wide ? scatter_wide_smem_bytes(pl.fanout) : scatter_smem_bytes(pl.fanout);
-    if (smem_scatter > 48 * 1024) {
-        if (pl.wide)
-            GJ_CUDA_TRY(cudaFuncSetAttribute(k_part_scatter_wide, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)smem_scatter));
-        else
-            GJ_CUDA_TRY(cudaFuncSetAttribute(k_part_scatter, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)smem_scatter));
-    }
     if (pl.wide)
         k_part_hist<kWideBlock><<<pl.nblocks, kWideBlock, smem_hist, s>>>(d_keys, m, pl.chunk, min_key, shift,
                                                                           pl.fanout, hist);
@@ -423,14 +487,47 @@ int range_partition_impl(const uint64_t* d_keys, uint64_t m, uint64_t min_key, u
         k_part_offsets<<<(pl.fanout + 256) / 256, 256, 0, s>>>(hist, pl.fanout, pl.nblocks, m, d_offsets);
         GJ_CUDA_TRY(cudaGetLastError());
     }
-    if (pl.wide)
-        k_part_scatter_wide<<<pl.nblocks, kWideBlock, smem_scatter, s>>>(d_keys, m, pl.chunk, min_key, shift, pl.fanout,
-                                                                         hist, row_base, d_out_keys, d_out_rows);
-    else
-        k_part_scatter<<<pl.nblocks, kScatterBlock, smem_scatter, s>>>(d_keys, m, pl.chunk, min_key, shift, pl.fanout,
-                                                                    hist, row_base, d_out_keys, d_out_rows);
-    GJ_CUDA_TRY(cudaGetLastError());
-    return GJ_OK;
+    const size_t smem = pl.wide ? scatter_wide_smem_bytes(pl.fanout) : scatter_smem_bytes(pl.fanout);
+    const partition_inverse iv = inverse ? *inverse : partition_inverse{};
+    auto launch = [&](auto kernel, int block) {
+        if (smem > 48 * 1024)
+            GJ_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        kernel<<<pl.nblocks, block, smem, s>>>(d_keys, m, pl.chunk, min_key, shift, pl.fanout, hist, row_base,
+                                               d_out_keys, d_out_rows, iv);
+        GJ_CUDA_TRY(cudaGetLastError());
+        return (int)GJ_OK;
+    };
+    if (pl.wide) return inverse ? launch(k_part_scatter_wide<true>, kWideBlock) : launch(k_part_scatter_wide<false>, kWideBlock);
+    return inverse ? launch(k_part_scatter<true>, kScatterBlock) : launch(k_part_scatter<false>, kScatterBlock);
+}
+
+bool carve_partition_inverse(void* ws, size_t ws_bytes, uint64_t m, uint32_t radix_bits, int sm_count,
+                             partition_inverse* out) {
+    const partition_plan pl = plan_partition(m ? m : 1, radix_bits, sm_count);
+    const uint64_t cells = (uint64_t)pl.nblocks * pl.tiles_per_chunk() * pl.fanout;
+    workspace_carver wc(ws, ws_bytes);
+    out->offsets = wc.take<uint16_t>(m);
+    out->delta = wc.take<uint32_t>(cells);
+    out->start = wc.take<uint16_t>(cells);
+    return out->offsets && out->delta && out->start;
+}
+
+int gather_values(const uint32_t* d_values, uint64_t m, uint32_t radix_bits, const partition_inverse& iv,
+                  uint32_t* d_out, cudaStream_t s) {
+    if (m == 0) return GJ_OK;
+    device_info di;
+    GJ_TRY(current_device_info(&di));
+    const partition_plan pl = plan_partition(m, radix_bits, di.sm_count);
+    const size_t smem = gather_smem_bytes(pl.tile(), pl.fanout);
+    auto launch = [&](auto kernel, int block) {
+        if (smem > 48 * 1024)
+            GJ_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        kernel<<<pl.nblocks * pl.tiles_per_chunk(), block, smem, s>>>(d_values, m, pl.chunk, pl.fanout,
+                                                                     pl.tiles_per_chunk(), iv, d_out);
+        GJ_CUDA_TRY(cudaGetLastError());
+        return (int)GJ_OK;
+    };
+    return pl.wide ? launch(k_part_gather<kWideBlock, 2>, kWideBlock) : launch(k_part_gather<kScatterBlock, 4>, kScatterBlock);
 }
 
 // key range used by the partitioned INLJ for an index (recorded at build)

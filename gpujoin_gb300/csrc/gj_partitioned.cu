@@ -82,6 +82,12 @@ constexpr int kProbeItems = 8;             // probes per thread and tile (one at
 constexpr uint32_t kProbeTile = kProbeBlock * kProbeItems;
 constexpr uint32_t kChunk = 4 * kProbeTile;  // probes per block
 
+// window size from which positions come back through the partition's inverse
+#ifndef GJ_GATHER_MIN
+#define GJ_GATHER_MIN (1ull << 22)
+#endif
+constexpr uint64_t kGatherMin = GJ_GATHER_MIN;
+
 enum probe_semantics : int { kSemNone = 0, kSemLowerBound = 1, kSemExact = 2 };
 
 // bucket of a key: (key - min) >> shift, clamped to [0, buckets - 1]
@@ -242,6 +248,7 @@ struct probe_args {
     uint64_t n;
     dir_geom g;
     uint32_t* positions;         // positions[row] = result, or null
+    uint32_t* values;            // values[value_index(i)] = result of relation entry i, or null (no rows then)
     uint2* pairs;                // (row, result) of the matches, or null
     unsigned long long* count;   // pairs appended at atomicAdd(count, ...)
 };
@@ -367,6 +374,17 @@ __global__ void __launch_bounds__(kProbeBlock, GJ_PROBE_BLOCKS) k_part_probe(con
                 }
             }
         }
+        if (a.values) {
+            // the tile's keys have all been read once every thread is here:
+            // its results take the first half of their room
+            __syncthreads();
+#pragma unroll
+            for (int k = 0; k < kProbeItems; ++k) {
+                const uint64_t i = t0 + (uint64_t)k * kProbeBlock + threadIdx.x;
+                if (valid[k]) a.values[value_index((uint32_t)i)] = res[k];
+            }
+            continue;
+        }
         // probe rows are read only now, when the results are written
         uint32_t row[kProbeItems];
 #pragma unroll
@@ -429,6 +447,7 @@ __global__ void __launch_bounds__(kProbeBlock, GJ_PROBE_BLOCKS) k_part_probe(con
 }
 static_assert(kProbeBlock / 32 * kProbeItems % 32 == 0, "the tile scan gives each lane whole counts");
 static_assert(kProbeItems % kProbeBatch == 0, "whole batches per tile");
+static_assert(kProbeTile == kValueTile, "a tile's values lie in the room of its own keys");
 
 // ---------------------------------------------------------------------------
 // host side
@@ -622,10 +641,19 @@ int gj_partitioned_inlj(const gj_index* index, const uint64_t* d_probes, uint64_
     const bool aligned = (reinterpret_cast<uintptr_t>(index->d_col) & 31) == 0;
     for (uint64_t off = 0; off < m; off += w) {
         const uint64_t len = std::min<uint64_t>(w, m - off);
-        GJ_TRY(range_partition_impl(d_probes + off, len, index->min_key, pshift, radix_bits, off, pkeys, prows,
-                                    nullptr, pws, pws_bytes, s));
         a.len = len;
+        // Positions alone come back to probe order through the partition's
+        // inverse, kept where the row ids would be, unless the window's
+        // positions are few enough to stay in L2 while they are stored one
+        // by one (or a high fanout leaves no room for the tiles' runs).
+        partition_inverse iv{};
+        const bool back = d_positions && !d_pairs && len >= kGatherMin &&
+                          carve_partition_inverse(prows, w * sizeof(uint32_t), len, radix_bits, di.sm_count, &iv);
+        GJ_TRY(range_partition_impl(d_probes + off, len, index->min_key, pshift, radix_bits, off, pkeys, prows,
+                                    nullptr, pws, pws_bytes, s, back ? &iv : nullptr));
+        a.values = back ? reinterpret_cast<uint32_t*>(pkeys) : nullptr;
         GJ_TRY(dispatch_probe(sem, aligned, a, s));
+        if (back) GJ_TRY(gather_values(a.values, len, radix_bits, iv, d_positions + off, s));
     }
     return GJ_OK;
 }

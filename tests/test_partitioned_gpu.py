@@ -106,3 +106,21 @@ def test_partitioned_skewed_probes(orc, gj, cuda, kind):
             order = np.argsort(a[:, 0], kind="stable")
             np.testing.assert_array_equal(a[order, 0], erows)
             np.testing.assert_array_equal(a[order, 1], epos)
+
+
+@pytest.mark.parametrize("radix_bits", [1, 5, 7, 8, 11, 12])
+@pytest.mark.parametrize("m,window", [((1 << 22) + 1, 0), (3 * (1 << 22) - 77, 1 << 22)])
+def test_positions_through_the_inverse(orc, gj, cuda, radix_bits, m, window):
+    # windows large enough for the gather pass that brings positions back to
+    # probe order (the last, shorter window stores them by row): one ragged
+    # window and several, through both scatter kernels, and a fanout whose
+    # runs do not fit beside the offsets
+    import torch
+
+    rng = np.random.default_rng(radix_bits)
+    col = column(rng, 300_007)
+    pr = probes_for(rng, col, m)[:m]
+    for kind in ("btree", "binary_search"):
+        ix = gj.make_index(kind).construct(None, to_dev(torch, col)).prepare_partitioned()
+        got, _, _ = ix.partitioned_inlj(to_dev(torch, pr), window_size=window, radix_bits=radix_bits)
+        np.testing.assert_array_equal(from_dev_u32(got), expected(orc, kind, col, pr))
