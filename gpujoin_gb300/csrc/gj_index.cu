@@ -80,6 +80,37 @@ __global__ void k_gather_fence(const uint64_t* __restrict__ col, uint64_t n, uin
     }
 }
 
+// key start table: pos[b] = the first key not below bucket b's first value
+// (binary search per bucket; n from the bucket past the last one on)
+__global__ void k_key_start(const uint64_t* __restrict__ col, uint64_t n, uint64_t min_key, uint32_t shift,
+                            uint32_t buckets, uint32_t entries, uint32_t* __restrict__ pos) {
+    for (uint32_t b = blockIdx.x * blockDim.x + threadIdx.x; b < entries; b += gridDim.x * blockDim.x)
+        pos[b] = b >= buckets ? (uint32_t)n
+                              : (uint32_t)lower_bound_branch_free(col, n, min_key + ((uint64_t)b << shift));
+}
+
+// sums[0] += column sectors the key start table's searches read, sums[1] +=
+// levels below the tree's start entry, over kStartSample keys of the column
+constexpr uint32_t kStartSample = 8192;
+__global__ void k_start_cost(key_start t, const uint64_t* __restrict__ col, uint32_t n, btree_view bt,
+                             unsigned long long* sums) {
+    const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
+    uint32_t loads = 0, level = 0;
+    if (j < kStartSample) {
+        // spread over the column, off the tree's node boundaries
+        const uint64_t key = col[((uint64_t)j * n + mix64(j) % n) / kStartSample];
+        bool eq;
+        start_lower_bound<false, true>(t, col, n, key, &eq, &loads);
+        if (bt.start) level = (uint32_t)(bt.start[2 * ((key - bt.min_key) >> bt.start_shift) + 1] >> 32);
+    }
+    loads = __reduce_add_sync(0xffffffffu, loads);
+    level = __reduce_add_sync(0xffffffffu, level);
+    if ((threadIdx.x & 31) == 0) {
+        atomicAdd(&sums[0], (unsigned long long)loads);
+        atomicAdd(&sums[1], (unsigned long long)level);
+    }
+}
+
 // start table of a B+tree: entry b = the deepest node shared by the exact
 // descents of every key of bucket b, [min + b * 2^shift, min + (b + 1) * 2^shift)
 // clamped to max (v reads every level from global memory: no shared cache)
@@ -258,6 +289,55 @@ int host_copy_of_column(const uint64_t* d_keys, const uint64_t* h_keys, uint64_t
     return GJ_OK;
 }
 
+// Key start table of 2^bits buckets (fewer for a narrow key range); use(loads,
+// level) decides from the sampled cost of its searches -- mean column sectors
+// read, and for a B+tree the mean level its lookups start at -- whether the
+// index keeps it.
+template <class Use>
+int build_key_start(gj_index* idx, uint32_t bits, cudaStream_t s, Use&& use) {
+    const uint64_t range = idx->max_key - idx->min_key;
+    const uint32_t used = range ? 64u - (uint32_t)__builtin_clzll(range) : 0u;
+    key_start t{};
+    t.min_key = idx->min_key;
+    t.range = range;
+    t.shift = used > bits ? used - bits : 0u;
+    t.inv_width = std::ldexp(1.0f, -(int)t.shift);
+    t.col_aligned = aligned32(idx->d_col);
+    const uint32_t buckets = (uint32_t)(range >> t.shift) + 1;
+    const uint32_t entries = (buckets + 1 + 3) & ~3u;  // whole 16-byte groups
+    void* p = nullptr;
+    GJ_TRY(device_alloc(idx, (size_t)entries * sizeof(uint32_t) + 2 * sizeof(unsigned long long), &p));
+    uint32_t* pos = static_cast<uint32_t*>(p);
+    unsigned long long* d_sums = reinterpret_cast<unsigned long long*>(pos + entries);
+    unsigned long long sums[2] = {0, 0};
+    k_key_start<<<(entries + 255) / 256, 256, 0, s>>>(idx->d_col, idx->n, t.min_key, t.shift, buckets, entries, pos);
+    GJ_CUDA_TRY(cudaGetLastError());
+    t.pos = pos;
+    GJ_CUDA_TRY(cudaMemsetAsync(d_sums, 0, sizeof(sums), s));
+    k_start_cost<<<kStartSample / 256, 256, 0, s>>>(t, idx->d_col, (uint32_t)idx->n, idx->bt, d_sums);
+    GJ_CUDA_TRY(cudaGetLastError());
+    GJ_CUDA_TRY(cudaMemcpyAsync(sums, d_sums, sizeof(sums), cudaMemcpyDeviceToHost, s));
+    GJ_CUDA_TRY(cudaStreamSynchronize(s));
+    if (!use((double)sums[0] / kStartSample, (double)sums[1] / kStartSample)) {
+        GJ_CUDA_TRY(cudaFree(p));
+        idx->allocations.pop_back();
+        return GJ_OK;
+    }
+    idx->ks = t;
+    idx->bytes += (size_t)entries * sizeof(uint32_t);
+    return GJ_OK;
+}
+
+// Bits of a key start table: about one bucket a key, at most 2^22 (16 MB).  A
+// larger table leaves L2 (2^26 probes into 2^23 keys: 770 us at 2^22, 865 at
+// 2^23, 1298 at 2^24), a smaller one leaves wider windows (2^26 keys: 2132 us
+// at 2^20, 1758 at 2^21, 1657 at 2^22).
+uint32_t key_start_bits(uint64_t n) {
+    uint32_t b = 1;
+    while (b < 22 && (1ull << b) < n) ++b;
+    return b;
+}
+
 int build_binary_search(gj_index* idx, cudaStream_t s) {
     idx->bs.col = idx->d_col;
     idx->bs.n = idx->n;
@@ -282,6 +362,8 @@ int build_binary_search(gj_index* idx, cudaStream_t s) {
     idx->bs.fence_shift = shift;
     idx->bs.fence_steps = steps;
     idx->bytes = (uint64_t)slots * sizeof(uint64_t);
+    if (idx->params.index_memory == GJ_INDEX_MEMORY_DEVICE)
+        GJ_TRY(build_key_start(idx, key_start_bits(idx->n), s, [](double, double) { return true; }));
     return GJ_OK;
 }
 
@@ -438,6 +520,19 @@ int build_btree(gj_index* idx, cudaStream_t s) {
     idx->bt.start_shift = shift;
     idx->bt.start_entries = (uint32_t)entries;
     idx->bytes += entries * 16;
+    // The default tree's scattered lookups go through a key start table, at
+    // leaf granularity, where that is faster: up to 2^24 keys (2^26 probes,
+    // table against nodes: 584 / 1104 us at 2^20 uniform keys, 928 / 1046 at
+    // 2^24), and above where the node table starts most lookups far from the
+    // leaves (2^26 clustered keys, mean level 4.5: 1965 / 16585 us).  Above
+    // 2^24 keys that spread evenly (mean level about 2) the nodes' single
+    // column sector wins (lognormal 2^26 keys: 1895 / 1572 us), and so they do
+    // where a column is so uneven that the table's windows take long searches.
+    if (W == kBtreeCompressed16 && L == 4 && idx->params.btree_start_bits == 0 &&
+        idx->params.index_memory == GJ_INDEX_MEMORY_DEVICE)
+        GJ_TRY(build_key_start(idx, key_start_bits(n), s, [&](double loads, double level) {
+            return loads <= 4.0 && (n <= (1ull << 24) || level >= 3.0);
+        }));
     return GJ_OK;
 }
 
@@ -465,6 +560,11 @@ int build_harmonia(gj_index* idx, const uint64_t* h_keys, cudaStream_t s) {
     idx->hm.n = idx->n;
     idx->hm.inner_size = ha.keys.size();
     idx->hm.depth = ha.depth;
+    // first child of the level's first node, less 33 times that node
+    for (uint64_t l = 0, first = 0; l + 1 < ha.depth; ++l) {
+        idx->hm_base.of[l + 1] = (int64_t)ha.children[first] - (int64_t)(kHarmoniaKeys + 1) * (int64_t)first;
+        first += ha.level_nodes[l];
+    }
     // shared-memory cache: whole top levels (keys + children) within the budget
     const uint64_t per_node = (kHarmoniaKeys + 1) * sizeof(uint64_t);
     uint64_t cached = 0;
@@ -515,6 +615,11 @@ int build_harmonia(gj_index* idx, const uint64_t* h_keys, cudaStream_t s) {
     idx->hm.start_shift = shift;
     idx->hm.start_entries = (uint32_t)entries;
     idx->bytes += entries * sizeof(uint64_t);
+    // as for the B+tree; 32-key nodes take about three sectors a level, so the
+    // table wins at every size (2^26 probes, table against nodes: 584 / 2135
+    // us at 2^20 keys, 1764 / 3781 at 2^26, clustered 1.97 / 4.44 ms)
+    if (idx->params.btree_start_bits == 0 && idx->params.index_memory == GJ_INDEX_MEMORY_DEVICE)
+        GJ_TRY(build_key_start(idx, key_start_bits(n), s, [](double loads, double) { return loads <= 4.0; }));
     return GJ_OK;
 }
 
@@ -530,7 +635,13 @@ int build_radix_spline_index(gj_index* idx, const uint64_t* h_keys, cudaStream_t
         pts[i].x = rs.sx[i];
         pts[i].y = rs.sy[i];
         pts[i].slope = i + 1 < pts.size() ? (rs.sy[i + 1] - rs.sy[i]) / (double)(rs.sx[i + 1] - rs.sx[i]) : 0.0;
-        pts[i].pad = 0;
+        pts[i].step = 0;
+        if (i + 1 < pts.size()) {
+            const uint64_t dx = rs.sx[i + 1] - rs.sx[i];
+            const uint32_t sh = (uint32_t)__builtin_clzll(dx);
+            const unsigned __int128 dy = (unsigned __int128)(uint64_t)(rs.sy[i + 1] - rs.sy[i]);
+            pts[i].step = (uint64_t)((dy << 64) / (dx << sh)) << 6 | sh;
+        }
     }
     void *pt = nullptr, *pp = nullptr;
     GJ_TRY(device_alloc(idx, rs.table.size() * sizeof(uint32_t), &pt));

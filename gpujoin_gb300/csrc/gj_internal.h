@@ -113,6 +113,8 @@ struct gj_index {
     gj::bs_view bs{};
     gj::btree_view bt{};
     gj::harmonia_view hm{};
+    gj::harmonia_child_base hm_base{};
+    gj::key_start ks{};  // key start table (binary search; default B+tree over a small column), or none
     gj::rs_view rs{};
     gj::learned_view ln{};
     gj::hash_view hs{};

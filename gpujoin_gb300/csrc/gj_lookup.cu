@@ -5,7 +5,10 @@
 
 namespace gj {
 
-int lookup_call_bs(const gj_index* idx, const lookup_call& c) { return run_call(op_bs{idx->bs}, idx, c); }
+int lookup_call_bs(const gj_index* idx, const lookup_call& c) {
+    if (idx->ks.pos) return run_call(op_start<false>{idx->ks, idx->d_col, (uint32_t)idx->n}, idx, c);
+    return run_call(op_bs{idx->bs}, idx, c);
+}
 int lookup_call_noop(const gj_index* idx, const lookup_call& c) { return run_call(op_noop{}, idx, c); }
 int lookup_call_hash(const gj_index* idx, const lookup_call& c) { return run_call(op_hash{idx->hs}, idx, c); }
 

@@ -10,6 +10,9 @@ int lookup_call_btree<7>(const gj_index* idx, const lookup_call& c) {
 
 template <>
 int lookup_call_btree<15>(const gj_index* idx, const lookup_call& c) {
+    // sorted tiles share the paths of a tree; they keep its nodes
+    const bool sorted = c.action == lookup_action::sorted_pairs || c.action == lookup_action::sorted_positions;
+    if (idx->ks.pos && !sorted) return run_call(op_start<true>{idx->ks, idx->d_col, (uint32_t)idx->n}, idx, c);
     return run_call(op_btree<15>{idx->bt}, idx, c);
 }
 

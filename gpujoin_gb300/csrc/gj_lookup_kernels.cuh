@@ -97,6 +97,8 @@ struct stage_desc {
 // and touch a slice of the tree, use the default class.
 struct op_bs {
     static constexpr int kMinBlocks = GJ_BLOCKS(8);
+    static constexpr int kLong = 2;
+    static constexpr bool kStaged = true;
     bs_view v;
     template <bool kScattered = true>
     __device__ __forceinline__ uint32_t lookup(const uint64_t* cache, uint64_t key) const {
@@ -104,16 +106,43 @@ struct op_bs {
     }
     __device__ __forceinline__ uint32_t operator()(const uint64_t* cache, uint64_t key) const { return lookup(cache, key); }
 };
+// lookups through the index's key start table: the lower bound (binary
+// search) or the position of an equal key (the default B+tree over a column
+// small enough for the table to replace its levels)
+template <bool kExact>
+struct op_start {
+    static constexpr int kMinBlocks = GJ_BLOCKS(8);
+    static constexpr int kLong = 2;
+    static constexpr bool kStaged = false;
+    key_start t;
+    const uint64_t* col;
+    uint32_t n;
+    template <bool kScattered = true>
+    __device__ __forceinline__ uint32_t lookup(const uint64_t*, uint64_t key) const {
+        bool eq;
+        const uint32_t lb = start_lower_bound<kScattered>(t, col, n, key, &eq);
+        return (kExact ? eq : lb < n) ? lb : kInvalid;
+    }
+    __device__ __forceinline__ uint32_t operator()(const uint64_t* cache, uint64_t key) const { return lookup(cache, key); }
+};
+// Trees: a scattered lookup starts at its bucket's entry of the start table,
+// nearly always below the levels that fit shared memory, so only the sorted
+// tiles (whose common node is searched from the root) stage them; the kernels
+// without them keep the room for L1 and have nothing to load before the
+// first probe.
+//
 // Sorted tiles: an op with a tile_hint searches once per tile for what all
 // keys of the tile's range share (for the B+tree: the deepest node on every
 // path) and starts each probe's search there.
 template <int W>
 struct op_btree {
     static constexpr int kMinBlocks = GJ_BLOCKS(8);
+    static constexpr int kLong = 8;
+    static constexpr bool kStaged = false;
     btree_view v;
     template <bool kScattered = true>
     __device__ __forceinline__ uint32_t lookup(const uint64_t* cache, uint64_t key) const {
-        return btree_lookup<W, kScattered>(v, cache, key);
+        return btree_lookup<W, kScattered, false>(v, cache, key);
     }
     __device__ __forceinline__ uint32_t operator()(const uint64_t* cache, uint64_t key) const { return lookup(cache, key); }
     using tile_hint = btree_cursor;
@@ -136,15 +165,20 @@ struct tile_hint_of<Op, std::void_t<typename Op::tile_hint>> {
 };
 struct op_harmonia {
     static constexpr int kMinBlocks = GJ_BLOCKS(8);
+    static constexpr int kLong = 2;
+    static constexpr bool kStaged = false;
     harmonia_view v;
+    harmonia_child_base base;
     template <bool kScattered = true>
     __device__ __forceinline__ uint32_t lookup(const uint64_t* cache, uint64_t key) const {
-        return harmonia_lookup<kScattered>(v, cache, key);
+        return harmonia_lookup<kScattered, false>(v, cache, key, &base);
     }
     __device__ __forceinline__ uint32_t operator()(const uint64_t* cache, uint64_t key) const { return lookup(cache, key); }
 };
 struct op_rs {
     static constexpr int kMinBlocks = GJ_BLOCKS(8);
+    static constexpr int kLong = 1;
+    static constexpr bool kStaged = false;
     rs_view v;
     template <bool kScattered = true>
     __device__ __forceinline__ uint32_t lookup(const uint64_t*, uint64_t key) const {
@@ -154,6 +188,8 @@ struct op_rs {
 };
 struct op_hash {
     static constexpr int kMinBlocks = GJ_BLOCKS(8);
+    static constexpr int kLong = 8;
+    static constexpr bool kStaged = false;
     hash_view v;
     template <bool kScattered = true>
     __device__ __forceinline__ uint32_t lookup(const uint64_t*, uint64_t key) const {
@@ -163,6 +199,8 @@ struct op_hash {
 };
 struct op_noop {
     static constexpr int kMinBlocks = GJ_BLOCKS(8);
+    static constexpr int kLong = 8;
+    static constexpr bool kStaged = false;
     template <bool kScattered = true>
     __device__ __forceinline__ uint32_t lookup(const uint64_t*, uint64_t) const { return kInvalid; }
     __device__ __forceinline__ uint32_t operator()(const uint64_t*, uint64_t) const { return kInvalid; }
@@ -171,11 +209,26 @@ struct op_noop {
 // FMAs read their weights from the constant bank
 struct op_learned {
     static constexpr int kMinBlocks = GJ_BLOCKS(4);
+    static constexpr int kLong = 8;
+    static constexpr bool kStaged = false;
     learned_view v;
     learned_root_params p;
     template <bool kScattered = true>
     __device__ __forceinline__ uint32_t lookup(const uint64_t*, uint64_t key) const {
         return learned_lookup<kScattered>(v, p.w, key);
+    }
+    __device__ __forceinline__ uint32_t operator()(const uint64_t* cache, uint64_t key) const { return lookup(cache, key); }
+};
+// linear and segment-table roots: no network to evaluate, twice the warps
+struct op_learned_plain {
+    static constexpr int kMinBlocks = GJ_BLOCKS(8);
+    static constexpr int kLong = 2;
+    static constexpr bool kStaged = false;
+    learned_view v;
+    float p[2];
+    template <bool kScattered = true>
+    __device__ __forceinline__ uint32_t lookup(const uint64_t*, uint64_t key) const {
+        return learned_lookup<kScattered, false>(v, p, key);
     }
     __device__ __forceinline__ uint32_t operator()(const uint64_t* cache, uint64_t key) const { return lookup(cache, key); }
 };
@@ -190,7 +243,7 @@ __device__ __forceinline__ void stage_cache(uint64_t* dst, const stage_desc& sd)
 // ---------------------------------------------------------------------------
 // plain lookup: out[i] = lookup(probes[i])
 // ---------------------------------------------------------------------------
-// One block per tile of kLookupItems * kBlock probes (item k of thread t is
+// One block per tile of kIt * kBlock probes (item k of thread t is
 // probe tile + k * kBlock + t: coalesced).  The grid is not persistent: the
 // hardware hands tiles to SMs as they free up, which balances SMs that run
 // at different speeds (near and far HBM of the two dies) without a counter.
@@ -198,50 +251,60 @@ __device__ __forceinline__ void stage_cache(uint64_t* dst, const stage_desc& sd)
 // dependent loads; occupancy, not per-thread interleaving, keeps many loads
 // in flight) and loads the next probe key before it searches the current
 // one.  No per-thread arrays: the search runs with few live registers.
-#ifndef GJ_LOOKUP_ITEMS
-#define GJ_LOOKUP_ITEMS 8
-#endif
-constexpr int kLookupItems = GJ_LOOKUP_ITEMS;
-constexpr uint32_t kLookupTile = kBlock * kLookupItems;
+
+
+// Whether a lookup launch gives its threads Op::kLong probes each, one after
+// another, or one.  One fills the chip from the fewest probes (65,536 probes
+// into 2^26 keys: 84 us in 2048-probe blocks, 10 in 256-probe blocks) and
+// keeps most loads in flight when the column's sectors come from DRAM (2^26
+// probes into 2^26 keys 1568 against 1654 us); several save a block's start
+// where the searches run from L2 (hash table of 2^20 keys 406 against 485 us
+// with 8).
+inline int long_blocks(uint64_t n, uint64_t m, bool* yes) {
+    device_info di;
+    GJ_TRY(current_device_info(&di));
+    *yes = n <= (1ull << 23) && m >= 16ull * di.sm_count * 8 * kBlock;  // 16 waves of a full chip
+    return GJ_OK;
+}
 
 __device__ __forceinline__ uint64_t load_probe(const uint64_t* p, uint64_t i, uint64_t m) {
     return i < m ? __ldcs(reinterpret_cast<const unsigned long long*>(p + i)) : 0ull;
 }
 
-template <class Op>
+template <class Op, int kIt>
 __global__ void __launch_bounds__(kBlock, Op::kMinBlocks) k_lookup(const __grid_constant__ Op op, const stage_desc sd,
                                                    const uint64_t* __restrict__ probes, uint64_t m,
                                                    uint32_t* __restrict__ out) {
     extern __shared__ __align__(16) uint64_t cache[];
-    stage_cache(cache, sd);
-    const uint64_t t0 = (uint64_t)blockIdx.x * kLookupTile + threadIdx.x;
+    if constexpr (Op::kStaged) stage_cache(cache, sd);
+    const uint64_t t0 = (uint64_t)blockIdx.x * (kBlock * kIt) + threadIdx.x;
     uint64_t next = load_probe(probes, t0, m);
 #pragma unroll 1
-    for (int k = 0; k < kLookupItems; ++k) {
+    for (int k = 0; k < kIt; ++k) {
         const uint64_t i = t0 + (uint64_t)k * kBlock;
         if (i >= m) break;
         const uint64_t key = next;
-        if (k + 1 < kLookupItems) next = load_probe(probes, i + kBlock, m);
+        if (k + 1 < kIt) next = load_probe(probes, i + kBlock, m);
         __stcs(out + i, op(cache, key));
     }
 }
 
 // scattered lookup over a partitioned relation: out[rows[i]] = lookup(keys[i])
-template <class Op>
+template <class Op, int kIt>
 __global__ void __launch_bounds__(kBlock, Op::kMinBlocks) k_scatter_lookup(const __grid_constant__ Op op, const stage_desc sd,
                                                            const uint64_t* __restrict__ keys,
                                                            const uint32_t* __restrict__ rows, uint64_t m,
                                                            uint32_t* __restrict__ out) {
     extern __shared__ __align__(16) uint64_t cache[];
-    stage_cache(cache, sd);
-    const uint64_t t0 = (uint64_t)blockIdx.x * kLookupTile + threadIdx.x;
+    if constexpr (Op::kStaged) stage_cache(cache, sd);
+    const uint64_t t0 = (uint64_t)blockIdx.x * (kBlock * kIt) + threadIdx.x;
     uint64_t next = load_probe(keys, t0, m);
 #pragma unroll 1
-    for (int k = 0; k < kLookupItems; ++k) {
+    for (int k = 0; k < kIt; ++k) {
         const uint64_t i = t0 + (uint64_t)k * kBlock;
         if (i >= m) break;
         const uint64_t key = next;
-        if (k + 1 < kLookupItems) next = load_probe(keys, i + kBlock, m);
+        if (k + 1 < kIt) next = load_probe(keys, i + kBlock, m);
         const uint32_t r = op.template lookup<false>(cache, key);
         out[__ldcs(rows + i)] = r;
     }
@@ -266,7 +329,7 @@ __global__ void __launch_bounds__(kBlock, Op::kMinBlocks) k_scatter_lookup(const
 // per 2^28 probes, against 18.7 with 4 and 21.4 with 16); GJ_PAIRS_ITEMS
 // overrides it in tuning builds
 #ifndef GJ_PAIRS_ITEMS
-#define GJ_PAIRS_ITEMS GJ_LOOKUP_ITEMS
+#define GJ_PAIRS_ITEMS 8
 #endif
 constexpr int kItems = GJ_PAIRS_ITEMS;
 constexpr int kCompactItems = 16;                // k_compact_pairs items per thread
@@ -459,7 +522,7 @@ __global__ void __launch_bounds__(kBlock, Op::kMinBlocks) k_pairs(const __grid_c
                                                   uint2* __restrict__ pairs, const uint64_t* __restrict__ d_base,
                                                   uint64_t* __restrict__ d_count, pairs_ws ws, uint32_t num_tiles) {
     extern __shared__ __align__(16) uint64_t cache[];
-    stage_cache(cache, sd);
+    if constexpr (Op::kStaged) stage_cache(cache, sd);
     const uint64_t base = d_base ? *d_base : 0ull;
     auto search = [&](uint64_t t0, uint32_t* s_pos) {
         uint64_t next = load_probe(probes, t0 + threadIdx.x, m);
@@ -732,14 +795,6 @@ stage_desc make_stage(const gj_index* idx) {
                 sd.words0 = idx->bt.cache_keys;
             }
             break;
-        case GJ_INDEX_HARMONIA:
-            if (idx->hm.cached_nodes) {
-                sd.src0 = idx->hm.keys;
-                sd.words0 = idx->hm.cached_nodes * kHarmoniaKeys;
-                sd.src1 = idx->hm.children;
-                sd.words1 = idx->hm.cached_nodes;
-            }
-            break;
         default:
             break;
     }
@@ -783,13 +838,19 @@ int grid_for(Kernel kernel, size_t smem, uint64_t work_items, int* grid) {
 }
 
 template <class Op>
-int run_lookup(const Op& op, const stage_desc& sd, const uint64_t* probes, uint64_t m, uint32_t* out, cudaStream_t s) {
-    const size_t smem = stage_bytes(sd);
-    GJ_TRY(prepare_smem(k_lookup<Op>, smem));
-    const uint64_t grid = (m + kLookupTile - 1) / kLookupTile;
-    k_lookup<Op><<<(unsigned)grid, kBlock, smem, s>>>(op, sd, probes, m, out);
-    GJ_CUDA_TRY(cudaGetLastError());
-    return GJ_OK;
+int run_lookup(const Op& op, const stage_desc& sd, uint64_t n, const uint64_t* probes, uint64_t m, uint32_t* out,
+               cudaStream_t s) {
+    const size_t smem = Op::kStaged ? stage_bytes(sd) : 0;
+    auto launch = [&](auto kernel, int items) {
+        GJ_TRY(prepare_smem(kernel, smem));
+        const uint64_t tile = (uint64_t)kBlock * items;
+        kernel<<<(unsigned)((m + tile - 1) / tile), kBlock, smem, s>>>(op, sd, probes, m, out);
+        GJ_CUDA_TRY(cudaGetLastError());
+        return (int)GJ_OK;
+    };
+    bool full = false;
+    GJ_TRY(long_blocks(n, m, &full));
+    return full ? launch(k_lookup<Op, Op::kLong>, Op::kLong) : launch(k_lookup<Op, 1>, 1);
 }
 
 template <class Op>
@@ -805,18 +866,23 @@ int run_sorted_lookup(const Op& op, const stage_desc& sd, const uint64_t* probes
 }
 
 template <class Op>
-int run_scatter(const Op& op, const stage_desc& sd, const uint64_t* keys, const uint32_t* rows, uint64_t m,
-                uint32_t* out, cudaStream_t s) {
-    const size_t smem = stage_bytes(sd);
-    GJ_TRY(prepare_smem(k_scatter_lookup<Op>, smem));
-    const uint64_t grid = (m + kLookupTile - 1) / kLookupTile;
-    k_scatter_lookup<Op><<<(unsigned)grid, kBlock, smem, s>>>(op, sd, keys, rows, m, out);
-    GJ_CUDA_TRY(cudaGetLastError());
-    return GJ_OK;
+int run_scatter(const Op& op, const stage_desc& sd, uint64_t n, const uint64_t* keys, const uint32_t* rows,
+                uint64_t m, uint32_t* out, cudaStream_t s) {
+    const size_t smem = Op::kStaged ? stage_bytes(sd) : 0;
+    auto launch = [&](auto kernel, int items) {
+        GJ_TRY(prepare_smem(kernel, smem));
+        const uint64_t tile = (uint64_t)kBlock * items;
+        kernel<<<(unsigned)((m + tile - 1) / tile), kBlock, smem, s>>>(op, sd, keys, rows, m, out);
+        GJ_CUDA_TRY(cudaGetLastError());
+        return (int)GJ_OK;
+    };
+    bool full = false;
+    GJ_TRY(long_blocks(n, m, &full));
+    return full ? launch(k_scatter_lookup<Op, Op::kLong>, Op::kLong) : launch(k_scatter_lookup<Op, 1>, 1);
 }
 
 template <class Op>
-int run_pairs(const Op& op, const stage_desc& sd, const uint64_t* probes, const uint32_t* rows, uint64_t m,
+int run_pairs(const Op& op, const stage_desc& sd, uint64_t n, const uint64_t* probes, const uint32_t* rows, uint64_t m,
               uint32_t* pairs, const uint64_t* d_base, uint64_t* d_count, void* ws, size_t ws_bytes, uint32_t* stash,
               cudaStream_t s, uint32_t spin_limit = 0, bool skip_first_tile = false, bool unordered = false) {
     const uint32_t num_tiles = (uint32_t)((m + kTile - 1) / kTile);
@@ -840,7 +906,7 @@ int run_pairs(const Op& op, const stage_desc& sd, const uint64_t* probes, const 
     // never publishes; every later tile's look-back runs out
     if (skip_first_tile) GJ_CUDA_TRY(cudaMemsetAsync(pw.tile_counter, 1, 1, s));
     if (stash) {
-        GJ_TRY(run_lookup(op, sd, probes, m, stash, s));
+        GJ_TRY(run_lookup(op, sd, n, probes, m, stash, s));
         const uint32_t compact_tiles = (uint32_t)((m + kCompactTile - 1) / kCompactTile);
         int grid = 0;
         GJ_TRY(grid_for(k_compact_pairs, 0, (uint64_t)compact_tiles * kBlock, &grid));
@@ -849,7 +915,7 @@ int run_pairs(const Op& op, const stage_desc& sd, const uint64_t* probes, const 
         GJ_CUDA_TRY(cudaGetLastError());
         return GJ_OK;
     }
-    const size_t smem = stage_bytes(sd);
+    const size_t smem = Op::kStaged ? stage_bytes(sd) : 0;
     int grid = 0;
     if (unordered) {
         GJ_TRY(grid_for(k_pairs<Op, false>, smem, (uint64_t)num_tiles * kBlock, &grid));
@@ -903,10 +969,10 @@ template <class Op>
 int run_call(const Op& op, const gj_index* idx, const lookup_call& c) {
     const stage_desc sd = make_stage(idx);
     switch (c.action) {
-        case lookup_action::positions: return run_lookup(op, sd, c.keys, c.m, c.out, c.s);
-        case lookup_action::scatter: return run_scatter(op, sd, c.keys, c.rows, c.m, c.out, c.s);
+        case lookup_action::positions: return run_lookup(op, sd, idx->n, c.keys, c.m, c.out, c.s);
+        case lookup_action::scatter: return run_scatter(op, sd, idx->n, c.keys, c.rows, c.m, c.out, c.s);
         case lookup_action::pairs:
-            return run_pairs(op, sd, c.keys, c.rows, c.m, c.out, c.d_base, c.d_count, c.ws, c.ws_bytes, c.stash, c.s,
+            return run_pairs(op, sd, idx->n, c.keys, c.rows, c.m, c.out, c.d_base, c.d_count, c.ws, c.ws_bytes, c.stash, c.s,
                              c.spin_limit, c.skip_first_tile, c.unordered);
         case lookup_action::sorted_pairs:
             return run_sorted_pairs(op, sd, c.keys, c.rows, c.m, c.out, c.d_base, c.d_count, c.ws, c.ws_bytes, c.s);

@@ -62,8 +62,13 @@ GJ_DEVICE_INLINE void ld_sector_64(const uint64_t* p, uint64_t (&k)[4]) {
 // tree (tens of MB, read by every probe) are kept over the column sectors a
 // probe reads once (hundreds of MB, random).  Loads carry an L2 cache policy;
 // no device-wide setting is involved.  Both classes serve scattered probes,
-// whose neighbouring sectors are of no use: their misses fill 64 bytes.
-enum l2_class : int { kL2Default = 0, kL2Keep = 1, kL2Stream = 2 };
+// whose neighbouring sectors are of no use: their misses fill 64 bytes.  The
+// exception is a column searched over a few sectors in a row (kL2StreamLine):
+// its misses fill the line, as the part serves about 43 G random DRAM accesses
+// per second of either size (2^26 probes into 2^24 keys through the key start
+// table 922 against 1027 us, RadixSpline 1624 against 1859; level with it at
+// 2^26 keys).
+enum l2_class : int { kL2Default = 0, kL2Keep = 1, kL2Stream = 2, kL2StreamLine = 3 };
 
 template <int kClass>
 GJ_DEVICE_INLINE uint64_t l2_policy() {
@@ -79,6 +84,10 @@ template <int kClass>
 GJ_DEVICE_INLINE void ld_sector_c(const uint64_t* p, uint64_t (&k)[4]) {
     if constexpr (kClass == kL2Default) {
         ld_sector(p, k);
+    } else if constexpr (kClass == kL2StreamLine) {
+        asm("ld.global.nc.L2::cache_hint.v4.u64 {%0, %1, %2, %3}, [%4], %5;"
+            : "=l"(k[0]), "=l"(k[1]), "=l"(k[2]), "=l"(k[3])
+            : "l"(p), "l"(l2_policy<kClass>()));
     } else {
         asm("ld.global.nc.L2::cache_hint.L2::64B.v4.u64 {%0, %1, %2, %3}, [%4], %5;"
             : "=l"(k[0]), "=l"(k[1]), "=l"(k[2]), "=l"(k[3])
@@ -189,6 +198,125 @@ GJ_DEVICE_INLINE uint64_t lower_bound_sectors(const uint64_t* arr, uint64_t arr_
             return r;
         }
     }
+}
+
+// Lower bound of key in a 32-byte aligned column of n < 2^32 keys, for a
+// caller that expects it in sectors [sl, sr] and near sector s of them.  While
+// the answer is elsewhere the search moves on from the sector it has read, by
+// the key's distance over the spacing of that sector's keys (twice at most:
+// exact at once in a run of equal steps, close where the column is smooth
+// nearby), then halves what is left: any column costs at most two loads more
+// than halving alone.  The sectors are read whole and compared whole -- keys
+// outside the caller's window are as good as those inside.
+// *edge: 0 when the answer is certain, 1 / 2 when it is the first key of
+// sector sl / the key behind sector sr, i.e. the bound within the sectors, and
+// the column's only if the caller's range holds.  *eq: the answer's key is
+// read and equals key.  loads counts the sectors read (build statistics).
+template <int kClass, bool kCount = false>
+GJ_DEVICE_INLINE uint32_t search_sectors(const uint64_t* col, uint32_t n, uint32_t sl, uint32_t sr, uint32_t s,
+                                         uint64_t key, bool* eq, uint32_t* edge, uint32_t* loads = nullptr) {
+    constexpr uint32_t kNear = 3;  // few sectors left: the next one, without arithmetic
+    const uint32_t sl0 = sl, sr0 = sr;
+    uint64_t right_key = 0;  // first key of sector sr + 1, once that has been read
+#pragma unroll 1
+    for (uint32_t step = 0;; ++step) {
+        const uint32_t s0 = s << 2;
+        uint64_t k[4];
+        if (n - s0 >= 4) {
+            ld_sector_c<kClass>(col + s0, k);
+        } else {
+#pragma unroll
+            for (uint32_t i = 0; i < 4; ++i) k[i] = (i < n - s0) ? ld_ro_c<kClass>(col + s0 + i) : ~0ull;
+        }
+        if constexpr (kCount) ++*loads;
+        const uint32_t below = (k[0] < key) + (k[1] < key) + (k[2] < key) + (k[3] < key);
+        if (below == 4) {
+            if (s == sr) {
+                *eq = sr != sr0 && right_key == key;
+                *edge = sr == sr0 ? 2u : 0u;
+                return s0 + 4;
+            }
+            sl = s + 1;
+            if (sr - sl < kNear) {
+                s = sl;
+                continue;
+            }
+            if (step < 2) {  // sectors past this one
+                const float d = __fdividef((float)(key - k[3]) * 0.75f, (float)(k[3] - k[0]));
+                s = sl + (uint32_t)fminf(d, (float)(sr - sl));
+                s = s > sr ? sr : s;
+                continue;
+            }
+        } else if (below == 0 && s != sl) {
+            right_key = k[0];
+            sr = s - 1;
+            if (sr - sl < kNear) {
+                s = sr;
+                continue;
+            }
+            if (step < 2) {
+                const float d = __fdividef((float)(k[0] - key) * 0.75f, (float)(k[3] - k[0]));
+                const uint32_t back = (uint32_t)fminf(d, (float)(sr - sl));
+                s = sr - (back < sr - sl ? back : sr - sl);
+                continue;
+            }
+        } else {
+            *eq = s0 + below < n && pick4(k, below) == key;
+            *edge = below == 0 && s == sl0 ? 1u : 0u;
+            return s0 + below;
+        }
+        s = (sl + sr) >> 1;
+    }
+}
+
+// ---------------------------------------------------------------------------
+// key start table: the key range [min_key, max_key] of a column cut into
+// buckets of 2^shift key values; pos[b] is the position of the first key not
+// below bucket b's first value (pos[buckets] = n, padded to whole groups of
+// four), so the lower bound of a key of bucket b lies in [pos[b], pos[b + 1]].
+// One load replaces the search above that window.  A narrow window is read
+// from its start; in a wide one the key's place in its bucket says where.
+// 2^26 Zipf(0.5) probes: binary search over 2^26 uniform keys 14.3 ms (sampled
+// keys in shared memory, then halving) against 1.57, at the part's random
+// access rate; over 2^20 keys 3.39 ms against 0.57.
+// ---------------------------------------------------------------------------
+struct key_start {
+    const uint32_t* pos;  // null: the index has none
+    uint64_t min_key;
+    uint64_t range;       // max_key - min_key
+    uint32_t shift;
+    uint32_t col_aligned;
+    float inv_width;      // 2^-shift
+};
+
+// lower bound (n past the last key); *eq: it is the position of an equal key
+template <bool kScattered = true, bool kCount = false>
+GJ_DEVICE_INLINE uint32_t start_lower_bound(const key_start& t, const uint64_t* col, uint32_t n, uint64_t key,
+                                            bool* eq, uint32_t* loads = nullptr) {
+    constexpr int kTable = kScattered ? kL2Keep : kL2Default;
+    constexpr int kColumn = kScattered ? kL2StreamLine : kL2Default;
+    *eq = false;
+    const uint64_t off = key - t.min_key;
+    if (off > t.range) return key < t.min_key ? 0u : n;
+    // entries b and b + 1: one 16-byte load unless b is the last of its four
+    const uint32_t b = (uint32_t)(off >> t.shift), q = b & 3u;
+    uint64_t e[2];
+    ld_pair_c<kTable>(reinterpret_cast<const uint64_t*>(t.pos + (b - q)), e);
+    const uint64_t w = q < 2 ? e[0] : e[1];
+    const uint32_t lo = (q & 1) ? (uint32_t)(w >> 32) : (uint32_t)w;
+    const uint32_t hi = q == 3 ? ld_ro(t.pos + b + 1) : (q & 1) ? (uint32_t)e[1] : (uint32_t)(w >> 32);
+    // the answer may be hi, the next bucket's first key: never an equal one
+    if (lo >= hi) return lo;
+    if (!t.col_aligned) return (uint32_t)lower_bound_sectors<kColumn>(col, n, lo, hi, key, false, eq);
+    const uint32_t sl = lo >> 2, sr = (hi - 1) >> 2;
+    uint32_t s = sl;
+    if (sr - sl > 1) {
+        const float in = (float)(off & ((1ull << t.shift) - 1)) * t.inv_width;  // place of the key in its bucket
+        s = (lo + (uint32_t)(in * (float)(hi - lo))) >> 2;
+        s = s > sr ? sr : s;
+    }
+    uint32_t edge;
+    return search_sectors<kColumn, kCount>(col, n, sl, sr, s, key, eq, &edge, loads);
 }
 
 // ---------------------------------------------------------------------------
@@ -397,16 +525,18 @@ GJ_DEVICE_INLINE uint32_t btree_cx_child(const btree_view& v, const uint32_t (&w
 
 // leaf reached for key through compressed nodes (open slots left, or exact),
 // starting at node j (base B) of level l; l = 0 means j is the leaf
-template <int W, int kInner, bool kExact>
+template <int W, int kInner, bool kExact, bool kCached = true>
 GJ_DEVICE_INLINE uint32_t btree_cx_descend(const btree_view& v, const uint64_t* cache, uint64_t key, int l,
                                            uint32_t j, uint64_t B) {
     constexpr int kLog = btree_cx_log<W>;
     const int first_global = (int)v.height - (int)v.cached_levels;
     uint64_t span = l >= 1 ? (uint64_t)v.leaf_keys << (kLog * (l - 1)) : 0;  // column keys under one child
     uint32_t w[8];
-    for (; l > first_global; --l, span >>= kLog) {
-        btree_cx_node<kInner>(v, cache, l, j, true, w);
-        j = (j << kLog) + btree_cx_child<W, kInner, kExact>(v, w, j, span, key, &B);
+    if constexpr (kCached) {
+        for (; l > first_global; --l, span >>= kLog) {
+            btree_cx_node<kInner>(v, cache, l, j, true, w);
+            j = (j << kLog) + btree_cx_child<W, kInner, kExact>(v, w, j, span, key, &B);
+        }
     }
     for (; l >= 1; --l, span >>= kLog) {
         btree_cx_node<kInner>(v, cache, l, j, false, w);
@@ -461,13 +591,14 @@ struct btree_cursor {
 
 GJ_DEVICE_INLINE btree_cursor btree_root(const btree_view& v) { return {v.min_key, 0u, (int32_t)v.height}; }
 
-template <int W, int kInner>
+template <int W, int kInner, bool kCached = true>
 GJ_DEVICE_INLINE uint32_t btree_plain_descend(const btree_view& v, const uint64_t* cache, uint64_t key, int l,
                                               uint32_t j) {
     constexpr uint32_t F = W + 1;
     // node and leaf numbers are below 2^32 (at most one leaf per key)
     const int first_global = (int)v.height - (int)v.cached_levels;  // levels <= this come from global memory
-    for (; l > first_global; --l) j = j * F + btree_node_search<W>(cache + v.smem_offset[l] + j * W, key, true);
+    if constexpr (kCached)
+        for (; l > first_global; --l) j = j * F + btree_node_search<W>(cache + v.smem_offset[l] + j * W, key, true);
     for (; l >= 1; --l) j = j * F + btree_node_search<W, kInner>(v.level[l] + (uint64_t)j * W, key, false);
     return j;
 }
@@ -478,8 +609,9 @@ GJ_DEVICE_INLINE uint32_t btree_plain_descend(const btree_view& v, const uint64_
 // of the inner levels: both use the default class then.
 //
 // The search starts at `from`, a node on the key's path (the root, or the
-// deepest node shared by the paths of a run of sorted probes).
-template <int W, bool kScattered = true>
+// deepest node shared by the paths of a run of sorted probes).  kCached: the
+// top cached_levels levels are in the shared cache (else cache is not read).
+template <int W, bool kScattered = true, bool kCached = true>
 GJ_DEVICE_INLINE uint32_t btree_lookup_from(const btree_view& v, const uint64_t* cache, uint64_t key,
                                             const btree_cursor& from) {
     constexpr int kInner = kScattered ? kL2Keep : kL2Default;
@@ -487,8 +619,8 @@ GJ_DEVICE_INLINE uint32_t btree_lookup_from(const btree_view& v, const uint64_t*
     constexpr bool kCompressed = W == (int)kBtreeCompressed || W == (int)kBtreeCompressed16;
     if (key > v.max_key || key < v.min_key) return kInvalid;
     uint64_t j;
-    if constexpr (kCompressed) j = btree_cx_descend<W, kInner, false>(v, cache, key, from.level, from.node, from.base);
-    else j = btree_plain_descend<W, kInner>(v, cache, key, from.level, from.node);
+    if constexpr (kCompressed) j = btree_cx_descend<W, kInner, false, kCached>(v, cache, key, from.level, from.node, from.base);
+    else j = btree_plain_descend<W, kInner, kCached>(v, cache, key, from.level, from.node);
     // leaf j: column slice [j*L, min(j*L + L, n))
     uint64_t base = j * v.leaf_keys;
     uint64_t end = base + v.leaf_keys < v.n ? base + v.leaf_keys : v.n;
@@ -508,7 +640,7 @@ GJ_DEVICE_INLINE uint32_t btree_lookup_from(const btree_view& v, const uint64_t*
     if constexpr (kCompressed) {
         // a wrong left turn: search again, open slots resolved exactly
         if (pos == end && end < v.n) {  // a wrong left turn: search again, open slots resolved exactly
-            j = btree_cx_descend<W, kInner, true>(v, cache, key, (int)v.height, 0u, v.min_key);
+            j = btree_cx_descend<W, kInner, true, kCached>(v, cache, key, (int)v.height, 0u, v.min_key);
             base = j * v.leaf_keys;
             end = base + v.leaf_keys < v.n ? base + v.leaf_keys : v.n;
             pos = lower_bound_sectors<kColumn>(v.col, v.n, base, end, key, v.col_aligned, &eq);
@@ -519,13 +651,13 @@ GJ_DEVICE_INLINE uint32_t btree_lookup_from(const btree_view& v, const uint64_t*
 
 // A scattered lookup starts at its key bucket's entry of the start table:
 // one 16-byte load in place of the levels above that node.
-template <int W, bool kScattered = true>
+template <int W, bool kScattered = true, bool kCached = true>
 GJ_DEVICE_INLINE uint32_t btree_lookup(const btree_view& v, const uint64_t* cache, uint64_t key) {
     if (key > v.max_key || key < v.min_key) return kInvalid;
-    if (v.start == nullptr) return btree_lookup_from<W, kScattered>(v, cache, key, btree_root(v));
+    if (v.start == nullptr) return btree_lookup_from<W, kScattered, kCached>(v, cache, key, btree_root(v));
     uint64_t e[2];
     ld_pair_c<kScattered ? kL2Keep : kL2Default>(v.start + 2 * ((key - v.min_key) >> v.start_shift), e);
-    return btree_lookup_from<W, kScattered>(v, cache, key, {e[0], (uint32_t)e[1], (int32_t)(e[1] >> 32)});
+    return btree_lookup_from<W, kScattered, kCached>(v, cache, key, {e[0], (uint32_t)e[1], (int32_t)(e[1] >> 32)});
 }
 
 // The deepest node on the paths of both lo and hi (lo <= hi): every key in
@@ -646,11 +778,21 @@ struct harmonia_view {
     uint32_t start_entries;
 };
 
+// A node's first child is 33 * node plus a constant of its level: every node
+// before it on the level is full.  The library's kernels carry the constants
+// (children is the same numbers as a table, for kernels that only have the
+// view).
+struct harmonia_child_base {
+    int64_t of[16];  // by level, root 1 (index 0 unused)
+};
+
 // Shared cache layout: cached_nodes * 32 keys, then cached_nodes children.
-// A node's child offset does not depend on the search, so it is loaded
-// alongside the node's keys.
-template <bool kScattered = true>
-GJ_DEVICE_INLINE uint32_t harmonia_lookup(const harmonia_view& v, const uint64_t* cache, uint64_t key) {
+// A node's child offset does not depend on the search: it is computed from
+// the level's constant, or loaded alongside the node's keys.
+// kCached: top levels may be staged in shared memory.
+template <bool kScattered = true, bool kCached = true>
+GJ_DEVICE_INLINE uint32_t harmonia_lookup(const harmonia_view& v, const uint64_t* cache, uint64_t key,
+                                          const harmonia_child_base* base = nullptr) {
     constexpr int kInner = kScattered ? kL2Keep : kL2Default;
     constexpr int kColumn = kScattered ? kL2Stream : kL2Default;
     constexpr uint32_t K = kHarmoniaKeys;
@@ -669,7 +811,7 @@ GJ_DEVICE_INLINE uint32_t harmonia_lookup(const harmonia_view& v, const uint64_t
     for (uint32_t d = d0; d < depth; ++d) {
         uint32_t lb;
         uint64_t child;
-        if (d <= v.cached_levels) {
+        if (kCached && d <= v.cached_levels) {
             const uint64_t* node = cache + pos * K;
             uint32_t c = 0;
 #pragma unroll
@@ -677,7 +819,7 @@ GJ_DEVICE_INLINE uint32_t harmonia_lookup(const harmonia_view& v, const uint64_t
             lb = c + ((node[c] < key) ? 1u : 0u);
             child = cache[(uint64_t)v.cached_nodes * K + pos];
         } else {
-            child = ld_ro_c<kInner>(v.children + pos);
+            child = base ? pos * (K + 1) + (uint64_t)base->of[d] : ld_ro_c<kInner>(v.children + pos);
             bool eq;
             lb = (uint32_t)lower_bound_sectors<kInner>(v.keys + pos * K, K, 0, K, key, true, &eq);
         }
@@ -821,12 +963,13 @@ GJ_DEVICE_INLINE uint32_t harmonia_lookup_cooperative(bool active, const harmoni
 // ---------------------------------------------------------------------------
 // A spline point (src/rs.cuh:22-52: Coord{x, y}) with the slope of the
 // segment to the next point, computed at build with the same double
-// division the estimate would make: one 32-byte sector, one load per segment.
+// division the estimate would make, and once more in fixed point: one 32-byte
+// sector, one load per segment.
 struct rs_point {
     uint64_t x;
-    double y;
+    double y;      // a position: a whole number below 2^32
     double slope;  // (y[i+1] - y[i]) / (x[i+1] - x[i]); 0 for the last point
-    uint64_t pad;
+    uint64_t step; // shift | floor(dy * 2^64 / (dx << shift)) << 6, dx << shift in [2^63, 2^64)
 };
 static_assert(sizeof(rs_point) == 32, "a spline point is one sector");
 
@@ -842,9 +985,18 @@ struct rs_view {
     uint32_t pad;
 };
 
-GJ_DEVICE_INLINE double rs_estimate(const rs_view& v, uint64_t key) {
-    if (key <= v.min_key) return 0.0;
-    if (key >= v.max_key) return (double)(v.n - 1);
+// a whole number below 2^53 held in a double, by its bits: GB300 runs double
+// arithmetic and conversions at a small fraction of its integer rate
+GJ_DEVICE_INLINE uint32_t whole_of_double(uint64_t bits) {
+    const uint32_t e = (uint32_t)(bits >> 52);
+    return e < 1023u ? 0u : (uint32_t)(((bits & ((1ull << 52) - 1)) | (1ull << 52)) >> (1075u - e));
+}
+
+// The spline's estimate of a key's position, rounded down and at most two
+// below the real value: y + (key - x) * slope in 64-bit fixed point.
+GJ_DEVICE_INLINE uint32_t rs_estimate(const rs_view& v, uint64_t key) {
+    if (key <= v.min_key) return 0;
+    if (key >= v.max_key) return (uint32_t)(v.n - 1);
     const uint64_t prefix = (key - v.min_key) >> v.shift;
     const uint32_t b = ld_ro(v.table + prefix);
     const uint32_t e = ld_ro(v.table + prefix + 1);
@@ -862,17 +1014,28 @@ GJ_DEVICE_INLINE double rs_estimate(const rs_view& v, uint64_t key) {
     // segment [lo - 1, lo]: its left point and precomputed slope
     uint64_t w[4];
     ld_sector(reinterpret_cast<const uint64_t*>(v.pts + lo - 1), w);
-    return __dadd_rn(__dmul_rn((double)(key - w[0]), __longlong_as_double((long long)w[2])),
-                     __longlong_as_double((long long)w[1]));
+    return whole_of_double(w[1]) + (uint32_t)__umul64hi((key - w[0]) << (w[3] & 63u), w[3] >> 6);
 }
 
-// lower bound inside [b, e), widened to the whole column when the window
-// does not bracket it (possible only for keys outside the column)
+// lower bound expected inside [b, e) and near `guess`, widened to the whole
+// column when the window turns out not to bracket it (possible only for keys
+// outside the column)
 template <bool kScattered = true>
-GJ_DEVICE_INLINE uint64_t window_lower_bound(const uint64_t* col, uint64_t n, uint64_t b, uint64_t e, uint64_t key,
-                                             bool aligned) {
+GJ_DEVICE_INLINE uint64_t window_lower_bound(const uint64_t* col, uint64_t n, uint64_t b, uint64_t e, uint64_t guess,
+                                             uint64_t key, bool aligned) {
+    constexpr int kColumn = kScattered ? kL2StreamLine : kL2Default;
     bool eq;
-    uint64_t pos = lower_bound_sectors<kScattered ? kL2Stream : kL2Default>(col, n, b, e, key, aligned, &eq);
+    uint64_t pos;
+    if (aligned && b < e) {
+        const uint32_t sl = (uint32_t)(b >> 2), sr = (uint32_t)((e - 1) >> 2);
+        const uint32_t s = (uint32_t)(guess >> 2);
+        uint32_t edge;
+        pos = search_sectors<kColumn>(col, (uint32_t)n, sl, sr, s < sl ? sl : s > sr ? sr : s, key, &eq, &edge);
+        if ((edge == 1 && pos > 0 && ld_ro(col + pos - 1) >= key) || (edge == 2 && pos < n && ld_ro(col + pos) < key))
+            pos = lower_bound_sectors(col, n, 0, n, key, aligned, &eq);
+        return pos;
+    }
+    pos = lower_bound_sectors<kColumn>(col, n, b, e, key, aligned, &eq);
     if ((pos == b && b > 0 && ld_ro(col + b - 1) >= key) || (pos == e && e < n && ld_ro(col + e) < key))
         pos = lower_bound_sectors(col, n, 0, n, key, aligned, &eq);
     return pos;
@@ -880,12 +1043,11 @@ GJ_DEVICE_INLINE uint64_t window_lower_bound(const uint64_t* col, uint64_t n, ui
 
 template <bool kScattered = true>
 GJ_DEVICE_INLINE uint32_t rs_lookup(const rs_view& v, uint64_t key) {
-    const double est = rs_estimate(v, key);
-    const double err = (double)v.max_error;
-    uint64_t b = est < err ? 0 : (uint64_t)(est - err);
-    uint64_t e = (est + err + 2 > (double)v.n) ? v.n : (uint64_t)(est + err + 2);
-    if (b > e) b = e;
-    const uint64_t pos = window_lower_bound<kScattered>(v.col, v.n, b, e, key, v.col_aligned);
+    const uint64_t est = rs_estimate(v, key), err = v.max_error;
+    // the real estimate lies in [est, est + 2]
+    const uint64_t b = est < err ? 0 : est - err;
+    const uint64_t e = est + err + 4 > v.n ? v.n : est + err + 4;
+    const uint64_t pos = window_lower_bound<kScattered>(v.col, v.n, b, e, est, key, v.col_aligned);
     return pos < v.n ? (uint32_t)pos : kInvalid;
 }
 
@@ -987,6 +1149,10 @@ GJ_DEVICE_INLINE float learned_norm(const learned_view& v, uint64_t key) {
 // below segment i's first key: the key CDF, exact at every segment end and
 // linear in between.  It reads the table from global memory (v.root), not
 // from `root`, which holds the by-value parameters of the other kinds.
+//
+// kMlp = false: the caller knows the root is not an MLP (its kernel then
+// needs half the registers).
+template <bool kMlp = true>
 GJ_DEVICE_INLINE uint32_t learned_route(const learned_view& v, const float* root, float x) {
     float r;
     if (v.root_kind == GJ_LEARNED_ROOT_SEGMENTS) {
@@ -994,7 +1160,7 @@ GJ_DEVICE_INLINE uint32_t learned_route(const learned_view& v, const float* root
         const uint32_t i = min((uint32_t)t, v.segments - 1);
         const float2 s = __ldg(reinterpret_cast<const float2*>(v.root) + i);
         r = fmaf(t - (float)i, s.y, s.x);
-    } else if (v.root_kind == GJ_LEARNED_ROOT_MLP)
+    } else if (kMlp && v.root_kind == GJ_LEARNED_ROOT_MLP)
         r = v.hidden <= 16 ? mlp_forward<16>(root, x) : mlp_forward<32>(root, x);
     else
         r = fmaf(root[0], x, root[1]);
@@ -1013,9 +1179,9 @@ GJ_DEVICE_INLINE int64_t learned_predict(const learned_leaf& lf, uint64_t key) {
     return (int64_t)lf.base + (int64_t)off;
 }
 
-template <bool kScattered = true>
+template <bool kScattered = true, bool kMlp = true>
 GJ_DEVICE_INLINE uint32_t learned_lookup(const learned_view& v, const float* root, uint64_t key) {
-    const uint32_t li = learned_route(v, root, learned_norm(v, key));
+    const uint32_t li = learned_route<kMlp>(v, root, learned_norm(v, key));
     uint64_t w[4];
     ld_sector_c<kScattered ? kL2Keep : kL2Default>(reinterpret_cast<const uint64_t*>(v.leaves + li), w);
     learned_leaf lf;
@@ -1033,7 +1199,9 @@ GJ_DEVICE_INLINE uint32_t learned_lookup(const learned_view& v, const float* roo
     lo = lo < 0 ? 0 : (lo > n ? n : lo);
     hi = hi < 0 ? 0 : (hi > n ? n : hi);
     if (lo > hi) lo = hi;
-    const uint64_t pos = window_lower_bound<kScattered>(v.col, v.n, (uint64_t)lo, (uint64_t)hi, key, v.col_aligned);
+    const int64_t at = pred < lo ? lo : pred > hi ? hi : pred;
+    const uint64_t pos =
+        window_lower_bound<kScattered>(v.col, v.n, (uint64_t)lo, (uint64_t)hi, (uint64_t)at, key, v.col_aligned);
     return pos < v.n ? (uint32_t)pos : kInvalid;
 }
 

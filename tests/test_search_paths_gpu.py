@@ -1,0 +1,75 @@
+"""Scattered lookups on the columns where the key start table, the searches
+from a guess and the launch shape can go wrong, against the oracle: columns
+of a few keys, sizes around a sector and a table group, runs of consecutive
+keys, two scales of clusters (wide windows the guess misses), the extreme
+keys, unaligned columns, and probe counts around a block and a launch-shape
+threshold."""
+import numpy as np
+import pytest
+
+from test_lookup_gpu import column, expected, from_dev_u32, probes_for, to_dev
+
+pytestmark = pytest.mark.gpu
+
+KINDS = ["binary_search", "btree", "harmonia", "radix_spline", "learned"]
+
+
+def _columns(case, rng):
+    if case == "tiny":
+        for n in (1, 2, 3, 4, 5, 7, 8, 9, 31, 33, 63, 64, 65):
+            yield column(rng, n)
+    elif case == "run":
+        yield np.arange(100, 100 + 4096, dtype=np.uint64)
+        yield np.arange((1 << 64) - 5000, (1 << 64) - 1, dtype=np.uint64)
+    elif case == "extremes":
+        mid = column(rng, 4094)
+        yield np.unique(np.concatenate([[0], mid, [(1 << 64) - 1]]).astype(np.uint64))
+        yield np.array([0, (1 << 64) - 1], dtype=np.uint64)
+    elif case == "two_scales":
+        # clusters of clusters: every bucket holds either nothing or far too much
+        big = np.sort(rng.choice(1 << 20, size=24, replace=False).astype(np.uint64)) << np.uint64(42)
+        small = np.sort(rng.choice(1 << 16, size=64, replace=False).astype(np.uint64)) << np.uint64(14)
+        fine = np.unique(rng.integers(0, 1 << 13, size=96, dtype=np.uint64))
+        yield np.unique((big[:, None, None] + small[None, :, None] + fine[None, None, :]).ravel())
+    else:  # "uniform"
+        for n in (1023, 1024, 1025, 100_003):
+            yield column(rng, n)
+
+
+@pytest.mark.parametrize("shift", [0, 1])
+@pytest.mark.parametrize("kind", KINDS)
+@pytest.mark.parametrize("case", ["tiny", "run", "extremes", "two_scales", "uniform"])
+def test_scattered_lookups(orc, gj, cuda, case, kind, shift):
+    import torch
+
+    rng = np.random.default_rng(len(case) * 7 + len(kind))
+    for col in _columns(case, rng):
+        if kind == "harmonia":
+            col = col[: len(col) // 32 * 32]
+            if not len(col):
+                continue
+        pr = probes_for(rng, col, 3000)
+        d = to_dev(torch, np.concatenate([np.zeros(4 - shift, dtype=np.uint64), col]))[4 - shift:]
+        assert (d.data_ptr() % 32 == 0) == (shift == 0)
+        ix = gj.make_index(kind).construct(None, d)
+        np.testing.assert_array_equal(from_dev_u32(ix.lookup(to_dev(torch, pr))), expected(orc, kind, col, pr),
+                                      err_msg=f"{len(col)} keys")
+
+
+@pytest.mark.parametrize("kind", ["btree", "hash", "learned"])
+@pytest.mark.parametrize("m", [255, 256, 257, 311_297, 16 * 152 * 8 * 256 - 1, 16 * 152 * 8 * 256 + 513])
+def test_launch_shapes(orc, gj, cuda, kind, m):
+    import torch
+
+    rng = np.random.default_rng(m)
+    col = column(rng, 40_000)
+    pr = rng.choice(col, size=m)
+    pr[::17] += np.uint64(1)
+    ix = gj.make_index(kind).construct(None, to_dev(torch, col))
+    d_pr = to_dev(torch, pr)
+    exp = expected(orc, kind, col, pr)
+    np.testing.assert_array_equal(from_dev_u32(ix.lookup(d_pr)), exp)
+    rows = torch.randperm(m, device="cuda").to(torch.int32)
+    out = torch.empty(m, dtype=torch.int32, device="cuda")
+    ix.partitioned_lookup(d_pr, rows, out)
+    np.testing.assert_array_equal(from_dev_u32(out)[rows.cpu().numpy()], exp)
