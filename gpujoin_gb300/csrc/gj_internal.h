@@ -173,10 +173,9 @@ int pairs_error_flag(void* ws, size_t ws_bytes, uint64_t m, unsigned int* flag, 
 size_t partition_ws_bytes(uint64_t m, uint32_t radix_bits, int sm_count);
 // The way back from a partitioned relation to probe order, left by a
 // partition pass that is given one (it then writes no row ids): every key's
-// offset inside its tile, and per tile and partition where the run went.
+// offset inside its tile, and per tile where its runs begin in its sorted order.
 struct partition_inverse {
     uint16_t* offsets;  // m, in relation order
-    uint32_t* delta;    // tiles x fanout
     uint16_t* start;    // tiles x fanout
 };
 // room for one of m probes inside ws; false when ws is too small for it
@@ -188,8 +187,9 @@ constexpr uint32_t kValueTile = 2048;
 __host__ __device__ inline uint64_t value_index(uint32_t d) {
     return (uint64_t)(d / kValueTile) * (2 * kValueTile) + d % kValueTile;
 }
-int gather_values(const uint32_t* d_values, uint64_t m, uint32_t radix_bits, const partition_inverse& iv,
-                  uint32_t* d_out, cudaStream_t s);
+// (ws: the partition pass's workspace, not written since)
+int gather_values(const uint32_t* d_values, uint64_t m, uint32_t radix_bits, void* ws, size_t ws_bytes,
+                  const partition_inverse& iv, uint32_t* d_out, cudaStream_t s);
 int range_partition_impl(const uint64_t* d_keys, uint64_t m, uint64_t min_key, uint32_t shift, uint32_t radix_bits,
                          uint64_t row_base, uint64_t* d_out_keys, uint32_t* d_out_rows, uint64_t* d_offsets, void* ws,
                          size_t ws_bytes, cudaStream_t s, const partition_inverse* inverse = nullptr);

@@ -9,10 +9,12 @@
 // maps onto one contiguous slice of the index and a window's lookups walk the
 // index in order (the slices stay resident in the 126 MB L2).
 //
-// A partition pass (all on the caller's stream):
-//   1. k_part_hist   per-block histograms of the keys
-//   2. scan          exclusive offsets, partition-major (p, block)
-//   3. k_part_scatter keys and row ids to their partition, in block order
+// The keys are cut into tiles.  A partition pass (all on the caller's stream):
+//   1. k_part_hist    per tile and partition, how many keys the tile's chunk
+//                     (a run of tiles, one block's) has before the tile
+//   2. k_part_base    where each chunk's keys start in each partition
+//   3. k_part_scatter keys and row ids to their partition, in tile order
+// and, for callers that want values back in probe order, k_part_gather.
 // The windowed partitioned INLJ that drives it is in gj_partitioned.cu.
 #include <cuda_runtime.h>
 
@@ -24,20 +26,7 @@
 namespace gj {
 namespace {
 
-constexpr int kPartBlock = 512;
 constexpr uint32_t kMaxRadixBits = 12;
-constexpr int kHistUnroll = 8;                                    // keys in flight per thread
-// scatter geometry: block size and resident blocks per SM (its register cap)
-#ifndef GJ_SCATTER_BLOCK
-#define GJ_SCATTER_BLOCK 512
-#endif
-#ifndef GJ_SCATTER_PER_SM
-#define GJ_SCATTER_PER_SM 3
-#endif
-constexpr int kScatterBlock = GJ_SCATTER_BLOCK;
-constexpr int kScatterPerSM = GJ_SCATTER_PER_SM;
-constexpr int kScatterItems = 8;                                  // keys per thread per tile
-constexpr uint32_t kScatterTile = kScatterBlock * kScatterItems;
 
 __device__ __forceinline__ uint32_t part_of(uint64_t key, uint64_t min_key, uint32_t shift, uint32_t fanout) {
     if (key <= min_key) return 0;
@@ -45,55 +34,81 @@ __device__ __forceinline__ uint32_t part_of(uint64_t key, uint64_t min_key, uint
     return p >= fanout ? fanout - 1 : (uint32_t)p;
 }
 
+// What the passes share.  The j-th key of tile t that goes to partition p
+// lands at before[t * fanout + p] + chunk_start[c * fanout + p] + part_start[p]
+// + j of the relation (c: the chunk of t), all below 2^32.
+struct part_tables {
+    uint32_t* before;       // tiles x fanout
+    uint32_t* chunk_start;  // chunks x fanout; the histogram leaves chunk counts, k_part_base their prefixes
+    uint32_t* part_start;   // fanout
+    uint32_t* done;         // blocks of k_part_base that are through
+    uint32_t tiles, tiles_per_chunk, chunks, fanout;
+};
+struct part_func {
+    uint64_t min_key;
+    uint32_t shift;
+};
+
 // sub-histograms per block: warps spread their shared-memory atomics over
 // several copies when the fanout is small (fewer same-address conflicts)
 __host__ __device__ __forceinline__ uint32_t hist_copies(uint32_t fanout) {
-    uint32_t c = 16;  // one per warp of kPartBlock
-    while (c > 1 && (size_t)c * fanout * sizeof(uint32_t) > 32768) c >>= 1;
+    uint32_t c = 16;
+    while (c > 1 && (size_t)c * fanout * sizeof(uint32_t) > 16384) c >>= 1;
     return c;
 }
 
-// hist[p * G + b] = number of keys of block b's chunk in partition p (kB
-// threads a block: 512, or 1024 when the scatter runs one block per SM)
-template <int kB>
-__global__ void __launch_bounds__(kB) k_part_hist(const uint64_t* __restrict__ keys, uint64_t m, uint64_t chunk,
-                                                  uint64_t min_key, uint32_t shift, uint32_t fanout,
-                                                  uint64_t* __restrict__ hist) {
-    extern __shared__ uint32_t s_hist[];
-    const uint32_t copies = hist_copies(fanout);
-    for (uint32_t p = threadIdx.x; p < fanout * copies; p += blockDim.x) s_hist[p] = 0;
-    __syncthreads();
-    uint32_t* mine = s_hist + ((threadIdx.x >> 5) & (copies - 1)) * fanout;
-    const uint64_t b0 = blockIdx.x * chunk, b1 = min(m, b0 + chunk);
+// One block per chunk, tile after tile; the histogram is double buffered, so
+// one barrier a tile suffices.  Bound by HBM (8 bytes a key).
+template <int kB, int kTile>
+__global__ void __launch_bounds__(kB) k_part_hist(const uint64_t* __restrict__ keys, uint64_t m, part_func f,
+                                                  part_tables t) {
+    constexpr int kIt = kTile / kB;
+    extern __shared__ uint32_t s_hist[];  // 2 x copies x fanout, then the chunk's counts so far
+    const uint32_t fanout = t.fanout, copies = hist_copies(fanout);
+    uint32_t* s_run = s_hist + 2 * copies * fanout;
+    for (uint32_t p = threadIdx.x; p < (2 * copies + 1) * fanout; p += kB) s_hist[p] = 0;
+    if (blockIdx.x == 0 && threadIdx.x == 0) *t.done = 0;
+    const uint32_t first = blockIdx.x * t.tiles_per_chunk, last = min(t.tiles, first + t.tiles_per_chunk);
     const unsigned long long* k64 = reinterpret_cast<const unsigned long long*>(keys);
-    for (uint64_t i = b0 + threadIdx.x; i < b1; i += (uint64_t)kB * kHistUnroll) {
-        uint64_t k[kHistUnroll];
+    uint64_t next[kIt];
+    auto load = [&](uint32_t tile) {
 #pragma unroll
-        for (int u = 0; u < kHistUnroll; ++u) {
-            const uint64_t j = i + (uint64_t)u * kB;
-            k[u] = j < b1 ? __ldcs(k64 + j) : 0ull;
+        for (int k = 0; k < kIt; ++k) {
+            const uint64_t i = (uint64_t)tile * kTile + k * kB + threadIdx.x;
+            next[k] = i < m ? __ldcs(k64 + i) : 0ull;
         }
+    };
+    load(first);
+    __syncthreads();
+    for (uint32_t tile = first; tile < last; ++tile) {
+        uint32_t* buf = s_hist + (tile & 1) * copies * fanout;
+        uint32_t* mine = buf + ((threadIdx.x >> 5) & (copies - 1)) * fanout;
+        uint64_t key[kIt];
 #pragma unroll
-        for (int u = 0; u < kHistUnroll; ++u)
-            if (i + (uint64_t)u * kB < b1) atomicAdd(&mine[part_of(k[u], min_key, shift, fanout)], 1u);
+        for (int k = 0; k < kIt; ++k) key[k] = next[k];
+        if (tile + 1 < last) load(tile + 1);
+#pragma unroll
+        for (int k = 0; k < kIt; ++k)
+            if ((uint64_t)tile * kTile + k * kB + threadIdx.x < m)
+                atomicAdd(&mine[part_of(key[k], f.min_key, f.shift, fanout)], 1u);
+        __syncthreads();
+        for (uint32_t p = threadIdx.x; p < fanout; p += kB) {
+            uint32_t c = 0;
+            for (uint32_t q = 0; q < copies; ++q) {
+                c += buf[q * fanout + p];
+                buf[q * fanout + p] = 0;  // for the tile after the next, behind the next barrier
+            }
+            const uint32_t run = s_run[p];
+            __stcs(t.before + (uint64_t)tile * fanout + p, run);
+            s_run[p] = run + c;
+        }
     }
     __syncthreads();
-    for (uint32_t p = threadIdx.x; p < fanout; p += blockDim.x) {
-        uint32_t c = 0;
-        for (uint32_t q = 0; q < copies; ++q) c += s_hist[q * fanout + p];
-        hist[(uint64_t)p * gridDim.x + blockIdx.x] = c;
-    }
-}
-
-// offsets[p] = start of partition p (inclusive scan of hist, read at the
-// previous partition's last block); offsets[fanout] = m
-__global__ void k_part_offsets(const uint64_t* __restrict__ incl, uint32_t fanout, uint32_t nblocks, uint64_t m,
-                               uint64_t* __restrict__ offsets) {
-    for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p <= fanout; p += gridDim.x * blockDim.x)
-        offsets[p] = p == 0 ? 0 : (p == fanout ? m : incl[(uint64_t)p * nblocks - 1]);
+    for (uint32_t p = threadIdx.x; p < fanout; p += kB) t.chunk_start[(uint64_t)blockIdx.x * fanout + p] = s_run[p];
 }
 
 // out[p] = sum of in[0..p) over count entries, by the whole block of kB threads
+// (in == out is fine)
 template <int kB>
 __device__ __forceinline__ void block_exclusive_scan(const uint32_t* in, uint32_t* out, uint32_t count) {
     __shared__ uint32_t s_warp[kB / 32];
@@ -106,8 +121,8 @@ __device__ __forceinline__ void block_exclusive_scan(const uint32_t* in, uint32_
     uint32_t incl = sum;
 #pragma unroll
     for (int d = 1; d < 32; d <<= 1) {
-        const uint32_t t = __shfl_up_sync(0xffffffffu, incl, d);
-        if (lane >= (uint32_t)d) incl += t;
+        const uint32_t v = __shfl_up_sync(0xffffffffu, incl, d);
+        if (lane >= (uint32_t)d) incl += v;
     }
     if (lane == 31) s_warp[warp] = incl;
     __syncthreads();
@@ -117,8 +132,8 @@ __device__ __forceinline__ void block_exclusive_scan(const uint32_t* in, uint32_
         uint32_t w = v;
 #pragma unroll
         for (int d = 1; d < 32; d <<= 1) {
-            const uint32_t t = __shfl_up_sync(0xffffffffu, w, d);
-            if (lane >= (uint32_t)d) w += t;
+            const uint32_t x = __shfl_up_sync(0xffffffffu, w, d);
+            if (lane >= (uint32_t)d) w += x;
         }
         if (lane < kWarps) s_warp[lane] = w - v;
     }
@@ -126,241 +141,145 @@ __device__ __forceinline__ void block_exclusive_scan(const uint32_t* in, uint32_
     uint32_t run = s_warp[warp] + incl - sum;
     for (uint32_t q = 0; q < per; ++q)
         if (begin + q < count) {
+            const uint32_t v = in[begin + q];
             out[begin + q] = run;
-            run += in[begin + q];
+            run += v;
         }
 }
 
-// Where tile t of the relation's runs went: the j-th key of the tile in
-// partition order lies at relation index delta[p] + j (modulo 2^32: m is below
-// it), p being the partition whose run [start[p], start[p + 1]) holds j.
-// Tiles are numbered block by block, every block's share rounded up to whole
-// tiles.
-__device__ __forceinline__ uint64_t tile_number(uint64_t t0, uint64_t b0, uint64_t chunk, uint32_t tile) {
-    return blockIdx.x * ((chunk + tile - 1) / tile) + (t0 - b0) / tile;
-}
-__device__ __forceinline__ void leave_run(const partition_inverse& iv, uint64_t tile, uint32_t fanout, uint32_t p,
-                                          uint64_t delta, uint32_t start) {
-    iv.delta[tile * fanout + p] = (uint32_t)delta;
-    iv.start[tile * fanout + p] = (uint16_t)start;
+// Chunk counts to chunk prefixes, 32 partitions a block (lane = partition, a
+// warp takes a run of chunks); the last block to finish scans the partitions'
+// totals into their starts.  offsets (optional): the same as 64-bit, and m.
+constexpr int kBaseBlock = 1024;
+__global__ void __launch_bounds__(kBaseBlock) k_part_base(part_tables t, uint64_t m, uint64_t* __restrict__ offsets) {
+    constexpr uint32_t kWarps = kBaseBlock / 32;
+    __shared__ uint32_t s_sum[kWarps][33];
+    __shared__ bool s_last;
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, fanout = t.fanout;
+    const uint32_t p = blockIdx.x * 32 + lane;
+    const uint32_t per = (t.chunks + kWarps - 1) / kWarps;
+    const uint32_t c0 = min(warp * per, t.chunks), c1 = min(c0 + per, t.chunks);
+    uint32_t sum = 0;
+    if (p < fanout)
+        for (uint32_t c = c0; c < c1; ++c) sum += t.chunk_start[(uint64_t)c * fanout + p];
+    s_sum[warp][lane] = sum;
+    __syncthreads();
+    uint32_t run = 0;
+    for (uint32_t w = 0; w < warp; ++w) run += s_sum[w][lane];
+    if (p < fanout) {
+        for (uint32_t c = c0; c < c1; ++c) {
+            const uint32_t v = t.chunk_start[(uint64_t)c * fanout + p];
+            t.chunk_start[(uint64_t)c * fanout + p] = run;
+            run += v;
+        }
+        if (warp == kWarps - 1) t.part_start[p] = run;  // the partition's size, for the last block
+    }
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) s_last = atomicAdd(t.done, 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    extern __shared__ uint32_t s_part[];  // fanout
+    for (uint32_t q = threadIdx.x; q < fanout; q += kBaseBlock) s_part[q] = __ldcg(t.part_start + q);
+    __syncthreads();
+    block_exclusive_scan<kBaseBlock>(s_part, s_part, fanout);
+    __syncthreads();
+    for (uint32_t q = threadIdx.x; q < fanout; q += kBaseBlock) {
+        t.part_start[q] = s_part[q];
+        if (offsets) offsets[q] = s_part[q];
+    }
+    if (offsets && threadIdx.x == 0) offsets[fanout] = m;
 }
 
-// Scatter block b's chunk.  The flat (partition, block) order of the scanned
-// histogram makes the start of cell c the inclusive sum of cell c - 1, so the
-// keys are read once.  Each tile of kScatterTile keys is first grouped by
-// partition in shared memory (a counting sort whose ranks come from
-// shared-memory atomics), then every partition's run of the tile is written
-// with consecutive threads on consecutive addresses: whole sectors instead of
-// one scattered 8-byte store per key.  The order inside a partition follows
-// the block and tile order; inside a tile it is not fixed.
-// kScatterPerSM resident blocks (the register cap; about 52 KB of shared
-// memory per 512-thread block for fanouts up to 2^8)
+__device__ __forceinline__ uint32_t run_start(const part_tables& t, uint32_t tile, uint32_t p) {
+    return __ldcs(t.before + (uint64_t)tile * t.fanout + p) +
+           __ldg(t.chunk_start + (uint64_t)(tile / t.tiles_per_chunk) * t.fanout + p) + __ldg(t.part_start + p);
+}
+
+// Scatter, one block per tile: the tile's keys are grouped by partition in
+// shared memory (a counting sort whose ranks come from shared-memory
+// atomics), then every partition's run is written with consecutive threads on
+// consecutive addresses.  The order inside a partition follows the tiles;
+// inside a tile it is not fixed.
+//
+// Bound by HBM (8 bytes read, 12 written a key; 10 for kInverse) where the
+// runs are long, i.e. at low fanouts, and by the sectors two runs share where
+// they are short.  A run ends inside a sector that the next tile's run
+// completes: tiles run in order, so the two writes meet in L2 shortly after
+// one another.  (With one block per chunk of consecutive tiles instead, as
+// many streams were open as blocks x partitions, more lines than L2 holds at
+// fanout 2^11, and each half-written sector cost a DRAM access of its own:
+// 2.58 ms per 2^27 keys.)  Independent tiles also let one block's loads
+// overlap another's writes on an SM without a register prefetch.
 //
 // kInverse: instead of row ids the relation gets each key's offset inside its
-// tile (16 bits), and the tile leaves where its runs went (iv): what
-// k_part_gather needs to bring results back to probe order.
-template <bool kInverse>
-__global__ void __launch_bounds__(kScatterBlock, kScatterPerSM) k_part_scatter(const uint64_t* __restrict__ keys, uint64_t m,
-                                                             uint64_t chunk, uint64_t min_key, uint32_t shift,
-                                                             uint32_t fanout, const uint64_t* __restrict__ incl,
-                                                             uint64_t row_base, uint64_t* __restrict__ out_keys,
+// tile (16 bits), and the tile leaves where its runs begin in its sorted
+// order: what k_part_gather needs to bring results back to probe order.
+template <int kB, int kIt, int kPerSM, bool kInverse>
+__global__ void __launch_bounds__(kB, kPerSM) k_part_scatter(const uint64_t* __restrict__ keys, uint64_t m, part_func f,
+                                                             part_tables t, uint64_t row_base,
+                                                             uint64_t* __restrict__ out_keys,
                                                              uint32_t* __restrict__ out_rows, partition_inverse iv) {
+    constexpr uint32_t kTile = kB * kIt;
+    static_assert(kTile <= (1u << 13) && (1u << kMaxRadixBits) <= (1u << 19), "slot packing");
     extern __shared__ unsigned long long s_mem[];
-    uint64_t* s_keys = reinterpret_cast<uint64_t*>(s_mem);                       // kScatterTile
-    unsigned long long* s_dst = s_mem + kScatterTile;                            // fanout: next output slot
-    uint32_t* s_rows = reinterpret_cast<uint32_t*>(s_dst + fanout);              // kScatterTile
-    uint32_t* s_cnt = s_rows + kScatterTile;                                     // fanout
-    uint32_t* s_start = s_cnt + fanout;                                          // fanout
-    unsigned long long* s_delta = reinterpret_cast<unsigned long long*>(s_start + fanout);  // fanout
-    for (uint32_t p = threadIdx.x; p < fanout; p += blockDim.x) {
-        const uint64_t cell = (uint64_t)p * gridDim.x + blockIdx.x;
-        s_dst[p] = cell == 0 ? 0ull : incl[cell - 1];
-    }
-    const unsigned long long* k64 = reinterpret_cast<const unsigned long long*>(keys);
-    const uint64_t b0 = blockIdx.x * chunk, b1 = min(m, b0 + chunk);
-    static_assert(kScatterTile <= (1u << 13) && (1u << kMaxRadixBits) <= (1u << 19), "slot packing");
-    for (uint64_t t0 = b0; t0 < b1; t0 += kScatterTile) {
-        const uint32_t tn = b1 - t0 < kScatterTile ? (uint32_t)(b1 - t0) : kScatterTile;
-        for (uint32_t p = threadIdx.x; p < fanout; p += blockDim.x) s_cnt[p] = 0;
-        __syncthreads();
-        uint64_t key[kScatterItems];
-        uint32_t slot[kScatterItems];  // partition << 13 | rank inside the tile's partition run
+    uint64_t* s_keys = reinterpret_cast<uint64_t*>(s_mem);            // kTile
+    uint32_t* s_start = reinterpret_cast<uint32_t*>(s_mem + kTile);   // fanout: counts, then starts in the tile
+    uint32_t* s_delta = s_start + t.fanout;                           // fanout: relation index less tile place
+    uint16_t* s_off = reinterpret_cast<uint16_t*>(s_delta + t.fanout);  // kTile
+    const uint32_t fanout = t.fanout, tile = blockIdx.x;
+    const uint64_t t0 = (uint64_t)tile * kTile;
+    const uint32_t tn = m - t0 < kTile ? (uint32_t)(m - t0) : kTile;
+    const unsigned long long* k64 = reinterpret_cast<const unsigned long long*>(keys) + t0;
+    uint64_t key[kIt];
 #pragma unroll
-        for (int k = 0; k < kScatterItems; ++k) {
-            const uint32_t j = k * kScatterBlock + threadIdx.x;
-            key[k] = j < tn ? __ldcs(k64 + t0 + j) : 0ull;
-        }
-#pragma unroll
-        for (int k = 0; k < kScatterItems; ++k) {
-            const uint32_t j = k * kScatterBlock + threadIdx.x;
-            const uint32_t p = part_of(key[k], min_key, shift, fanout);
-            slot[k] = j < tn ? (p << 13) | atomicAdd(&s_cnt[p], 1u) : 0u;
-        }
-        __syncthreads();
-        block_exclusive_scan<kScatterBlock>(s_cnt, s_start, fanout);
-        __syncthreads();
-#pragma unroll
-        for (int k = 0; k < kScatterItems; ++k) {
-            const uint32_t j = k * kScatterBlock + threadIdx.x;
-            if (j < tn) {
-                const uint32_t q = s_start[slot[k] >> 13] + (slot[k] & ((1u << 13) - 1));
-                s_keys[q] = key[k];
-                s_rows[q] = kInverse ? j : (uint32_t)(row_base + t0 + j);
-            }
-        }
-        // output index of the tile's j-th sorted key = s_delta[p] + j
-        for (uint32_t p = threadIdx.x; p < fanout; p += blockDim.x) {
-            s_delta[p] = s_dst[p] - s_start[p];
-            if constexpr (kInverse) leave_run(iv, tile_number(t0, b0, chunk, kScatterTile), fanout, p, s_delta[p], s_start[p]);
-        }
-        __syncthreads();
-        for (uint32_t j = threadIdx.x; j < tn; j += kScatterBlock) {
-            const uint64_t k = s_keys[j];
-            const uint64_t d = s_delta[part_of(k, min_key, shift, fanout)] + j;
-            __stcg(reinterpret_cast<unsigned long long*>(out_keys) + d, (unsigned long long)k);
-            if constexpr (kInverse) iv.offsets[d] = (uint16_t)s_rows[j];
-            else __stcg(out_rows + d, s_rows[j]);
-        }
-        __syncthreads();
-        for (uint32_t p = threadIdx.x; p < fanout; p += blockDim.x) s_dst[p] += s_cnt[p];
-        __syncthreads();
+    for (int k = 0; k < kIt; ++k) {
+        const uint32_t j = k * kB + threadIdx.x;
+        key[k] = j < tn ? __ldcs(k64 + j) : 0ull;
     }
-}
-
-size_t scatter_smem_bytes(uint32_t fanout) {
-    return (size_t)kScatterTile * (sizeof(uint64_t) + sizeof(uint32_t)) + (size_t)fanout * (8 + 4 + 4 + 8);
-}
-
-// The scatter for fanouts of 2^8 and more: the same counting sort per tile,
-// with tiles large enough that a partition's run in a tile covers whole
-// sectors (8192 keys: 32 a partition at 2^8, 8 at 2^10, 2 at 2^12), one
-// 1024-thread block per SM, and the next tile's keys loaded into registers
-// while the current tile is sorted and written (measured at fanout 2^8:
-// 11.33 against 12.46 ms for the partitioned step with the 4K-tile kernel).  A key's place in the tile
-// is kept as a 16-bit offset (its row is row_base + tile start + offset).
-// fanout from which the wide scatter runs; GJ_WIDE_RADIX_BITS overrides it
-// in tuning builds
-#ifndef GJ_WIDE_RADIX_BITS
-#define GJ_WIDE_RADIX_BITS 8
-#endif
-constexpr uint32_t kWideRadixBits = GJ_WIDE_RADIX_BITS;
-// block size, resident blocks per SM and the register prefetch of the next
-// tile (one 1024-thread block with the prefetch measured fastest: 10.63 ms
-// per partitioned step of 2^29 probes, against 11.71 for two 1024-thread
-// blocks without it and 11.18 / 12.47 for two 768-thread blocks without /
-// with it); GJ_WIDE_BLOCK / GJ_WIDE_PER_SM / GJ_WIDE_PREFETCH override them
-// in tuning builds
-#ifndef GJ_WIDE_BLOCK
-#define GJ_WIDE_BLOCK 1024
-#endif
-#ifndef GJ_WIDE_PER_SM
-#define GJ_WIDE_PER_SM 1
-#endif
-#ifndef GJ_WIDE_PREFETCH
-#define GJ_WIDE_PREFETCH 1
-#endif
-constexpr int kWideBlock = GJ_WIDE_BLOCK;
-constexpr int kWidePerSM = GJ_WIDE_PER_SM;
-constexpr int kWideItems = 8;
-constexpr uint32_t kWideTile = kWideBlock * kWideItems;
-
-template <bool kInverse>
-__global__ void __launch_bounds__(kWideBlock, kWidePerSM) k_part_scatter_wide(const uint64_t* __restrict__ keys, uint64_t m,
-                                                                     uint64_t chunk, uint64_t min_key, uint32_t shift,
-                                                                     uint32_t fanout, const uint64_t* __restrict__ incl,
-                                                                     uint64_t row_base, uint64_t* __restrict__ out_keys,
-                                                                     uint32_t* __restrict__ out_rows, partition_inverse iv) {
-    extern __shared__ unsigned long long s_mem[];
-    uint64_t* s_keys = reinterpret_cast<uint64_t*>(s_mem);             // kWideTile
-    unsigned long long* s_dst = s_mem + kWideTile;                     // fanout: next output slot
-    uint32_t* s_cnt = reinterpret_cast<uint32_t*>(s_dst + fanout);     // fanout
-    uint32_t* s_start = s_cnt + fanout;                                // fanout
-    unsigned long long* s_delta = reinterpret_cast<unsigned long long*>(s_start + fanout);  // fanout
-    uint32_t* s_meta = reinterpret_cast<uint32_t*>(s_delta + fanout);  // kWideTile: partition << 16 | offset
-    for (uint32_t p = threadIdx.x; p < fanout; p += kWideBlock) {
-        const uint64_t cell = (uint64_t)p * gridDim.x + blockIdx.x;
-        s_dst[p] = cell == 0 ? 0ull : incl[cell - 1];
-        s_cnt[p] = 0;
+    for (uint32_t p = threadIdx.x; p < fanout; p += kB) {
+        s_start[p] = 0;
+        s_delta[p] = run_start(t, tile, p);
     }
-    const unsigned long long* k64 = reinterpret_cast<const unsigned long long*>(keys);
-    const uint64_t b0 = blockIdx.x * chunk, b1 = min(m, b0 + chunk);
-    static_assert(kWideTile <= (1u << 13) && (1u << kMaxRadixBits) <= (1u << 19), "slot packing");
-    static_assert(kWideTile <= (1u << 16) && (1u << kMaxRadixBits) <= (1u << 16), "16-bit tile offsets and partitions");
-#if GJ_WIDE_PREFETCH
-    uint64_t next[kWideItems];
-#pragma unroll
-    for (int k = 0; k < kWideItems; ++k) {
-        const uint64_t i = b0 + (uint64_t)k * kWideBlock + threadIdx.x;
-        next[k] = i < b1 ? __ldcs(k64 + i) : 0ull;
-    }
-#endif
     __syncthreads();
-    for (uint64_t t0 = b0; t0 < b1; t0 += kWideTile) {
-        const uint32_t tn = b1 - t0 < kWideTile ? (uint32_t)(b1 - t0) : kWideTile;
-        uint64_t key[kWideItems];
-#if GJ_WIDE_PREFETCH
+    uint32_t slot[kIt];  // partition << 13 | rank inside the tile's partition run
 #pragma unroll
-        for (int k = 0; k < kWideItems; ++k) key[k] = next[k];
-        const uint64_t t1 = t0 + kWideTile;
+    for (int k = 0; k < kIt; ++k) {
+        const uint32_t p = part_of(key[k], f.min_key, f.shift, fanout);
+        slot[k] = (uint32_t)(k * kB + threadIdx.x) < tn ? (p << 13) | atomicAdd(&s_start[p], 1u) : 0u;
+    }
+    __syncthreads();
+    block_exclusive_scan<kB>(s_start, s_start, fanout);
+    __syncthreads();
 #pragma unroll
-        for (int k = 0; k < kWideItems; ++k) {
-            const uint64_t i = t1 + (uint64_t)k * kWideBlock + threadIdx.x;
-            next[k] = i < b1 ? __ldcs(k64 + i) : 0ull;
+    for (int k = 0; k < kIt; ++k) {
+        const uint32_t j = k * kB + threadIdx.x;
+        if (j < tn) {
+            const uint32_t q = s_start[slot[k] >> 13] + (slot[k] & ((1u << 13) - 1));
+            s_keys[q] = key[k];
+            s_off[q] = (uint16_t)j;
         }
-#else
+    }
+    for (uint32_t p = threadIdx.x; p < fanout; p += kB) {
+        s_delta[p] -= s_start[p];
+        if constexpr (kInverse) iv.start[(uint64_t)tile * fanout + p] = (uint16_t)s_start[p];
+    }
+    __syncthreads();
 #pragma unroll
-        for (int k = 0; k < kWideItems; ++k) {
-            const uint64_t i = t0 + (uint64_t)k * kWideBlock + threadIdx.x;
-            key[k] = i < b1 ? __ldcs(k64 + i) : 0ull;
+    for (int k = 0; k < kIt; ++k) {
+        const uint32_t j = k * kB + threadIdx.x;
+        if (j < tn) {
+            const uint64_t x = s_keys[j];
+            const uint32_t d = s_delta[part_of(x, f.min_key, f.shift, fanout)] + j;
+            __stcg(reinterpret_cast<unsigned long long*>(out_keys) + d, (unsigned long long)x);
+            if constexpr (kInverse) __stcg(reinterpret_cast<unsigned short*>(iv.offsets) + d, s_off[j]);
+            else __stcg(out_rows + d, (uint32_t)(row_base + t0 + s_off[j]));
         }
-#endif
-        uint32_t slot[kWideItems];  // partition << 13 | rank inside the tile's partition run
-#pragma unroll
-        for (int k = 0; k < kWideItems; ++k) {
-            const uint32_t j = k * kWideBlock + threadIdx.x;
-            const uint32_t p = part_of(key[k], min_key, shift, fanout);
-            slot[k] = j < tn ? (p << 13) | atomicAdd(&s_cnt[p], 1u) : 0u;
-        }
-        __syncthreads();
-        block_exclusive_scan<kWideBlock>(s_cnt, s_start, fanout);
-        __syncthreads();
-#pragma unroll
-        for (int k = 0; k < kWideItems; ++k) {
-            const uint32_t j = k * kWideBlock + threadIdx.x;
-            if (j < tn) {
-                const uint32_t q = s_start[slot[k] >> 13] + (slot[k] & ((1u << 13) - 1));
-                s_keys[q] = key[k];
-                s_meta[q] = ((slot[k] >> 13) << 16) | j;
-            }
-        }
-        // output index of the tile's j-th sorted key = s_delta[p] + j
-        for (uint32_t p = threadIdx.x; p < fanout; p += kWideBlock) {
-            s_delta[p] = s_dst[p] - s_start[p];
-            if constexpr (kInverse) leave_run(iv, tile_number(t0, b0, chunk, kWideTile), fanout, p, s_delta[p], s_start[p]);
-        }
-        __syncthreads();
-        for (uint32_t j = threadIdx.x; j < tn; j += kWideBlock) {
-            const uint64_t k = s_keys[j];
-            // the partition and the tile offset were stored with the key
-            const uint32_t meta = s_meta[j];
-            const uint64_t d = s_delta[meta >> 16] + j;
-            __stcg(reinterpret_cast<unsigned long long*>(out_keys) + d, (unsigned long long)k);
-            if constexpr (kInverse) iv.offsets[d] = (uint16_t)meta;
-            else __stcg(out_rows + d, (uint32_t)(row_base + t0 + (meta & 0xFFFFu)));
-        }
-        __syncthreads();
-        for (uint32_t p = threadIdx.x; p < fanout; p += kWideBlock) {
-            s_dst[p] += s_cnt[p];
-            s_cnt[p] = 0;
-        }
-        __syncthreads();
     }
 }
 
-size_t scatter_wide_smem_bytes(uint32_t fanout) {
-    return (size_t)kWideTile * (sizeof(uint64_t) + sizeof(uint32_t)) +
-           (size_t)fanout * (8 + 4 + 4 + 8);
-}
+size_t scatter_smem_bytes(uint32_t tile, uint32_t fanout) { return (size_t)tile * 10 + (size_t)fanout * 8; }
 
 // The scatter backwards for values of the relation: out[row] = the value of
 // the probe that came from row.  A tile's values are read where the scatter
@@ -375,34 +294,33 @@ size_t scatter_wide_smem_bytes(uint32_t fanout) {
 // the other's writes.
 // values is dense per kValueTile relation entries, at a stride of twice that
 // (each tile's values lie in the first half of the room its keys took).
-template <int kB, int kPerSM>
-__global__ void __launch_bounds__(kB, kPerSM) k_part_gather(const uint32_t* __restrict__ values, uint64_t m, uint64_t chunk,
-                                                     uint32_t fanout, uint32_t tiles_per_chunk, partition_inverse iv,
-                                                     uint32_t* __restrict__ out) {
-    constexpr uint32_t kTile = kB * 8;
+template <int kB, int kIt, int kPerSM>
+__global__ void __launch_bounds__(kB, kPerSM) k_part_gather(const uint32_t* __restrict__ values, uint64_t m,
+                                                            part_tables t, partition_inverse iv,
+                                                            uint32_t* __restrict__ out) {
+    constexpr uint32_t kTile = kB * kIt;
     extern __shared__ unsigned long long s_mem[];
+    const uint32_t fanout = t.fanout, tile = blockIdx.x;
     uint32_t* s_out = reinterpret_cast<uint32_t*>(s_mem);              // kTile
     uint32_t* s_delta = s_out + kTile;                                 // fanout
     uint16_t* s_start = reinterpret_cast<uint16_t*>(s_delta + fanout); // fanout + 2
     uint16_t* s_part = s_start + fanout + 2;                           // kTile: partition of sorted place j
-    const uint64_t b0 = blockIdx.x / tiles_per_chunk * chunk, b1 = min(m, b0 + chunk);
-    const uint64_t t0 = b0 + (uint64_t)(blockIdx.x % tiles_per_chunk) * kTile;
-    if (t0 >= b1) return;
-    const uint32_t tn = b1 - t0 < kTile ? (uint32_t)(b1 - t0) : kTile;
-    const uint64_t cell = (uint64_t)blockIdx.x * fanout;
+    const uint64_t t0 = (uint64_t)tile * kTile;
+    const uint32_t tn = m - t0 < kTile ? (uint32_t)(m - t0) : kTile;
     for (uint32_t p = threadIdx.x; p < fanout; p += kB) {
-        s_delta[p] = __ldcs(iv.delta + cell + p);
-        s_start[p] = __ldcs(iv.start + cell + p);
+        const uint16_t at = __ldcs(iv.start + (uint64_t)tile * fanout + p);
+        s_delta[p] = run_start(t, tile, p) - at;
+        s_start[p] = at;
     }
     if (threadIdx.x == 0) s_start[fanout] = (uint16_t)tn;
     __syncthreads();
     for (uint32_t p = threadIdx.x >> 5; p < fanout; p += kB / 32)
         for (uint32_t j = s_start[p] + (threadIdx.x & 31); j < s_start[p + 1]; j += 32) s_part[j] = (uint16_t)p;
     __syncthreads();
-    uint32_t v[8];
-    uint16_t o[8];
+    uint32_t v[kIt];
+    uint16_t o[kIt];
 #pragma unroll
-    for (int k = 0; k < 8; ++k) {
+    for (int k = 0; k < kIt; ++k) {
         const uint32_t j = k * kB + threadIdx.x;
         if (j < tn) {
             const uint32_t d = s_delta[s_part[j]] + j;
@@ -411,11 +329,11 @@ __global__ void __launch_bounds__(kB, kPerSM) k_part_gather(const uint32_t* __re
         }
     }
 #pragma unroll
-    for (int k = 0; k < 8; ++k)
+    for (int k = 0; k < kIt; ++k)
         if (k * kB + threadIdx.x < tn) s_out[o[k]] = v[k];
     __syncthreads();
 #pragma unroll
-    for (int k = 0; k < 8; ++k) {
+    for (int k = 0; k < kIt; ++k) {
         const uint32_t j = k * kB + threadIdx.x;
         if (j < tn) __stcs(out + t0 + j, s_out[j]);
     }
@@ -425,34 +343,76 @@ size_t gather_smem_bytes(uint32_t tile, uint32_t fanout) {
     return (size_t)tile * (4 + 2) + (size_t)fanout * 4 + ((size_t)fanout + 2) * 2;
 }
 
+// Tile geometry.  4096 keys by blocks of 512 threads, three on an SM, up to
+// fanout 2^8; from 2^9 on 8192 keys (a run of the tile then still covers
+// sectors), 512 threads, two on an SM, unless that leaves SMs without a tile.
+// Scatter plus gather of 2^28 keys, small / large tiles: 1892 / 2013 us at
+// 2^8, 2806 / 2211 at 2^9; 1024 threads on a large tile cost 2136 at 2^8 (32
+// registers, spills), four small blocks an SM 1822 against 1447 at 2^5.
+// All three passes of 2^28 keys at 2^5 / 2^8 / 2^11: 1543 / 1828 / 5506 us
+// before, 1293 / 1475 / 2781 now.
+constexpr uint32_t kWideTile = 8192, kTile = 4096;
+constexpr uint32_t kWideRadixBits = 9;
+constexpr int kTileBlock = 512, kHistBlock = 1024;
+constexpr uint32_t kHistPerSM = 2;
+
 struct partition_plan {
-    uint32_t fanout, nblocks;
-    uint64_t chunk;
-    bool wide;
-    uint32_t tile() const { return wide ? kWideTile : kScatterTile; }
-    uint32_t tiles_per_chunk() const { return (uint32_t)((chunk + tile() - 1) / tile()); }
+    uint32_t fanout, tile, tiles, tiles_per_chunk, chunks;
+    bool wide() const { return tile == kWideTile; }
 };
 
-partition_plan plan_partition(uint64_t m, uint32_t radix_bits, int sm_count) {
+partition_plan plan_of(uint64_t m, uint32_t radix_bits, int sm_count, bool wide) {
     partition_plan pl;
     pl.fanout = 1u << radix_bits;
-    pl.wide = radix_bits >= kWideRadixBits;
-    // the scatter kernel's resident blocks
-    uint64_t nb = (uint64_t)sm_count * (pl.wide ? kWidePerSM : kScatterPerSM);
-    const uint64_t min_chunk = 4096;
-    if (nb * min_chunk > m) nb = std::max<uint64_t>(1, (m + min_chunk - 1) / min_chunk);
-    pl.chunk = (m + nb - 1) / nb;
-    pl.nblocks = (uint32_t)((m + pl.chunk - 1) / pl.chunk);
-    if (pl.nblocks == 0) pl.nblocks = 1;
+    pl.tile = wide ? kWideTile : kTile;
+    pl.tiles = (uint32_t)((m + pl.tile - 1) / pl.tile);
+    const uint32_t want = (uint32_t)sm_count * kHistPerSM;
+    pl.tiles_per_chunk = std::max(1u, (pl.tiles + want - 1) / want);
+    pl.chunks = (pl.tiles + pl.tiles_per_chunk - 1) / pl.tiles_per_chunk;
     return pl;
+}
+
+uint64_t wide_from(int sm_count) { return 2ull * sm_count * kWideTile; }
+
+partition_plan plan_partition(uint64_t m, uint32_t radix_bits, int sm_count) {
+    return plan_of(m, radix_bits, sm_count, radix_bits >= kWideRadixBits && m >= wide_from(sm_count));
+}
+
+size_t plan_bytes(const partition_plan& pl) {
+    return workspace_carver::need({(size_t)pl.tiles * pl.fanout * 4, (size_t)pl.chunks * pl.fanout * 4,
+                                   (size_t)pl.fanout * 4, 4});
+}
+
+bool carve_tables(void* ws, size_t ws_bytes, const partition_plan& pl, part_tables* t) {
+    workspace_carver wc(ws, ws_bytes);
+    t->before = wc.take<uint32_t>((size_t)pl.tiles * pl.fanout);
+    t->chunk_start = wc.take<uint32_t>((size_t)pl.chunks * pl.fanout);
+    t->part_start = wc.take<uint32_t>(pl.fanout);
+    t->done = wc.take<uint32_t>(1);
+    t->tiles = pl.tiles;
+    t->tiles_per_chunk = pl.tiles_per_chunk;
+    t->chunks = pl.chunks;
+    t->fanout = pl.fanout;
+    return t->before && t->chunk_start && t->part_start && t->done;
+}
+
+template <class Kernel, class... Args>
+int launch(Kernel kernel, uint32_t grid, int block, size_t smem, cudaStream_t s, Args... args) {
+    if (smem > 40 * 1024)  // with the kernels' static part, near the 48 KB allowed without asking
+        GJ_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    kernel<<<grid, block, smem, s>>>(args...);
+    GJ_CUDA_TRY(cudaGetLastError());
+    return GJ_OK;
 }
 
 }  // namespace
 
+// the workspace of a window of m keys also serves any shorter window
 size_t partition_ws_bytes(uint64_t m, uint32_t radix_bits, int sm_count) {
-    const partition_plan pl = plan_partition(m ? m : 1, radix_bits, sm_count);
-    const uint64_t cells = (uint64_t)pl.fanout * pl.nblocks;
-    return workspace_carver::need({cells * sizeof(uint64_t), scan_workspace_bytes(cells)});
+    if (m == 0) m = 1;
+    const size_t bytes = plan_bytes(plan_partition(m, radix_bits, sm_count));
+    const uint64_t narrow = std::min(m, wide_from(sm_count));
+    return std::max(bytes, plan_bytes(plan_of(narrow, radix_bits, sm_count, false)));
 }
 
 int range_partition_impl(const uint64_t* d_keys, uint64_t m, uint64_t min_key, uint32_t shift, uint32_t radix_bits,
@@ -461,11 +421,8 @@ int range_partition_impl(const uint64_t* d_keys, uint64_t m, uint64_t min_key, u
     device_info di;
     GJ_TRY(current_device_info(&di));
     const partition_plan pl = plan_partition(m ? m : 1, radix_bits, di.sm_count);
-    const uint64_t cells = (uint64_t)pl.fanout * pl.nblocks;
-    workspace_carver wc(ws, ws_bytes);
-    uint64_t* hist = wc.take<uint64_t>(cells);
-    void* scan_ws = wc.take<char>(scan_workspace_bytes(cells));
-    if (!hist || !scan_ws) {
+    part_tables t;
+    if (!carve_tables(ws, ws_bytes, pl, &t)) {
         set_error("range partition: workspace of %zu bytes is smaller than the %zu required", ws_bytes,
                   partition_ws_bytes(m, radix_bits, di.sm_count));
         return GJ_ERR_WORKSPACE;
@@ -474,60 +431,48 @@ int range_partition_impl(const uint64_t* d_keys, uint64_t m, uint64_t min_key, u
         if (d_offsets) GJ_CUDA_TRY(cudaMemsetAsync(d_offsets, 0, ((size_t)pl.fanout + 1) * sizeof(uint64_t), s));
         return GJ_OK;
     }
-    const size_t smem_hist = (size_t)pl.fanout * hist_copies(pl.fanout) * sizeof(uint32_t);
-    if (pl.wide)
-        k_part_hist<kWideBlock><<<pl.nblocks, kWideBlock, smem_hist, s>>>(d_keys, m, pl.chunk, min_key, shift,
-                                                                          pl.fanout, hist);
-    else
-        k_part_hist<kPartBlock><<<pl.nblocks, kPartBlock, smem_hist, s>>>(d_keys, m, pl.chunk, min_key, shift,
-                                                                          pl.fanout, hist);
-    GJ_CUDA_TRY(cudaGetLastError());
-    GJ_TRY(inclusive_scan_sum(hist, cells, scan_ws, scan_workspace_bytes(cells), s));
-    if (d_offsets) {
-        k_part_offsets<<<(pl.fanout + 256) / 256, 256, 0, s>>>(hist, pl.fanout, pl.nblocks, m, d_offsets);
-        GJ_CUDA_TRY(cudaGetLastError());
-    }
-    const size_t smem = pl.wide ? scatter_wide_smem_bytes(pl.fanout) : scatter_smem_bytes(pl.fanout);
+    const part_func f{min_key, shift};
+    const size_t hist_smem = (2 * (size_t)hist_copies(pl.fanout) + 1) * pl.fanout * sizeof(uint32_t);
+    GJ_TRY(pl.wide() ? launch(k_part_hist<kHistBlock, kWideTile>, pl.chunks, kHistBlock, hist_smem, s, d_keys, m, f, t)
+                     : launch(k_part_hist<kHistBlock, kTile>, pl.chunks, kHistBlock, hist_smem, s, d_keys, m, f, t));
+    GJ_TRY(launch(k_part_base, (pl.fanout + 31) / 32, kBaseBlock, pl.fanout * sizeof(uint32_t), s, t, m, d_offsets));
+    const size_t smem = scatter_smem_bytes(pl.tile, pl.fanout);
     const partition_inverse iv = inverse ? *inverse : partition_inverse{};
-    auto launch = [&](auto kernel, int block) {
-        if (smem > 48 * 1024)
-            GJ_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        kernel<<<pl.nblocks, block, smem, s>>>(d_keys, m, pl.chunk, min_key, shift, pl.fanout, hist, row_base,
-                                               d_out_keys, d_out_rows, iv);
-        GJ_CUDA_TRY(cudaGetLastError());
-        return (int)GJ_OK;
+    auto scatter = [&](auto kernel, int block) {
+        return launch(kernel, pl.tiles, block, smem, s, d_keys, m, f, t, row_base, d_out_keys, d_out_rows, iv);
     };
-    if (pl.wide) return inverse ? launch(k_part_scatter_wide<true>, kWideBlock) : launch(k_part_scatter_wide<false>, kWideBlock);
-    return inverse ? launch(k_part_scatter<true>, kScatterBlock) : launch(k_part_scatter<false>, kScatterBlock);
+    constexpr int kWideIt = kWideTile / kTileBlock, kIt = kTile / kTileBlock;
+    if (pl.wide())
+        return inverse ? scatter(k_part_scatter<kTileBlock, kWideIt, 2, true>, kTileBlock)
+                       : scatter(k_part_scatter<kTileBlock, kWideIt, 2, false>, kTileBlock);
+    return inverse ? scatter(k_part_scatter<kTileBlock, kIt, 3, true>, kTileBlock)
+                   : scatter(k_part_scatter<kTileBlock, kIt, 3, false>, kTileBlock);
 }
 
 bool carve_partition_inverse(void* ws, size_t ws_bytes, uint64_t m, uint32_t radix_bits, int sm_count,
                              partition_inverse* out) {
     const partition_plan pl = plan_partition(m ? m : 1, radix_bits, sm_count);
-    const uint64_t cells = (uint64_t)pl.nblocks * pl.tiles_per_chunk() * pl.fanout;
     workspace_carver wc(ws, ws_bytes);
     out->offsets = wc.take<uint16_t>(m);
-    out->delta = wc.take<uint32_t>(cells);
-    out->start = wc.take<uint16_t>(cells);
-    return out->offsets && out->delta && out->start;
+    out->start = wc.take<uint16_t>((size_t)pl.tiles * pl.fanout);
+    return out->offsets && out->start;
 }
 
-int gather_values(const uint32_t* d_values, uint64_t m, uint32_t radix_bits, const partition_inverse& iv,
-                  uint32_t* d_out, cudaStream_t s) {
+int gather_values(const uint32_t* d_values, uint64_t m, uint32_t radix_bits, void* ws, size_t ws_bytes,
+                  const partition_inverse& iv, uint32_t* d_out, cudaStream_t s) {
     if (m == 0) return GJ_OK;
     device_info di;
     GJ_TRY(current_device_info(&di));
     const partition_plan pl = plan_partition(m, radix_bits, di.sm_count);
-    const size_t smem = gather_smem_bytes(pl.tile(), pl.fanout);
-    auto launch = [&](auto kernel, int block) {
-        if (smem > 48 * 1024)
-            GJ_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        kernel<<<pl.nblocks * pl.tiles_per_chunk(), block, smem, s>>>(d_values, m, pl.chunk, pl.fanout,
-                                                                     pl.tiles_per_chunk(), iv, d_out);
-        GJ_CUDA_TRY(cudaGetLastError());
-        return (int)GJ_OK;
-    };
-    return pl.wide ? launch(k_part_gather<kWideBlock, 2>, kWideBlock) : launch(k_part_gather<kScatterBlock, 4>, kScatterBlock);
+    part_tables t;
+    if (!carve_tables(ws, ws_bytes, pl, &t)) {
+        set_error("partition gather: workspace of %zu bytes is too small", ws_bytes);
+        return GJ_ERR_WORKSPACE;
+    }
+    const size_t smem = gather_smem_bytes(pl.tile, pl.fanout);
+    constexpr int kWideIt = kWideTile / kTileBlock, kIt = kTile / kTileBlock;
+    return pl.wide() ? launch(k_part_gather<kTileBlock, kWideIt, 3>, pl.tiles, kTileBlock, smem, s, d_values, m, t, iv, d_out)
+                     : launch(k_part_gather<kTileBlock, kIt, 4>, pl.tiles, kTileBlock, smem, s, d_values, m, t, iv, d_out);
 }
 
 // key range used by the partitioned INLJ for an index (recorded at build)

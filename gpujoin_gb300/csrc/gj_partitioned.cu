@@ -645,7 +645,7 @@ int gj_partitioned_inlj(const gj_index* index, const uint64_t* d_probes, uint64_
         // Positions alone come back to probe order through the partition's
         // inverse, kept where the row ids would be, unless the window's
         // positions are few enough to stay in L2 while they are stored one
-        // by one (or a high fanout leaves no room for the tiles' runs).
+        // by one.
         partition_inverse iv{};
         const bool back = d_positions && !d_pairs && len >= kGatherMin &&
                           carve_partition_inverse(prows, w * sizeof(uint32_t), len, radix_bits, di.sm_count, &iv);
@@ -653,7 +653,7 @@ int gj_partitioned_inlj(const gj_index* index, const uint64_t* d_probes, uint64_
                                     nullptr, pws, pws_bytes, s, back ? &iv : nullptr));
         a.values = back ? reinterpret_cast<uint32_t*>(pkeys) : nullptr;
         GJ_TRY(dispatch_probe(sem, aligned, a, s));
-        if (back) GJ_TRY(gather_values(a.values, len, radix_bits, iv, d_positions + off, s));
+        if (back) GJ_TRY(gather_values(a.values, len, radix_bits, pws, pws_bytes, iv, d_positions + off, s));
     }
     return GJ_OK;
 }

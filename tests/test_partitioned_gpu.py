@@ -108,6 +108,32 @@ def test_partitioned_skewed_probes(orc, gj, cuda, kind):
             np.testing.assert_array_equal(a[order, 1], epos)
 
 
+@pytest.mark.parametrize("radix_bits", range(1, 13))
+@pytest.mark.parametrize("m", [1, 4095, 4096, 4097, 70_001, 2 * 152 * 8192 + 8191])
+def test_range_partition_layout(gj, cuda, radix_bits, m):
+    # the relation itself: partitions in key order, whole and disjoint, the
+    # tuples of earlier tiles first, and every row id with its own key; both
+    # tile sizes, every fanout (shared memory up to its limits)
+    import torch
+
+    g = torch.Generator(device="cuda")
+    g.manual_seed(radix_bits * 1000 + m)
+    keys = torch.randint(0, 1 << 40, (m,), generator=g, device="cuda", dtype=torch.int64)
+    keys[: m // 3] = keys[: m // 3] % 1000  # a crowded partition
+    low, shift = 500, 40 - radix_bits
+    rel = gj.range_partition(keys, low, shift, radix_bits)
+    part = torch.clamp((keys - low).clamp(min=0) >> shift, max=(1 << radix_bits) - 1)
+    sizes = torch.bincount(part, minlength=1 << radix_bits)
+    assert int(rel.offsets[0]) == 0 and torch.equal(rel.offsets[1:], torch.cumsum(sizes, 0))
+    rows = rel.rows.to(torch.int64)
+    assert torch.equal(torch.sort(rows)[0], torch.arange(m, device="cuda"))
+    assert torch.equal(keys[rows], rel.keys)
+    assert torch.equal(part[rows], torch.sort(part)[0])
+    tile = rows // 8192  # chunks of whole tiles of either size come in order
+    order = part[rows] * (1 << 20) + tile
+    assert bool((order[1:] >= order[:-1]).all())
+
+
 @pytest.mark.parametrize("radix_bits", [1, 5, 7, 8, 11, 12])
 @pytest.mark.parametrize("m,window", [((1 << 22) + 1, 0), (3 * (1 << 22) - 77, 1 << 22)])
 def test_positions_through_the_inverse(orc, gj, cuda, radix_bits, m, window):
