@@ -30,12 +30,27 @@
 namespace gj {
 namespace {
 
+// resident blocks per SM (the register cap: 32); 512 batches over eight
+// indexes took 4222 us with every kind's search inlined in one loop (and no
+// cap), with a loop per kind 2501 / 2195 / 2061 / 2032 at 4 / 5 / 6 / 8
+constexpr int kBatchPerSM = 8;
 constexpr int kBatchBlock = 256;
 
+// What a tile's searches need to know of its index.  The common kinds have a
+// loop of their own in the kernel; the rest (trees that search their nodes,
+// MLP roots, indexes in host memory) share one behind a call, so that their
+// registers are not everyone's.
+enum view_kind : int32_t { kViewStartExact, kViewStartLower, kViewSpline, kViewLearned, kViewHash, kViewOther };
+struct start_view {
+    key_start t;
+    const uint64_t* col;
+    uint32_t n;
+};
 struct any_view {
-    int32_t type;
-    uint32_t pad;
+    int32_t kind;
+    int32_t type;  // kViewOther: the index type
     union {
+        start_view st;
         bs_view bs;
         btree_view bt;
         harmonia_view hm;
@@ -60,7 +75,7 @@ __device__ __forceinline__ uint64_t globaltimer_ns() {
     return t;
 }
 
-__device__ __forceinline__ uint32_t any_lookup(const any_view& v, const float* root, uint64_t key) {
+__device__ __noinline__ uint32_t other_lookup(const any_view& v, const float* root, uint64_t key) {
     switch (v.type) {
         case GJ_INDEX_BINARY_SEARCH: return bs_lookup(v.u.bs, nullptr, key);
         case GJ_INDEX_BTREE:
@@ -74,17 +89,30 @@ __device__ __forceinline__ uint32_t any_lookup(const any_view& v, const float* r
                 default: return btree_lookup<64>(v.u.bt, nullptr, key);
             }
         case GJ_INDEX_HARMONIA: return harmonia_lookup(v.u.hm, nullptr, key);
-        case GJ_INDEX_RADIX_SPLINE: return rs_lookup(v.u.rs, key);
         case GJ_INDEX_LEARNED: return learned_lookup(v.u.ln, root, key);
-        case GJ_INDEX_HASH: return hash_lookup(v.u.hs, key);
         default: return kInvalid;
+    }
+}
+
+// out[j] = lookup(probes[j]) for the tile's probes [first, last)
+template <class Lookup>
+__device__ __forceinline__ void search_tile(const uint64_t* __restrict__ probes, uint32_t* __restrict__ out,
+                                            uint64_t first, uint64_t last, Lookup&& lookup) {
+    uint64_t j = first + threadIdx.x;
+    uint64_t next = j < last ? __ldcs(reinterpret_cast<const unsigned long long*>(probes + j)) : 0ull;
+#pragma unroll 1
+    for (; j < last; j += kBatchBlock) {
+        const uint64_t key = next;
+        if (j + kBatchBlock < last)
+            next = __ldcs(reinterpret_cast<const unsigned long long*>(probes + j + kBatchBlock));
+        __stcs(out + j, lookup(key));
     }
 }
 
 // The block stages the view of its tile's index (and a learned index's root
 // parameters) in shared memory; consecutive tiles of one batch reuse them.
 template <int kItems>
-__global__ void __launch_bounds__(kBatchBlock) k_batch(const any_view* __restrict__ views,
+__global__ void __launch_bounds__(kBatchBlock, kBatchPerSM) k_batch(const any_view* __restrict__ views,
                                                        const batch_desc* __restrict__ batches,
                                                        const uint32_t* __restrict__ tile_batch, uint32_t total_tiles,
                                                        const uint64_t* __restrict__ probes,
@@ -119,14 +147,38 @@ __global__ void __launch_bounds__(kBatchBlock) k_batch(const any_view* __restric
         }
         const uint64_t first = (tile - bd.tile_begin) * kTile;
         const uint64_t last = min(bd.size, first + kTile);
-        uint64_t j = first + threadIdx.x;
-        uint64_t next = j < last ? __ldcs(reinterpret_cast<const unsigned long long*>(probes + bd.offset + j)) : 0ull;
-#pragma unroll 1
-        for (; j < last; j += kBatchBlock) {
-            const uint64_t key = next;
-            if (j + kBatchBlock < last)
-                next = __ldcs(reinterpret_cast<const unsigned long long*>(probes + bd.offset + j + kBatchBlock));
-            __stcs(out + bd.offset + j, any_lookup(s_view, s_root, key));
+        const uint64_t* tile_probes = probes + bd.offset;
+        uint32_t* tile_out = out + bd.offset;
+        switch (s_view.kind) {
+            case kViewStartExact:
+                search_tile(tile_probes, tile_out, first, last, [&](uint64_t key) {
+                    bool eq;
+                    const uint32_t lb = start_lower_bound(s_view.u.st.t, s_view.u.st.col, s_view.u.st.n, key, &eq);
+                    return eq ? lb : kInvalid;
+                });
+                break;
+            case kViewStartLower:
+                search_tile(tile_probes, tile_out, first, last, [&](uint64_t key) {
+                    bool eq;
+                    const uint32_t lb = start_lower_bound(s_view.u.st.t, s_view.u.st.col, s_view.u.st.n, key, &eq);
+                    return lb < s_view.u.st.n ? lb : kInvalid;
+                });
+                break;
+            case kViewSpline:
+                search_tile(tile_probes, tile_out, first, last,
+                            [&](uint64_t key) { return rs_lookup(s_view.u.rs, key); });
+                break;
+            case kViewLearned:
+                search_tile(tile_probes, tile_out, first, last,
+                            [&](uint64_t key) { return learned_lookup<true, false>(s_view.u.ln, s_root, key); });
+                break;
+            case kViewHash:
+                search_tile(tile_probes, tile_out, first, last,
+                            [&](uint64_t key) { return hash_lookup(s_view.u.hs, key); });
+                break;
+            default:
+                search_tile(tile_probes, tile_out, first, last,
+                            [&](uint64_t key) { return other_lookup(s_view, s_root, key); });
         }
         __syncthreads();
         if (threadIdx.x == 0 && done_ns) {
@@ -339,15 +391,23 @@ int gj_batch_plan_create(gj_index* const* indexes, uint32_t num_indexes, const u
         const gj_index* ix = indexes[i];
         any_view& v = views[i];
         std::memset(&v, 0, sizeof(v));
+        v.kind = kViewOther;
         v.type = ix->type;
         switch (ix->type) {
             case GJ_INDEX_BINARY_SEARCH: v.u.bs = ix->bs; v.u.bs.fence_slots = 0; break;
             case GJ_INDEX_BTREE: v.u.bt = ix->bt; v.u.bt.cached_levels = 0; break;
             case GJ_INDEX_HARMONIA: v.u.hm = ix->hm; v.u.hm.cached_nodes = 0; v.u.hm.cached_levels = 0; break;
-            case GJ_INDEX_RADIX_SPLINE: v.u.rs = ix->rs; break;
-            case GJ_INDEX_LEARNED: v.u.ln = ix->ln; break;
-            case GJ_INDEX_HASH: v.u.hs = ix->hs; break;
+            case GJ_INDEX_RADIX_SPLINE: v.kind = kViewSpline; v.u.rs = ix->rs; break;
+            case GJ_INDEX_LEARNED:
+                if (ix->ln.root_kind != GJ_LEARNED_ROOT_MLP) v.kind = kViewLearned;
+                v.u.ln = ix->ln;
+                break;
+            case GJ_INDEX_HASH: v.kind = kViewHash; v.u.hs = ix->hs; break;
             default: break;
+        }
+        if (ix->ks.pos) {
+            v.kind = ix->type == GJ_INDEX_BINARY_SEARCH ? kViewStartLower : kViewStartExact;
+            v.u.st = {ix->ks, ix->d_col, (uint32_t)ix->n};
         }
     }
     if (cudaMemcpyAsync(pl->d_views, views.data(), views.size() * sizeof(any_view), cudaMemcpyHostToDevice, s) !=
