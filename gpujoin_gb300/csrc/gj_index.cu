@@ -12,6 +12,7 @@
 #include <cstring>
 #include <memory>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "gj_internal.h"
@@ -289,25 +290,64 @@ int host_copy_of_column(const uint64_t* d_keys, const uint64_t* h_keys, uint64_t
     return GJ_OK;
 }
 
+// Bits of a key start table: about one bucket a key, at most 2^22 (16 MB).  A
+// larger table leaves L2 (2^26 probes into 2^23 keys: 770 us at 2^22, 865 at
+// 2^23, 1298 at 2^24), a smaller one leaves wider windows (2^26 keys: 2132 us
+// at 2^20, 1758 at 2^21, 1657 at 2^22).
+uint32_t key_start_bits(uint64_t n) {
+    uint32_t b = 1;
+    while (b < 22 && (1ull << b) < n) ++b;
+    return b;
+}
+
+// device memory that is freed unless it is handed on
+struct spare_memory {
+    void* p = nullptr;
+    spare_memory() = default;
+    spare_memory(const spare_memory&) = delete;
+    ~spare_memory() { cudaFree(p); }
+    int take(size_t bytes) {
+        const cudaError_t e = cudaMalloc(&p, bytes);
+        if (e == cudaSuccess) return GJ_OK;
+        p = nullptr;
+        set_error("cudaMalloc(%zu) failed: %s", bytes, cudaGetErrorString(e));
+        return e == cudaErrorMemoryAllocation ? GJ_ERR_OUT_OF_MEMORY : GJ_ERR_CUDA;
+    }
+    void* release() {
+        void* q = p;
+        p = nullptr;
+        return q;
+    }
+};
+
+uint32_t key_start_shift(uint64_t range, uint32_t bits) {
+    const uint32_t used = range ? 64u - (uint32_t)__builtin_clzll(range) : 0u;
+    return used > bits ? used - bits : 0u;
+}
+// the table in whole 16-byte groups, and the two sums of the cost sample
+size_t key_start_bytes(const gj_index* idx, uint32_t bits) {
+    const uint64_t range = idx->max_key - idx->min_key;
+    const uint64_t buckets = (range >> key_start_shift(range, bits)) + 1;
+    return ((buckets + 1 + 3) & ~3ull) * sizeof(uint32_t) + 2 * sizeof(unsigned long long);
+}
+
 // Key start table of 2^bits buckets (fewer for a narrow key range); use(loads,
 // level) decides from the sampled cost of its searches -- mean column sectors
 // read, and for a B+tree the mean level its lookups start at -- whether the
 // index keeps it.
 template <class Use>
-int build_key_start(gj_index* idx, uint32_t bits, cudaStream_t s, Use&& use) {
+int build_key_start(gj_index* idx, uint32_t bits, cudaStream_t s, spare_memory&& spare, Use&& use) {
     const uint64_t range = idx->max_key - idx->min_key;
-    const uint32_t used = range ? 64u - (uint32_t)__builtin_clzll(range) : 0u;
     key_start t{};
     t.min_key = idx->min_key;
     t.range = range;
-    t.shift = used > bits ? used - bits : 0u;
+    t.shift = key_start_shift(range, bits);
     t.inv_width = std::ldexp(1.0f, -(int)t.shift);
     t.col_aligned = aligned32(idx->d_col);
     const uint32_t buckets = (uint32_t)(range >> t.shift) + 1;
     const uint32_t entries = (buckets + 1 + 3) & ~3u;  // whole 16-byte groups
-    void* p = nullptr;
-    GJ_TRY(device_alloc(idx, (size_t)entries * sizeof(uint32_t) + 2 * sizeof(unsigned long long), &p));
-    uint32_t* pos = static_cast<uint32_t*>(p);
+    if (!spare.p) GJ_TRY(spare.take(key_start_bytes(idx, bits)));
+    uint32_t* pos = static_cast<uint32_t*>(spare.p);
     unsigned long long* d_sums = reinterpret_cast<unsigned long long*>(pos + entries);
     unsigned long long sums[2] = {0, 0};
     k_key_start<<<(entries + 255) / 256, 256, 0, s>>>(idx->d_col, idx->n, t.min_key, t.shift, buckets, entries, pos);
@@ -318,24 +358,11 @@ int build_key_start(gj_index* idx, uint32_t bits, cudaStream_t s, Use&& use) {
     GJ_CUDA_TRY(cudaGetLastError());
     GJ_CUDA_TRY(cudaMemcpyAsync(sums, d_sums, sizeof(sums), cudaMemcpyDeviceToHost, s));
     GJ_CUDA_TRY(cudaStreamSynchronize(s));
-    if (!use((double)sums[0] / kStartSample, (double)sums[1] / kStartSample)) {
-        GJ_CUDA_TRY(cudaFree(p));
-        idx->allocations.pop_back();
-        return GJ_OK;
-    }
+    if (!use((double)sums[0] / kStartSample, (double)sums[1] / kStartSample)) return GJ_OK;
+    idx->allocations.push_back(spare.release());
     idx->ks = t;
     idx->bytes += (size_t)entries * sizeof(uint32_t);
     return GJ_OK;
-}
-
-// Bits of a key start table: about one bucket a key, at most 2^22 (16 MB).  A
-// larger table leaves L2 (2^26 probes into 2^23 keys: 770 us at 2^22, 865 at
-// 2^23, 1298 at 2^24), a smaller one leaves wider windows (2^26 keys: 2132 us
-// at 2^20, 1758 at 2^21, 1657 at 2^22).
-uint32_t key_start_bits(uint64_t n) {
-    uint32_t b = 1;
-    while (b < 22 && (1ull << b) < n) ++b;
-    return b;
 }
 
 int build_binary_search(gj_index* idx, cudaStream_t s) {
@@ -363,7 +390,7 @@ int build_binary_search(gj_index* idx, cudaStream_t s) {
     idx->bs.fence_steps = steps;
     idx->bytes = (uint64_t)slots * sizeof(uint64_t);
     if (idx->params.index_memory == GJ_INDEX_MEMORY_DEVICE)
-        GJ_TRY(build_key_start(idx, key_start_bits(idx->n), s, [](double, double) { return true; }));
+        GJ_TRY(build_key_start(idx, key_start_bits(idx->n), s, spare_memory(), [](double, double) { return true; }));
     return GJ_OK;
 }
 
@@ -403,19 +430,19 @@ int build_btree(gj_index* idx, cudaStream_t s) {
     void* p = nullptr;
     GJ_TRY(device_alloc(idx, total * sizeof(uint64_t), &p));
     uint64_t* base = static_cast<uint64_t*>(p);
-    uint64_t min_key = 0;
-    GJ_CUDA_TRY(cudaMemcpyAsync(&min_key, idx->d_col, sizeof(uint64_t), cudaMemcpyDefault, s));
+    // scattered lookups may get a key start table (below)
+    const bool candidate = W == kBtreeCompressed16 && L == 4 && idx->params.btree_start_bits == 0 &&
+                           idx->params.index_memory == GJ_INDEX_MEMORY_DEVICE;
+    spare_memory spare;
+    const uint64_t min_key = idx->min_key, maxk = idx->max_key;
     if (compressed) {
         // top down: a node's base comes from its parent's encoding
         uint64_t* bases[2] = {nullptr, nullptr};
-        cudaError_t e = cudaMalloc(reinterpret_cast<void**>(&bases[0]), nodes[1] * sizeof(uint64_t));
-        if (e == cudaSuccess) e = cudaMalloc(reinterpret_cast<void**>(&bases[1]), nodes[1] * sizeof(uint64_t));
-        if (e != cudaSuccess) {
-            cudaFree(bases[0]);
-            set_error("btree: scratch allocation failed: %s", cudaGetErrorString(e));
-            return GJ_ERR_OUT_OF_MEMORY;
-        }
-        GJ_CUDA_TRY(cudaStreamSynchronize(s));  // min_key
+        // the room of the key start table, when one follows
+        GJ_TRY(spare.take(std::max<size_t>(2 * nodes[1] * sizeof(uint64_t),
+                                           candidate ? key_start_bytes(idx, key_start_bits(n)) : 0)));
+        bases[0] = static_cast<uint64_t*>(spare.p);
+        bases[1] = bases[0] + nodes[1];
         int rc = GJ_OK;
         for (uint32_t l = height; l >= 1 && rc == GJ_OK; --l) {
             const uint64_t span = (uint64_t)L << (fan_log * (l - 1));
@@ -437,14 +464,7 @@ int build_btree(gj_index* idx, cudaStream_t s) {
             }
             idx->bt.level[l] = base + offset[l];
         }
-        const cudaError_t se = cudaStreamSynchronize(s);
-        cudaFree(bases[0]);
-        cudaFree(bases[1]);
         GJ_TRY(rc);
-        if (se != cudaSuccess) {
-            set_error("btree: encoding failed: %s", cudaGetErrorString(se));
-            return GJ_ERR_CUDA;
-        }
     } else {
         uint64_t span = L;  // column keys below one child of a level-1 node
         for (uint32_t l = 1; l <= height; ++l) {
@@ -474,9 +494,6 @@ int build_btree(gj_index* idx, cudaStream_t s) {
     idx->bt.node_keys = W;
     idx->bt.leaf_keys = L;
     idx->bt.col_aligned = aligned32(idx->d_col);
-    uint64_t maxk = 0;
-    GJ_CUDA_TRY(cudaMemcpyAsync(&maxk, idx->d_col + n - 1, sizeof(uint64_t), cudaMemcpyDefault, s));
-    GJ_CUDA_TRY(cudaStreamSynchronize(s));
     idx->bt.max_key = maxk;
     idx->bt.min_key = min_key;
     idx->bytes = total * sizeof(uint64_t);
@@ -515,7 +532,6 @@ int build_btree(gj_index* idx, cudaStream_t s) {
         default: k_btree_start<64><<<grid, 256, 0, s>>>(tv, entries, table); break;
     }
     GJ_CUDA_TRY(cudaGetLastError());
-    GJ_CUDA_TRY(cudaStreamSynchronize(s));
     idx->bt.start = table;
     idx->bt.start_shift = shift;
     idx->bt.start_entries = (uint32_t)entries;
@@ -528,11 +544,12 @@ int build_btree(gj_index* idx, cudaStream_t s) {
     // 2^24 keys that spread evenly (mean level about 2) the nodes' single
     // column sector wins (lognormal 2^26 keys: 1895 / 1572 us), and so they do
     // where a column is so uneven that the table's windows take long searches.
-    if (W == kBtreeCompressed16 && L == 4 && idx->params.btree_start_bits == 0 &&
-        idx->params.index_memory == GJ_INDEX_MEMORY_DEVICE)
-        GJ_TRY(build_key_start(idx, key_start_bits(n), s, [&](double loads, double level) {
+    if (candidate)
+        GJ_TRY(build_key_start(idx, key_start_bits(n), s, std::move(spare), [&](double loads, double level) {
             return loads <= 4.0 && (n <= (1ull << 24) || level >= 3.0);
         }));
+    else
+        GJ_CUDA_TRY(cudaStreamSynchronize(s));  // before the scratch is freed
     return GJ_OK;
 }
 
@@ -619,7 +636,7 @@ int build_harmonia(gj_index* idx, const uint64_t* h_keys, cudaStream_t s) {
     // table wins at every size (2^26 probes, table against nodes: 584 / 2135
     // us at 2^20 keys, 1764 / 3781 at 2^26, clustered 1.97 / 4.44 ms)
     if (idx->params.btree_start_bits == 0 && idx->params.index_memory == GJ_INDEX_MEMORY_DEVICE)
-        GJ_TRY(build_key_start(idx, key_start_bits(n), s, [](double loads, double) { return loads <= 4.0; }));
+        GJ_TRY(build_key_start(idx, key_start_bits(n), s, spare_memory(), [](double loads, double) { return loads <= 4.0; }));
     return GJ_OK;
 }
 
