@@ -7,14 +7,17 @@
 // query (src/tpch/cpu_only.cpp:230-275): rows pass when lo <= date < hi (the
 // GPU kernels of the reference test `date >= upper`, a bug not reproduced).
 //
-// Each block scans a tile of fact rows, compacts the rows that pass the date
-// filter into shared memory (ballot + popc), and only then probes the index
-// with the compacted rows, so warps stay full during the lookups (the role of
-// ij_np_lane_refill_scan_lookup, src/tpch/tpch_14_ij.cu:466-566).  Sums are
-// integer, so the result does not depend on the order of the atomics.
+// Each warp filters a run of fact rows and compacts the rows that pass into
+// shared memory, and only then probes the index with them, so its lanes stay
+// full during the lookups (the role of ij_np_lane_refill_scan_lookup,
+// src/tpch/tpch_14_ij.cu:466-566).  Sums are integer, so the result does not
+// depend on the order of the atomics.
 #include <cuda_runtime.h>
 
+#include <algorithm>
+#include <atomic>
 #include <cstdint>
+#include <type_traits>
 
 #include "gj_internal.h"
 
@@ -22,80 +25,11 @@ namespace gj {
 namespace {
 
 constexpr int kJoinBlock = 256;
-constexpr int kJoinItems = 16;
-constexpr int kJoinTile = kJoinBlock * kJoinItems;
 
-template <class Lookup>
-__global__ void __launch_bounds__(kJoinBlock) k_star_join(const Lookup lookup, const uint64_t* __restrict__ dim_col,
-                                                          const uint32_t* __restrict__ fk,
-                                                          const uint32_t* __restrict__ date,
-                                                          const int64_t* __restrict__ price,
-                                                          const int64_t* __restrict__ disc, uint64_t nfact,
-                                                          const uint8_t* __restrict__ flag, uint32_t lo, uint32_t hi,
-                                                          unsigned long long* __restrict__ out) {
-    __shared__ uint32_t s_rows[kJoinTile];
-    __shared__ uint32_t s_warp[kJoinBlock / 32];
-    __shared__ uint32_t s_count;
+// the sums of the block's threads into out, one atomic each
+__device__ __forceinline__ void add_sums(unsigned long long num, unsigned long long den,
+                                         unsigned long long* __restrict__ out) {
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    unsigned long long num = 0, den = 0;
-    const uint64_t tiles = (nfact + kJoinTile - 1) / kJoinTile;
-    for (uint64_t t = blockIdx.x; t < tiles; t += gridDim.x) {
-        const uint64_t base = t * kJoinTile;
-        // 1. filter + compact (rows in tile order)
-        uint32_t selected = 0;
-        uint32_t local[kJoinItems];
-#pragma unroll
-        for (int k = 0; k < kJoinItems; ++k) {
-            const uint64_t i = base + (uint64_t)k * kJoinBlock + threadIdx.x;
-            bool pass = false;
-            if (i < nfact) {
-                const uint32_t d = __ldcs(date + i);
-                pass = (d >= lo) && (d < hi);
-            }
-            local[k] = pass ? 1u : 0u;
-            selected += local[k];
-        }
-        uint32_t incl = selected;
-#pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-            const uint32_t v = __shfl_up_sync(0xffffffffu, incl, d);
-            if (lane >= (uint32_t)d) incl += v;
-        }
-        if (lane == 31) s_warp[warp] = incl;
-        __syncthreads();
-        if (warp == 0) {
-            uint32_t w = lane < kJoinBlock / 32 ? s_warp[lane] : 0u;
-            uint32_t wi = w;
-#pragma unroll
-            for (int d = 1; d < 32; d <<= 1) {
-                const uint32_t v = __shfl_up_sync(0xffffffffu, wi, d);
-                if (lane >= (uint32_t)d) wi += v;
-            }
-            if (lane < kJoinBlock / 32) s_warp[lane] = wi - w;
-            if (lane == kJoinBlock / 32 - 1) s_count = wi;
-        }
-        __syncthreads();
-        uint32_t o = s_warp[warp] + incl - selected;
-#pragma unroll
-        for (int k = 0; k < kJoinItems; ++k)
-            if (local[k]) s_rows[o++] = (uint32_t)(k * kJoinBlock + threadIdx.x);
-        __syncthreads();
-        // 2. probe the compacted rows
-        const uint32_t cnt = s_count;
-        for (uint32_t r = threadIdx.x; r < cnt; r += kJoinBlock) {
-            const uint64_t i = base + s_rows[r];
-            const uint64_t key = __ldg(fk + i);
-            const uint32_t pos = lookup(key);
-            if (pos != kInvalid && __ldg(reinterpret_cast<const unsigned long long*>(dim_col) + pos) == key) {
-                const int64_t summand = __ldg(reinterpret_cast<const long long*>(price) + i) *
-                                        (100 - __ldg(reinterpret_cast<const long long*>(disc) + i));
-                den += (unsigned long long)summand;
-                if (__ldg(flag + pos)) num += (unsigned long long)summand;
-            }
-        }
-        __syncthreads();
-    }
-    // block reduction, one atomic per sum per block
 #pragma unroll
     for (int d = 16; d > 0; d >>= 1) {
         num += __shfl_down_sync(0xffffffffu, num, d);
@@ -113,9 +47,81 @@ __global__ void __launch_bounds__(kJoinBlock) k_star_join(const Lookup lookup, c
             a += s_num[w];
             b += s_den[w];
         }
-        atomicAdd(&out[0], a);
-        atomicAdd(&out[1], b);
+        if (a) atomicAdd(&out[0], a);
+        if (b) atomicAdd(&out[1], b);
     }
+}
+
+// Warps work alone, each on runs of kV * 128 rows (kV 16-byte loads of dates
+// a lane, all in flight).  At 6M rows and a month's window the whole call is
+// a few memory latencies long: the dates, then per passing row the foreign
+// key with price and discount beside it, the index, the flag.  So there are
+// no block barriers on the way, one run of 1024 rows a warp covers such a
+// table in one wave, and short tables take runs of 256.  (Block tiles of 4096
+// rows with a block-wide scan took 15.3 us and a second, nearly empty wave.)
+// kVec: the dates are 16-byte aligned.
+template <class Lookup, int kV, bool kVec>
+__global__ void __launch_bounds__(kJoinBlock, kV > 4 ? 5 : 6) k_star_join(
+    const __grid_constant__ Lookup lookup, const uint32_t* __restrict__ fk, const uint32_t* __restrict__ date,
+    const int64_t* __restrict__ price, const int64_t* __restrict__ disc, uint64_t nfact,
+    const uint8_t* __restrict__ flag, uint32_t lo, uint32_t hi, unsigned long long* __restrict__ out) {
+    constexpr uint32_t kRun = kV * 128;
+    __shared__ uint16_t s_rows[kJoinBlock / 32][kRun];
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint16_t* rows = s_rows[warp];
+    unsigned long long num = 0, den = 0;
+    const uint64_t step = (uint64_t)gridDim.x * (kJoinBlock / 32) * kRun;
+    for (uint64_t base = ((uint64_t)blockIdx.x * (kJoinBlock / 32) + warp) * kRun; base < nfact; base += step) {
+        uint32_t pass = 0;  // bit 4 k + c: row base + 128 k + 4 lane + c
+        if (kVec && nfact - base >= kRun) {
+            uint4 d[kV];
+#pragma unroll
+            for (int k = 0; k < kV; ++k)
+                d[k] = __ldcs(reinterpret_cast<const uint4*>(date + base + k * 128) + lane);
+#pragma unroll
+            for (int k = 0; k < kV; ++k) {
+                const uint32_t b = (d[k].x >= lo && d[k].x < hi ? 1u : 0u) | (d[k].y >= lo && d[k].y < hi ? 2u : 0u) |
+                                   (d[k].z >= lo && d[k].z < hi ? 4u : 0u) | (d[k].w >= lo && d[k].w < hi ? 8u : 0u);
+                pass |= b << (4 * k);
+            }
+        } else {
+#pragma unroll 1
+            for (int k = 0; k < 4 * kV; ++k) {
+                const uint64_t i = base + (k >> 2) * 128 + 4 * lane + (k & 3);
+                if (i < nfact) {
+                    const uint32_t d = __ldcs(date + i);
+                    pass |= (d >= lo && d < hi ? 1u : 0u) << k;
+                }
+            }
+        }
+        const uint32_t mine = __popc(pass);
+        uint32_t incl = mine;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const uint32_t v = __shfl_up_sync(0xffffffffu, incl, d);
+            if (lane >= (uint32_t)d) incl += v;
+        }
+        const uint32_t count = __shfl_sync(0xffffffffu, incl, 31);
+        for (uint32_t o = incl - mine; pass; pass &= pass - 1, ++o) {
+            const uint32_t b = __ffs(pass) - 1;
+            rows[o] = (uint16_t)((b >> 2) * 128 + 4 * lane + (b & 3));
+        }
+        __syncwarp();
+        for (uint32_t r = lane; r < count; r += 32) {
+            const uint64_t i = base + rows[r];
+            const uint64_t key = __ldg(fk + i);
+            const int64_t p = __ldg(reinterpret_cast<const long long*>(price) + i);
+            const int64_t q = __ldg(reinterpret_cast<const long long*>(disc) + i);
+            const uint32_t pos = lookup(key);
+            if (pos != kInvalid) {
+                const int64_t summand = p * (100 - q);
+                den += (unsigned long long)summand;
+                if (__ldg(flag + pos)) num += (unsigned long long)summand;
+            }
+        }
+        __syncwarp();  // the rows are overwritten by the next run
+    }
+    add_sums(num, den, out);
 }
 
 // The reference's pipelined order, ij_pbws (src/tpch/tpch_14_ij.cu:95-362):
@@ -151,7 +157,7 @@ __device__ __forceinline__ void block_bitonic_sort(unsigned long long* s, uint32
 }
 
 template <class Lookup>
-__global__ void __launch_bounds__(kJoinBlock) k_star_join_sorted(const Lookup lookup, const uint64_t* __restrict__ dim_col,
+__global__ void __launch_bounds__(kJoinBlock) k_star_join_sorted(const __grid_constant__ Lookup lookup,
                                                                  const uint32_t* __restrict__ fk,
                                                                  const uint32_t* __restrict__ date,
                                                                  const int64_t* __restrict__ price,
@@ -226,7 +232,7 @@ __global__ void __launch_bounds__(kJoinBlock) k_star_join_sorted(const Lookup lo
                 const unsigned long long e = s_buf[j];
                 const uint64_t key = e >> 32, i = (uint32_t)e;
                 const uint32_t pos = lookup(key);
-                if (pos != kInvalid && __ldg(reinterpret_cast<const unsigned long long*>(dim_col) + pos) == key) {
+                if (pos != kInvalid) {
                     const int64_t summand = __ldg(reinterpret_cast<const long long*>(price) + i) *
                                             (100 - __ldg(reinterpret_cast<const long long*>(disc) + i));
                     den += (unsigned long long)summand;
@@ -239,53 +245,69 @@ __global__ void __launch_bounds__(kJoinBlock) k_star_join_sorted(const Lookup lo
         }
         if (!more) break;
     }
-#pragma unroll
-    for (int d = 16; d > 0; d >>= 1) {
-        num += __shfl_down_sync(0xffffffffu, num, d);
-        den += __shfl_down_sync(0xffffffffu, den, d);
-    }
-    __shared__ unsigned long long s_num[kJoinBlock / 32], s_den[kJoinBlock / 32];
-    if (lane == 0) {
-        s_num[warp] = num;
-        s_den[warp] = den;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        unsigned long long a = 0, b = 0;
-        for (int w = 0; w < kJoinBlock / 32; ++w) {
-            a += s_num[w];
-            b += s_den[w];
-        }
-        atomicAdd(&out[0], a);
-        atomicAdd(&out[1], b);
-    }
+    add_sums(num, den, out);
 }
 static_assert(kSortBatch + kSortTile <= kSortCap, "a batch plus one tile fits the buffer");
 
+// lookups of a foreign key: the position of the equal dimension key, or
+// kInvalid.  Nothing is staged in shared memory: every level comes from
+// global memory.
+struct join_start {
+    key_start t;
+    const uint64_t* col;
+    uint32_t n;
+    __device__ __forceinline__ uint32_t operator()(uint64_t key) const {
+        bool eq;
+        const uint32_t lb = start_lower_bound(t, col, n, key, &eq);
+        return eq ? lb : kInvalid;
+    }
+};
 template <int W>
 struct join_btree {
     btree_view v;
-    __device__ __forceinline__ uint32_t operator()(uint64_t key) const { return btree_lookup<W>(v, nullptr, key); }
+    __device__ __forceinline__ uint32_t operator()(uint64_t key) const {
+        return btree_lookup<W, true, false>(v, nullptr, key);
+    }
 };
 struct join_harmonia {
     harmonia_view v;
-    __device__ __forceinline__ uint32_t operator()(uint64_t key) const { return harmonia_lookup(v, nullptr, key); }
+    __device__ __forceinline__ uint32_t operator()(uint64_t key) const {
+        return harmonia_lookup<true, false>(v, nullptr, key);
+    }
 };
+__device__ __forceinline__ uint32_t if_equal(const uint64_t* col, uint32_t pos, uint64_t key) {
+    return pos != kInvalid && ld_ro(col + pos) == key ? pos : kInvalid;
+}
 struct join_bs {
     bs_view v;
     __device__ __forceinline__ uint32_t operator()(uint64_t key) const {
         bs_view u = v;
         u.fence_slots = 0;  // no shared cache in this kernel
-        return bs_lookup(u, nullptr, key);
+        return if_equal(v.col, bs_lookup(u, nullptr, key), key);
     }
 };
 struct join_rs {
     rs_view v;
-    __device__ __forceinline__ uint32_t operator()(uint64_t key) const { return rs_lookup(v, key); }
+    __device__ __forceinline__ uint32_t operator()(uint64_t key) const { return if_equal(v.col, rs_lookup(v, key), key); }
 };
 
+// Resident blocks per SM of a kernel, asked once per device: the query costs
+// as much as a launch, and the joins that care take about 10 us.
+template <class Lookup, int kWhich, class Kernel>
+int resident_blocks(Kernel kernel, int device, int* per_sm) {
+    static std::atomic<int> known[64];  // by device (0: not asked yet); one array per kernel
+    int n = known[device].load(std::memory_order_relaxed);
+    if (n == 0) {
+        GJ_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, kJoinBlock, 0));
+        if (n < 1) n = 1;
+        known[device].store(n, std::memory_order_relaxed);
+    }
+    *per_sm = n;
+    return GJ_OK;
+}
+
 template <class Lookup>
-int run_star_join_sorted(const Lookup& l, const gj_index* idx, const uint32_t* fk, const uint32_t* date,
+int run_star_join_sorted(const Lookup& l, const uint32_t* fk, const uint32_t* date,
                          const int64_t* price, const int64_t* disc, uint64_t nfact, const uint8_t* flag, uint32_t lo,
                          uint32_t hi, int64_t* out, cudaStream_t s) {
     GJ_CUDA_TRY(cudaMemsetAsync(out, 0, 2 * sizeof(int64_t), s));
@@ -293,34 +315,42 @@ int run_star_join_sorted(const Lookup& l, const gj_index* idx, const uint32_t* f
     device_info di;
     GJ_TRY(current_device_info(&di));
     int per_sm = 0;
-    GJ_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_star_join_sorted<Lookup>, kJoinBlock, 0));
-    uint64_t grid = (uint64_t)di.sm_count * (per_sm > 0 ? per_sm : 1);
+    GJ_TRY((resident_blocks<Lookup, 0>(k_star_join_sorted<Lookup>, di.device, &per_sm)));
+    uint64_t grid = (uint64_t)di.sm_count * per_sm;
     const uint64_t tiles = (nfact + kSortTile - 1) / kSortTile;
     if (grid > tiles) grid = tiles;
-    k_star_join_sorted<Lookup><<<(unsigned)grid, kJoinBlock, 0, s>>>(l, idx->d_col, fk, date, price, disc, nfact, flag,
-                                                                     lo, hi, reinterpret_cast<unsigned long long*>(out));
+    k_star_join_sorted<Lookup><<<(unsigned)grid, kJoinBlock, 0, s>>>(l, fk, date, price, disc, nfact, flag, lo, hi,
+                                                                     reinterpret_cast<unsigned long long*>(out));
     GJ_CUDA_TRY(cudaGetLastError());
     return GJ_OK;
 }
 
 template <class Lookup>
-int run_star_join(const Lookup& l, const gj_index* idx, const uint32_t* fk, const uint32_t* date, const int64_t* price,
+int run_star_join(const Lookup& l, const uint32_t* fk, const uint32_t* date, const int64_t* price,
                   const int64_t* disc, uint64_t nfact, const uint8_t* flag, uint32_t lo, uint32_t hi, int64_t* out,
                   cudaStream_t s, bool sorted = false) {
-    if (sorted) return run_star_join_sorted(l, idx, fk, date, price, disc, nfact, flag, lo, hi, out, s);
+    if (sorted) return run_star_join_sorted(l, fk, date, price, disc, nfact, flag, lo, hi, out, s);
     GJ_CUDA_TRY(cudaMemsetAsync(out, 0, 2 * sizeof(int64_t), s));
     if (nfact == 0) return GJ_OK;
     device_info di;
     GJ_TRY(current_device_info(&di));
-    int per_sm = 0;
-    GJ_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_star_join<Lookup>, kJoinBlock, 0));
-    uint64_t grid = (uint64_t)di.sm_count * (per_sm > 0 ? per_sm : 1);
-    const uint64_t tiles = (nfact + kJoinTile - 1) / kJoinTile;
-    if (grid > tiles) grid = tiles;
-    k_star_join<Lookup><<<(unsigned)grid, kJoinBlock, 0, s>>>(l, idx->d_col, fk, date, price, disc, nfact, flag, lo, hi,
-                                                             reinterpret_cast<unsigned long long*>(out));
-    GJ_CUDA_TRY(cudaGetLastError());
-    return GJ_OK;
+    auto launch = [&](auto kernel, auto which, uint64_t run) {
+        int per_sm = 0;
+        GJ_TRY((resident_blocks<Lookup, decltype(which)::value>(kernel, di.device, &per_sm)));
+        const uint64_t blocks = (nfact + run * (kJoinBlock / 32) - 1) / (run * (kJoinBlock / 32));
+        const uint64_t grid = std::min<uint64_t>((uint64_t)di.sm_count * per_sm, blocks);
+        kernel<<<(unsigned)grid, kJoinBlock, 0, s>>>(l, fk, date, price, disc, nfact, flag, lo, hi,
+                                                     reinterpret_cast<unsigned long long*>(out));
+        GJ_CUDA_TRY(cudaGetLastError());
+        return (int)GJ_OK;
+    };
+    using std::integral_constant;
+    if ((reinterpret_cast<uintptr_t>(date) & 15) != 0)
+        return launch(k_star_join<Lookup, 2, false>, integral_constant<int, 1>{}, 256);
+    // long runs once they fill half the chip's warps
+    if (nfact >= (uint64_t)di.sm_count * 24 * 1024)
+        return launch(k_star_join<Lookup, 8, true>, integral_constant<int, 2>{}, 1024);
+    return launch(k_star_join<Lookup, 2, true>, integral_constant<int, 3>{}, 256);
 }
 
 }  // namespace
@@ -340,7 +370,9 @@ int star_join(const gj_index* dim_index, const uint32_t* d_fk, const uint32_t* d
     }
     cudaStream_t s = as_stream(stream);
     const gj_index* idx = dim_index;
-    // this kernel stages nothing in shared memory: every level comes from global memory
+    if (idx->ks.pos)
+        return run_star_join(join_start{idx->ks, idx->d_col, (uint32_t)idx->n}, d_fk, d_date, d_price, d_discount,
+                             nfact, d_dim_flag, lo, hi, d_out, s, sorted);
     btree_view bt = idx->bt;
     bt.cached_levels = 0;
     harmonia_view hm = idx->hm;
@@ -349,17 +381,17 @@ int star_join(const gj_index* dim_index, const uint32_t* d_fk, const uint32_t* d
     switch (idx->type) {
         case GJ_INDEX_BTREE:
             return btree_dispatch(idx->bt.node_keys, [&](auto w) {
-                return run_star_join(join_btree<decltype(w)::value>{bt}, idx, d_fk, d_date, d_price, d_discount,
+                return run_star_join(join_btree<decltype(w)::value>{bt}, d_fk, d_date, d_price, d_discount,
                                      nfact, d_dim_flag, lo, hi, d_out, s, sorted);
             });
         case GJ_INDEX_HARMONIA:
-            return run_star_join(join_harmonia{hm}, idx, d_fk, d_date, d_price, d_discount, nfact, d_dim_flag, lo, hi,
+            return run_star_join(join_harmonia{hm}, d_fk, d_date, d_price, d_discount, nfact, d_dim_flag, lo, hi,
                                  d_out, s, sorted);
         case GJ_INDEX_BINARY_SEARCH:
-            return run_star_join(join_bs{idx->bs}, idx, d_fk, d_date, d_price, d_discount, nfact, d_dim_flag, lo, hi,
+            return run_star_join(join_bs{idx->bs}, d_fk, d_date, d_price, d_discount, nfact, d_dim_flag, lo, hi,
                                  d_out, s, sorted);
         case GJ_INDEX_RADIX_SPLINE:
-            return run_star_join(join_rs{idx->rs}, idx, d_fk, d_date, d_price, d_discount, nfact, d_dim_flag, lo, hi,
+            return run_star_join(join_rs{idx->rs}, d_fk, d_date, d_price, d_discount, nfact, d_dim_flag, lo, hi,
                                  d_out, s, sorted);
         default:
             set_error("gj_star_join_sum: the dimension index must be btree, harmonia, binary_search or radix_spline");
