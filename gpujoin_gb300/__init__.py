@@ -212,17 +212,31 @@ def _check(rc: int) -> None:
         raise GJError(rc, msg.decode() if msg else "")
 
 
-def _torch():
-    import torch
+_TORCH = None
+_RAW_STREAM = None  # (current device, its current stream's handle), where torch exposes them without objects
 
-    return torch
+
+def _torch():
+    global _TORCH, _RAW_STREAM
+    if _TORCH is None:
+        import torch
+
+        _TORCH = torch
+        dev = getattr(torch._C, "_cuda_getDevice", None)
+        raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+        if dev is not None and raw is not None:
+            _RAW_STREAM = (dev, raw)
+    return _TORCH
 
 
 def _stream(stream=None) -> int:
-    torch = _torch()
-    if stream is None:
-        stream = torch.cuda.current_stream()
-    return stream.cuda_stream
+    """Handle of the given stream, else of the current device's current stream."""
+    if stream is not None:
+        return stream.cuda_stream
+    torch = _TORCH or _torch()
+    if _RAW_STREAM is not None and torch.cuda.is_initialized():
+        return _RAW_STREAM[1](_RAW_STREAM[0]())
+    return torch.cuda.current_stream().cuda_stream
 
 
 def _hptr(t) -> int:
@@ -245,8 +259,7 @@ def _ptr(t) -> Optional[int]:
 
 
 def _empty(n: int, dtype, device):
-    torch = _torch()
-    return torch.empty(n, dtype=dtype, device=device)
+    return (_TORCH or _torch()).empty(n, dtype=dtype, device=device)
 
 
 def _workspace(nbytes: int, device):
@@ -353,7 +366,7 @@ class abstract_index:
         if out_pairs is None:
             out_pairs = _empty(2 * max(m, 1), torch.int32, dev)
         if out_count is None:
-            out_count = torch.zeros(1, dtype=torch.int64, device=dev)
+            out_count = _empty(1, torch.int64, dev)
         if workspace is None:
             need = _sz(0)
             _check(lib().gj_inlj_pairs_workspace_size(m, ctypes.byref(need)))
@@ -391,7 +404,7 @@ class abstract_index:
         if out_pairs is None:
             out_pairs = _empty(2 * max(m, 1), torch.int32, dev)
         if out_count is None:
-            out_count = torch.zeros(1, dtype=torch.int64, device=dev)
+            out_count = _empty(1, torch.int64, dev)
         if workspace is None:
             need = _sz(0)
             _check(lib().gj_inlj_pairs_workspace_size(m, ctypes.byref(need)))
@@ -463,7 +476,7 @@ class abstract_index:
         window = window_size if window_size else max(m, 1)
         pos = _empty(m, torch.int32, dev) if positions else None
         prs = _empty(2 * max(m, 1), torch.int32, dev) if pairs else None
-        cnt = torch.zeros(1, dtype=torch.int64, device=dev) if pairs else None
+        cnt = _empty(1, torch.int64, dev) if pairs else None  # the call starts it at 0
         if workspace is None:
             need = _sz(0)
             _check(lib().gj_partitioned_inlj_workspace_size(self.handle, window, radix_bits, ctypes.byref(need)))
@@ -663,7 +676,7 @@ def star_join_sum(dim_index: abstract_index, d_fk, d_date, d_price, d_discount, 
     sorted_batches: the reference's pipelined ij_pbws order (gj_star_join_sum_sorted)."""
     torch = _torch()
     if out is None:
-        out = torch.zeros(2, dtype=torch.int64, device=d_fk.device)
+        out = torch.empty(2, dtype=torch.int64, device=d_fk.device)  # overwritten by the call
     fn = lib().gj_star_join_sum_sorted if sorted_batches else lib().gj_star_join_sum
     _check(fn(dim_index.handle, _ptr(d_fk), _ptr(d_date), _ptr(d_price), _ptr(d_discount), d_fk.numel(),
               _ptr(d_dim_flag), lo, hi, _ptr(out), _stream(stream)))

@@ -10,8 +10,11 @@
 #include <algorithm>
 #include <cstdarg>
 #include <cstring>
+#include <map>
 #include <memory>
+#include <mutex>
 #include <string>
+#include <tuple>
 #include <utility>
 #include <vector>
 
@@ -57,6 +60,37 @@ int current_device_info(device_info* out) {
         cache[dev] = di;
     }
     *out = cache[dev];
+    return GJ_OK;
+}
+
+namespace {
+std::mutex g_kernel_mutex;
+std::map<std::pair<int, const void*>, size_t> g_kernel_smem;                               // limit raised to
+std::map<std::tuple<int, const void*, int, size_t>, int> g_kernel_resident;  // by block and dynamic smem
+}  // namespace
+
+int kernel_smem(const void* kernel, size_t smem) {
+    int dev = 0;
+    GJ_CUDA_TRY(cudaGetDevice(&dev));
+    std::lock_guard<std::mutex> lock(g_kernel_mutex);
+    size_t& raised = g_kernel_smem[{dev, kernel}];
+    if (smem > raised) {
+        GJ_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        raised = smem;
+    }
+    return GJ_OK;
+}
+
+int kernel_resident(const void* kernel, int block, size_t smem, int* per_sm) {
+    int dev = 0;
+    GJ_CUDA_TRY(cudaGetDevice(&dev));
+    std::lock_guard<std::mutex> lock(g_kernel_mutex);
+    int& n = g_kernel_resident[{dev, kernel, block, smem}];
+    if (n == 0) {
+        GJ_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, block, smem));
+        if (n < 1) n = 1;
+    }
+    *per_sm = n;
     return GJ_OK;
 }
 
@@ -870,6 +904,11 @@ int gj_index_build(int type, const uint64_t* d_keys, const uint64_t* h_keys, uin
     idx->d_col = d_keys;
     idx->params = p;
     GJ_CUDA_TRY(cudaGetDevice(&idx->device));
+    cudaPointerAttributes where;
+    if (d_keys && cudaPointerGetAttributes(&where, d_keys) == cudaSuccess)
+        idx->in_hbm = where.type == cudaMemoryTypeDevice && p.index_memory == GJ_INDEX_MEMORY_DEVICE;
+    else
+        cudaGetLastError();
 
     if (type != GJ_INDEX_NO_OP && n > 1) {
         unsigned long long* d_bad = nullptr;
@@ -1040,8 +1079,8 @@ int gj_inlj_pairs(const gj_index* index, const uint64_t* d_probes, uint64_t m, u
         set_error("gj_inlj_pairs: probe rows must fit 32 bits");
         return GJ_ERR_TOO_LARGE;
     }
-    // positions are parked in the upper half of the pairs buffer (2m u32)
-    return launch_pairs(index, d_probes, m, nullptr, d_pairs, nullptr, d_count, d_workspace, workspace_bytes,
+    // few probes park their positions in the upper half of the pairs buffer (2m u32)
+    return launch_pairs(index, d_probes, m, d_pairs, d_count, d_workspace, workspace_bytes,
                         d_pairs ? d_pairs + m : nullptr, as_stream(stream));
 }
 
@@ -1082,8 +1121,7 @@ int gj_inlj_pairs_sorted(const gj_index* index, const uint64_t* d_probes, uint64
         set_error("gj_inlj_pairs_sorted: probe rows must fit 32 bits");
         return GJ_ERR_TOO_LARGE;
     }
-    return launch_partitioned_pairs(index, d_probes, nullptr, m, d_pairs, nullptr, d_count, d_workspace,
-                                    workspace_bytes, as_stream(stream));
+    return launch_sorted_pairs(index, d_probes, m, d_pairs, d_count, d_workspace, workspace_bytes, as_stream(stream));
 }
 
 // device address of a caller buffer the GPU may touch: pinned or registered
@@ -1155,9 +1193,8 @@ static int host_pairs(const char* name, bool ordered, const gj_index* index, con
     if (!ordered)
         return launch_pairs_unordered(index, static_cast<const uint64_t*>(probes), m, static_cast<uint32_t*>(pairs),
                                       static_cast<uint64_t*>(count), d_workspace, workspace_bytes, as_stream(stream));
-    return launch_pairs(index, static_cast<const uint64_t*>(probes), m, nullptr, static_cast<uint32_t*>(pairs),
-                        nullptr, static_cast<uint64_t*>(count), d_workspace, workspace_bytes, nullptr,
-                        as_stream(stream));
+    return launch_pairs(index, static_cast<const uint64_t*>(probes), m, static_cast<uint32_t*>(pairs),
+                        static_cast<uint64_t*>(count), d_workspace, workspace_bytes, nullptr, as_stream(stream));
 }
 
 int gj_inlj_pairs_host(const gj_index* index, const uint64_t* h_probes, uint64_t m, uint32_t* h_pairs,

@@ -54,6 +54,13 @@ struct device_info {
 };
 int current_device_info(device_info* out);
 
+// Launch settings of a kernel on the current device, asked of the runtime once
+// and remembered: either question costs about as much as a launch.
+// kernel_smem raises the kernel's dynamic shared memory limit to smem where
+// it is lower; kernel_resident is the resident blocks per SM (at least 1).
+int kernel_smem(const void* kernel, size_t smem);
+int kernel_resident(const void* kernel, int block, size_t smem, int* per_sm);
+
 // aligned carve-out of a caller workspace
 struct workspace_carver {
     char* base;
@@ -103,6 +110,7 @@ struct gj_index {
     uint64_t n = 0;
     int device = 0;
     const uint64_t* d_col = nullptr;
+    bool in_hbm = false;  // the column and the index's own arrays are device memory
     uint64_t min_key = 0, max_key = 0;  // d_col[0], d_col[n - 1] (0 when empty)
     uint64_t bytes = 0;  // memory_consumption
     uint64_t host_bytes = 0;  // of which in pinned host memory
@@ -140,21 +148,16 @@ int launch_lookup(const gj_index* idx, const uint64_t* d_probes, uint64_t m, uin
 int launch_sorted_lookup(const gj_index* idx, const uint64_t* d_probes, uint64_t m, uint32_t* d_out, cudaStream_t s);
 int launch_scatter_lookup(const gj_index* idx, const uint64_t* d_keys, const uint32_t* d_rows, uint64_t m,
                           uint32_t* d_out, cudaStream_t s);
-// Pairs are written from offset *d_base (0 if null); *d_count = base +
-// matches.  With d_stash the probes take two passes (search, then ordered
-// compaction) and their positions are parked in d_stash: m u32 inside the
-// pairs buffer at or after u32 index 2 * (largest possible base) + m, so
-// that pair o only overlaps stash entries j <= o.  Without it, one pass.
-int launch_pairs(const gj_index* idx, const uint64_t* d_probes, uint64_t m, const uint32_t* d_rows,
-                 uint32_t* d_pairs, const uint64_t* d_base, uint64_t* d_count, void* ws, size_t ws_bytes,
-                 uint32_t* d_stash, cudaStream_t s);
-// Pairs of a partitioned relation (keys grouped by key range, row ids
-// attached): every tile of probes is sorted by key before it is searched.
-// Pairs are appended at *d_base; the order inside a tile is not fixed.
-// Workspace: pairs_workspace_bytes(m).
-int launch_partitioned_pairs(const gj_index* idx, const uint64_t* d_keys, const uint32_t* d_rows, uint64_t m,
-                             uint32_t* d_pairs, const uint64_t* d_base, uint64_t* d_count, void* ws, size_t ws_bytes,
-                             cudaStream_t s);
+// Pairs in probe order, *d_count = matches.  d_stash: room for m u32
+// positions at u32 index m of the pairs buffer (calls of few probes take two
+// passes through it), or null for buffers in host memory (always one pass).
+int launch_pairs(const gj_index* idx, const uint64_t* d_probes, uint64_t m, uint32_t* d_pairs, uint64_t* d_count,
+                 void* ws, size_t ws_bytes, uint32_t* d_stash, cudaStream_t s);
+// Pairs from block-wise sorted probes: every tile is sorted by key before it
+// is searched.  Tiles come in probe order, inside a tile pairs come in key
+// order.  Workspace: pairs_workspace_bytes(m).
+int launch_sorted_pairs(const gj_index* idx, const uint64_t* d_probes, uint64_t m, uint32_t* d_pairs, uint64_t* d_count,
+                        void* ws, size_t ws_bytes, cudaStream_t s);
 size_t pairs_workspace_bytes(uint64_t m);
 // launch_pairs for the test of the bounded waits: look-backs give up after
 // spin_limit polls, and tile 0 is never claimed (so every wait runs out)

@@ -15,9 +15,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
-#include <atomic>
 #include <cstdint>
-#include <type_traits>
 
 #include "gj_internal.h"
 
@@ -291,21 +289,6 @@ struct join_rs {
     __device__ __forceinline__ uint32_t operator()(uint64_t key) const { return if_equal(v.col, rs_lookup(v, key), key); }
 };
 
-// Resident blocks per SM of a kernel, asked once per device: the query costs
-// as much as a launch, and the joins that care take about 10 us.
-template <class Lookup, int kWhich, class Kernel>
-int resident_blocks(Kernel kernel, int device, int* per_sm) {
-    static std::atomic<int> known[64];  // by device (0: not asked yet); one array per kernel
-    int n = known[device].load(std::memory_order_relaxed);
-    if (n == 0) {
-        GJ_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, kJoinBlock, 0));
-        if (n < 1) n = 1;
-        known[device].store(n, std::memory_order_relaxed);
-    }
-    *per_sm = n;
-    return GJ_OK;
-}
-
 template <class Lookup>
 int run_star_join_sorted(const Lookup& l, const uint32_t* fk, const uint32_t* date,
                          const int64_t* price, const int64_t* disc, uint64_t nfact, const uint8_t* flag, uint32_t lo,
@@ -315,7 +298,7 @@ int run_star_join_sorted(const Lookup& l, const uint32_t* fk, const uint32_t* da
     device_info di;
     GJ_TRY(current_device_info(&di));
     int per_sm = 0;
-    GJ_TRY((resident_blocks<Lookup, 0>(k_star_join_sorted<Lookup>, di.device, &per_sm)));
+    GJ_TRY(kernel_resident(reinterpret_cast<const void*>(k_star_join_sorted<Lookup>), kJoinBlock, 0, &per_sm));
     uint64_t grid = (uint64_t)di.sm_count * per_sm;
     const uint64_t tiles = (nfact + kSortTile - 1) / kSortTile;
     if (grid > tiles) grid = tiles;
@@ -334,9 +317,9 @@ int run_star_join(const Lookup& l, const uint32_t* fk, const uint32_t* date, con
     if (nfact == 0) return GJ_OK;
     device_info di;
     GJ_TRY(current_device_info(&di));
-    auto launch = [&](auto kernel, auto which, uint64_t run) {
+    auto launch = [&](auto kernel, uint64_t run) {
         int per_sm = 0;
-        GJ_TRY((resident_blocks<Lookup, decltype(which)::value>(kernel, di.device, &per_sm)));
+        GJ_TRY(kernel_resident(reinterpret_cast<const void*>(kernel), kJoinBlock, 0, &per_sm));
         const uint64_t blocks = (nfact + run * (kJoinBlock / 32) - 1) / (run * (kJoinBlock / 32));
         const uint64_t grid = std::min<uint64_t>((uint64_t)di.sm_count * per_sm, blocks);
         kernel<<<(unsigned)grid, kJoinBlock, 0, s>>>(l, fk, date, price, disc, nfact, flag, lo, hi,
@@ -344,13 +327,12 @@ int run_star_join(const Lookup& l, const uint32_t* fk, const uint32_t* date, con
         GJ_CUDA_TRY(cudaGetLastError());
         return (int)GJ_OK;
     };
-    using std::integral_constant;
     if ((reinterpret_cast<uintptr_t>(date) & 15) != 0)
-        return launch(k_star_join<Lookup, 2, false>, integral_constant<int, 1>{}, 256);
+        return launch(k_star_join<Lookup, 2, false>, 256);
     // long runs once they fill half the chip's warps
     if (nfact >= (uint64_t)di.sm_count * 24 * 1024)
-        return launch(k_star_join<Lookup, 8, true>, integral_constant<int, 2>{}, 1024);
-    return launch(k_star_join<Lookup, 2, true>, integral_constant<int, 3>{}, 256);
+        return launch(k_star_join<Lookup, 8, true>, 1024);
+    return launch(k_star_join<Lookup, 2, true>, 256);
 }
 
 }  // namespace

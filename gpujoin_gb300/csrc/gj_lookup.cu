@@ -38,39 +38,33 @@ size_t pairs_workspace_bytes(uint64_t m) {
 
 int launch_lookup(const gj_index* idx, const uint64_t* d_probes, uint64_t m, uint32_t* d_out, cudaStream_t s) {
     if (m == 0) return GJ_OK;
-    return dispatch(idx, {lookup_action::positions, d_probes, nullptr, m, d_out, nullptr, nullptr, nullptr, 0,
-                          nullptr, s});
+    return dispatch(idx, {lookup_action::positions, d_probes, nullptr, m, d_out, nullptr, nullptr, 0, nullptr, s});
 }
 
 int launch_sorted_lookup(const gj_index* idx, const uint64_t* d_probes, uint64_t m, uint32_t* d_out, cudaStream_t s) {
     if (m == 0) return GJ_OK;
-    return dispatch(idx, {lookup_action::sorted_positions, d_probes, nullptr, m, d_out, nullptr, nullptr, nullptr, 0,
-                          nullptr, s});
+    return dispatch(idx, {lookup_action::sorted_positions, d_probes, nullptr, m, d_out, nullptr, nullptr, 0, nullptr, s});
 }
 
 int launch_scatter_lookup(const gj_index* idx, const uint64_t* d_keys, const uint32_t* d_rows, uint64_t m,
                           uint32_t* d_out, cudaStream_t s) {
     if (m == 0) return GJ_OK;
-    return dispatch(idx, {lookup_action::scatter, d_keys, d_rows, m, d_out, nullptr, nullptr, nullptr, 0, nullptr, s});
+    return dispatch(idx, {lookup_action::scatter, d_keys, d_rows, m, d_out, nullptr, nullptr, 0, nullptr, s});
 }
 
-int launch_pairs(const gj_index* idx, const uint64_t* d_probes, uint64_t m, const uint32_t* d_rows, uint32_t* d_pairs,
-                 const uint64_t* d_base, uint64_t* d_count, void* ws, size_t ws_bytes, uint32_t* d_stash,
-                 cudaStream_t s) {
-    return dispatch(idx, {lookup_action::pairs, d_probes, d_rows, m, d_pairs, d_base, d_count, ws, ws_bytes, d_stash,
-                          s});
+int launch_pairs(const gj_index* idx, const uint64_t* d_probes, uint64_t m, uint32_t* d_pairs, uint64_t* d_count,
+                 void* ws, size_t ws_bytes, uint32_t* d_stash, cudaStream_t s) {
+    return dispatch(idx, {lookup_action::pairs, d_probes, nullptr, m, d_pairs, d_count, ws, ws_bytes, d_stash, s});
 }
 
-int launch_partitioned_pairs(const gj_index* idx, const uint64_t* d_keys, const uint32_t* d_rows, uint64_t m,
-                             uint32_t* d_pairs, const uint64_t* d_base, uint64_t* d_count, void* ws, size_t ws_bytes,
-                             cudaStream_t s) {
-    return dispatch(idx, {lookup_action::sorted_pairs, d_keys, d_rows, m, d_pairs, d_base, d_count, ws, ws_bytes,
-                          nullptr, s});
+int launch_sorted_pairs(const gj_index* idx, const uint64_t* d_probes, uint64_t m, uint32_t* d_pairs, uint64_t* d_count,
+                        void* ws, size_t ws_bytes, cudaStream_t s) {
+    return dispatch(idx, {lookup_action::sorted_pairs, d_probes, nullptr, m, d_pairs, d_count, ws, ws_bytes, nullptr, s});
 }
 
 int launch_pairs_stalled(const gj_index* idx, const uint64_t* d_probes, uint64_t m, uint32_t* d_pairs,
                          uint64_t* d_count, void* ws, size_t ws_bytes, uint32_t spin_limit, cudaStream_t s) {
-    lookup_call c{lookup_action::pairs, d_probes, nullptr, m, d_pairs, nullptr, d_count, ws, ws_bytes,
+    lookup_call c{lookup_action::pairs, d_probes, nullptr, m, d_pairs, d_count, ws, ws_bytes,
                   d_pairs ? d_pairs + m : nullptr, s};
     c.spin_limit = spin_limit;
     c.skip_first_tile = true;
@@ -79,7 +73,7 @@ int launch_pairs_stalled(const gj_index* idx, const uint64_t* d_probes, uint64_t
 
 int launch_pairs_unordered(const gj_index* idx, const uint64_t* d_probes, uint64_t m, uint32_t* d_pairs,
                            uint64_t* d_count, void* ws, size_t ws_bytes, cudaStream_t s) {
-    lookup_call c{lookup_action::pairs, d_probes, nullptr, m, d_pairs, nullptr, d_count, ws, ws_bytes, nullptr, s};
+    lookup_call c{lookup_action::pairs, d_probes, nullptr, m, d_pairs, d_count, ws, ws_bytes, nullptr, s};
     c.unordered = true;
     return dispatch(idx, c);
 }

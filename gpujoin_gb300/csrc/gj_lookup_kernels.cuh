@@ -15,8 +15,6 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
-#include <map>
-#include <mutex>
 #include <type_traits>
 #include <utility>
 
@@ -29,14 +27,13 @@ enum class lookup_action { positions, scatter, pairs, sorted_pairs, sorted_posit
 struct lookup_call {
     lookup_action action;
     const uint64_t* keys;  // probes, or the keys of a partitioned relation
-    const uint32_t* rows;  // row ids (partitioned relation) or null
+    const uint32_t* rows;  // row ids of a partitioned relation (scatter), else null
     uint64_t m;
     uint32_t* out;         // positions (positions, scatter) or pairs
-    const uint64_t* d_base;
     uint64_t* d_count;
     void* ws;
     size_t ws_bytes;
-    uint32_t* stash;       // pairs: two-pass positions buffer, or null
+    uint32_t* stash;       // pairs: room for m positions (two passes), or null (host buffers)
     cudaStream_t s;
     // test hook of the bounded waits (gj_debug_inlj_pairs_stalled): a spin
     // limit other than kSpinLimit (0 = default) and a first tile left
@@ -260,10 +257,11 @@ __device__ __forceinline__ void stage_cache(uint64_t* dst, const stage_desc& sd)
 // probes into 2^26 keys 1568 against 1654 us); several save a block's start
 // where the searches run from L2 (hash table of 2^20 keys 406 against 485 us
 // with 8).
+constexpr uint64_t kL2Keys = 1ull << 23;  // columns of up to 64 MB stay in L2
 inline int long_blocks(uint64_t n, uint64_t m, bool* yes) {
     device_info di;
     GJ_TRY(current_device_info(&di));
-    *yes = n <= (1ull << 23) && m >= 16ull * di.sm_count * 8 * kBlock;  // 16 waves of a full chip
+    *yes = n <= kL2Keys && m >= 16ull * di.sm_count * 8 * kBlock;  // 16 waves of a full chip
     return GJ_OK;
 }
 
@@ -319,22 +317,23 @@ __global__ void __launch_bounds__(kBlock, Op::kMinBlocks) k_scatter_lookup(const
 // bounded anyway; on expiry the kernel raises the error flag (GJ_ERR_TIMEOUT
 // on the host) and stops writing.
 //
-// Plain probes take two passes: k_lookup writes the positions to the upper
-// half of the pairs buffer (the caller provides 2m u32), then
-// k_compact_pairs turns them into pairs.  The search pass has no block
-// barriers, and the compaction is a streaming pass.  Probes of a partitioned
-// relation (row ids, appended behind *d_base) take the single-pass k_pairs.
-// k_pairs items per thread (8 measured fastest for gj_inlj_pairs_host, whose
-// tiles read their probes from and write their pairs to host memory: 15.2 ms
-// per 2^28 probes, against 18.7 with 4 and 21.4 with 16); GJ_PAIRS_ITEMS
-// overrides it in tuning builds
-#ifndef GJ_PAIRS_ITEMS
-#define GJ_PAIRS_ITEMS 8
-#endif
-constexpr int kItems = GJ_PAIRS_ITEMS;
+// From kSinglePassMin probes on, k_pairs searches and places tile by tile.
+// Fewer take two passes, k_lookup with one probe a thread -- the positions go
+// to the upper half of the pairs buffer (the caller provides 2m u32) -- and
+// k_compact_pairs: 16,384 probes into 2^26 keys 18.7 us against 23.3 in tiles
+// of four probes a thread, 2^18 probes 25 against 28, 2^20 50.1 against 49.7.
+// Large calls save the positions' way through memory: 2^28 probes into a hash
+// table of 2^26 keys 6631 against 6081 us, into the B+tree 6856 against 6678.
+constexpr uint64_t kSinglePassMin = 1ull << 18;
+// probes a thread of k_pairs: 8 for long calls into a column that stays in L2
+// (hash table of 2^20 keys 2027 against 2212 us per 2^28 probes with 4), 4
+// where its sectors come from DRAM (learned index over 2^26 keys 8514 against
+// 8647 with 8) and for calls too short to fill the chip with long tiles (2^18
+// probes into 2^14 keys 14.8 against 18.9) or whose probes come over the host
+// link (33.3 M 1697 against 1773)
+constexpr int kItems = 8, kFewItems = 4;
 constexpr int kCompactItems = 16;                // k_compact_pairs items per thread
-static_assert(kItems >= 4 && (kItems & (kItems - 1)) == 0, "the pairs scan needs a power-of-two item count >= 4");
-constexpr uint32_t kTile = kBlock * kItems;
+static_assert(kFewItems >= 4, "the pairs scan gives each lane of a warp whole counts");
 // the workspace holds one state per kStateTile probes: enough for the
 // smallest tile of any pairs kernel, at the same offsets for all of them
 constexpr uint32_t kStateTile = kBlock * 4;
@@ -488,8 +487,7 @@ __device__ __forceinline__ void publish_tile(tile_pairs<kIt>& t, uint32_t tile, 
 // false when the kernel must stop (look-back timed out).
 template <int kIt, class RowOf>
 __device__ __forceinline__ bool place_tile(const tile_pairs<kIt>& t, RowOf&& row_of, uint32_t tile, uint2* pairs,
-                                           uint64_t base, uint64_t* __restrict__ d_count, const pairs_ws& ws,
-                                           uint32_t num_tiles) {
+                                           uint64_t* __restrict__ d_count, const pairs_ws& ws, uint32_t num_tiles) {
     __shared__ unsigned long long s_prefix;
     __shared__ int s_abort;
     if (threadIdx.x < 32) {
@@ -503,12 +501,12 @@ __device__ __forceinline__ bool place_tile(const tile_pairs<kIt>& t, RowOf&& row
                 atomicExch(&ws.tile_state[tile], kFlagPrefix | (prefix + t.total));
             s_abort = ok ? 0 : 1;
             s_prefix = prefix;
-            if (ok && tile == num_tiles - 1) *d_count = base + prefix + t.total;
+            if (ok && tile == num_tiles - 1) *d_count = prefix + t.total;
         }
     }
     __syncthreads();
     if (s_abort) return false;
-    write_tile(t, row_of, tile, pairs, base + s_prefix);
+    write_tile(t, row_of, tile, pairs, s_prefix);
     __syncthreads();
     return true;
 }
@@ -522,13 +520,13 @@ __device__ __forceinline__ bool place_tile(const tile_pairs<kIt>& t, RowOf&& row
 // pairs (src/tpch/tpch_14_ij.cu:371-407) -- and the last tile to finish
 // writes the count.
 template <int kIt, bool kOrdered = true, class Fill, class RowOf>
-__device__ __forceinline__ bool pairs_tile(Fill&& fill, RowOf&& row_of, uint32_t tile, uint2* pairs, uint64_t base,
+__device__ __forceinline__ bool pairs_tile(Fill&& fill, RowOf&& row_of, uint32_t tile, uint2* pairs,
                                            uint64_t* __restrict__ d_count, const pairs_ws& ws, uint32_t num_tiles) {
     __shared__ tile_pairs<kIt> t;
     fill((uint64_t)tile * (kBlock * kIt), t.pos);
     if constexpr (kOrdered) {
         publish_tile(t, tile, ws);
-        return place_tile(t, row_of, tile, pairs, base, d_count, ws, num_tiles);
+        return place_tile(t, row_of, tile, pairs, d_count, ws, num_tiles);
     } else {
         __shared__ unsigned long long s_first;
         count_tile(t, [&](unsigned long long total) {
@@ -537,11 +535,11 @@ __device__ __forceinline__ bool pairs_tile(Fill&& fill, RowOf&& row_of, uint32_t
                 __threadfence();  // this tile's total is counted before it counts as done
                 if (atomicAdd(&ws.totals[1], 1ull) == (unsigned long long)num_tiles - 1ull) {
                     __threadfence();
-                    *d_count = base + atomicAdd(&ws.totals[0], 0ull);
+                    *d_count = atomicAdd(&ws.totals[0], 0ull);
                 }
             }
         });
-        write_tile(t, row_of, tile, pairs, base + s_first);
+        write_tile(t, row_of, tile, pairs, s_first);
         __syncthreads();
         return true;
     }
@@ -554,17 +552,27 @@ __device__ __forceinline__ uint32_t claim_tile(const pairs_ws& ws) {
     return s_tile;
 }
 
+// The block that claims tile 0 writes an empty count before its own count is
+// published, so that a caller's fresh counter reads 0 even where a
+// look-back times out (the last tile overwrites it behind that publication).
+__device__ __forceinline__ void start_count(uint32_t tile, uint64_t* d_count) {
+    if (tile == 0 && threadIdx.x == 0) {
+        *d_count = 0;
+        __threadfence();
+    }
+}
+
 
 // Single pass: search and place pairs tile by tile.  Unordered, a tile is
-// written as soon as it is searched.  Ordered (host buffers), a block
-// publishes its tile's count, searches its next tile, and only then looks
+// written as soon as it is searched.  Ordered, a block publishes its tile's count, searches its next tile, and only then looks
 // back for the first tile's place and writes it: the counts of the
 // predecessors have arrived by then, where a block that looked back at once
-// sat idle until the slowest tile before it had come over the host link.
+// sat idle until the slowest tile before it was searched (or its probes had
+// come over the host link).
 // (33.3 M probes from host memory: 2109 us, 1808 with the write put off.)
 // Every look-back ends: it needs the counts of earlier tiles, which their
 // blocks publish before they wait for anything.
-template <class Op, bool kOrdered>
+template <class Op, bool kOrdered, int kIt>
 __global__ void __launch_bounds__(kBlock, Op::kMinBlocks) k_pairs(const __grid_constant__ Op op, const stage_desc sd, const uint64_t* __restrict__ probes,
                                                   uint64_t m, uint2* __restrict__ pairs,
                                                   uint64_t* __restrict__ d_count, pairs_ws ws, uint32_t num_tiles) {
@@ -573,10 +581,10 @@ __global__ void __launch_bounds__(kBlock, Op::kMinBlocks) k_pairs(const __grid_c
     auto search = [&](uint64_t t0, uint32_t* s_pos) {
         uint64_t next = load_probe(probes, t0 + threadIdx.x, m);
 #pragma unroll 1
-        for (int k = 0; k < kItems; ++k) {
+        for (int k = 0; k < kIt; ++k) {
             const uint64_t i = t0 + (uint64_t)k * kBlock + threadIdx.x;
             const uint64_t key = next;
-            if (k + 1 < kItems) next = load_probe(probes, i + kBlock, m);
+            if (k + 1 < kIt) next = load_probe(probes, i + kBlock, m);
             s_pos[k * kBlock + threadIdx.x] = i < m ? op(cache, key) : kInvalid;
         }
     };
@@ -585,18 +593,19 @@ __global__ void __launch_bounds__(kBlock, Op::kMinBlocks) k_pairs(const __grid_c
         for (;;) {
             const uint32_t tile = claim_tile(ws);
             if (tile >= num_tiles) break;
-            if (!pairs_tile<kItems, false>(search, row_of, tile, pairs, 0, d_count, ws, num_tiles)) break;
+            if (!pairs_tile<kIt, false>(search, row_of, tile, pairs, d_count, ws, num_tiles)) break;
         }
     } else {
-        __shared__ tile_pairs<kItems> s_tile[2];
+        __shared__ tile_pairs<kIt> s_tile[2];
         uint32_t pending = num_tiles;  // searched tile still to be written, in the other buffer
         for (uint32_t cur = 0;; cur ^= 1) {
             const uint32_t tile = claim_tile(ws);
             if (tile < num_tiles) {
-                search((uint64_t)tile * kTile, s_tile[cur].pos);
-                publish_tile<kItems>(s_tile[cur], tile, ws);
+                start_count(tile, d_count);
+                search((uint64_t)tile * (kBlock * kIt), s_tile[cur].pos);
+                publish_tile<kIt>(s_tile[cur], tile, ws);
             }
-            if (pending < num_tiles && !place_tile<kItems>(s_tile[cur ^ 1], row_of, pending, pairs, 0, d_count, ws, num_tiles)) break;
+            if (pending < num_tiles && !place_tile<kIt>(s_tile[cur ^ 1], row_of, pending, pairs, d_count, ws, num_tiles)) break;
             pending = tile;
             if (tile >= num_tiles) break;
         }
@@ -604,18 +613,15 @@ __global__ void __launch_bounds__(kBlock, Op::kMinBlocks) k_pairs(const __grid_c
 }
 
 // Second pass of the two-pass pairs: compact the positions k_lookup wrote
-// to the stash into pairs at *d_base + (rank of the match).  The stash lies
-// inside the pairs buffer, placed so that the u32 words of pair o only reach
-// stash entries j <= o: a tile writes pairs only after every earlier tile
+// to the stash into pairs at the rank of the match.  The stash is the upper
+// half of the pairs buffer, so the u32 words of pair o only reach stash
+// entries j <= o: a tile writes pairs only after every earlier tile
 // has published its count, i.e. after every earlier tile has read its
 // positions, so no position is overwritten before it is read.  (stash and
 // pairs alias, so neither is __restrict__.)
-__global__ void __launch_bounds__(kBlock) k_compact_pairs(const uint32_t* stash, const uint32_t* __restrict__ rows,
-                                                          uint64_t m, uint2* pairs,
-                                                          const uint64_t* __restrict__ d_base,
+__global__ void __launch_bounds__(kBlock) k_compact_pairs(const uint32_t* stash, uint64_t m, uint2* pairs,
                                                           uint64_t* __restrict__ d_count, pairs_ws ws,
                                                           uint32_t num_tiles) {
-    const uint64_t base = d_base ? *d_base : 0ull;
     auto load = [&](uint64_t t0, uint32_t* s_pos) {
 #pragma unroll
         for (int k = 0; k < kCompactItems; ++k) {
@@ -623,17 +629,17 @@ __global__ void __launch_bounds__(kBlock) k_compact_pairs(const uint32_t* stash,
             s_pos[k * kBlock + threadIdx.x] = i < m ? __ldcs(stash + i) : kInvalid;
         }
     };
+    auto row_of = [&](int, uint64_t i) { return (uint32_t)i; };
     for (;;) {
         const uint32_t tile = claim_tile(ws);
         if (tile >= num_tiles) break;
-        auto row_of = [&](int, uint64_t i) { return rows ? __ldcs(rows + i) : (uint32_t)i; };
-        if (!pairs_tile<kCompactItems>(load, row_of, tile, pairs, base, d_count, ws, num_tiles)) break;
+        start_count(tile, d_count);
+        if (!pairs_tile<kCompactItems>(load, row_of, tile, pairs, d_count, ws, num_tiles)) break;
     }
 }
 
-// Pairs of a partitioned relation (probes grouped by key range, rows
-// attached).  Each tile of kTile probes is first sorted by key in shared
-// memory -- a counting sort over kSortBuckets equal-width buckets of the
+// Pairs from block-wise sorted probes.  Each tile of kSortTile probes is first
+// sorted by key in shared memory -- a counting sort over kSortBuckets equal-width buckets of the
 // tile's key range -- and then searched in that order: neighbouring lanes
 // follow the same path through the upper index levels, and a warp-wide load
 // of one sector serves all lanes that ask for it.  Pairs leave in tile order
@@ -642,7 +648,7 @@ __global__ void __launch_bounds__(kBlock) k_compact_pairs(const uint32_t* stash,
 constexpr int kSortItems = 4;                        // probes per thread and tile
 constexpr uint32_t kSortTile = kBlock * kSortItems;  // 1024
 constexpr uint32_t kSortBuckets = kSortTile;
-static_assert(kStateTile <= kSortTile && kStateTile <= kTile && kStateTile <= kCompactTile,
+static_assert(kStateTile <= kSortTile && kStateTile <= kBlock * kFewItems && kStateTile <= kCompactTile,
               "the workspace needs a state per tile of every pairs kernel");
 
 __device__ __forceinline__ unsigned bit_length(uint64_t v) { return v ? 64u - (unsigned)__clzll(v) : 0u; }
@@ -763,29 +769,19 @@ __device__ __forceinline__ uint32_t sorted_lookup(const Op& op, const uint64_t* 
 }
 
 // about 21 KB of shared memory per block; 6 resident blocks (40 registers),
-// fewer for index kinds compiled for fewer.  kRows = false: no row ids, the
-// row of probe i is i (plain probes in sorted tiles).
-template <class Op, bool kRows>
+// fewer for index kinds compiled for fewer.
+template <class Op>
 __global__ void __launch_bounds__(kBlock, Op::kMinBlocks < 6 ? Op::kMinBlocks : 6) k_sorted_pairs(const __grid_constant__ Op op, const stage_desc sd,
-                                                         const uint64_t* __restrict__ keys,
-                                                         const uint32_t* __restrict__ rows, uint64_t m,
-                                                         uint2* __restrict__ pairs,
-                                                         const uint64_t* __restrict__ d_base,
-                                                         uint64_t* __restrict__ d_count, pairs_ws ws,
-                                                         uint32_t num_tiles) {
+                                                         const uint64_t* __restrict__ keys, uint64_t m,
+                                                         uint2* __restrict__ pairs, uint64_t* __restrict__ d_count,
+                                                         pairs_ws ws, uint32_t num_tiles) {
     extern __shared__ __align__(16) uint64_t cache[];
     using hint_t = typename tile_hint_of<Op>::type;
     __shared__ sorted_tile_smem<hint_t> t;
     stage_cache(cache, sd);
-    const uint64_t base = d_base ? *d_base : 0ull;
     auto fill = [&](uint64_t t0, uint32_t* s_pos) {
         const uint32_t tn = m - t0 < kSortTile ? (uint32_t)(m - t0) : kSortTile;
-        sort_tile(op, cache, keys, t0, tn,
-                  [&](uint32_t j) {
-                      if constexpr (kRows) return __ldcs(rows + t0 + j);
-                      else return (uint32_t)(t0 + j);
-                  },
-                  t);
+        sort_tile(op, cache, keys, t0, tn, [&](uint32_t j) { return (uint32_t)(t0 + j); }, t);
         const hint_t h = t.hint;
 #pragma unroll 1
         for (int k = 0; k < kSortItems; ++k) {
@@ -797,7 +793,8 @@ __global__ void __launch_bounds__(kBlock, Op::kMinBlocks < 6 ? Op::kMinBlocks : 
     for (;;) {
         const uint32_t tile = claim_tile(ws);
         if (tile >= num_tiles) break;
-        if (!pairs_tile<kSortItems>(fill, row_of, tile, pairs, base, d_count, ws, num_tiles)) break;
+        start_count(tile, d_count);
+        if (!pairs_tile<kSortItems>(fill, row_of, tile, pairs, d_count, ws, num_tiles)) break;
     }
 }
 
@@ -864,33 +861,20 @@ stage_desc make_stage(const gj_index* idx) {
 
 size_t stage_bytes(const stage_desc& sd) { return (size_t)(sd.words0 + sd.words1) * sizeof(uint64_t); }
 
+// a kernel's staged cache (smem bytes) beside its static shared memory, which
+// together may pass the 48 KB allowed without asking
 template <class Kernel>
-int prepare_smem(Kernel kernel, size_t smem) {
-    // Static plus dynamic shared memory above 48 KB needs the kernel's
-    // dynamic limit raised first; the limit set so far is remembered per
-    // (device, kernel), so the attribute call is made once per new maximum.
-    if (smem == 0) return GJ_OK;
-    int dev = 0;
-    GJ_CUDA_TRY(cudaGetDevice(&dev));
-    static std::mutex mu;
-    static std::map<std::pair<int, const void*>, size_t> raised;
-    std::lock_guard<std::mutex> lock(mu);
-    size_t& cur = raised[{dev, reinterpret_cast<const void*>(kernel)}];
-    if (smem > cur) {
-        GJ_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        cur = smem;
-    }
-    return GJ_OK;
+int kernel_staged(Kernel kernel, size_t smem) {
+    return smem ? kernel_smem(reinterpret_cast<const void*>(kernel), smem) : GJ_OK;
 }
 
 template <class Kernel>
 int grid_for(Kernel kernel, size_t smem, uint64_t work_items, int* grid) {
     device_info di;
     GJ_TRY(current_device_info(&di));
-    GJ_TRY(prepare_smem(kernel, smem));
+    GJ_TRY(kernel_staged(kernel, smem));
     int per_sm = 0;
-    GJ_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kBlock, smem));
-    if (per_sm < 1) per_sm = 1;
+    GJ_TRY(kernel_resident(reinterpret_cast<const void*>(kernel), kBlock, smem, &per_sm));
     uint64_t g = (uint64_t)di.sm_count * per_sm;
     const uint64_t need = (work_items + kBlock - 1) / kBlock;
     if (need < g) g = need ? need : 1;
@@ -903,7 +887,7 @@ int run_lookup(const Op& op, const stage_desc& sd, uint64_t n, const uint64_t* p
                cudaStream_t s) {
     const size_t smem = Op::kStaged ? stage_bytes(sd) : 0;
     auto launch = [&](auto kernel, int items) {
-        GJ_TRY(prepare_smem(kernel, smem));
+        GJ_TRY(kernel_staged(kernel, smem));
         const uint64_t tile = (uint64_t)kBlock * items;
         kernel<<<(unsigned)((m + tile - 1) / tile), kBlock, smem, s>>>(op, sd, probes, m, out);
         GJ_CUDA_TRY(cudaGetLastError());
@@ -918,7 +902,7 @@ template <class Op>
 int run_sorted_lookup(const Op& op, const stage_desc& sd, const uint64_t* probes, uint64_t m, uint32_t* out,
                       cudaStream_t s) {
     const size_t smem = stage_bytes(sd);
-    GJ_TRY(prepare_smem(k_sorted_lookup<Op>, smem));
+    GJ_TRY(kernel_staged(k_sorted_lookup<Op>, smem));
     const uint64_t per_block = (uint64_t)kSortTile * kSortedLookupTiles;
     const uint64_t grid = (m + per_block - 1) / per_block;
     k_sorted_lookup<Op><<<(unsigned)grid, kBlock, smem, s>>>(op, sd, probes, m, out);
@@ -931,7 +915,7 @@ int run_scatter(const Op& op, const stage_desc& sd, uint64_t n, const uint64_t* 
                 uint64_t m, uint32_t* out, cudaStream_t s) {
     const size_t smem = Op::kStaged ? stage_bytes(sd) : 0;
     auto launch = [&](auto kernel, int items) {
-        GJ_TRY(prepare_smem(kernel, smem));
+        GJ_TRY(kernel_staged(kernel, smem));
         const uint64_t tile = (uint64_t)kBlock * items;
         kernel<<<(unsigned)((m + tile - 1) / tile), kBlock, smem, s>>>(op, sd, keys, rows, m, out);
         GJ_CUDA_TRY(cudaGetLastError());
@@ -943,10 +927,9 @@ int run_scatter(const Op& op, const stage_desc& sd, uint64_t n, const uint64_t* 
 }
 
 template <class Op>
-int run_pairs(const Op& op, const stage_desc& sd, uint64_t n, const uint64_t* probes, const uint32_t* rows, uint64_t m,
-              uint32_t* pairs, const uint64_t* d_base, uint64_t* d_count, void* ws, size_t ws_bytes, uint32_t* stash,
-              cudaStream_t s, uint32_t spin_limit = 0, bool skip_first_tile = false, bool unordered = false) {
-    const uint32_t num_tiles = (uint32_t)((m + kTile - 1) / kTile);
+int run_pairs(const Op& op, const stage_desc& sd, uint64_t n, const uint64_t* probes, uint64_t m, uint32_t* pairs,
+              uint64_t* d_count, void* ws, size_t ws_bytes, uint32_t* stash, cudaStream_t s, uint32_t spin_limit = 0,
+              bool skip_first_tile = false, bool unordered = false) {
     pairs_ws pw;
     size_t used = 0;
     if (!carve_pairs_ws(ws, ws_bytes, m, &pw, &used)) {
@@ -955,10 +938,7 @@ int run_pairs(const Op& op, const stage_desc& sd, uint64_t n, const uint64_t* pr
         return GJ_ERR_WORKSPACE;
     }
     if (m == 0) {
-        if (d_base && d_base != d_count)
-            GJ_CUDA_TRY(cudaMemcpyAsync(d_count, d_base, sizeof(uint64_t), cudaMemcpyDeviceToDevice, s));
-        else if (!d_base)
-            GJ_CUDA_TRY(cudaMemsetAsync(d_count, 0, sizeof(uint64_t), s));
+        GJ_CUDA_TRY(cudaMemsetAsync(d_count, 0, sizeof(uint64_t), s));
         return GJ_OK;
     }
     GJ_CUDA_TRY(cudaMemsetAsync(ws, 0, used, s));
@@ -966,63 +946,51 @@ int run_pairs(const Op& op, const stage_desc& sd, uint64_t n, const uint64_t* pr
     // test hook: the tile counter starts at 1, so tile 0 is never claimed and
     // never publishes; every later tile's look-back runs out
     if (skip_first_tile) GJ_CUDA_TRY(cudaMemsetAsync(pw.tile_counter, 1, 1, s));
-    if (stash) {
+    if (stash && m < kSinglePassMin) {
         GJ_TRY(run_lookup(op, sd, n, probes, m, stash, s));
         const uint32_t compact_tiles = (uint32_t)((m + kCompactTile - 1) / kCompactTile);
         int grid = 0;
         GJ_TRY(grid_for(k_compact_pairs, 0, (uint64_t)compact_tiles * kBlock, &grid));
-        k_compact_pairs<<<grid, kBlock, 0, s>>>(stash, rows, m, reinterpret_cast<uint2*>(pairs), d_base, d_count, pw,
-                                                compact_tiles);
+        k_compact_pairs<<<grid, kBlock, 0, s>>>(stash, m, reinterpret_cast<uint2*>(pairs), d_count, pw, compact_tiles);
         GJ_CUDA_TRY(cudaGetLastError());
         return GJ_OK;
     }
     const size_t smem = Op::kStaged ? stage_bytes(sd) : 0;
-    int grid = 0;
-    if (rows || d_base) {
-        set_error("inlj pairs: the single pass takes plain probes");
-        return GJ_ERR_UNSUPPORTED;
-    }
-    auto single = [&](auto kernel) {
+    auto single = [&](auto kernel, uint32_t items) {
+        const uint32_t num_tiles = (uint32_t)((m + kBlock * items - 1) / (kBlock * items));
+        int grid = 0;
         GJ_TRY(grid_for(kernel, smem, (uint64_t)num_tiles * kBlock, &grid));
         kernel<<<grid, kBlock, smem, s>>>(op, sd, probes, m, reinterpret_cast<uint2*>(pairs), d_count, pw, num_tiles);
+        GJ_CUDA_TRY(cudaGetLastError());
         return (int)GJ_OK;
     };
-    GJ_TRY(unordered ? single(k_pairs<Op, false>) : single(k_pairs<Op, true>));
-    GJ_CUDA_TRY(cudaGetLastError());
-    return GJ_OK;
+    if (unordered) return single(k_pairs<Op, false, kItems>, kItems);
+    // (stash null: host buffers)
+    if (!stash || n > kL2Keys || m < (1ull << 22)) return single(k_pairs<Op, true, kFewItems>, kFewItems);
+    return single(k_pairs<Op, true, kItems>, kItems);
 }
 
 template <class Op>
-int run_sorted_pairs(const Op& op, const stage_desc& sd, const uint64_t* keys, const uint32_t* rows, uint64_t m,
-                     uint32_t* pairs, const uint64_t* d_base, uint64_t* d_count, void* ws, size_t ws_bytes,
-                     cudaStream_t s) {
+int run_sorted_pairs(const Op& op, const stage_desc& sd, const uint64_t* probes, uint64_t m, uint32_t* pairs,
+                     uint64_t* d_count, void* ws, size_t ws_bytes, cudaStream_t s) {
     const uint32_t num_tiles = (uint32_t)((m + kSortTile - 1) / kSortTile);
     pairs_ws pw;
     size_t used = 0;
     if (!carve_pairs_ws(ws, ws_bytes, m, &pw, &used)) {
-        set_error("partitioned pairs: workspace of %zu bytes is smaller than the %zu required", ws_bytes,
+        set_error("sorted pairs: workspace of %zu bytes is smaller than the %zu required", ws_bytes,
                   pairs_workspace_bytes(m));
         return GJ_ERR_WORKSPACE;
     }
     if (m == 0) {
-        if (d_base && d_base != d_count)
-            GJ_CUDA_TRY(cudaMemcpyAsync(d_count, d_base, sizeof(uint64_t), cudaMemcpyDeviceToDevice, s));
-        else if (!d_base)
-            GJ_CUDA_TRY(cudaMemsetAsync(d_count, 0, sizeof(uint64_t), s));
+        GJ_CUDA_TRY(cudaMemsetAsync(d_count, 0, sizeof(uint64_t), s));
         return GJ_OK;
     }
     GJ_CUDA_TRY(cudaMemsetAsync(ws, 0, used, s));
     const size_t smem = stage_bytes(sd);
     int grid = 0;
-    if (rows) {
-        GJ_TRY(grid_for(k_sorted_pairs<Op, true>, smem, (uint64_t)num_tiles * kBlock, &grid));
-        k_sorted_pairs<Op, true><<<grid, kBlock, smem, s>>>(op, sd, keys, rows, m, reinterpret_cast<uint2*>(pairs),
-                                                            d_base, d_count, pw, num_tiles);
-    } else {
-        GJ_TRY(grid_for(k_sorted_pairs<Op, false>, smem, (uint64_t)num_tiles * kBlock, &grid));
-        k_sorted_pairs<Op, false><<<grid, kBlock, smem, s>>>(op, sd, keys, rows, m, reinterpret_cast<uint2*>(pairs),
-                                                             d_base, d_count, pw, num_tiles);
-    }
+    GJ_TRY(grid_for(k_sorted_pairs<Op>, smem, (uint64_t)num_tiles * kBlock, &grid));
+    k_sorted_pairs<Op><<<grid, kBlock, smem, s>>>(op, sd, probes, m, reinterpret_cast<uint2*>(pairs), d_count, pw,
+                                                  num_tiles);
     GJ_CUDA_TRY(cudaGetLastError());
     return GJ_OK;
 }
@@ -1034,10 +1002,10 @@ int run_call(const Op& op, const gj_index* idx, const lookup_call& c) {
         case lookup_action::positions: return run_lookup(op, sd, idx->n, c.keys, c.m, c.out, c.s);
         case lookup_action::scatter: return run_scatter(op, sd, idx->n, c.keys, c.rows, c.m, c.out, c.s);
         case lookup_action::pairs:
-            return run_pairs(op, sd, idx->n, c.keys, c.rows, c.m, c.out, c.d_base, c.d_count, c.ws, c.ws_bytes, c.stash, c.s,
-                             c.spin_limit, c.skip_first_tile, c.unordered);
+            return run_pairs(op, sd, idx->n, c.keys, c.m, c.out, c.d_count, c.ws, c.ws_bytes, c.stash, c.s, c.spin_limit,
+                             c.skip_first_tile, c.unordered);
         case lookup_action::sorted_pairs:
-            return run_sorted_pairs(op, sd, c.keys, c.rows, c.m, c.out, c.d_base, c.d_count, c.ws, c.ws_bytes, c.s);
+            return run_sorted_pairs(op, sd, c.keys, c.m, c.out, c.d_count, c.ws, c.ws_bytes, c.s);
         case lookup_action::sorted_positions: return run_sorted_lookup(op, sd, c.keys, c.m, c.out, c.s);
     }
     set_error("probe kernels: unknown action");

@@ -399,7 +399,7 @@ bool carve_tables(void* ws, size_t ws_bytes, const partition_plan& pl, part_tabl
 template <class Kernel, class... Args>
 int launch(Kernel kernel, uint32_t grid, int block, size_t smem, cudaStream_t s, Args... args) {
     if (smem > 40 * 1024)  // with the kernels' static part, near the 48 KB allowed without asking
-        GJ_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        GJ_TRY(kernel_smem(reinterpret_cast<const void*>(kernel), smem));
     kernel<<<grid, block, smem, s>>>(args...);
     GJ_CUDA_TRY(cudaGetLastError());
     return GJ_OK;
