@@ -83,10 +83,9 @@ constexpr uint32_t kProbeTile = kProbeBlock * kProbeItems;
 constexpr uint32_t kChunk = 4 * kProbeTile;  // probes per block
 
 // window size from which positions come back through the partition's inverse
-#ifndef GJ_GATHER_MIN
-#define GJ_GATHER_MIN (1ull << 22)
-#endif
-constexpr uint64_t kGatherMin = GJ_GATHER_MIN;
+// (below it a window's positions stay in L2: 151 us either way at 2^22 probes
+// into 2^22 keys, at 2^23 224 against 240, at 2^25 664 against 984)
+constexpr uint64_t kGatherMin = 1ull << 22;
 
 enum probe_semantics : int { kSemNone = 0, kSemLowerBound = 1, kSemExact = 2 };
 
@@ -369,7 +368,15 @@ __global__ void __launch_bounds__(kProbeBlock, GJ_PROBE_BLOCKS) k_part_probe(con
                     bool eq = false;
                     const uint64_t lo = (uint64_t)slo[k] << 2;
                     const uint64_t hi = (((uint64_t)shi[k] + 1) << 2) < a.n ? ((uint64_t)shi[k] + 1) << 2 : a.n;
-                    const uint64_t lb = lower_bound_sectors(a.col, a.n, lo, hi, key[k], kAligned, &eq);
+                    uint64_t lb = lo;
+                    if (kAligned && lo < hi) {
+                        // a crowded bucket: from its middle, by the spacing of the keys met
+                        uint32_t edge;
+                        lb = search_sectors<kL2Default>(a.col, (uint32_t)a.n, slo[k], (uint32_t)((hi - 1) >> 2),
+                                                        (uint32_t)((lo + hi) >> 3), key[k], &eq, &edge);
+                    } else {
+                        lb = lower_bound_sectors(a.col, a.n, lo, hi, key[k], kAligned, &eq);
+                    }
                     if (lb < a.n && (kSem == kSemLowerBound || eq)) res[r + k] = (uint32_t)lb;
                 }
             }
@@ -516,6 +523,29 @@ int dispatch_probe(int sem, bool aligned, const probe_args& a, cudaStream_t s) {
     return aligned ? launch_probe<kSemLowerBound, true>(a, s) : launch_probe<kSemLowerBound, false>(a, s);
 }
 
+// Whether the plain lookup returns a window's positions sooner than
+// partitioning it: partitioning pays once the column is far larger than L2 and
+// the window has probes enough per column line (2^26 uniform keys, default
+// B+tree, plain / partitioned: 107 / 271 us for 2^22 probes, 774 / 867 for
+// 2^25, 1538 / 1346 for 2^26; 2^28 keys 1292 / 1396 for 2^25, 5135 / 3393 for
+// 2^27; 2^25 lognormal keys 5391 / 6180 for 2^28, uniform 5280 / 4746; up to
+// 2^24 keys plain wins at every window).  Index kinds whose plain search is
+// long (RadixSpline, trees without a start table, MLP roots) only come out
+// ahead in windows too short to fill the chip's passes (RadixSpline over 2^26
+// keys: 231 / 271 us for 2^22 probes, 890 / 580 for 2^24).
+bool plain_lookup_wins(const gj_index* idx, uint64_t len) {
+    if (!idx->in_hbm) return false;
+    bool short_search = idx->ks.pos != nullptr;
+    switch (idx->type) {
+        case GJ_INDEX_NO_OP:
+        case GJ_INDEX_HASH: short_search = true; break;
+        case GJ_INDEX_BTREE: short_search |= idx->bt.node_keys == kBtreeCompressed16; break;
+        case GJ_INDEX_LEARNED: short_search = idx->ln.root_kind != GJ_LEARNED_ROOT_MLP; break;
+        default: break;
+    }
+    return len < (1ull << 22) || (short_search && (idx->n <= (1ull << 25) || len < 3 * (1ull << 24)));
+}
+
 // the directory of an index into dir (L.dir_entries entries)
 int build_directory(const gj_index* idx, const partitioned_layout& L, uint32_t* dir, uint32_t* tiles,
                     cudaStream_t s) {
@@ -624,7 +654,9 @@ int gj_partitioned_inlj(const gj_index* index, const uint64_t* d_probes, uint64_
     if (m == 0) return GJ_OK;
 
     const int sem = semantics_of(index);
-    if (sem != kSemNone && !prepared) GJ_TRY(build_directory(index, L, dir, tiles, s));
+    const bool positions_only = d_positions && !d_pairs;
+    const bool plain_windows = positions_only && plain_lookup_wins(index, std::min(w, m));
+    if (sem != kSemNone && !prepared && !plain_windows) GJ_TRY(build_directory(index, L, dir, tiles, s));
     const uint32_t pshift = shift_for(index->min_key, index->max_key, radix_bits);
     probe_args a;
     a.pkeys = pkeys;
@@ -641,13 +673,17 @@ int gj_partitioned_inlj(const gj_index* index, const uint64_t* d_probes, uint64_
     const bool aligned = (reinterpret_cast<uintptr_t>(index->d_col) & 31) == 0;
     for (uint64_t off = 0; off < m; off += w) {
         const uint64_t len = std::min<uint64_t>(w, m - off);
+        if (plain_windows) {
+            GJ_TRY(launch_lookup(index, d_probes + off, len, d_positions + off, s));
+            continue;
+        }
         a.len = len;
         // Positions alone come back to probe order through the partition's
         // inverse, kept where the row ids would be, unless the window's
         // positions are few enough to stay in L2 while they are stored one
         // by one.
         partition_inverse iv{};
-        const bool back = d_positions && !d_pairs && len >= kGatherMin &&
+        const bool back = positions_only && len >= kGatherMin &&
                           carve_partition_inverse(prows, w * sizeof(uint32_t), len, radix_bits, di.sm_count, &iv);
         GJ_TRY(range_partition_impl(d_probes + off, len, index->min_key, pshift, radix_bits, off, pkeys, prows,
                                     nullptr, pws, pws_bytes, s, back ? &iv : nullptr));

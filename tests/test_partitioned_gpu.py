@@ -146,7 +146,8 @@ def test_positions_through_the_inverse(orc, gj, cuda, radix_bits, m, window):
     rng = np.random.default_rng(radix_bits)
     col = column(rng, 300_007)
     pr = probes_for(rng, col, m)[:m]
-    for kind in ("btree", "binary_search"):
-        ix = gj.make_index(kind).construct(None, to_dev(torch, col)).prepare_partitioned()
+    # kinds whose plain lookup is not taken for windows of this size, and one for which it is
+    for kind, params in (("radix_spline", {}), ("btree", {"btree_node_keys": 8}), ("btree", {})):
+        ix = gj.make_index(kind, **params).construct(None, to_dev(torch, col)).prepare_partitioned()
         got, _, _ = ix.partitioned_inlj(to_dev(torch, pr), window_size=window, radix_bits=radix_bits)
         np.testing.assert_array_equal(from_dev_u32(got), expected(orc, kind, col, pr))
