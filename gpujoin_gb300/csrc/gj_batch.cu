@@ -30,10 +30,10 @@
 namespace gj {
 namespace {
 
-// resident blocks per SM (the register cap: 32); 512 batches over eight
+// resident blocks per SM (the register cap: 40); 512 batches over eight
 // indexes took 4222 us with every kind's search inlined in one loop (and no
-// cap), with a loop per kind 2501 / 2195 / 2061 / 2032 at 4 / 5 / 6 / 8
-constexpr int kBatchPerSM = 8;
+// cap), with a loop per kind 2200 / 2136 / 2182 at 5 / 6 / 8
+constexpr int kBatchPerSM = 6;
 constexpr int kBatchBlock = 256;
 
 // What a tile's searches need to know of its index.  The common kinds have a

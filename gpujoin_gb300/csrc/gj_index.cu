@@ -115,13 +115,25 @@ __global__ void k_gather_fence(const uint64_t* __restrict__ col, uint64_t n, uin
     }
 }
 
-// key start table: pos[b] = the first key not below bucket b's first value
-// (binary search per bucket; n from the bucket past the last one on)
+// key start table: the first key not below each bucket's first value (binary
+// search per bucket; n from the bucket past the last one on), with the
+// bucket's count where entries are packed; clears the sums of the cost sample
 __global__ void k_key_start(const uint64_t* __restrict__ col, uint64_t n, uint64_t min_key, uint32_t shift,
-                            uint32_t buckets, uint32_t entries, uint32_t* __restrict__ pos) {
-    for (uint32_t b = blockIdx.x * blockDim.x + threadIdx.x; b < entries; b += gridDim.x * blockDim.x)
-        pos[b] = b >= buckets ? (uint32_t)n
-                              : (uint32_t)lower_bound_branch_free(col, n, min_key + ((uint64_t)b << shift));
+                            uint32_t buckets, uint32_t entries, uint32_t packed, uint32_t* __restrict__ pos,
+                            unsigned long long* __restrict__ sums) {
+    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t < 2) sums[t] = 0;
+    for (uint32_t b = t; b < entries; b += gridDim.x * blockDim.x) {
+        const uint64_t first = min_key + ((uint64_t)b << shift);
+        const uint64_t lo = b >= buckets ? n : lower_bound_branch_free(col, n, first);
+        uint32_t e = (uint32_t)lo;
+        if (packed && b < buckets) {
+            const uint64_t rest =
+                b + 1 == buckets ? n - lo : lower_bound_branch_free(col + lo, n - lo, first + (1ull << shift));
+            e |= (rest < kStartWide ? (uint32_t)rest : kStartWide) << kStartPosBits;
+        }
+        pos[b] = e;
+    }
 }
 
 // sums[0] += column sectors the key start table's searches read, sums[1] +=
@@ -384,10 +396,11 @@ int build_key_start(gj_index* idx, uint32_t bits, cudaStream_t s, spare_memory&&
     uint32_t* pos = static_cast<uint32_t*>(spare.p);
     unsigned long long* d_sums = reinterpret_cast<unsigned long long*>(pos + entries);
     unsigned long long sums[2] = {0, 0};
-    k_key_start<<<(entries + 255) / 256, 256, 0, s>>>(idx->d_col, idx->n, t.min_key, t.shift, buckets, entries, pos);
+    t.packed = idx->n <= kStartPackedKeys ? 1u : 0u;
+    k_key_start<<<(entries + 255) / 256, 256, 0, s>>>(idx->d_col, idx->n, t.min_key, t.shift, buckets, entries,
+                                                     t.packed, pos, d_sums);
     GJ_CUDA_TRY(cudaGetLastError());
     t.pos = pos;
-    GJ_CUDA_TRY(cudaMemsetAsync(d_sums, 0, sizeof(sums), s));
     k_start_cost<<<kStartSample / 256, 256, 0, s>>>(t, idx->d_col, (uint32_t)idx->n, idx->bt, d_sums);
     GJ_CUDA_TRY(cudaGetLastError());
     GJ_CUDA_TRY(cudaMemcpyAsync(sums, d_sums, sizeof(sums), cudaMemcpyDeviceToHost, s));

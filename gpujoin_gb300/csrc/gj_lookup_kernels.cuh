@@ -94,7 +94,7 @@ struct stage_desc {
 // and touch a slice of the tree, use the default class.
 struct op_bs {
     static constexpr int kMinBlocks = GJ_BLOCKS(8);
-    static constexpr int kLong = 2;
+    static constexpr int kLong = 4;
     static constexpr bool kStaged = true;
     bs_view v;
     template <bool kScattered = true>
@@ -109,7 +109,7 @@ struct op_bs {
 template <bool kExact>
 struct op_start {
     static constexpr int kMinBlocks = GJ_BLOCKS(8);
-    static constexpr int kLong = 2;
+    static constexpr int kLong = 4;
     static constexpr bool kStaged = false;
     key_start t;
     const uint64_t* col;
@@ -162,7 +162,7 @@ struct tile_hint_of<Op, std::void_t<typename Op::tile_hint>> {
 };
 struct op_harmonia {
     static constexpr int kMinBlocks = GJ_BLOCKS(8);
-    static constexpr int kLong = 2;
+    static constexpr int kLong = 4;
     static constexpr bool kStaged = false;
     harmonia_view v;
     harmonia_child_base base;
@@ -219,7 +219,7 @@ struct op_learned {
 // linear and segment-table roots: no network to evaluate, twice the warps
 struct op_learned_plain {
     static constexpr int kMinBlocks = GJ_BLOCKS(8);
-    static constexpr int kLong = 2;
+    static constexpr int kLong = 4;
     static constexpr bool kStaged = false;
     learned_view v;
     float p[2];
@@ -256,7 +256,8 @@ __device__ __forceinline__ void stage_cache(uint64_t* dst, const stage_desc& sd)
 // keeps most loads in flight when the column's sectors come from DRAM (2^26
 // probes into 2^26 keys 1568 against 1654 us); several save a block's start
 // where the searches run from L2 (hash table of 2^20 keys 406 against 485 us
-// with 8).
+// with 8, key start table 534 against 569 with 4; RadixSpline, whose registers
+// then spill, is level or slower).
 constexpr uint64_t kL2Keys = 1ull << 23;  // columns of up to 64 MB stay in L2
 inline int long_blocks(uint64_t n, uint64_t m, bool* yes) {
     device_info di;

@@ -141,6 +141,17 @@ GJ_DEVICE_INLINE uint64_t pick4(const uint64_t (&k)[4], uint32_t i) {
     return (i & 2) ? hi : lo;
 }
 
+// Keys of a sorted sector below key, by halving in registers; *eq: one of them
+// equals it (the one at the returned place).
+GJ_DEVICE_INLINE uint32_t sector_rank(const uint64_t (&k)[4], uint64_t key, bool* eq) {
+    const bool p = k[1] < key;
+    const uint64_t a = p ? k[2] : k[0], b = p ? k[3] : k[1];
+    const bool q = a < key;
+    const uint64_t c = q ? b : a;
+    *eq = c == key;
+    return (p ? 2u : 0u) + (q ? 1u : 0u) + (c < key ? 1u : 0u);
+}
+
 // Lower bound of key in arr[lo, hi) by a binary search over the 32-byte
 // sectors that cover the range.  arr must be 32-byte aligned when aligned is
 // set; arr_n is the number of valid entries of arr (a sector that reaches
@@ -229,7 +240,8 @@ GJ_DEVICE_INLINE uint32_t search_sectors(const uint64_t* col, uint32_t n, uint32
             for (uint32_t i = 0; i < 4; ++i) k[i] = (i < n - s0) ? ld_ro_c<kClass>(col + s0 + i) : ~0ull;
         }
         if constexpr (kCount) ++*loads;
-        const uint32_t below = (k[0] < key) + (k[1] < key) + (k[2] < key) + (k[3] < key);
+        bool at;
+        const uint32_t below = sector_rank(k, key, &at);
         if (below == 4) {
             if (s == sr) {
                 *eq = sr != sr0 && right_key == key;
@@ -261,7 +273,7 @@ GJ_DEVICE_INLINE uint32_t search_sectors(const uint64_t* col, uint32_t n, uint32
                 continue;
             }
         } else {
-            *eq = s0 + below < n && pick4(k, below) == key;
+            *eq = at && s0 + below < n;
             *edge = below == 0 && s == sl0 ? 1u : 0u;
             return s0 + below;
         }
@@ -276,6 +288,9 @@ GJ_DEVICE_INLINE uint32_t search_sectors(const uint64_t* col, uint32_t n, uint32
 // four), so the lower bound of a key of bucket b lies in [pos[b], pos[b + 1]].
 // One load replaces the search above that window.  A narrow window is read
 // from its start; in a wide one the key's place in its bucket says where.
+// Up to 2^24 keys an entry also carries its bucket's count, pos | count << 25
+// (kStartWide: too many, the next entry has the end), and a lookup reads 4
+// bytes; these lookups run from L2 and are bound by instruction issue.
 // 2^26 Zipf(0.5) probes: binary search over 2^26 uniform keys 14.3 ms (sampled
 // keys in shared memory, then halving) against 1.57, at the part's random
 // access rate; over 2^20 keys 3.39 ms against 0.57.
@@ -287,7 +302,22 @@ struct key_start {
     uint32_t shift;
     uint32_t col_aligned;
     float inv_width;      // 2^-shift
+    uint32_t packed;      // entries carry counts
 };
+constexpr uint64_t kStartPackedKeys = 1ull << 24;
+constexpr uint32_t kStartPosBits = 25, kStartPosMask = (1u << kStartPosBits) - 1;
+constexpr uint32_t kStartWide = (1u << (32 - kStartPosBits)) - 1;
+
+template <int kClass>
+GJ_DEVICE_INLINE uint32_t ld_start(const uint32_t* p) {
+    if constexpr (kClass == kL2Default) {
+        return ld_ro(p);
+    } else {
+        uint32_t v;
+        asm("ld.global.nc.L2::cache_hint.L2::64B.u32 %0, [%1], %2;" : "=r"(v) : "l"(p), "l"(l2_policy<kClass>()));
+        return v;
+    }
+}
 
 // lower bound (n past the last key); *eq: it is the position of an equal key
 template <bool kScattered = true, bool kCount = false>
@@ -298,13 +328,22 @@ GJ_DEVICE_INLINE uint32_t start_lower_bound(const key_start& t, const uint64_t* 
     *eq = false;
     const uint64_t off = key - t.min_key;
     if (off > t.range) return key < t.min_key ? 0u : n;
-    // entries b and b + 1: one 16-byte load unless b is the last of its four
-    const uint32_t b = (uint32_t)(off >> t.shift), q = b & 3u;
-    uint64_t e[2];
-    ld_pair_c<kTable>(reinterpret_cast<const uint64_t*>(t.pos + (b - q)), e);
-    const uint64_t w = q < 2 ? e[0] : e[1];
-    const uint32_t lo = (q & 1) ? (uint32_t)(w >> 32) : (uint32_t)w;
-    const uint32_t hi = q == 3 ? ld_ro(t.pos + b + 1) : (q & 1) ? (uint32_t)e[1] : (uint32_t)(w >> 32);
+    const uint32_t b = (uint32_t)(off >> t.shift);
+    uint32_t lo, hi;
+    if (t.packed) {
+        const uint32_t e = ld_start<kTable>(t.pos + b);
+        lo = e & kStartPosMask;
+        hi = lo + (e >> kStartPosBits);
+        if ((e >> kStartPosBits) == kStartWide) hi = ld_start<kTable>(t.pos + b + 1) & kStartPosMask;
+    } else {
+        // entries b and b + 1: one 16-byte load unless b is the last of its four
+        const uint32_t q = b & 3u;
+        uint64_t e[2];
+        ld_pair_c<kTable>(reinterpret_cast<const uint64_t*>(t.pos + (b - q)), e);
+        const uint64_t w = q < 2 ? e[0] : e[1];
+        lo = (q & 1) ? (uint32_t)(w >> 32) : (uint32_t)w;
+        hi = q == 3 ? ld_ro(t.pos + b + 1) : (q & 1) ? (uint32_t)e[1] : (uint32_t)(w >> 32);
+    }
     // the answer may be hi, the next bucket's first key: never an equal one
     if (lo >= hi) return lo;
     if (!t.col_aligned) return (uint32_t)lower_bound_sectors<kColumn>(col, n, lo, hi, key, false, eq);
@@ -630,10 +669,8 @@ GJ_DEVICE_INLINE uint32_t btree_lookup_from(const btree_view& v, const uint64_t*
         // a full leaf of one aligned sector: one load, four compares
         uint64_t k[4];
         ld_sector_c<kColumn>(v.col + base, k);
-        const uint32_t below = (k[0] < key ? 1u : 0u) + (k[1] < key ? 1u : 0u) + (k[2] < key ? 1u : 0u) +
-                               (k[3] < key ? 1u : 0u);
+        const uint32_t below = sector_rank(k, key, &eq);
         pos = base + below;
-        eq = below < 4 && pick4(k, below & 3u) == key;
     } else {
         pos = lower_bound_sectors<kColumn>(v.col, v.n, base, end, key, v.col_aligned, &eq);
     }
@@ -1026,7 +1063,11 @@ GJ_DEVICE_INLINE uint64_t window_lower_bound(const uint64_t* col, uint64_t n, ui
     constexpr int kColumn = kScattered ? kL2StreamLine : kL2Default;
     bool eq;
     uint64_t pos;
-    if (aligned && b < e) {
+    // A column larger than L2 is searched from the guess, which saves DRAM
+    // accesses (learned index over 2^26 keys 2191 against 2066 us per 2^26
+    // probes); one that fits is halved, which saves instructions (2^20 keys
+    // 790 against 884 us, RadixSpline 1292 against 1333).
+    if (aligned && b < e && n > (1ull << 23)) {
         const uint32_t sl = (uint32_t)(b >> 2), sr = (uint32_t)((e - 1) >> 2);
         const uint32_t s = (uint32_t)(guess >> 2);
         uint32_t edge;
