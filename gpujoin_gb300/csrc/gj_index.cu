@@ -115,6 +115,9 @@ __global__ void k_gather_fence(const uint64_t* __restrict__ col, uint64_t n, uin
     }
 }
 
+constexpr uint32_t kStartSample = 8192;  // keys sampled for a key start table's cost
+constexpr int kStartSums = 3;
+
 // key start table: the first key not below each bucket's first value (binary
 // search per bucket; n from the bucket past the last one on), with the
 // bucket's count where entries are packed; clears the sums of the cost sample
@@ -122,7 +125,7 @@ __global__ void k_key_start(const uint64_t* __restrict__ col, uint64_t n, uint64
                             uint32_t buckets, uint32_t entries, uint32_t packed, uint32_t* __restrict__ pos,
                             unsigned long long* __restrict__ sums) {
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t < 2) sums[t] = 0;
+    if (t < kStartSums) sums[t] = 0;
     for (uint32_t b = t; b < entries; b += gridDim.x * blockDim.x) {
         const uint64_t first = min_key + ((uint64_t)b << shift);
         const uint64_t lo = b >= buckets ? n : lower_bound_branch_free(col, n, first);
@@ -136,25 +139,31 @@ __global__ void k_key_start(const uint64_t* __restrict__ col, uint64_t n, uint64
     }
 }
 
-// sums[0] += column sectors the key start table's searches read, sums[1] +=
-// levels below the tree's start entry, over kStartSample keys of the column
-constexpr uint32_t kStartSample = 8192;
+// over kStartSample keys of the column: sums[0] += column sectors the key start
+// table's searches read, sums[1] += levels below the tree's start entry,
+// sums[2] += windows of three sectors or more
 __global__ void k_start_cost(key_start t, const uint64_t* __restrict__ col, uint32_t n, btree_view bt,
                              unsigned long long* sums) {
     const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
     uint32_t loads = 0, level = 0;
+    bool is_wide = false;
     if (j < kStartSample) {
         // spread over the column, off the tree's node boundaries
         const uint64_t key = col[((uint64_t)j * n + mix64(j) % n) / kStartSample];
         bool eq;
         start_lower_bound<false, true>(t, col, n, key, &eq, &loads);
+        uint32_t lo, hi;
+        start_window<kL2Default>(t, (uint32_t)((key - t.min_key) >> t.shift), &lo, &hi);
+        is_wide = lo < hi && ((hi - 1) >> 2) - (lo >> 2) > 1;
         if (bt.start) level = (uint32_t)(bt.start[2 * ((key - bt.min_key) >> bt.start_shift) + 1] >> 32);
     }
+    const uint32_t wide = __popc(__ballot_sync(0xffffffffu, is_wide));
     loads = __reduce_add_sync(0xffffffffu, loads);
     level = __reduce_add_sync(0xffffffffu, level);
     if ((threadIdx.x & 31) == 0) {
         atomicAdd(&sums[0], (unsigned long long)loads);
         atomicAdd(&sums[1], (unsigned long long)level);
+        atomicAdd(&sums[2], (unsigned long long)wide);
     }
 }
 
@@ -370,11 +379,11 @@ uint32_t key_start_shift(uint64_t range, uint32_t bits) {
     const uint32_t used = range ? 64u - (uint32_t)__builtin_clzll(range) : 0u;
     return used > bits ? used - bits : 0u;
 }
-// the table in whole 16-byte groups, and the two sums of the cost sample
+// the table in whole 16-byte groups, and the sums of the cost sample
 size_t key_start_bytes(const gj_index* idx, uint32_t bits) {
     const uint64_t range = idx->max_key - idx->min_key;
     const uint64_t buckets = (range >> key_start_shift(range, bits)) + 1;
-    return ((buckets + 1 + 3) & ~3ull) * sizeof(uint32_t) + 2 * sizeof(unsigned long long);
+    return ((buckets + 1 + 3) & ~3ull) * sizeof(uint32_t) + kStartSums * sizeof(unsigned long long);
 }
 
 // Key start table of 2^bits buckets (fewer for a narrow key range); use(loads,
@@ -395,7 +404,7 @@ int build_key_start(gj_index* idx, uint32_t bits, cudaStream_t s, spare_memory&&
     if (!spare.p) GJ_TRY(spare.take(key_start_bytes(idx, bits)));
     uint32_t* pos = static_cast<uint32_t*>(spare.p);
     unsigned long long* d_sums = reinterpret_cast<unsigned long long*>(pos + entries);
-    unsigned long long sums[2] = {0, 0};
+    unsigned long long sums[kStartSums] = {};
     t.packed = idx->n <= kStartPackedKeys ? 1u : 0u;
     k_key_start<<<(entries + 255) / 256, 256, 0, s>>>(idx->d_col, idx->n, t.min_key, t.shift, buckets, entries,
                                                      t.packed, pos, d_sums);
@@ -406,6 +415,7 @@ int build_key_start(gj_index* idx, uint32_t bits, cudaStream_t s, spare_memory&&
     GJ_CUDA_TRY(cudaMemcpyAsync(sums, d_sums, sizeof(sums), cudaMemcpyDeviceToHost, s));
     GJ_CUDA_TRY(cudaStreamSynchronize(s));
     if (!use((double)sums[0] / kStartSample, (double)sums[1] / kStartSample)) return GJ_OK;
+    t.narrow = sums[2] <= kStartSample / 256 ? 1u : 0u;
     idx->allocations.push_back(spare.release());
     idx->ks = t;
     idx->bytes += (size_t)entries * sizeof(uint32_t);
