@@ -186,7 +186,7 @@ bool carve_partition_inverse(void* ws, size_t ws_bytes, uint64_t m, uint32_t rad
                              partition_inverse* out);
 // d_out[row] = value of the probe of that row, for values in relation order:
 // entry d of the relation has its value at d_values[value_index(d)]
-constexpr uint32_t kValueTile = 2048;
+constexpr uint32_t kValueTile = 256;
 __host__ __device__ inline uint64_t value_index(uint32_t d) {
     return (uint64_t)(d / kValueTile) * (2 * kValueTile) + d % kValueTile;
 }

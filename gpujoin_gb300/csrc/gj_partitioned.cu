@@ -247,7 +247,7 @@ struct probe_args {
     uint64_t n;
     dir_geom g;
     uint32_t* positions;         // positions[row] = result, or null
-    uint32_t* values;            // values[value_index(i)] = result of relation entry i, or null (no rows then)
+    uint32_t* values;            // values[value_index(i)] = result of relation entry i (k_part_values), or null
     uint2* pairs;                // (row, result) of the matches, or null
     unsigned long long* count;   // pairs appended at atomicAdd(count, ...)
 };
@@ -381,17 +381,6 @@ __global__ void __launch_bounds__(kProbeBlock, GJ_PROBE_BLOCKS) k_part_probe(con
                 }
             }
         }
-        if (a.values) {
-            // the tile's keys have all been read once every thread is here:
-            // its results take the first half of their room
-            __syncthreads();
-#pragma unroll
-            for (int k = 0; k < kProbeItems; ++k) {
-                const uint64_t i = t0 + (uint64_t)k * kProbeBlock + threadIdx.x;
-                if (valid[k]) a.values[value_index((uint32_t)i)] = res[k];
-            }
-            continue;
-        }
         // probe rows are read only now, when the results are written
         uint32_t row[kProbeItems];
 #pragma unroll
@@ -454,7 +443,56 @@ __global__ void __launch_bounds__(kProbeBlock, GJ_PROBE_BLOCKS) k_part_probe(con
 }
 static_assert(kProbeBlock / 32 * kProbeItems % 32 == 0, "the tile scan gives each lane whole counts");
 static_assert(kProbeItems % kProbeBatch == 0, "whole batches per tile");
-static_assert(kProbeTile == kValueTile, "a tile's values lie in the room of its own keys");
+
+// Positions of a window that k_part_gather brings back to probe order: the
+// result of relation entry i goes to a.values, over the keys of its block, all
+// of which have been read by then.  One probe a thread at 32 registers: the
+// search is the same two or three L2 sectors as in k_part_probe, whose 24
+// warps an SM (pairs, eight results a thread) keep fewer of them in flight
+// (2^29 probes into 2^28 keys 6.10 ms there).
+template <int kSem, bool kAligned>
+__global__ void __launch_bounds__(kValueTile, 8) k_part_values(const __grid_constant__ probe_args a) {
+    const uint64_t i = (uint64_t)blockIdx.x * kValueTile + threadIdx.x;
+    const uint64_t key = i < a.len ? __ldcs(reinterpret_cast<const unsigned long long*>(a.pkeys) + i) : 0ull;
+    __syncthreads();
+    if (i >= a.len) return;
+    uint32_t res = kInvalid;
+    if constexpr (kSem != kSemNone) {
+        const uint32_t n = (uint32_t)a.n;
+        const uint32_t b = bucket_of(key, a.g);
+        const uint32_t slo = __ldg(a.dir + b);
+        bool eq = false;
+        uint32_t lb = n;
+        if constexpr (kAligned) {
+            // the bucket's first sector, then the one behind it: a key of
+            // either that is not below the probe settles it, so the bucket's
+            // end is only read for what is left
+            const uint32_t last = (n - 1) >> 2;
+            if (slo <= last) {
+                uint64_t k[4];
+                ld_column_sector<kL2Default>(a.col, n, slo, k);
+                uint32_t below = sector_rank(k, key, &eq);
+                lb = (slo << 2) + below;
+                if (below == 4 && slo < last) {
+                    ld_column_sector<kL2Default>(a.col, n, slo + 1, k);
+                    below = sector_rank(k, key, &eq);
+                    lb += below;
+                    const uint32_t shi = below == 4 ? min(__ldg(a.dir + b + 1), last) : 0u;
+                    if (shi > slo + 1) {
+                        uint32_t edge;
+                        lb = search_sectors<kL2Default>(a.col, n, slo + 2, shi, slo + 2 + (shi - slo - 2) / 2, key, &eq,
+                                                        &edge);
+                    }
+                }
+            }
+        } else {
+            const uint64_t lo = (uint64_t)slo << 2, end = ((uint64_t)__ldg(a.dir + b + 1) + 1) << 2;
+            lb = (uint32_t)lower_bound_sectors(a.col, n, lo, end < n ? end : n, key, false, &eq);
+        }
+        if (lb < n && (kSem == kSemLowerBound || eq)) res = lb;
+    }
+    __stcs(a.values + value_index((uint32_t)i), res);
+}
 
 // ---------------------------------------------------------------------------
 // host side
@@ -511,6 +549,11 @@ size_t partitioned_ws_bytes(const partitioned_layout& L, int sm_count, bool prep
 
 template <int kSem, bool kAligned>
 int launch_probe(const probe_args& a, cudaStream_t s) {
+    if (a.values) {
+        k_part_values<kSem, kAligned><<<(unsigned)((a.len + kValueTile - 1) / kValueTile), kValueTile, 0, s>>>(a);
+        GJ_CUDA_TRY(cudaGetLastError());
+        return GJ_OK;
+    }
     const uint64_t grid = (a.len + kChunk - 1) / kChunk;
     k_part_probe<kSem, kAligned><<<(unsigned)grid, kProbeBlock, 0, s>>>(a);
     GJ_CUDA_TRY(cudaGetLastError());
