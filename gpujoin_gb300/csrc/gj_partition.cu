@@ -482,12 +482,14 @@ void index_key_range(const gj_index* idx, uint64_t* min_key, uint64_t* max_key) 
 }
 
 uint32_t default_radix_bits(uint64_t n) {
-    // about 2^20 index keys (8 MB of column, 4 MB of directory) per partition,
+    // about 2^21 index keys (16 MB of column, 8 MB of directory) per partition,
     // fanout within [2^5, 2^12]: a partition's slices stay in L2 while it is
-    // probed, and the scatter's runs stay long (measured best: 2^5-2^6 at
-    // 2^26 keys, 2^7-2^8 at 2^28)
+    // probed, and the scatter's runs stay long.  Positions of 2^29 probes into
+    // 2^28 uniform keys 9.9 / 8.8 / 9.1 / 9.8 ms at 2^5 .. 2^8, lognormal (whose
+    // fullest partitions hold many times the mean) 15.5 / 12.4 / 10.5 / 10.5;
+    // 2^28 into 2^26 keys 4.34 / 4.42 / 4.52 / 4.81 and 5.18 / 4.91 / 4.90 / 5.13.
     uint32_t b = 5;
-    while (b < kMaxRadixBits && (n >> b) > (1ull << 20)) ++b;
+    while (b < kMaxRadixBits && (n >> b) > (1ull << 21)) ++b;
     return b;
 }
 
