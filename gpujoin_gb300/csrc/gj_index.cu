@@ -714,7 +714,11 @@ int build_radix_spline_index(gj_index* idx, const uint64_t* h_keys, cudaStream_t
             const uint64_t dx = rs.sx[i + 1] - rs.sx[i];
             const uint32_t sh = (uint32_t)__builtin_clzll(dx);
             const unsigned __int128 dy = (unsigned __int128)(uint64_t)(rs.sy[i + 1] - rs.sy[i]);
-            pts[i].step = (uint64_t)((dy << 64) / (dx << sh)) << 6 | sh;
+            const float rate = (float)(pts[i].slope * 0.25);
+            uint32_t bits = 0;
+            std::memcpy(&bits, &rate, sizeof(bits));
+            // dy <= dx: the quotient is at most 2^34 - 1 wide
+            pts[i].step = (uint64_t)(bits >> 8) << 40 | (uint64_t)((dy << 64) / (dx << sh)) << 6 | sh;
         }
     }
     void *pt = nullptr, *pp = nullptr;

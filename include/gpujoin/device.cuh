@@ -231,13 +231,17 @@ GJ_DEVICE_INLINE void ld_column_sector(const uint64_t* col, uint32_t n, uint32_t
 // nearby), then halves what is left: any column costs at most two loads more
 // than halving alone.  The sectors are read whole and compared whole -- keys
 // outside the caller's window are as good as those inside.
+// kRate: the caller knows the spacing (rate sectors per unit of key, a
+// spline's or a model's slope), which is cheaper and steadier than that of
+// three gaps.
 // *edge: 0 when the answer is certain, 1 / 2 when it is the first key of
 // sector sl / the key behind sector sr, i.e. the bound within the sectors, and
 // the column's only if the caller's range holds.  *eq: the answer's key is
 // read and equals key.  loads counts the sectors read (build statistics).
-template <int kClass, bool kCount = false>
+template <int kClass, bool kCount = false, bool kRate = false>
 GJ_DEVICE_INLINE uint32_t search_sectors(const uint64_t* col, uint32_t n, uint32_t sl, uint32_t sr, uint32_t s,
-                                         uint64_t key, bool* eq, uint32_t* edge, uint32_t* loads = nullptr) {
+                                         uint64_t key, bool* eq, uint32_t* edge, uint32_t* loads = nullptr,
+                                         float rate = 0.f) {
     constexpr uint32_t kNear = 3;  // few sectors left: the next one, without arithmetic
     const uint32_t sl0 = sl, sr0 = sr;
     uint64_t right_key = 0;  // first key of sector sr + 1, once that has been read
@@ -261,7 +265,8 @@ GJ_DEVICE_INLINE uint32_t search_sectors(const uint64_t* col, uint32_t n, uint32
                 continue;
             }
             if (step < 2) {  // sectors past this one
-                const float d = __fdividef((float)(key - k[3]) * 0.75f, (float)(k[3] - k[0]));
+                const float d = kRate ? (float)(key - k[3]) * rate
+                                      : __fdividef((float)(key - k[3]) * 0.75f, (float)(k[3] - k[0]));
                 s = sl + (uint32_t)fminf(d, (float)(sr - sl));
                 s = s > sr ? sr : s;
                 continue;
@@ -274,7 +279,8 @@ GJ_DEVICE_INLINE uint32_t search_sectors(const uint64_t* col, uint32_t n, uint32
                 continue;
             }
             if (step < 2) {
-                const float d = __fdividef((float)(k[0] - key) * 0.75f, (float)(k[3] - k[0]));
+                const float d = kRate ? (float)(k[0] - key) * rate
+                                      : __fdividef((float)(k[0] - key) * 0.75f, (float)(k[3] - k[0]));
                 const uint32_t back = (uint32_t)fminf(d, (float)(sr - sl));
                 s = sr - (back < sr - sl ? back : sr - sl);
                 continue;
@@ -1037,7 +1043,8 @@ struct rs_point {
     uint64_t x;
     double y;      // a position: a whole number below 2^32
     double slope;  // (y[i+1] - y[i]) / (x[i+1] - x[i]); 0 for the last point
-    uint64_t step; // shift | floor(dy * 2^64 / (dx << shift)) << 6, dx << shift in [2^63, 2^64)
+    uint64_t step; // shift | floor(dy * 2^64 / (dx << shift)) << 6, dx << shift in [2^63, 2^64), and from
+                   // bit 40 on the upper 24 bits of dy / dx / 4 as a float (sectors per unit of key)
 };
 static_assert(sizeof(rs_point) == 32, "a spline point is one sector");
 
@@ -1061,18 +1068,24 @@ GJ_DEVICE_INLINE uint32_t whole_of_double(uint64_t bits) {
 }
 
 // The spline's estimate of a key's position, rounded down and at most two
-// below the real value: y + (key - x) * slope in 64-bit fixed point.
-GJ_DEVICE_INLINE uint32_t rs_estimate(const rs_view& v, uint64_t key) {
+// below the real value: y + (key - x) * slope in 64-bit fixed point.  *rate:
+// the segment's sectors per unit of key.
+GJ_DEVICE_INLINE uint32_t rs_estimate(const rs_view& v, uint64_t key, float* rate) {
+    *rate = 0.f;
     if (key <= v.min_key) return 0;
     if (key >= v.max_key) return (uint32_t)(v.n - 1);
     const uint64_t prefix = (key - v.min_key) >> v.shift;
     const uint32_t b = ld_ro(v.table + prefix);
     const uint32_t e = ld_ro(v.table + prefix + 1);
-    // first spline point with x >= key in [b, e)
-    uint32_t lo = b, cnt = e - b;
+    // first spline point with x >= key in [b, e); w: the last point read, if
+    // it lies before the key (one point is the usual range)
+    uint32_t lo = b, cnt = e - b, have = 0xFFFFFFFFu;
+    uint64_t w[4];
     while (cnt > 0) {
         const uint32_t step = cnt >> 1, mid = lo + step;
-        if (ld_ro(&v.pts[mid].x) < key) {
+        ld_sector(reinterpret_cast<const uint64_t*>(v.pts + mid), w);
+        have = mid;
+        if (w[0] < key) {
             lo = mid + 1;
             cnt -= step + 1;
         } else {
@@ -1080,29 +1093,32 @@ GJ_DEVICE_INLINE uint32_t rs_estimate(const rs_view& v, uint64_t key) {
         }
     }
     // segment [lo - 1, lo]: its left point and precomputed slope
-    uint64_t w[4];
-    ld_sector(reinterpret_cast<const uint64_t*>(v.pts + lo - 1), w);
-    return whole_of_double(w[1]) + (uint32_t)__umul64hi((key - w[0]) << (w[3] & 63u), w[3] >> 6);
+    if (have != lo - 1) ld_sector(reinterpret_cast<const uint64_t*>(v.pts + lo - 1), w);
+    *rate = __uint_as_float((uint32_t)(w[3] >> 40) << 8);
+    return whole_of_double(w[1]) + (uint32_t)__umul64hi((key - w[0]) << (w[3] & 63u), (w[3] >> 6) & ((1ull << 34) - 1));
 }
 
 // lower bound expected inside [b, e) and near `guess`, widened to the whole
 // column when the window turns out not to bracket it (possible only for keys
 // outside the column)
-template <bool kScattered = true>
+template <bool kScattered, uint32_t kLogKeys>
 GJ_DEVICE_INLINE uint64_t window_lower_bound(const uint64_t* col, uint64_t n, uint64_t b, uint64_t e, uint64_t guess,
-                                             uint64_t key, bool aligned) {
+                                             float rate, uint64_t key, bool aligned) {
     constexpr int kColumn = kScattered ? kL2StreamLine : kL2Default;
     bool eq;
     uint64_t pos;
-    // A column larger than L2 is searched from the guess, which saves DRAM
-    // accesses (learned index over 2^26 keys 2191 against 2066 us per 2^26
-    // probes); one that fits is halved, which saves instructions (2^20 keys
-    // 790 against 884 us, RadixSpline 1292 against 1333).
-    if (aligned && b < e && n > (1ull << 23)) {
+    // Columns of more than 2^kLogKeys keys are searched from the guess, smaller
+    // ones are halved: the guess saves sectors, halving instructions.  A
+    // spline's window is 66 keys wide (2^26 probes: 2^16 clustered keys 1205
+    // us halved, 1370 from the guess; 2^20 uniform keys 1292 / 1182, 2^26 keys
+    // 3533 / 2921), a learned leaf's about 14 (2^20 keys 787 / 833, 2^26 keys
+    // 2191 / 2043).
+    if (aligned && b < e && n > (1ull << kLogKeys)) {
         const uint32_t sl = (uint32_t)(b >> 2), sr = (uint32_t)((e - 1) >> 2);
         const uint32_t s = (uint32_t)(guess >> 2);
         uint32_t edge;
-        pos = search_sectors<kColumn>(col, (uint32_t)n, sl, sr, s < sl ? sl : s > sr ? sr : s, key, &eq, &edge);
+        pos = search_sectors<kColumn, false, true>(col, (uint32_t)n, sl, sr, s < sl ? sl : s > sr ? sr : s, key, &eq,
+                                                   &edge, nullptr, rate);
         if ((edge == 1 && pos > 0 && ld_ro(col + pos - 1) >= key) || (edge == 2 && pos < n && ld_ro(col + pos) < key))
             pos = lower_bound_sectors(col, n, 0, n, key, aligned, &eq);
         return pos;
@@ -1115,11 +1131,12 @@ GJ_DEVICE_INLINE uint64_t window_lower_bound(const uint64_t* col, uint64_t n, ui
 
 template <bool kScattered = true>
 GJ_DEVICE_INLINE uint32_t rs_lookup(const rs_view& v, uint64_t key) {
-    const uint64_t est = rs_estimate(v, key), err = v.max_error;
+    float rate;
+    const uint64_t est = rs_estimate(v, key, &rate), err = v.max_error;
     // the real estimate lies in [est, est + 2]
     const uint64_t b = est < err ? 0 : est - err;
     const uint64_t e = est + err + 4 > v.n ? v.n : est + err + 4;
-    const uint64_t pos = window_lower_bound<kScattered>(v.col, v.n, b, e, est, key, v.col_aligned);
+    const uint64_t pos = window_lower_bound<kScattered, 17>(v.col, v.n, b, e, est, rate, key, v.col_aligned);
     return pos < v.n ? (uint32_t)pos : kInvalid;
 }
 
@@ -1273,7 +1290,8 @@ GJ_DEVICE_INLINE uint32_t learned_lookup(const learned_view& v, const float* roo
     if (lo > hi) lo = hi;
     const int64_t at = pred < lo ? lo : pred > hi ? hi : pred;
     const uint64_t pos =
-        window_lower_bound<kScattered>(v.col, v.n, (uint64_t)lo, (uint64_t)hi, (uint64_t)at, key, v.col_aligned);
+        window_lower_bound<kScattered, 23>(v.col, v.n, (uint64_t)lo, (uint64_t)hi, (uint64_t)at, lf.slope * 0.25f, key,
+                                       v.col_aligned);
     return pos < v.n ? (uint32_t)pos : kInvalid;
 }
 
