@@ -10,7 +10,7 @@
 // (gj_batch_plan_run_graph).
 //
 // mode 0: one persistent kernel.  All batches are cut into tiles of
-//         kBatchBlock * tile_items probes; blocks claim tiles in order from an
+//         kBatchBlock * tile_items probes; blocks claim tiles, index by index, from an
 //         atomic counter, so small batches never wait behind a kernel
 //         boundary and no SM idles at batch tails.
 // mode 1: one lookup launch per batch -- the baseline the persistent kernel
@@ -19,6 +19,7 @@
 // latency percentiles.  The tile shape is the plan's autotuned parameter.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdint>
 #include <cstring>
 #include <new>
@@ -272,8 +273,16 @@ int plan_alloc(T** p, size_t count) {
 int plan_layout(gj_batch_plan* pl, uint32_t items, cudaStream_t s) {
     const uint64_t tile_probes = (uint64_t)kBatchBlock * items;
     std::vector<batch_desc> descs(pl->num_batches);
+    // Tiles of one index follow each other (in batch order): the blocks of the
+    // chip search one or two indexes at a time, whose columns and tables then
+    // stay in L2, where all of a stream's would not (512 batches over eight
+    // indexes, about 400 MB: 1588 us, 2079 in batch order).
+    std::vector<uint32_t> order(pl->num_batches);
+    for (uint32_t b = 0; b < pl->num_batches; ++b) order[b] = b;
+    std::stable_sort(order.begin(), order.end(),
+                     [&](uint32_t a, uint32_t b) { return pl->batch_index[a] < pl->batch_index[b]; });
     uint64_t tiles = 0;
-    for (uint32_t b = 0; b < pl->num_batches; ++b) {
+    for (const uint32_t b : order) {
         descs[b].offset = pl->offset[b];
         descs[b].size = pl->size[b];
         descs[b].tile_begin = tiles;
