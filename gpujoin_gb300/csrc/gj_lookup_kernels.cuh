@@ -270,12 +270,17 @@ __device__ __forceinline__ uint64_t load_probe(const uint64_t* p, uint64_t i, ui
     return i < m ? __ldcs(reinterpret_cast<const unsigned long long*>(p + i)) : 0ull;
 }
 
-template <class Op, int kIt>
+// kClear: the launch also clears words 64-bit words of clear, the state of
+// the compaction that follows it, in place of a memset of its own.
+template <class Op, int kIt, bool kClear = false>
 __global__ void __launch_bounds__(kBlock, Op::kMinBlocks) k_lookup(const __grid_constant__ Op op, const stage_desc sd,
                                                    const uint64_t* __restrict__ probes, uint64_t m,
-                                                   uint32_t* __restrict__ out) {
+                                                   uint32_t* __restrict__ out, unsigned long long* clear,
+                                                   uint32_t words) {
     extern __shared__ __align__(16) uint64_t cache[];
     if constexpr (Op::kStaged) stage_cache(cache, sd);
+    if constexpr (kClear)
+        for (uint32_t w = blockIdx.x * kBlock + threadIdx.x; w < words; w += gridDim.x * kBlock) clear[w] = 0;
     const uint64_t t0 = (uint64_t)blockIdx.x * (kBlock * kIt) + threadIdx.x;
     uint64_t next = load_probe(probes, t0, m);
 #pragma unroll 1
@@ -885,15 +890,16 @@ int grid_for(Kernel kernel, size_t smem, uint64_t work_items, int* grid) {
 
 template <class Op>
 int run_lookup(const Op& op, const stage_desc& sd, uint64_t n, const uint64_t* probes, uint64_t m, uint32_t* out,
-               cudaStream_t s) {
+               cudaStream_t s, unsigned long long* clear = nullptr, uint32_t words = 0) {
     const size_t smem = Op::kStaged ? stage_bytes(sd) : 0;
     auto launch = [&](auto kernel, int items) {
         GJ_TRY(kernel_staged(kernel, smem));
         const uint64_t tile = (uint64_t)kBlock * items;
-        kernel<<<(unsigned)((m + tile - 1) / tile), kBlock, smem, s>>>(op, sd, probes, m, out);
+        kernel<<<(unsigned)((m + tile - 1) / tile), kBlock, smem, s>>>(op, sd, probes, m, out, clear, words);
         GJ_CUDA_TRY(cudaGetLastError());
         return (int)GJ_OK;
     };
+    if (clear) return launch(k_lookup<Op, 1, true>, 1);
     bool full = false;
     GJ_TRY(long_blocks(n, m, &full));
     return full ? launch(k_lookup<Op, Op::kLong>, Op::kLong) : launch(k_lookup<Op, 1>, 1);
@@ -942,13 +948,17 @@ int run_pairs(const Op& op, const stage_desc& sd, uint64_t n, const uint64_t* pr
         GJ_CUDA_TRY(cudaMemsetAsync(d_count, 0, sizeof(uint64_t), s));
         return GJ_OK;
     }
-    GJ_CUDA_TRY(cudaMemsetAsync(ws, 0, used, s));
     if (spin_limit) pw.spin_limit = spin_limit;
+    const bool two_passes = stash && m < kSinglePassMin;
+    // the state lies in whole 64-bit words at the head of the workspace
+    if (two_passes)
+        GJ_TRY(run_lookup(op, sd, n, probes, m, stash, s, pw.tile_state, (uint32_t)(used / 8)));
+    else
+        GJ_CUDA_TRY(cudaMemsetAsync(ws, 0, used, s));
     // test hook: the tile counter starts at 1, so tile 0 is never claimed and
     // never publishes; every later tile's look-back runs out
     if (skip_first_tile) GJ_CUDA_TRY(cudaMemsetAsync(pw.tile_counter, 1, 1, s));
-    if (stash && m < kSinglePassMin) {
-        GJ_TRY(run_lookup(op, sd, n, probes, m, stash, s));
+    if (two_passes) {
         const uint32_t compact_tiles = (uint32_t)((m + kCompactTile - 1) / kCompactTile);
         int grid = 0;
         GJ_TRY(grid_for(k_compact_pairs, 0, (uint64_t)compact_tiles * kBlock, &grid));
