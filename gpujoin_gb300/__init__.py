@@ -369,7 +369,8 @@ class abstract_index:
             out_count = _empty(1, torch.int64, dev)
         if workspace is None:
             need = _sz(0)
-            _check(lib().gj_inlj_pairs_workspace_size(m, ctypes.byref(need)))
+            size = lib().gj_inlj_pairs_workspace_size if ordered else lib().gj_inlj_pairs_host_workspace_size
+            _check(size(m, ctypes.byref(need)))
             workspace = _workspace(need.value, dev)
         fn = lib().gj_inlj_pairs if ordered else lib().gj_inlj_pairs_unordered
         _check(fn(self.handle, _ptr(d_probes), m, _ptr(out_pairs), _ptr(out_count), _ptr(workspace),
@@ -407,7 +408,7 @@ class abstract_index:
             out_count = _empty(1, torch.int64, dev)
         if workspace is None:
             need = _sz(0)
-            _check(lib().gj_inlj_pairs_workspace_size(m, ctypes.byref(need)))
+            _check(lib().gj_inlj_pairs_host_workspace_size(m, ctypes.byref(need)))  # no room to partition
             workspace = _workspace(need.value, dev)
         _check(lib().gj_inlj_pairs_sorted(self.handle, _ptr(d_probes), m, _ptr(out_pairs), _ptr(out_count),
                                           _ptr(workspace), workspace.numel(), _stream(stream)))

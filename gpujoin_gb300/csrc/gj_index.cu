@@ -389,7 +389,7 @@ size_t key_start_bytes(const gj_index* idx, uint32_t bits) {
 // Key start table of 2^bits buckets (fewer for a narrow key range); use(loads,
 // level) decides from the sampled cost of its searches -- mean column sectors
 // read, and for a B+tree the mean level its lookups start at -- whether the
-// index keeps it.
+// index's scattered lookups go through it.
 template <class Use>
 int build_key_start(gj_index* idx, uint32_t bits, cudaStream_t s, spare_memory&& spare, Use&& use) {
     const uint64_t range = idx->max_key - idx->min_key;
@@ -414,10 +414,11 @@ int build_key_start(gj_index* idx, uint32_t bits, cudaStream_t s, spare_memory&&
     GJ_CUDA_TRY(cudaGetLastError());
     GJ_CUDA_TRY(cudaMemcpyAsync(sums, d_sums, sizeof(sums), cudaMemcpyDeviceToHost, s));
     GJ_CUDA_TRY(cudaStreamSynchronize(s));
-    if (!use((double)sums[0] / kStartSample, (double)sums[1] / kStartSample)) return GJ_OK;
     t.narrow = sums[2] <= kStartSample / 256 ? 1u : 0u;
     idx->allocations.push_back(spare.release());
-    idx->ks = t;
+    idx->rel = t;
+    idx->rel_loads = (double)sums[0] / kStartSample;
+    if (use(idx->rel_loads, (double)sums[1] / kStartSample)) idx->ks = t;
     idx->bytes += (size_t)entries * sizeof(uint32_t);
     return GJ_OK;
 }
@@ -969,6 +970,10 @@ int gj_index_build(int type, const uint64_t* d_keys, const uint64_t* h_keys, uin
         case GJ_INDEX_HASH: rc = build_hash(idx.get(), s); break;
         case GJ_INDEX_NO_OP: break;
     }
+    // large ordered-pairs calls partition their probes and search through a
+    // key start table, whatever the kind
+    if (rc == GJ_OK && type != GJ_INDEX_NO_OP && idx->in_hbm && n > partition_pairs_keys(type) && !idx->rel.pos)
+        rc = build_key_start(idx.get(), key_start_bits(n), s, spare_memory(), [](double, double) { return false; });
     if (rc == GJ_OK) {
         cudaError_t e = cudaStreamSynchronize(s);
         if (e != cudaSuccess) {
@@ -1094,7 +1099,7 @@ int gj_index_lookup(const gj_index* index, const uint64_t* d_probes, uint64_t m,
 
 int gj_inlj_pairs_workspace_size(uint64_t m, size_t* bytes) {
     GJ_CHECK_ARG(bytes, "gj_inlj_pairs_workspace_size: null argument");
-    *bytes = pairs_workspace_bytes(m);
+    *bytes = pairs_workspace_bytes(m) + pairs_partition_bytes(m);
     return GJ_OK;
 }
 

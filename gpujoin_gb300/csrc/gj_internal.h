@@ -122,7 +122,11 @@ struct gj_index {
     gj::btree_view bt{};
     gj::harmonia_view hm{};
     gj::harmonia_child_base hm_base{};
-    gj::key_start ks{};  // key start table (binary search; default B+tree over a small column), or none
+    gj::key_start ks{};  // key start table of scattered lookups (binary search, Harmonia, default B+tree where
+                         // it beats the nodes), or none
+    gj::key_start rel{};     // key start table for probes grouped by key range (the same where there is one, else
+                             // one of its own over a large column), or none
+    double rel_loads = 0.0;  // column sectors its searches read on average
     gj::rs_view rs{};
     gj::learned_view ln{};
     gj::hash_view hs{};
@@ -159,6 +163,21 @@ int launch_pairs(const gj_index* idx, const uint64_t* d_probes, uint64_t m, uint
 int launch_sorted_pairs(const gj_index* idx, const uint64_t* d_probes, uint64_t m, uint32_t* d_pairs, uint64_t* d_count,
                         void* ws, size_t ws_bytes, cudaStream_t s);
 size_t pairs_workspace_bytes(uint64_t m);
+// Pairs in probe order by way of a partition (gj_partition.cu), for calls
+// where that is sooner and whose workspace has room beyond
+// pairs_workspace_bytes: *taken tells whether the call was.
+constexpr uint64_t kPartitionPairsMin = 1ull << 25, kPartitionPairsMax = 1ull << 29;  // probes
+// column keys above which such calls are made: kinds whose plain search reads
+// one random sector of a table or a spline's and a column's gain from fewer
+// (2^28 probes into 2^24 keys: hash table 5145, RadixSpline 5900, learned 5063
+// us plain, 4570 by partition; B+tree 4237)
+inline uint64_t partition_pairs_keys(int type) {
+    const bool tree = type == GJ_INDEX_BTREE || type == GJ_INDEX_HARMONIA || type == GJ_INDEX_BINARY_SEARCH;
+    return tree ? 3ull << 23 : 3ull << 22;
+}
+size_t pairs_partition_bytes(uint64_t m);
+int launch_pairs_by_partition(const gj_index* idx, const uint64_t* d_probes, uint64_t m, uint32_t* d_pairs,
+                              uint64_t* d_count, void* ws, size_t ws_bytes, cudaStream_t s, bool* taken);
 // launch_pairs for the test of the bounded waits: look-backs give up after
 // spin_limit polls, and tile 0 is never claimed (so every wait runs out)
 int launch_pairs_stalled(const gj_index* idx, const uint64_t* d_probes, uint64_t m, uint32_t* d_pairs,

@@ -54,6 +54,11 @@ int launch_scatter_lookup(const gj_index* idx, const uint64_t* d_keys, const uin
 
 int launch_pairs(const gj_index* idx, const uint64_t* d_probes, uint64_t m, uint32_t* d_pairs, uint64_t* d_count,
                  void* ws, size_t ws_bytes, uint32_t* d_stash, cudaStream_t s) {
+    if (d_stash) {
+        bool taken = false;
+        GJ_TRY(launch_pairs_by_partition(idx, d_probes, m, d_pairs, d_count, ws, ws_bytes, s, &taken));
+        if (taken) return GJ_OK;
+    }
     return dispatch(idx, {lookup_action::pairs, d_probes, nullptr, m, d_pairs, d_count, ws, ws_bytes, d_stash, s});
 }
 

@@ -21,7 +21,7 @@
 #include <algorithm>
 #include <cstdint>
 
-#include "gj_internal.h"
+#include "gj_lookup_kernels.cuh"  // pairs_tile and its state
 
 namespace gj {
 namespace {
@@ -339,6 +339,79 @@ __global__ void __launch_bounds__(kB, kPerSM) k_part_gather(const uint32_t* __re
     }
 }
 
+// values[i] = result of relation entry i through the index's key start table;
+// neighbouring probes share its and the column's lines in L2
+template <bool kExact>
+__global__ void __launch_bounds__(kBlock, 8) k_relation_values(const __grid_constant__ key_start t,
+                                                               const uint64_t* __restrict__ col, uint32_t n,
+                                                               const uint64_t* __restrict__ keys, uint64_t m,
+                                                               uint32_t* __restrict__ values) {
+    const uint64_t i = (uint64_t)blockIdx.x * kBlock + threadIdx.x;
+    if (i >= m) return;
+    bool eq;
+    const uint32_t lb =
+        start_lower_bound<false>(t, col, n, __ldcs(reinterpret_cast<const unsigned long long*>(keys) + i), &eq);
+    __stcs(values + i, (kExact ? eq : lb < n) ? lb : kInvalid);
+}
+
+// k_part_gather into ordered pairs: a block claims tiles in order, gathers a
+// tile's values into probe order and places its pairs behind those of the
+// tiles before it.  6 bytes read and up to 8 written a probe.
+constexpr int kGatherItems = 16;
+constexpr uint32_t kGatherTile = kBlock * kGatherItems;
+__global__ void __launch_bounds__(kBlock, 6) k_gather_pairs(const uint32_t* __restrict__ values, uint64_t m,
+                                                            part_tables t, partition_inverse iv,
+                                                            uint2* __restrict__ pairs, uint64_t* __restrict__ d_count,
+                                                            pairs_ws ws) {
+    extern __shared__ unsigned long long s_mem[];
+    const uint32_t fanout = t.fanout;
+    uint32_t* s_delta = reinterpret_cast<uint32_t*>(s_mem);            // fanout
+    uint16_t* s_start = reinterpret_cast<uint16_t*>(s_delta + fanout); // fanout + 2
+    uint16_t* s_part = s_start + fanout + 2;                           // kGatherTile
+    auto gather = [&](uint64_t t0, uint32_t* pos) {
+        const uint32_t tile = (uint32_t)(t0 / kGatherTile);
+        const uint32_t tn = m - t0 < kGatherTile ? (uint32_t)(m - t0) : kGatherTile;
+        for (uint32_t p = threadIdx.x; p < fanout; p += kBlock) {
+            const uint16_t at = __ldcs(iv.start + (uint64_t)tile * fanout + p);
+            s_delta[p] = run_start(t, tile, p) - at;
+            s_start[p] = at;
+        }
+        if (threadIdx.x == 0) s_start[fanout] = (uint16_t)tn;
+        __syncthreads();
+        for (uint32_t p = threadIdx.x >> 5; p < fanout; p += kBlock / 32)
+            for (uint32_t j = s_start[p] + (threadIdx.x & 31); j < s_start[p + 1]; j += 32) s_part[j] = (uint16_t)p;
+        __syncthreads();
+#pragma unroll 1
+        for (uint32_t j0 = threadIdx.x; j0 < kGatherTile; j0 += 8 * kBlock) {
+            uint32_t v[8];
+            uint16_t o[8];
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+                const uint32_t j = j0 + k * kBlock;
+                if (j < tn) {
+                    const uint32_t d = s_delta[s_part[j]] + j;
+                    v[k] = __ldcs(values + d);
+                    o[k] = __ldcs(iv.offsets + d);
+                }
+            }
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+                const uint32_t j = j0 + k * kBlock;
+                if (j < tn) pos[o[k]] = v[k];
+                else pos[j] = kInvalid;
+            }
+        }
+        __syncthreads();
+    };
+    auto row_of = [&](int, uint64_t i) { return (uint32_t)i; };
+    for (;;) {
+        const uint32_t tile = claim_tile(ws);
+        if (tile >= t.tiles) break;
+        start_count(tile, d_count);
+        if (!pairs_tile<kGatherItems>(gather, row_of, tile, pairs, d_count, ws, t.tiles)) break;
+    }
+}
+
 size_t gather_smem_bytes(uint32_t tile, uint32_t fanout) {
     return (size_t)tile * (4 + 2) + (size_t)fanout * 4 + ((size_t)fanout + 2) * 2;
 }
@@ -473,6 +546,90 @@ int gather_values(const uint32_t* d_values, uint64_t m, uint32_t radix_bits, voi
     constexpr int kWideIt = kWideTile / kTileBlock, kIt = kTile / kTileBlock;
     return pl.wide() ? launch(k_part_gather<kTileBlock, kWideIt, 3>, pl.tiles, kTileBlock, smem, s, d_values, m, t, iv, d_out)
                      : launch(k_part_gather<kTileBlock, kIt, 4>, pl.tiles, kTileBlock, smem, s, d_values, m, t, iv, d_out);
+}
+
+namespace {
+constexpr uint32_t kPairsRadixBits = 8;  // the most of a call's partition (small tiles)
+// scratch of an ordered-pairs call by partition, behind pairs_workspace_bytes
+struct pairs_scratch {
+    void* tables;
+    size_t table_bytes;
+    uint32_t* values;
+    void* inverse;
+    size_t inverse_bytes;
+};
+size_t pairs_inverse_bytes(uint64_t m) {
+    return workspace_carver::need({m * 2, (m / kTile + 1) * (2ull << kPairsRadixBits)});
+}
+}  // namespace
+
+size_t pairs_partition_bytes(uint64_t m) {
+    if (m < kPartitionPairsMin || m > kPartitionPairsMax) return 0;
+    // no device is asked: more SMs than there are only make the tables larger
+    return workspace_carver::need({partition_ws_bytes(m, kPairsRadixBits, 256) + (1u << 20), m * 4,
+                                   pairs_inverse_bytes(m)});
+}
+
+// Taken by large calls into columns far larger than L2: the partition, the
+// probes from L2 and the gather cost less than a random DRAM access a probe.
+// B+tree, plain / by partition: 2^28 probes into 2^26 uniform keys 6687 / 4998
+// us (histogram 349, scatter 911, probes 2956, gather 835), 50 M 1284 / 1026;
+// lognormal 6675 / 6083; 2^25 keys 5711 / 4679, 2^24 keys 4237 / 4567; 2^29
+// into 2^28 keys 21.5 / 12.4 ms.  The relation's keys lie in the pairs buffer,
+// which has 8 bytes a probe and is not written before the gather.  Columns
+// whose table windows take long searches are left to the plain pairs: at once
+// below 2^26 keys (2^25 clustered keys 5505 / 5955), where those searches
+// dwarf the rest above (2^26 clustered keys 8628 / 5972).  A hash table is one
+// random sector whatever the column, so only short searches beat it (50 M
+// probes into 2^24 / 2^26 / 2^28 uniform keys 988 / 921, 1163 / 1026 and 1243 /
+// 1328).  34 M probes are about where lognormal columns break even (2^25 keys
+// 754 / 752; 2^26 865 / 839, 24 M 629 / 622).
+int launch_pairs_by_partition(const gj_index* idx, const uint64_t* d_probes, uint64_t m, uint32_t* d_pairs,
+                              uint64_t* d_count, void* ws, size_t ws_bytes, cudaStream_t s, bool* taken) {
+    *taken = false;
+    if (m < kPartitionPairsMin || m > kPartitionPairsMax || idx->n <= partition_pairs_keys(idx->type) || !idx->in_hbm ||
+        !idx->rel.pos || !idx->rel.col_aligned)
+        return GJ_OK;
+    const double most = idx->type == GJ_INDEX_HASH ? 2.0 : idx->n < (1ull << 26) ? 2.5 : 4.0;
+    if (idx->rel_loads > most) return GJ_OK;
+    const uint32_t bits = std::min(default_radix_bits(idx->n), kPairsRadixBits);
+    device_info di;
+    GJ_TRY(current_device_info(&di));
+    const size_t head = pairs_workspace_bytes(m);
+    if (ws_bytes <= head) return GJ_OK;
+    pairs_ws pw;
+    size_t used = 0;
+    if (!carve_pairs_ws(ws, head, m, &pw, &used)) return GJ_OK;
+    workspace_carver wc(static_cast<char*>(ws) + head, ws_bytes - head);
+    pairs_scratch sc;
+    sc.table_bytes = partition_ws_bytes(m, bits, di.sm_count);
+    sc.tables = wc.take<char>(sc.table_bytes);
+    sc.values = wc.take<uint32_t>(m);
+    sc.inverse_bytes = pairs_inverse_bytes(m);
+    sc.inverse = wc.take<char>(sc.inverse_bytes);
+    partition_inverse iv{};
+    part_tables t;
+    const partition_plan pl = plan_partition(m, bits, di.sm_count);
+    if (!sc.tables || !sc.values || !sc.inverse ||
+        !carve_partition_inverse(sc.inverse, sc.inverse_bytes, m, bits, di.sm_count, &iv) ||
+        !carve_tables(sc.tables, sc.table_bytes, pl, &t))
+        return GJ_OK;
+    static_assert(kGatherTile == kTile, "the gather's tiles are the scatter's");
+    *taken = true;
+    uint64_t* keys = reinterpret_cast<uint64_t*>(d_pairs);
+    GJ_CUDA_TRY(cudaMemsetAsync(ws, 0, used, s));
+    GJ_TRY(range_partition_impl(d_probes, m, idx->min_key, shift_for(idx->min_key, idx->max_key, bits), bits, 0, keys,
+                                nullptr, nullptr, sc.tables, sc.table_bytes, s, &iv));
+    const uint32_t blocks = (uint32_t)((m + kBlock - 1) / kBlock);
+    const bool exact =
+        idx->type == GJ_INDEX_BTREE || idx->type == GJ_INDEX_HARMONIA || idx->type == GJ_INDEX_HASH;
+    GJ_TRY(launch(exact ? k_relation_values<true> : k_relation_values<false>, blocks, kBlock, 0, s, idx->rel, idx->d_col,
+                  (uint32_t)idx->n, static_cast<const uint64_t*>(keys), m, sc.values));
+    const size_t smem = (size_t)pl.fanout * 4 + ((size_t)pl.fanout + 2) * 2 + kGatherTile * 2;
+    int grid = 0;
+    GJ_TRY(grid_for(k_gather_pairs, smem, (uint64_t)pl.tiles * kBlock, &grid));
+    return launch(k_gather_pairs, (uint32_t)grid, kBlock, smem, s, static_cast<const uint32_t*>(sc.values), m, t, iv,
+                  reinterpret_cast<uint2*>(d_pairs), d_count, pw);
 }
 
 // key range used by the partitioned INLJ for an index (recorded at build)

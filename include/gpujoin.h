@@ -174,7 +174,10 @@ int gj_index_lookup(const gj_index* index, const uint64_t* d_probes, uint64_t m,
  * (probe row, build position) pair -- two uint32 at d_pairs[2k], [2k+1] --
  * per probe with a result, in probe order (deterministic; the reference's
  * order follows its atomics).  *d_count (device) receives the pair count.
- * d_pairs must hold 2*m uint32.  Workspace: gj_inlj_pairs_workspace_size. */
+ * d_pairs must hold 2*m uint32.  Workspace: gj_inlj_pairs_workspace_size,
+ * which from 2^25 to 2^29 probes includes room (about 6.2 bytes a probe)
+ * with which calls into columns far larger than L2 partition their probes
+ * first; gj_inlj_pairs_host_workspace_size bytes serve every call without. */
 int gj_inlj_pairs_workspace_size(uint64_t m, size_t* bytes);
 int gj_inlj_pairs(const gj_index* index, const uint64_t* d_probes, uint64_t m, uint32_t* d_pairs,
                   uint64_t* d_count, void* d_workspace, size_t workspace_bytes, void* stream);

@@ -286,3 +286,33 @@ def test_inlj_pairs_large(orc, gj, cuda, m):
     rows2, pos2 = pairs_of(out2, cnt2)
     np.testing.assert_array_equal(rows2, erows)
     np.testing.assert_array_equal(pos2, epos)
+
+
+@pytest.mark.parametrize("kind", ["btree", "binary_search", "harmonia", "radix_spline", "learned", "hash"])
+@pytest.mark.parametrize("dist", ["DIST_UNIFORM", "DIST_LOGNORMAL"])
+@pytest.mark.parametrize("m", [3 << 24, (3 << 24) + 4097])
+def test_pairs_by_partition(gj, cuda, kind, dist, m):
+    # calls large enough to partition their probes first: the same pairs, in
+    # probe order, as the index's own lookups give, on the offered workspace
+    # and on one that has no room for it
+    import torch
+
+    n = (1 << 25) + 64
+    keys = gj.generate_sorted_keys(n, getattr(gj, dist), 1 << 63, seed=5)
+    ix = gj.make_index(kind).construct(None, keys)
+    probes = gj.generate_probes(keys, m, theta=0.5, absent_fraction=0.1, seed=6)
+    probes[:4] = torch.tensor([0, 1, -1, -2], dtype=torch.int64, device="cuda")  # both ends of the key range
+    pos = ix.lookup(probes)
+    rows = torch.nonzero(pos != -1).flatten()
+    small, offered = ctypes.c_size_t(0), ctypes.c_size_t(0)
+    gj.lib().gj_inlj_pairs_host_workspace_size(m, ctypes.byref(small))
+    gj.lib().gj_inlj_pairs_workspace_size(m, ctypes.byref(offered))
+    assert offered.value > 6 * m > small.value
+    for nbytes in (offered.value, small.value):
+        ws = torch.full((nbytes,), 0xA5, dtype=torch.uint8, device="cuda")
+        pairs, count = ix.inlj_pairs(probes, workspace=ws)
+        ix.inlj_pairs_status(ws, m)
+        assert int(count) == rows.numel()
+        got = pairs[: 2 * int(count)].view(-1, 2)
+        assert torch.equal(got[:, 0].to(torch.int64), rows)
+        assert torch.equal(got[:, 1], pos[rows])
