@@ -177,6 +177,25 @@ def profile_traffic(kernel_tag: str):
 # ---------------------------------------------------------------------------
 # GPU arm
 # ---------------------------------------------------------------------------
+def count_launches(fn):
+    """Kernels of the library that one call of fn launches, counted (not timed)
+    by the profiler outside any timed region; None where it cannot trace."""
+    import torch
+
+    try:
+        from torch.profiler import ProfilerActivity, profile
+
+        fn()
+        torch.cuda.synchronize()
+        with profile(activities=[ProfilerActivity.CUDA]) as prof:
+            fn()
+            torch.cuda.synchronize()
+        found = sum(e.count for e in prof.key_averages() if "gj::" in e.key)
+        return found or None
+    except Exception:
+        return None
+
+
 def time_steps(fn, steps: int, warmup: int, stream, world: int, device):
     """Run warmup untimed steps, then time exactly `steps` steps with CUDA
     events on `stream`, bracketed by barrier + synchronize; returns ms."""
@@ -670,28 +689,32 @@ def inlj_workload(args, world, rank, device, stream):
                                                 "api": "gj_inlj_pairs_unordered (device buffers)",
                                                 "pairs": d_count, "parity": d_parity}}}
 
-    # Roofline of the dominant kernel.  A pairs step is two launches: the
-    # search pass (k_lookup: probe key in, one 32-byte leaf sector, u32
-    # position out to the upper half of the pairs buffer) and the ordered
-    # compaction (u32 in, 8-byte pair out).  The search pass is timed on its
-    # own here -- the same kernel on the same probes and output location, CUDA
-    # events on the same stream; its algorithmic bytes are 8 + 32 + 4 per probe.
+    # Roofline of the step.  A pairs step of this size partitions its probes
+    # first: histogram (8 B read a probe), scatter (8 read, key and 16-bit tile
+    # offset written), probes (key read, u32 position written; the index and
+    # the column come from L2, each read from HBM about once), gather (position
+    # and offset read, pair written) -- or, where the call stays plain, one
+    # launch: probe in, one 32-byte column sector, pair out.  Beside it the
+    # plain lookup of the same probes into positions, timed on its own: one
+    # random column sector a probe.
     peak, peak_kind = measured_peak()
     lookup_bytes_per_probe = bytes_per_probe - 4
+    per_step = count_launches(lambda: headline_ix.inlj_pairs(probes, pairs, count, ws))
+    step_bytes = bytes_per_probe if per_step is not None and per_step < 4 else 52 + 8.0 * n / m
     lookup_ms = time_steps(lambda: headline_ix.lookup(probes, out=pairs[m:]), args.steps, args.warmup, stream, world,
                            device)
     lookup_ms = max_over_ranks(lookup_ms, world, device) / args.steps
-    achieved = lookup_bytes_per_probe * m / (lookup_ms / 1e3) / 1e9
-    traffic = profile_traffic(f"k_lookup_{headline_index}_n{args.n_log2}_m{args.m_log2}")
     step_ms = headline_ms / args.steps
+    achieved = step_bytes * m / (step_ms / 1e3) / 1e9
     roofline = {"bound": "hbm", "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
-                "frac": round(achieved / peak, 4), "traffic": traffic,
+                "frac": round(achieved / peak, 4), "traffic": None,
                 "peak_source": f"{peak_kind} hbm_gbs (copy, burst)",
-                "kernel": f"k_lookup<{headline_index}> (search pass of the pairs step)",
-                "kernel_ms": round(lookup_ms, 4), "kernel_share_of_step": round(lookup_ms / step_ms, 3),
-                "bytes_per_probe": lookup_bytes_per_probe,
-                "step_bytes_per_probe": bytes_per_probe,
-                "step_achieved": round(bytes_per_probe * m / (step_ms / 1e3) / 1e9, 1)}
+                "kernel": "the whole pairs step", "bytes_per_probe": step_bytes, "launches_per_step": per_step,
+                "plain_lookup": {
+                    "kernel": f"k_lookup<{headline_index}> (positions of the same probes)",
+                    "kernel_ms": round(lookup_ms, 4), "bytes_per_probe": lookup_bytes_per_probe,
+                    "achieved": round(lookup_bytes_per_probe * m / (lookup_ms / 1e3) / 1e9, 1),
+                    "traffic": profile_traffic(f"k_lookup_{headline_index}_n{args.n_log2}_m{args.m_log2}")}}
     # index path: the L2 sectors the search pass reads per probe (ncu,
     # lts__t_sectors_srcunit_tex_op_read at 2^24 probes of the same index),
     # times 32 B, over the live kernel time
@@ -700,7 +723,7 @@ def inlj_workload(args, world, rank, device, stream):
         path_gbs = l2_sectors * 32 * m / (lookup_ms / 1e3) / 1e9
         roofline["index_path"] = {"l2_sectors_per_probe": l2_sectors, "bytes_per_probe": round(l2_sectors * 32, 1),
                                   "l2_to_sm_gbs": round(path_gbs, 1),
-                                  "note": "L2-to-SM bytes of the search pass (ncu sectors x 32 B over the live "
+                                  "note": "L2-to-SM bytes of the plain lookup (ncu sectors x 32 B over the live "
                                           "kernel time); most index reads are L2 hits"}
     # the second roofline of scattered probes: each needs at least one random
     # 32-byte sector of a column larger than L2, so probes/s <= random
@@ -749,7 +772,7 @@ def inlj_workload(args, world, rank, device, stream):
         "roofline": roofline,
         "cpu_baseline": cpu,
         "e2e": e2e,
-        "gpu_launches": 2 * args.steps,
+        "gpu_launches": (per_step or 1) * args.steps,
         "clocks": clocks,
     }
     if rank == 0 and world == 1 and not args.no_extras:
@@ -827,9 +850,11 @@ def partitioned_measure(args, world, device, stream, n_log2, m_log2, steps, kind
         parity = check_pairs_sample(pairs, count, m, keys.cpu().numpy().view(np.uint64),
                                     probes.cpu().numpy().view(np.uint64), args.parity_sample, args.seed + 7, sem)
         parity["semantics"] = sem
-    # the same probes through the unpartitioned pairs kernel, for comparison
+    # the same probes through the unpartitioned pairs kernel, for comparison (a
+    # workspace without the room to partition)
+    launches = count_launches(step)
     pw = ctypes.c_size_t()
-    gj.lib().gj_inlj_pairs_workspace_size(m, ctypes.byref(pw))
+    gj.lib().gj_inlj_pairs_host_workspace_size(m, ctypes.byref(pw))
     pws = torch.empty(pw.value, dtype=torch.uint8, device=device)
     plain_steps = max(2, steps // 2)
     plain_ms = time_steps(lambda: ix.inlj_pairs(probes, pairs, count, pws), plain_steps, 1, stream, world,
@@ -846,7 +871,7 @@ def partitioned_measure(args, world, device, stream, n_log2, m_log2, steps, kind
            "roofline": {"bound": "hbm", "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
                         "frac": round(achieved / peak, 4), "bytes_per_probe": bpp,
                         "peak_source": f"{peak_kind} hbm_gbs (copy, burst)"},
-           "launches_per_step": 3 + ((m + window - 1) // window) * 8, "clocks": clocks}
+           "launches_per_step": launches, "clocks": clocks}
     # The probe pass reads its index slices from L2 (a partition's directory
     # and column slice stay resident while its probes run), one random
     # 32-byte sector per request; so its floor is the L2 rate of random
@@ -892,7 +917,7 @@ def partitioned_workload(args, world, rank, device, stream):
         f"partitioned INLJ: {r['build_keys']} uniform uint64 keys (2^{n_log2}), {r['probes']} Zipf({args.theta}) "
         f"probes (2^{m_log2}), {kind}, range partition 2^{r['radix_bits']}, window {r['window']}",
         {"partitioned": r, "parity": r["parity"], "roofline": dict(r["roofline"], traffic=None),
-         "gpu_launches": args.steps * r["launches_per_step"], "clocks": r["clocks"], "cpu_baseline": None,
+         "gpu_launches": args.steps * (r["launches_per_step"] or 1), "clocks": r["clocks"], "cpu_baseline": None,
          "e2e": None})
 
 
