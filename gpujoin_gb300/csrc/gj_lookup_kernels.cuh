@@ -7,8 +7,10 @@
 // partitioned_lookup_kernel (src/index_lookup_partitioning.cu:218-248) and
 // ij_lookup_kernel (src/tpch/tpch_14_ij.cu:371-407).
 //
-// Each kernel stages the upper part of the index (B+tree top levels,
-// Harmonia top nodes, the sampled binary-search keys) into shared memory once
+// Lookups of scattered probes start at an entry of a start table (key start
+// table, B+tree or Harmonia node table) and stage nothing; the sampled keys
+// of a binary search without a table, and the top B+tree levels that the
+// sorted-tile kernels descend once a tile, are staged in shared memory once
 // per block.  Probe keys are streamed with evict-first loads, results with
 // streaming stores.
 #pragma once
@@ -33,7 +35,7 @@ struct lookup_call {
     uint64_t* d_count;
     void* ws;
     size_t ws_bytes;
-    uint32_t* stash;       // pairs: room for m positions (two passes), or null (host buffers)
+    uint32_t* stash;       // pairs: room for m positions (for two passes), or null (host buffers)
     cudaStream_t s;
     // test hook of the bounded waits (gj_debug_inlj_pairs_stalled): a spin
     // limit other than kSpinLimit (0 = default) and a first tile left
@@ -330,6 +332,10 @@ __global__ void __launch_bounds__(kBlock, Op::kMinBlocks) k_scatter_lookup(const
 // of four probes a thread, 2^18 probes 25 against 28, 2^20 50.1 against 49.7.
 // Large calls save the positions' way through memory: 2^28 probes into a hash
 // table of 2^26 keys 6631 against 6081 us, into the B+tree 6856 against 6678.
+// An index in host memory keeps the two passes at every size (host_index
+// below): each lookup waits on the link several times, and k_pairs' barriers
+// make a whole block wait for its slowest (2^22 probes into a B+tree of 2^20
+// keys 2325 us in two passes, 2692 in one).
 constexpr uint64_t kSinglePassMin = 1ull << 18;
 // probes a thread of k_pairs: 8 for long calls into a column that stays in L2
 // (hash table of 2^20 keys 2027 against 2212 us per 2^28 probes with 4), 4
@@ -784,7 +790,7 @@ __global__ void __launch_bounds__(kBlock, Op::kMinBlocks < 6 ? Op::kMinBlocks : 
     extern __shared__ __align__(16) uint64_t cache[];
     using hint_t = typename tile_hint_of<Op>::type;
     __shared__ sorted_tile_smem<hint_t> t;
-    stage_cache(cache, sd);
+    stage_cache(cache, sd);  // the tiles' hints read it
     auto fill = [&](uint64_t t0, uint32_t* s_pos) {
         const uint32_t tn = m - t0 < kSortTile ? (uint32_t)(m - t0) : kSortTile;
         sort_tile(op, cache, keys, t0, tn, [&](uint32_t j) { return (uint32_t)(t0 + j); }, t);
@@ -819,7 +825,7 @@ __global__ void __launch_bounds__(kBlock, Op::kMinBlocks < 6 ? Op::kMinBlocks : 
     using hint_t = typename tile_hint_of<Op>::type;
     __shared__ sorted_tile_smem<hint_t> t;
     __shared__ uint32_t s_pos[kSortTile];
-    stage_cache(cache, sd);
+    stage_cache(cache, sd);  // the tiles' hints read it
     for (uint32_t r = 0; r < kSortedLookupTiles; ++r) {
         const uint64_t t0 = ((uint64_t)blockIdx.x * kSortedLookupTiles + r) * kSortTile;
         if (t0 >= m) break;
@@ -936,7 +942,7 @@ int run_scatter(const Op& op, const stage_desc& sd, uint64_t n, const uint64_t* 
 template <class Op>
 int run_pairs(const Op& op, const stage_desc& sd, uint64_t n, const uint64_t* probes, uint64_t m, uint32_t* pairs,
               uint64_t* d_count, void* ws, size_t ws_bytes, uint32_t* stash, cudaStream_t s, uint32_t spin_limit = 0,
-              bool skip_first_tile = false, bool unordered = false) {
+              bool skip_first_tile = false, bool unordered = false, bool host_index = false) {
     pairs_ws pw;
     size_t used = 0;
     if (!carve_pairs_ws(ws, ws_bytes, m, &pw, &used)) {
@@ -949,7 +955,7 @@ int run_pairs(const Op& op, const stage_desc& sd, uint64_t n, const uint64_t* pr
         return GJ_OK;
     }
     if (spin_limit) pw.spin_limit = spin_limit;
-    const bool two_passes = stash && m < kSinglePassMin;
+    const bool two_passes = stash && (m < kSinglePassMin || host_index);
     // the state lies in whole 64-bit words at the head of the workspace
     if (two_passes)
         GJ_TRY(run_lookup(op, sd, n, probes, m, stash, s, pw.tile_state, (uint32_t)(used / 8)));
@@ -1014,7 +1020,7 @@ int run_call(const Op& op, const gj_index* idx, const lookup_call& c) {
         case lookup_action::scatter: return run_scatter(op, sd, idx->n, c.keys, c.rows, c.m, c.out, c.s);
         case lookup_action::pairs:
             return run_pairs(op, sd, idx->n, c.keys, c.m, c.out, c.d_count, c.ws, c.ws_bytes, c.stash, c.s, c.spin_limit,
-                             c.skip_first_tile, c.unordered);
+                             c.skip_first_tile, c.unordered, idx->params.index_memory == GJ_INDEX_MEMORY_HOST);
         case lookup_action::sorted_pairs:
             return run_sorted_pairs(op, sd, c.keys, c.m, c.out, c.d_count, c.ws, c.ws_bytes, c.s);
         case lookup_action::sorted_positions: return run_sorted_lookup(op, sd, c.keys, c.m, c.out, c.s);

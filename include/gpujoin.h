@@ -86,8 +86,10 @@ typedef struct gj_index_params {
                                    one 32-byte sector) */
     uint32_t rs_radix_bits;     /* RadixSpline radix table bits (default 18) */
     uint32_t rs_max_error;      /* RadixSpline spline error (default 32) */
-    uint32_t bs_cache_keys;     /* binary search: sampled keys staged in shared memory (default 4096, 0 = off) */
-    uint32_t smem_cache_bytes;  /* B+tree / Harmonia: upper levels staged in shared memory (default 16384) */
+    uint32_t bs_cache_keys;     /* binary search: sampled keys staged in shared memory where no key start table
+                                   serves the lookup (index in host memory) (default 4096, 0 = off) */
+    uint32_t smem_cache_bytes;  /* B+tree: upper levels staged in shared memory by the sorted-tile kernels
+                                   (default 16384) */
     uint32_t learned_leaves;    /* learned index: linear leaf models (default 0: about 128 keys per leaf, a
                                    power of two in [2^10, 2^20]) */
     uint32_t learned_root;      /* GJ_LEARNED_ROOT_LINEAR, _MLP, _SEGMENTS or _AUTO (default AUTO) */
@@ -244,8 +246,9 @@ int gj_inlj_pairs_host(const gj_index* index, const uint64_t* h_probes, uint64_t
  * atomicAdd per tile, as the reference's join kernels place theirs,
  * src/tpch/tpch_14_ij.cu:371-407) instead of in probe order: the same set
  * of pairs and the same count, with no tile waiting for its predecessors
- * (19 % faster on GB300 for 2^28 probes: the link, not the ordering, is the
- * limit).  Same arguments and workspace; nothing waits, so
+ * (the link is the limit of both forms: 21.2 against 21.1 G probes/s on
+ * GB300 for 2^28 probes, where gj_inlj_pairs_host searches its next tile
+ * while the counts before the last one arrive).  Same arguments and workspace; nothing waits, so
  * gj_inlj_pairs_status has nothing to report. */
 int gj_inlj_pairs_host_unordered(const gj_index* index, const uint64_t* h_probes, uint64_t m, uint32_t* h_pairs,
                                  uint64_t* h_count, void* d_workspace, size_t workspace_bytes, void* stream);
@@ -323,7 +326,8 @@ int gj_partitioned_lookup(const gj_index* index, const uint64_t* d_part_keys, co
  * windows of window_size probes; each window is range-partitioned on the
  * index's key range and every partition is probed against its slice of the
  * index's column through a partition directory built once per call (each
- * index kind's result semantics kept).  Emits d_positions in probe order
+ * index kind's result semantics kept; positions alone, d_pairs == NULL, take
+ * gj_index_lookup's search window by window where that is sooner).  Emits d_positions in probe order
  * (equal to gj_index_lookup) when d_positions != NULL, and/or the (row, pos)
  * pairs of the matches when d_pairs != NULL (*d_count = number of pairs);
  * the set of pairs is fixed, their order is not (tiles of a window append
