@@ -120,15 +120,22 @@ constexpr int kStartSums = 3;
 
 // key start table: the first key not below each bucket's first value (binary
 // search per bucket; n from the bucket past the last one on), with the
-// bucket's count where entries are packed; clears the sums of the cost sample
+// bucket's count where entries are packed; clears the sums of the cost sample.
+// guide: an unpacked table over 2^guide_log of these buckets each, or null;
+// a bucket is then searched between the guide's entries
 __global__ void k_key_start(const uint64_t* __restrict__ col, uint64_t n, uint64_t min_key, uint32_t shift,
-                            uint32_t buckets, uint32_t entries, uint32_t packed, uint32_t* __restrict__ pos,
-                            unsigned long long* __restrict__ sums) {
+                            uint32_t buckets, uint32_t entries, uint32_t packed, const uint32_t* __restrict__ guide,
+                            uint32_t guide_log, uint32_t* __restrict__ pos, unsigned long long* __restrict__ sums) {
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t < kStartSums) sums[t] = 0;
     for (uint32_t b = t; b < entries; b += gridDim.x * blockDim.x) {
         const uint64_t first = min_key + ((uint64_t)b << shift);
-        const uint64_t lo = b >= buckets ? n : lower_bound_branch_free(col, n, first);
+        uint64_t from = 0, upto = n;
+        if (guide && b < buckets) {
+            from = guide[b >> guide_log];
+            upto = guide[(b >> guide_log) + 1];
+        }
+        const uint64_t lo = b >= buckets ? n : from + lower_bound_branch_free(col + from, upto - from, first);
         uint32_t e = (uint32_t)lo;
         if (packed && b < buckets) {
             const uint64_t rest =
@@ -379,11 +386,13 @@ uint32_t key_start_shift(uint64_t range, uint32_t bits) {
     const uint32_t used = range ? 64u - (uint32_t)__builtin_clzll(range) : 0u;
     return used > bits ? used - bits : 0u;
 }
-// the table in whole 16-byte groups, and the sums of the cost sample
+// a bucket each and the closing entry, in whole 16-byte groups
+uint64_t key_start_entries(uint64_t range, uint32_t shift) { return ((range >> shift) + 1 + 1 + 3) & ~3ull; }
+// the table and the sums of the cost sample
 size_t key_start_bytes(const gj_index* idx, uint32_t bits) {
     const uint64_t range = idx->max_key - idx->min_key;
-    const uint64_t buckets = (range >> key_start_shift(range, bits)) + 1;
-    return ((buckets + 1 + 3) & ~3ull) * sizeof(uint32_t) + kStartSums * sizeof(unsigned long long);
+    return key_start_entries(range, key_start_shift(range, bits)) * sizeof(uint32_t) +
+           kStartSums * sizeof(unsigned long long);
 }
 
 // Key start table of 2^bits buckets (fewer for a narrow key range); use(loads,
@@ -391,7 +400,8 @@ size_t key_start_bytes(const gj_index* idx, uint32_t bits) {
 // read, and for a B+tree the mean level its lookups start at -- whether the
 // index's scattered lookups go through it.
 template <class Use>
-int build_key_start(gj_index* idx, uint32_t bits, cudaStream_t s, spare_memory&& spare, Use&& use) {
+int build_key_start(gj_index* idx, uint32_t bits, cudaStream_t s, spare_memory&& spare, Use&& use,
+                    const key_start* guide = nullptr) {
     const uint64_t range = idx->max_key - idx->min_key;
     key_start t{};
     t.min_key = idx->min_key;
@@ -400,14 +410,15 @@ int build_key_start(gj_index* idx, uint32_t bits, cudaStream_t s, spare_memory&&
     t.inv_width = std::ldexp(1.0f, -(int)t.shift);
     t.col_aligned = aligned32(idx->d_col);
     const uint32_t buckets = (uint32_t)(range >> t.shift) + 1;
-    const uint32_t entries = (buckets + 1 + 3) & ~3u;  // whole 16-byte groups
+    const uint32_t entries = (uint32_t)key_start_entries(range, t.shift);
     if (!spare.p) GJ_TRY(spare.take(key_start_bytes(idx, bits)));
     uint32_t* pos = static_cast<uint32_t*>(spare.p);
     unsigned long long* d_sums = reinterpret_cast<unsigned long long*>(pos + entries);
     unsigned long long sums[kStartSums] = {};
     t.packed = idx->n <= kStartPackedKeys ? 1u : 0u;
     k_key_start<<<(entries + 255) / 256, 256, 0, s>>>(idx->d_col, idx->n, t.min_key, t.shift, buckets, entries,
-                                                     t.packed, pos, d_sums);
+                                                     t.packed, guide ? guide->pos : nullptr,
+                                                     guide ? guide->shift - t.shift : 0u, pos, d_sums);
     GJ_CUDA_TRY(cudaGetLastError());
     t.pos = pos;
     k_start_cost<<<kStartSample / 256, 256, 0, s>>>(t, idx->d_col, (uint32_t)idx->n, idx->bt, d_sums);
@@ -420,6 +431,40 @@ int build_key_start(gj_index* idx, uint32_t bits, cudaStream_t s, spare_memory&&
     idx->rel_loads = (double)sums[0] / kStartSample;
     if (use(idx->rel_loads, (double)sums[1] / kStartSample)) idx->ks = t;
     idx->bytes += (size_t)entries * sizeof(uint32_t);
+    return GJ_OK;
+}
+
+// The table large ordered-pairs calls search through (idx->rel), whatever the
+// kind.  A partition's probes share its slice of the table in L2, so above
+// 2^24 keys it is finer than a scattered lookup's: two to four keys a bucket,
+// at most 2^25 buckets (128 MB).  2^28 probes with 2^22 / 2^24 / 2^25 buckets:
+// 2^26 uniform keys 5019 / 4753 / 4656 us, lognormal 6115 / 5449 / 5240, 2^28
+// uniform keys 6305 / 5398 / 5117; the index takes 0.4 to 0.6 ms longer to
+// build.  The coarse table guides the finer one's build.  The coarse one is
+// given back unless lookups go through it; the finer one where it saves less
+// than a twentieth of the column loads (clustered keys: nothing).
+int build_partition_start(gj_index* idx, cudaStream_t s) {
+    const uint64_t n = idx->n;
+    if (!idx->rel.pos)
+        GJ_TRY(build_key_start(idx, key_start_bits(n), s, spare_memory(), [](double, double) { return false; }));
+    uint32_t bits = 1;
+    while (bits < 25 && (2ull << bits) < n) ++bits;
+    const key_start coarse = idx->rel;
+    const double coarse_loads = idx->rel_loads;
+    if (n <= kStartPackedKeys || coarse.shift <= key_start_shift(coarse.range, bits)) return GJ_OK;
+    GJ_TRY(build_key_start(idx, bits, s, spare_memory(), [](double, double) { return false; }, &coarse));
+    const key_start fine = idx->rel;
+    const bool keep = idx->rel_loads < 0.95 * coarse_loads;
+    if (!keep) {
+        idx->rel = coarse;
+        idx->rel_loads = coarse_loads;
+    }
+    const key_start& out = keep ? coarse : fine;  // no longer searched for pairs
+    if (idx->ks.pos == out.pos) return GJ_OK;
+    void* p = const_cast<uint32_t*>(out.pos);
+    idx->allocations.erase(std::find(idx->allocations.begin(), idx->allocations.end(), p));
+    idx->bytes -= key_start_entries(out.range, out.shift) * sizeof(uint32_t);
+    GJ_CUDA_TRY(cudaFree(p));
     return GJ_OK;
 }
 
@@ -971,10 +1016,8 @@ int gj_index_build(int type, const uint64_t* d_keys, const uint64_t* h_keys, uin
         case GJ_INDEX_HASH: rc = build_hash(idx.get(), s); break;
         case GJ_INDEX_NO_OP: break;
     }
-    // large ordered-pairs calls partition their probes and search through a
-    // key start table, whatever the kind
-    if (rc == GJ_OK && type != GJ_INDEX_NO_OP && idx->in_hbm && n > partition_pairs_keys(type) && !idx->rel.pos)
-        rc = build_key_start(idx.get(), key_start_bits(n), s, spare_memory(), [](double, double) { return false; });
+    if (rc == GJ_OK && type != GJ_INDEX_NO_OP && idx->in_hbm && n > partition_pairs_keys(type))
+        rc = build_partition_start(idx.get(), s);
     if (rc == GJ_OK) {
         cudaError_t e = cudaStreamSynchronize(s);
         if (e != cudaSuccess) {

@@ -573,9 +573,10 @@ size_t pairs_partition_bytes(uint64_t m) {
 // Taken by large calls into columns far larger than L2: the partition, the
 // probes from L2 and the gather cost less than a random DRAM access a probe.
 // B+tree, plain / by partition: 2^28 probes into 2^26 uniform keys 6687 / 4998
-// us (histogram 349, scatter 911, probes 2956, gather 835), 50 M 1284 / 1026;
-// lognormal 6675 / 6083; 2^25 keys 5711 / 4679, 2^24 keys 4237 / 4567; 2^29
-// into 2^28 keys 21.5 / 12.4 ms.  The relation's keys lie in the pairs buffer,
+// us (histogram 349, scatter 911, probes 2956, gather 835; 4625 since the
+// probes' table is finer than the lookups'), 50 M 1284 / 1026; lognormal 6675
+// / 6083 (5219); 2^25 keys 5711 / 4679, 2^24 keys 4237 / 4567; 2^29 into 2^28
+// keys 21.5 / 12.4 ms (2^28 probes 6.27 ms, 5.09 with the finer table).  The relation's keys lie in the pairs buffer,
 // which has 8 bytes a probe and is not written before the gather.  Columns
 // whose table windows take long searches are left to the plain pairs: at once
 // below 2^26 keys (2^25 clustered keys 5505 / 5955), where those searches

@@ -316,3 +316,30 @@ def test_pairs_by_partition(gj, cuda, kind, dist, m):
         got = pairs[: 2 * int(count)].view(-1, 2)
         assert torch.equal(got[:, 0].to(torch.int64), rows)
         assert torch.equal(got[:, 1], pos[rows])
+
+
+@pytest.mark.parametrize("kind", ["btree", "binary_search", "hash"])
+@pytest.mark.parametrize("column", ["clusters", "dense", "end_of_range"])
+def test_pairs_by_partition_start_tables(gj, cuda, kind, column):
+    # columns for which the partitioned pairs' table stays the lookups' own
+    # (clusters), has two keys a bucket (dense) or ends at the largest key with
+    # nearly all keys in its first buckets (end_of_range)
+    import torch
+
+    m = (1 << 25) + 257
+    if column == "clusters":
+        keys = gj.generate_sorted_keys(1 << 26, gj.DIST_CLUSTERS, 1 << 63, seed=5)
+    else:
+        keys = torch.arange((1 << 25) + 64, dtype=torch.int64, device="cuda") + 7
+        if column == "end_of_range":
+            keys[-1] = -1  # 2^64 - 1
+    ix = gj.make_index(kind).construct(None, keys)
+    probes = gj.generate_probes(keys, m, theta=0.5, absent_fraction=0.1 if column == "clusters" else 0.0, seed=6)
+    probes[:6] = torch.tensor([0, 6, 7, -1, -2, (1 << 25) + 71], dtype=torch.int64, device="cuda")
+    pos = ix.lookup(probes)
+    rows = torch.nonzero(pos != -1).flatten()
+    pairs, count = ix.inlj_pairs(probes)
+    assert int(count) == rows.numel()
+    got = pairs[: 2 * int(count)].view(-1, 2)
+    assert torch.equal(got[:, 0].to(torch.int64), rows)
+    assert torch.equal(got[:, 1], pos[rows])
