@@ -259,12 +259,18 @@ __device__ __forceinline__ void stage_cache(uint64_t* dst, const stage_desc& sd)
 // probes into 2^26 keys 1568 against 1654 us); several save a block's start
 // where the searches run from L2 (hash table of 2^20 keys 406 against 485 us
 // with 8, key start table 534 against 569 with 4; RadixSpline, whose registers
-// then spill, is level or slower).
+// then spill, is level or slower).  Plain lookups take several up to 2^24 keys,
+// where most sectors still hit L2 (24 M probes with 1 / 4: B+tree, uniform
+// probes 358 / 352 us, Zipf(1.25) 212 / 189), and into a hash table, whose
+// search is one load, at any size (2^26 keys with 1 / 4 / 8: uniform 548 / 559
+// / 567, Zipf(1.25), which L1 and L2 serve, 160 / 133 / 132).
 constexpr uint64_t kL2Keys = 1ull << 23;  // columns of up to 64 MB stay in L2
-inline int long_blocks(uint64_t n, uint64_t m, bool* yes) {
+template <class Op>
+constexpr uint64_t kLookupLongKeys = std::is_same<Op, op_hash>::value ? UINT64_MAX : 1ull << 24;
+inline int long_blocks(uint64_t n, uint64_t m, bool* yes, uint64_t keys = kL2Keys) {
     device_info di;
     GJ_TRY(current_device_info(&di));
-    *yes = n <= kL2Keys && m >= 16ull * di.sm_count * 8 * kBlock;  // 16 waves of a full chip
+    *yes = n <= keys && m >= 16ull * di.sm_count * 8 * kBlock;  // 16 waves of a full chip
     return GJ_OK;
 }
 
@@ -907,7 +913,7 @@ int run_lookup(const Op& op, const stage_desc& sd, uint64_t n, const uint64_t* p
     };
     if (clear) return launch(k_lookup<Op, 1, true>, 1);
     bool full = false;
-    GJ_TRY(long_blocks(n, m, &full));
+    GJ_TRY(long_blocks(n, m, &full, kLookupLongKeys<Op>));
     return full ? launch(k_lookup<Op, Op::kLong>, Op::kLong) : launch(k_lookup<Op, 1>, 1);
 }
 
