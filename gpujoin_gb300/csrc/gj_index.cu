@@ -1016,7 +1016,7 @@ int gj_index_build(int type, const uint64_t* d_keys, const uint64_t* h_keys, uin
         case GJ_INDEX_HASH: rc = build_hash(idx.get(), s); break;
         case GJ_INDEX_NO_OP: break;
     }
-    if (rc == GJ_OK && type != GJ_INDEX_NO_OP && idx->in_hbm && n > partition_pairs_keys(type))
+    if (rc == GJ_OK && type != GJ_INDEX_NO_OP && type != GJ_INDEX_HASH && idx->in_hbm && n > partition_pairs_keys(type))
         rc = build_partition_start(idx.get(), s);
     if (rc == GJ_OK) {
         cudaError_t e = cudaStreamSynchronize(s);

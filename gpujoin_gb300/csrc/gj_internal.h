@@ -167,10 +167,10 @@ size_t pairs_workspace_bytes(uint64_t m);
 // where that is sooner and whose workspace has room beyond
 // pairs_workspace_bytes: *taken tells whether the call was.
 constexpr uint64_t kPartitionPairsMin = 1ull << 25, kPartitionPairsMax = 1ull << 29;  // probes
-// column keys above which such calls are made: kinds whose plain search reads
-// one random sector of a table or a spline's and a column's gain from fewer
-// (2^28 probes into 2^24 keys: hash table 5145, RadixSpline 5900, learned 5063
-// us plain, 4570 by partition; B+tree 4237)
+// column keys above which such calls are made (hash tables never): kinds whose
+// plain search reads a spline's or a leaf's and a column's sector gain from
+// fewer (2^28 probes into 2^24 keys: RadixSpline 5900, learned 5063 us plain,
+// 4570 by partition; B+tree 4237)
 inline uint64_t partition_pairs_keys(int type) {
     const bool tree = type == GJ_INDEX_BTREE || type == GJ_INDEX_HARMONIA || type == GJ_INDEX_BINARY_SEARCH;
     return tree ? 3ull << 23 : 3ull << 22;

@@ -987,9 +987,15 @@ int run_pairs(const Op& op, const stage_desc& sd, uint64_t n, const uint64_t* pr
         GJ_CUDA_TRY(cudaGetLastError());
         return (int)GJ_OK;
     };
+    // a short call ends with its longest chain of searches (100,000 probes into a
+    // RadixSpline of 2^26 keys 52 us with 8 a thread, 30 with 4)
+    if (unordered && m < (1ull << 22)) return single(k_pairs<Op, false, kFewItems>, kFewItems);
     if (unordered) return single(k_pairs<Op, false, kItems>, kItems);
-    // (stash null: host buffers)
-    if (!stash || n > kL2Keys || m < (1ull << 22)) return single(k_pairs<Op, true, kFewItems>, kFewItems);
+    // (stash null: host buffers; a hash table's one load a search leaves less to
+    // wait for: 10^8 probes into 2^26 keys with 4 / 8 a thread, uniform 2295 /
+    // 2304 us, Zipf(1.25) 726 / 655)
+    const bool far = n > kL2Keys && !std::is_same<Op, op_hash>::value;
+    if (!stash || far || m < (1ull << 22)) return single(k_pairs<Op, true, kFewItems>, kFewItems);
     return single(k_pairs<Op, true, kItems>, kItems);
 }
 

@@ -580,10 +580,14 @@ size_t pairs_partition_bytes(uint64_t m) {
 // which has 8 bytes a probe and is not written before the gather.  Columns
 // whose table windows take long searches are left to the plain pairs: at once
 // below 2^26 keys (2^25 clustered keys 5505 / 5955), where those searches
-// dwarf the rest above (2^26 clustered keys 8628 / 5972).  A hash table is one
-// random sector whatever the column, so only short searches beat it (50 M
-// probes into 2^24 / 2^26 / 2^28 uniform keys 988 / 921, 1163 / 1026 and 1243 /
-// 1328).  34 M probes are about where lognormal columns break even (2^25 keys
+// dwarf the rest above (2^26 clustered keys 8628 / 5972).  Skewed probes, which L1
+// and L2 serve, gain little from the partition or lose: hash tables, whose plain
+// search is one load, are never partitioned (10^8 Zipf(1.25) probes into 2^26
+// keys 655 / 1561), the learned index, whose leaves know clustered keys, only
+// where the table's searches are short (2^25 clustered keys 1061 / 2148).  For
+// trees over uniform keys both are level (1596 / 1562); over lognormal keys the
+// partition costs a tenth there (1634 / 1806) and saves a quarter at even
+// probes (2692 / 2013).  34 M probes are about where lognormal columns break even (2^25 keys
 // 754 / 752; 2^26 865 / 839, 24 M 629 / 622).
 int launch_pairs_by_partition(const gj_index* idx, const uint64_t* d_probes, uint64_t m, uint32_t* d_pairs,
                               uint64_t* d_count, void* ws, size_t ws_bytes, cudaStream_t s, bool* taken) {
@@ -591,8 +595,8 @@ int launch_pairs_by_partition(const gj_index* idx, const uint64_t* d_probes, uin
     if (m < kPartitionPairsMin || m > kPartitionPairsMax || idx->n <= partition_pairs_keys(idx->type) || !idx->in_hbm ||
         !idx->rel.pos || !idx->rel.col_aligned)
         return GJ_OK;
-    const double most = idx->type == GJ_INDEX_HASH ? 2.0 : idx->n < (1ull << 26) ? 2.5 : 4.0;
-    if (idx->rel_loads > most) return GJ_OK;
+    const double most = idx->type == GJ_INDEX_LEARNED || idx->n < (1ull << 26) ? 2.0 : 4.0;
+    if (idx->type == GJ_INDEX_HASH || idx->rel_loads > most) return GJ_OK;
     const uint32_t bits = std::min(default_radix_bits(idx->n), kPairsRadixBits);
     device_info di;
     GJ_TRY(current_device_info(&di));
