@@ -144,6 +144,7 @@ _SIGNATURES = {
     "gj_inlj_pairs_host_unordered": (_i32, [_vp, _vp, _u64, _vp, _vp, _vp, _sz, _vp]),
     "gj_inlj_pairs_noalloc": (_i32, [_vp, _vp, _u64, _vp, _vp, _vp]),
     "gj_partition_workspace_size": (_i32, [_u64, _u32, ctypes.POINTER(_sz)]),
+    "gj_debug_partition_bytes": (_i32, [_u64, _u32, _u32, ctypes.POINTER(_sz), ctypes.POINTER(_sz)]),
     "gj_index_key_range": (_i32, [_vp, ctypes.POINTER(_u64), ctypes.POINTER(_u64)]),
     "gj_index_lookup_cooperative": (_i32, [_vp, _vp, _u64, _vp, _u32, _vp]),
     "gj_partition_shift": (_i32, [_u64, _u64, _u32, ctypes.POINTER(_u32)]),

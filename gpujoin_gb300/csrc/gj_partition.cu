@@ -447,12 +447,18 @@ partition_plan plan_of(uint64_t m, uint32_t radix_bits, int sm_count, bool wide)
 
 uint64_t wide_from(int sm_count) { return 2ull * sm_count * kWideTile; }
 
+// The chunk rows of a plan's tables by the most its tiles can need: the chunk
+// count itself falls where a chunk takes one more tile, the most never does.
+uint32_t chunk_rows(const partition_plan& pl, int sm_count) {
+    return std::min(pl.tiles, (uint32_t)sm_count * kHistPerSM);
+}
+
 partition_plan plan_partition(uint64_t m, uint32_t radix_bits, int sm_count) {
     return plan_of(m, radix_bits, sm_count, radix_bits >= kWideRadixBits && m >= wide_from(sm_count));
 }
 
-size_t plan_bytes(const partition_plan& pl) {
-    return workspace_carver::need({(size_t)pl.tiles * pl.fanout * 4, (size_t)pl.chunks * pl.fanout * 4,
+size_t plan_bytes(const partition_plan& pl, uint32_t rows) {
+    return workspace_carver::need({(size_t)pl.tiles * pl.fanout * 4, (size_t)rows * pl.fanout * 4,
                                    (size_t)pl.fanout * 4, 4});
 }
 
@@ -480,12 +486,14 @@ int launch(Kernel kernel, uint32_t grid, int block, size_t smem, cudaStream_t s,
 
 }  // namespace
 
-// the workspace of a window of m keys also serves any shorter window
+// The workspace of a window of m keys also serves any shorter window: tiles
+// and chunk_rows only grow with m inside a tile size, and the windows of the
+// other size below m need at most what wide_from keys in small tiles do.
 size_t partition_ws_bytes(uint64_t m, uint32_t radix_bits, int sm_count) {
     if (m == 0) m = 1;
-    const size_t bytes = plan_bytes(plan_partition(m, radix_bits, sm_count));
-    const uint64_t narrow = std::min(m, wide_from(sm_count));
-    return std::max(bytes, plan_bytes(plan_of(narrow, radix_bits, sm_count, false)));
+    const partition_plan own = plan_partition(m, radix_bits, sm_count);
+    const partition_plan narrow = plan_of(std::min(m, wide_from(sm_count)), radix_bits, sm_count, false);
+    return std::max(plan_bytes(own, chunk_rows(own, sm_count)), plan_bytes(narrow, chunk_rows(narrow, sm_count)));
 }
 
 int range_partition_impl(const uint64_t* d_keys, uint64_t m, uint64_t min_key, uint32_t shift, uint32_t radix_bits,
@@ -673,6 +681,16 @@ int gj_partition_workspace_size(uint64_t m, uint32_t radix_bits, size_t* bytes) 
     device_info di;
     GJ_TRY(current_device_info(&di));
     *bytes = partition_ws_bytes(m, radix_bits, di.sm_count);
+    return GJ_OK;
+}
+
+int gj_debug_partition_bytes(uint64_t m, uint32_t radix_bits, uint32_t sm_count, size_t* reserved, size_t* used) {
+    GJ_CHECK_ARG(reserved && used, "gj_debug_partition_bytes: null argument");
+    GJ_CHECK_ARG(radix_bits >= 1 && radix_bits <= kMaxRadixBits, "gj_debug_partition_bytes: radix_bits not in [1, 12]");
+    GJ_CHECK_ARG(sm_count >= 1 && sm_count <= 1024, "gj_debug_partition_bytes: sm_count not in [1, 1024]");
+    const partition_plan pl = plan_partition(m ? m : 1, radix_bits, (int)sm_count);
+    *reserved = partition_ws_bytes(m, radix_bits, (int)sm_count);
+    *used = plan_bytes(pl, pl.chunks);
     return GJ_OK;
 }
 

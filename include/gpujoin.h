@@ -305,8 +305,13 @@ int gj_inlj_pairs_noalloc(const gj_index* index, const uint64_t* d_probes, uint6
  * partition 0.  Partitions follow each other in key order; inside a
  * partition the tuples of earlier probe chunks come first, the order within
  * one chunk is not fixed.  d_out_keys / d_out_rows hold m entries, d_offsets
- * 2^radix_bits + 1.  radix_bits in [1, 12]. */
+ * 2^radix_bits + 1.  radix_bits in [1, 12].  The workspace of m keys serves
+ * every call of fewer keys at the same fanout too. */
 int gj_partition_workspace_size(uint64_t m, uint32_t radix_bits, size_t* bytes);
+/* Test hook of that size, on the host alone: for a device of sm_count SMs,
+ * what gj_partition_workspace_size gives for m keys and what a call of exactly
+ * m keys carves out of its workspace. */
+int gj_debug_partition_bytes(uint64_t m, uint32_t radix_bits, uint32_t sm_count, size_t* reserved, size_t* used);
 /* The key range an index was built over (its column's first and last key),
  * from which its partitions are cut; no counterpart in the reference, whose
  * partitioning uses fixed key bits (src/index_lookup_new.cu:63-67). */

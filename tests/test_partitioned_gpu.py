@@ -7,6 +7,8 @@ keys, probes outside the key range, several windows, and the directory
 built per call or kept with the index.
 Positions must equal the oracle's per probe row, the pairs as a set (their
 order across tiles is not fixed)."""
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -151,3 +153,43 @@ def test_positions_through_the_inverse(orc, gj, cuda, radix_bits, m, window):
         ix = gj.make_index(kind, **params).construct(None, to_dev(torch, col)).prepare_partitioned()
         got, _, _ = ix.partitioned_inlj(to_dev(torch, pr), window_size=window, radix_bits=radix_bits)
         np.testing.assert_array_equal(from_dev_u32(got), expected(orc, kind, col, pr))
+
+
+@pytest.mark.parametrize("kind,window,m,bits,pairs", [("btree", 1_300_000, 2_500_000, 0, True),
+                                                      ("hash", 1_500_000, 2_700_000, 5, True),
+                                                      ("radix_spline", 5_000_000, 9_900_000, 0, False),
+                                                      ("btree", 2_600_000, 5_050_000, 11, True)])
+def test_uneven_windows(orc, gj, cuda, kind, window, m, bits, pairs):
+    # a last window a little shorter than the others, whose tiles form more
+    # chunks than a whole window's
+    import torch
+
+    rng = np.random.default_rng(m)
+    col = column(rng, 300_007)
+    pr = probes_for(rng, col, m)[:m]
+    ix = gj.make_index(kind).construct(None, to_dev(torch, col))
+    pos, prs, cnt = ix.partitioned_inlj(to_dev(torch, pr), window_size=window, radix_bits=bits, positions=True,
+                                        pairs=pairs)
+    exp = expected(orc, kind, col, pr)
+    np.testing.assert_array_equal(from_dev_u32(pos), exp)
+    if pairs:
+        erows, epos = orc.pairs_from_positions(exp)
+        a = prs[: 2 * int(cnt.item())].cpu().numpy().view(np.uint32).reshape(-1, 2)
+        a = a[np.argsort(a[:, 0], kind="stable")]
+        np.testing.assert_array_equal(a[:, 0], erows)
+        np.testing.assert_array_equal(a[:, 1], epos)
+
+
+@pytest.mark.parametrize("bits", [1, 5, 8, 9, 11, 12])
+def test_range_partition_with_a_larger_workspace(gj, cuda, bits):
+    # one workspace, sized for the largest batch, for batches of every size below
+    import torch
+
+    for most, m in ((1_300_000, 1_200_000), (2_600_000, 2_489_000), (5_000_000, 4_950_000)):
+        need = ctypes.c_size_t(0)
+        assert gj.lib().gj_partition_workspace_size(most, bits, ctypes.byref(need)) == 0
+        ws = torch.empty(need.value, dtype=torch.uint8, device="cuda")
+        keys = torch.arange(m, device="cuda", dtype=torch.int64) * 7 % m
+        rel = gj.range_partition(keys, 0, max(0, m.bit_length() - bits), bits, workspace=ws)
+        assert torch.equal(keys[rel.rows.to(torch.int64)], rel.keys)
+        assert torch.equal(torch.sort(rel.rows.to(torch.int64))[0], torch.arange(m, device="cuda"))
