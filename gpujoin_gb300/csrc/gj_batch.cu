@@ -295,10 +295,17 @@ int plan_layout(gj_batch_plan* pl, uint32_t items, cudaStream_t s) {
         return GJ_ERR_TOO_LARGE;
     }
     if (tiles > pl->tile_map_capacity) {
+        uint32_t* map = nullptr;
+        GJ_TRY(plan_alloc(&map, tiles));  // the plan keeps its layout where this fails
         cudaFree(pl->d_tile_batch);
-        pl->d_tile_batch = nullptr;
-        GJ_TRY(plan_alloc(&pl->d_tile_batch, tiles));
+        pl->d_tile_batch = map;
         pl->tile_map_capacity = tiles;
+    }
+    // a captured run launches with the layout it was captured from: its tile
+    // map, tile count and grid
+    if (pl->exec) {
+        cudaGraphExecDestroy(pl->exec);
+        pl->exec = nullptr;
     }
     GJ_CUDA_TRY(cudaMemcpyAsync(pl->d_batches, descs.data(), descs.size() * sizeof(batch_desc), cudaMemcpyHostToDevice,
                                 s));

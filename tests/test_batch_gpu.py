@@ -92,3 +92,28 @@ def test_batch_plan_arguments(gj, cuda):
     assert gj.lib().gj_batch_plan_free(None) == 0
     assert gj.lib().gj_batch_plan_run(None, None, None, 0, None, None) == 1
     del ctypes
+
+
+@pytest.mark.parametrize("mode", [0, 1])
+def test_batch_graph_after_autotune(orc, gj, cuda, mode):
+    # a run captured before autotune, which lays the plan's tiles out anew
+    # (in another tile map, as small tiles need a larger one), asked for again
+    # with the same buffers
+    import torch
+
+    rng = np.random.default_rng(7)
+    keys = gj.generate_sorted_keys(1 << 16, 0, 1 << 63, seed=3)
+    ix = gj.make_index("btree").construct(None, keys)
+    sizes = rng.integers(1, 60_000, 40).astype(np.uint64)
+    offs = np.concatenate([[0], np.cumsum(sizes)[:-1]]).astype(np.uint64)
+    probes = gj.generate_probes(keys, int(sizes.sum()), theta=0.5, absent_fraction=0.1, seed=4)
+    exp = orc.exact_lookup(keys.cpu().numpy().view(np.uint64), probes.cpu().numpy().view(np.uint64))
+    plan = gj.batch_plan([ix], np.zeros(40, dtype=np.uint32), offs, sizes)
+    out = torch.empty(probes.numel(), dtype=torch.int32, device="cuda")
+    for _ in range(3):
+        out.fill_(-7)
+        plan.run_graph(probes, out, mode)
+        torch.cuda.synchronize()
+        np.testing.assert_array_equal(from_dev_u32(out), exp)
+        plan.autotune(probes, out)
+    plan.free()
