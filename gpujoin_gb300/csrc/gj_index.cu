@@ -753,19 +753,16 @@ int build_radix_spline_index(gj_index* idx, const uint64_t* h_keys, cudaStream_t
     // points with the slope of their segment (the estimate's division, done once)
     std::vector<rs_point> pts(rs.sx.size());
     for (size_t i = 0; i < pts.size(); ++i) {
-        pts[i].x = rs.sx[i];
-        pts[i].y = rs.sy[i];
-        pts[i].slope = i + 1 < pts.size() ? (rs.sy[i + 1] - rs.sy[i]) / (double)(rs.sx[i + 1] - rs.sx[i]) : 0.0;
-        pts[i].step = 0;
+        pts[i] = rs_point{rs.sx[i], rs.sy[i], 0, 0};
         if (i + 1 < pts.size()) {
-            const uint64_t dx = rs.sx[i + 1] - rs.sx[i];
-            const uint32_t sh = (uint32_t)__builtin_clzll(dx);
-            const unsigned __int128 dy = (unsigned __int128)(uint64_t)(rs.sy[i + 1] - rs.sy[i]);
-            const float rate = (float)(pts[i].slope * 0.25);
+            const uint64_t dx = rs.sx[i + 1] - rs.sx[i], dy = (uint64_t)(rs.sy[i + 1] - rs.sy[i]);
+            // 1 <= dy <= dx, so the quotient is below 2^64
+            const uint32_t sh = (uint32_t)__builtin_clzll(dx), up = (uint32_t)__builtin_clzll(dy) - 1;
+            const float rate = (float)((double)dy / (double)dx * 0.25);
             uint32_t bits = 0;
             std::memcpy(&bits, &rate, sizeof(bits));
-            // dy <= dx: the quotient is at most 2^34 - 1 wide
-            pts[i].step = (uint64_t)(bits >> 8) << 40 | (uint64_t)((dy << 64) / (dx << sh)) << 6 | sh;
+            pts[i].slope = (uint64_t)(((unsigned __int128)(dy << up) << 64) / (dx << sh));
+            pts[i].code = (uint64_t)bits << 32 | up << 6 | sh;
         }
     }
     void *pt = nullptr, *pp = nullptr;

@@ -1036,15 +1036,15 @@ GJ_DEVICE_INLINE uint32_t harmonia_lookup_cooperative(bool active, const harmoni
 // RadixSpline (src/rs.cuh:118-154, window src/indexes.cuh:205-215)
 // ---------------------------------------------------------------------------
 // A spline point (src/rs.cuh:22-52: Coord{x, y}) with the slope of the
-// segment to the next point, computed at build with the same double
-// division the estimate would make, and once more in fixed point: one 32-byte
-// sector, one load per segment.
+// segment to the next point: one 32-byte sector, one load per segment.  The
+// slope is kept in fixed point with at least 62 significant bits, more than
+// the double quotient of the reference's estimate has.
 struct rs_point {
     uint64_t x;
-    double y;      // a position: a whole number below 2^32
-    double slope;  // (y[i+1] - y[i]) / (x[i+1] - x[i]); 0 for the last point
-    uint64_t step; // shift | floor(dy * 2^64 / (dx << shift)) << 6, dx << shift in [2^63, 2^64), and from
-                   // bit 40 on the upper 24 bits of dy / dx / 4 as a float (sectors per unit of key)
+    double y;        // a position: a whole number below 2^32
+    uint64_t slope;  // floor(dy * 2^(64 + t) / (dx << s)); dx << s in [2^63, 2^64), dy << t in [2^62, 2^63);
+                     // 0 for the last point
+    uint64_t code;   // s | t << 6 | the float dy / dx / 4 (sectors per unit of key) << 32
 };
 static_assert(sizeof(rs_point) == 32, "a spline point is one sector");
 
@@ -1067,9 +1067,9 @@ GJ_DEVICE_INLINE uint32_t whole_of_double(uint64_t bits) {
     return e < 1023u ? 0u : (uint32_t)(((bits & ((1ull << 52) - 1)) | (1ull << 52)) >> (1075u - e));
 }
 
-// The spline's estimate of a key's position, rounded down and at most two
-// below the real value: y + (key - x) * slope in 64-bit fixed point.  *rate:
-// the segment's sectors per unit of key.
+// The spline's estimate of a key's position: y + (key - x) * slope rounded
+// down, in 64-bit fixed point (less than 2^-30 of a position is lost before the
+// rounding).  *rate: the segment's sectors per unit of key.
 GJ_DEVICE_INLINE uint32_t rs_estimate(const rs_view& v, uint64_t key, float* rate) {
     *rate = 0.f;
     if (key <= v.min_key) return 0;
@@ -1094,8 +1094,9 @@ GJ_DEVICE_INLINE uint32_t rs_estimate(const rs_view& v, uint64_t key, float* rat
     }
     // segment [lo - 1, lo]: its left point and precomputed slope
     if (have != lo - 1) ld_sector(reinterpret_cast<const uint64_t*>(v.pts + lo - 1), w);
-    *rate = __uint_as_float((uint32_t)(w[3] >> 40) << 8);
-    return whole_of_double(w[1]) + (uint32_t)__umul64hi((key - w[0]) << (w[3] & 63u), (w[3] >> 6) & ((1ull << 34) - 1));
+    *rate = __uint_as_float((uint32_t)(w[3] >> 32));
+    const uint32_t code = (uint32_t)w[3];
+    return whole_of_double(w[1]) + (uint32_t)(__umul64hi((key - w[0]) << (code & 63u), w[2]) >> ((code >> 6) & 63u));
 }
 
 // lower bound expected inside [b, e) and near `guess`, widened to the whole
@@ -1133,9 +1134,10 @@ template <bool kScattered = true>
 GJ_DEVICE_INLINE uint32_t rs_lookup(const rs_view& v, uint64_t key) {
     float rate;
     const uint64_t est = rs_estimate(v, key, &rate), err = v.max_error;
-    // the real estimate lies in [est, est + 2]
+    // the real estimate lies less than 1 + 2^-30 above est, and the reference
+    // searches [estimate - err, estimate + err + 2) (src/indexes.cuh:207-214)
     const uint64_t b = est < err ? 0 : est - err;
-    const uint64_t e = est + err + 4 > v.n ? v.n : est + err + 4;
+    const uint64_t e = est + err + 3 > v.n ? v.n : est + err + 3;
     const uint64_t pos = window_lower_bound<kScattered, 17>(v.col, v.n, b, e, est, rate, key, v.col_aligned);
     return pos < v.n ? (uint32_t)pos : kInvalid;
 }
