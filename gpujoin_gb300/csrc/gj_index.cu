@@ -434,6 +434,21 @@ int build_key_start(gj_index* idx, uint32_t bits, cudaStream_t s, spare_memory&&
     return GJ_OK;
 }
 
+void drop_start(gj_index* idx, const key_start& t) {
+    void* p = const_cast<uint32_t*>(t.pos);
+    idx->allocations.erase(std::find(idx->allocations.begin(), idx->allocations.end(), p));
+    idx->bytes -= key_start_entries(t.range, t.shift) * sizeof(uint32_t);
+    cudaFree(p);
+}
+
+// a table for ordered pairs (idx->rel) that no call of the index can take
+void drop_unread_start(gj_index* idx) {
+    if (!idx->rel.pos || partitions_pairs(idx)) return;
+    if (idx->rel.pos != idx->ks.pos) drop_start(idx, idx->rel);
+    idx->rel = key_start{};
+    idx->rel_loads = 0.0;
+}
+
 // The table large ordered-pairs calls search through (idx->rel), whatever the
 // kind.  A partition's probes share its slice of the table in L2, so above
 // 2^24 keys it is finer than a scattered lookup's: two to four keys a bucket,
@@ -460,11 +475,7 @@ int build_partition_start(gj_index* idx, cudaStream_t s) {
         idx->rel_loads = coarse_loads;
     }
     const key_start& out = keep ? coarse : fine;  // no longer searched for pairs
-    if (idx->ks.pos == out.pos) return GJ_OK;
-    void* p = const_cast<uint32_t*>(out.pos);
-    idx->allocations.erase(std::find(idx->allocations.begin(), idx->allocations.end(), p));
-    idx->bytes -= key_start_entries(out.range, out.shift) * sizeof(uint32_t);
-    GJ_CUDA_TRY(cudaFree(p));
+    if (idx->ks.pos != out.pos) drop_start(idx, out);
     return GJ_OK;
 }
 
@@ -537,15 +548,18 @@ int build_btree(gj_index* idx, cudaStream_t s) {
     // lies behind the host link: the tree reads one sector of it a lookup, the
     // table's search 1.3 (2^24 keys in host memory, 2^24 probes: 3707 / 4882 us)
     const bool candidate = W == kBtreeCompressed16 && L == 4 && idx->params.btree_start_bits == 0 && idx->in_hbm;
-    spare_memory spare;
+    spare_memory spare, encoding;
     const uint64_t min_key = idx->min_key, maxk = idx->max_key;
     if (compressed) {
         // top down: a node's base comes from its parent's encoding
         uint64_t* bases[2] = {nullptr, nullptr};
-        // the room of the key start table, when one follows
-        GJ_TRY(spare.take(std::max<size_t>(2 * nodes[1] * sizeof(uint64_t),
-                                           candidate ? key_start_bytes(idx, key_start_bits(n)) : 0)));
-        bases[0] = static_cast<uint64_t*>(spare.p);
+        // in the room of the key start table, when one follows that is not
+        // smaller (columns above 2^26 keys: the table takes memory of its own)
+        const size_t scratch = 2 * nodes[1] * sizeof(uint64_t);
+        const size_t table = candidate ? key_start_bytes(idx, key_start_bits(n)) : 0;
+        spare_memory& room = table >= scratch ? spare : encoding;
+        GJ_TRY(room.take(std::max(scratch, table >= scratch ? table : size_t(0))));
+        bases[0] = static_cast<uint64_t*>(room.p);
         bases[1] = bases[0] + nodes[1];
         int rc = GJ_OK;
         for (uint32_t l = height; l >= 1 && rc == GJ_OK; --l) {
@@ -1013,8 +1027,8 @@ int gj_index_build(int type, const uint64_t* d_keys, const uint64_t* h_keys, uin
         case GJ_INDEX_HASH: rc = build_hash(idx.get(), s); break;
         case GJ_INDEX_NO_OP: break;
     }
-    if (rc == GJ_OK && type != GJ_INDEX_NO_OP && type != GJ_INDEX_HASH && idx->in_hbm && n > partition_pairs_keys(type))
-        rc = build_partition_start(idx.get(), s);
+    if (rc == GJ_OK && may_partition_pairs(idx.get())) rc = build_partition_start(idx.get(), s);
+    if (rc == GJ_OK) drop_unread_start(idx.get());
     if (rc == GJ_OK) {
         cudaError_t e = cudaStreamSynchronize(s);
         if (e != cudaSuccess) {

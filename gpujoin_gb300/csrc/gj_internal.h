@@ -176,6 +176,11 @@ inline uint64_t partition_pairs_keys(int type) {
     return tree ? 3ull << 23 : 3ull << 22;
 }
 size_t pairs_partition_bytes(uint64_t m);
+// whether a call of an index can be made so: by its column and kind alone
+// (hash tables, whose plain search is one load, never are), and with the table
+// its build found
+bool may_partition_pairs(const gj_index* idx);
+bool partitions_pairs(const gj_index* idx);
 int launch_pairs_by_partition(const gj_index* idx, const uint64_t* d_probes, uint64_t m, uint32_t* d_pairs,
                               uint64_t* d_count, void* ws, size_t ws_bytes, cudaStream_t s, bool* taken);
 // launch_pairs for the test of the bounded waits: look-backs give up after

@@ -597,14 +597,20 @@ size_t pairs_partition_bytes(uint64_t m) {
 // partition costs a tenth there (1634 / 1806) and saves a quarter at even
 // probes (2692 / 2013).  34 M probes are about where lognormal columns break even (2^25 keys
 // 754 / 752; 2^26 865 / 839, 24 M 629 / 622).
+bool may_partition_pairs(const gj_index* idx) {
+    return idx->type != GJ_INDEX_NO_OP && idx->type != GJ_INDEX_HASH && idx->in_hbm &&
+           (reinterpret_cast<uintptr_t>(idx->d_col) & 31) == 0 && idx->n > partition_pairs_keys(idx->type);
+}
+
+bool partitions_pairs(const gj_index* idx) {
+    const double most = idx->type == GJ_INDEX_LEARNED || idx->n < (1ull << 26) ? 2.0 : 4.0;
+    return may_partition_pairs(idx) && idx->rel.pos && idx->rel_loads <= most;
+}
+
 int launch_pairs_by_partition(const gj_index* idx, const uint64_t* d_probes, uint64_t m, uint32_t* d_pairs,
                               uint64_t* d_count, void* ws, size_t ws_bytes, cudaStream_t s, bool* taken) {
     *taken = false;
-    if (m < kPartitionPairsMin || m > kPartitionPairsMax || idx->n <= partition_pairs_keys(idx->type) || !idx->in_hbm ||
-        !idx->rel.pos || !idx->rel.col_aligned)
-        return GJ_OK;
-    const double most = idx->type == GJ_INDEX_LEARNED || idx->n < (1ull << 26) ? 2.0 : 4.0;
-    if (idx->type == GJ_INDEX_HASH || idx->rel_loads > most) return GJ_OK;
+    if (m < kPartitionPairsMin || m > kPartitionPairsMax || !partitions_pairs(idx)) return GJ_OK;
     const uint32_t bits = std::min(default_radix_bits(idx->n), kPairsRadixBits);
     device_info di;
     GJ_TRY(current_device_info(&di));
@@ -634,8 +640,7 @@ int launch_pairs_by_partition(const gj_index* idx, const uint64_t* d_probes, uin
     GJ_TRY(range_partition_impl(d_probes, m, idx->min_key, shift_for(idx->min_key, idx->max_key, bits), bits, 0, keys,
                                 nullptr, nullptr, sc.tables, sc.table_bytes, s, &iv));
     const uint32_t blocks = (uint32_t)((m + kBlock - 1) / kBlock);
-    const bool exact =
-        idx->type == GJ_INDEX_BTREE || idx->type == GJ_INDEX_HARMONIA || idx->type == GJ_INDEX_HASH;
+    const bool exact = idx->type == GJ_INDEX_BTREE || idx->type == GJ_INDEX_HARMONIA;
     GJ_TRY(launch(exact ? k_relation_values<true> : k_relation_values<false>, blocks, kBlock, 0, s, idx->rel, idx->d_col,
                   (uint32_t)idx->n, static_cast<const uint64_t*>(keys), m, sc.values));
     const size_t smem = (size_t)pl.fanout * 4 + ((size_t)pl.fanout + 2) * 2 + kGatherTile * 2;
