@@ -124,6 +124,7 @@ _SIGNATURES = {
     "gj_parse_index_type": (_i32, [ctypes.c_char_p, ctypes.POINTER(_i32)]),
     "gj_index_type_name": (ctypes.c_char_p, [_i32]),
     "gj_index_build": (_i32, [_i32, _vp, _vp, _u64, ctypes.POINTER(gj_index_params), _vp, ctypes.POINTER(_vp)]),
+    "gj_debug_start_tables": (_u64, [_sz]),
     "gj_index_free": (_i32, [_vp]),
     "gj_index_memory_consumption": (_u64, [_vp]),
     "gj_index_host_memory": (_u64, [_vp]),

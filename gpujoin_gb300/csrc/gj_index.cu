@@ -362,6 +362,10 @@ uint32_t key_start_bits(uint64_t n) {
     return b;
 }
 
+// gj_debug_start_tables
+thread_local size_t g_table_limit = SIZE_MAX;
+thread_local uint64_t g_tables_taken = 0;
+
 // device memory that is freed unless it is handed on
 struct spare_memory {
     void* p = nullptr;
@@ -372,8 +376,18 @@ struct spare_memory {
         const cudaError_t e = cudaMalloc(&p, bytes);
         if (e == cudaSuccess) return GJ_OK;
         p = nullptr;
+        cudaGetLastError();  // the caller may go on without this memory
         set_error("cudaMalloc(%zu) failed: %s", bytes, cudaGetErrorString(e));
         return e == cudaErrorMemoryAllocation ? GJ_ERR_OUT_OF_MEMORY : GJ_ERR_CUDA;
+    }
+    int take_table(size_t bytes) {
+        if (bytes > g_table_limit) {
+            set_error("key start table of %zu bytes: no memory (gj_debug_start_tables)", bytes);
+            return GJ_ERR_OUT_OF_MEMORY;
+        }
+        GJ_TRY(take(bytes));
+        ++g_tables_taken;
+        return GJ_OK;
     }
     void* release() {
         void* q = p;
@@ -398,7 +412,8 @@ size_t key_start_bytes(const gj_index* idx, uint32_t bits) {
 // Key start table of 2^bits buckets (fewer for a narrow key range); use(loads,
 // level) decides from the sampled cost of its searches -- mean column sectors
 // read, and for a B+tree the mean level its lookups start at -- whether the
-// index's scattered lookups go through it.
+// index's scattered lookups go through it.  The index works without its table,
+// only slower: a device too full for one is no error.
 template <class Use>
 int build_key_start(gj_index* idx, uint32_t bits, cudaStream_t s, spare_memory&& spare, Use&& use,
                     const key_start* guide = nullptr) {
@@ -411,7 +426,10 @@ int build_key_start(gj_index* idx, uint32_t bits, cudaStream_t s, spare_memory&&
     t.col_aligned = aligned32(idx->d_col);
     const uint32_t buckets = (uint32_t)(range >> t.shift) + 1;
     const uint32_t entries = (uint32_t)key_start_entries(range, t.shift);
-    if (!spare.p) GJ_TRY(spare.take(key_start_bytes(idx, bits)));
+    if (!spare.p) {
+        const int rc = spare.take_table(key_start_bytes(idx, bits));
+        if (rc != GJ_OK) return rc == GJ_ERR_OUT_OF_MEMORY ? GJ_OK : rc;
+    }
     uint32_t* pos = static_cast<uint32_t*>(spare.p);
     unsigned long long* d_sums = reinterpret_cast<unsigned long long*>(pos + entries);
     unsigned long long sums[kStartSums] = {};
@@ -466,9 +484,10 @@ int build_partition_start(gj_index* idx, cudaStream_t s) {
     while (bits < 25 && (2ull << bits) < n) ++bits;
     const key_start coarse = idx->rel;
     const double coarse_loads = idx->rel_loads;
-    if (n <= kStartPackedKeys || coarse.shift <= key_start_shift(coarse.range, bits)) return GJ_OK;
+    if (!coarse.pos || n <= kStartPackedKeys || coarse.shift <= key_start_shift(coarse.range, bits)) return GJ_OK;
     GJ_TRY(build_key_start(idx, bits, s, spare_memory(), [](double, double) { return false; }, &coarse));
     const key_start fine = idx->rel;
+    if (fine.pos == coarse.pos) return GJ_OK;  // no memory for the finer one
     const bool keep = idx->rel_loads < 0.95 * coarse_loads;
     if (!keep) {
         idx->rel = coarse;
@@ -476,6 +495,12 @@ int build_partition_start(gj_index* idx, cudaStream_t s) {
     }
     const key_start& out = keep ? coarse : fine;  // no longer searched for pairs
     if (idx->ks.pos != out.pos) drop_start(idx, out);
+    return GJ_OK;
+}
+
+int finish_pairs_table(gj_index* idx, cudaStream_t s) {
+    if (may_partition_pairs(idx)) GJ_TRY(build_partition_start(idx, s));
+    drop_unread_start(idx);
     return GJ_OK;
 }
 
@@ -557,9 +582,9 @@ int build_btree(gj_index* idx, cudaStream_t s) {
         // smaller (columns above 2^26 keys: the table takes memory of its own)
         const size_t scratch = 2 * nodes[1] * sizeof(uint64_t);
         const size_t table = candidate ? key_start_bytes(idx, key_start_bits(n)) : 0;
-        spare_memory& room = table >= scratch ? spare : encoding;
-        GJ_TRY(room.take(std::max(scratch, table >= scratch ? table : size_t(0))));
-        bases[0] = static_cast<uint64_t*>(room.p);
+        if (table >= scratch && spare.take_table(table) != GJ_OK) spare.p = nullptr;
+        if (!spare.p) GJ_TRY(encoding.take(scratch));
+        bases[0] = static_cast<uint64_t*>(spare.p ? spare.p : encoding.p);
         bases[1] = bases[0] + nodes[1];
         int rc = GJ_OK;
         for (uint32_t l = height; l >= 1 && rc == GJ_OK; --l) {
@@ -666,8 +691,7 @@ int build_btree(gj_index* idx, cudaStream_t s) {
         GJ_TRY(build_key_start(idx, key_start_bits(n), s, std::move(spare), [&](double loads, double level) {
             return loads <= 4.0 && (n <= (1ull << 24) || level >= 3.0);
         }));
-    else
-        GJ_CUDA_TRY(cudaStreamSynchronize(s));  // before the scratch is freed
+    GJ_CUDA_TRY(cudaStreamSynchronize(s));  // before the scratch is freed
     return GJ_OK;
 }
 
@@ -924,8 +948,9 @@ const char* gj_index_type_name(int type) {
     }
 }
 
-int gj_index_build(int type, const uint64_t* d_keys, const uint64_t* h_keys, uint64_t n,
-                   const gj_index_params* params, void* stream, gj_index** out_index) {
+// (pairs_table: with the key start table of its large ordered-pairs calls)
+static int build_index(int type, const uint64_t* d_keys, const uint64_t* h_keys, uint64_t n,
+                       const gj_index_params* params, bool pairs_table, void* stream, gj_index** out_index) {
     GJ_CHECK_ARG(out_index, "gj_index_build: out_index is null");
     *out_index = nullptr;
     GJ_CHECK_ARG(gj_index_type_name(type) != nullptr, "gj_index_build: unknown index type");
@@ -963,7 +988,7 @@ int gj_index_build(int type, const uint64_t* d_keys, const uint64_t* h_keys, uin
             gj_index_params pc = p;
             pc.learned_root = roots[i];
             if (widths[i]) pc.learned_hidden = widths[i];
-            const int rc = gj_index_build(type, d_keys, h_keys, n, &pc, stream, &cand[i]);
+            const int rc = build_index(type, d_keys, h_keys, n, &pc, false, stream, &cand[i]);
             if (rc != GJ_OK) {
                 for (gj_index* c : cand) gj_index_free(c);
                 return rc;
@@ -980,6 +1005,12 @@ int gj_index_build(int type, const uint64_t* d_keys, const uint64_t* h_keys, uin
         }
         for (int i = 0; i < kCand; ++i)
             if (i != keep) gj_index_free(cand[i]);
+        // the table depends on the column alone: one for the root that is kept
+        const int rc = finish_pairs_table(cand[keep], s);
+        if (rc != GJ_OK) {
+            gj_index_free(cand[keep]);
+            return rc;
+        }
         *out_index = cand[keep];
         return GJ_OK;
     }
@@ -1027,8 +1058,7 @@ int gj_index_build(int type, const uint64_t* d_keys, const uint64_t* h_keys, uin
         case GJ_INDEX_HASH: rc = build_hash(idx.get(), s); break;
         case GJ_INDEX_NO_OP: break;
     }
-    if (rc == GJ_OK && may_partition_pairs(idx.get())) rc = build_partition_start(idx.get(), s);
-    if (rc == GJ_OK) drop_unread_start(idx.get());
+    if (rc == GJ_OK && pairs_table) rc = finish_pairs_table(idx.get(), s);
     if (rc == GJ_OK) {
         cudaError_t e = cudaStreamSynchronize(s);
         if (e != cudaSuccess) {
@@ -1043,6 +1073,18 @@ int gj_index_build(int type, const uint64_t* d_keys, const uint64_t* h_keys, uin
     }
     *out_index = idx.release();
     return GJ_OK;
+}
+
+int gj_index_build(int type, const uint64_t* d_keys, const uint64_t* h_keys, uint64_t n,
+                   const gj_index_params* params, void* stream, gj_index** out_index) {
+    return build_index(type, d_keys, h_keys, n, params, true, stream, out_index);
+}
+
+uint64_t gj_debug_start_tables(size_t max_bytes) {
+    g_table_limit = max_bytes;
+    const uint64_t taken = g_tables_taken;
+    g_tables_taken = 0;
+    return taken;
 }
 
 int gj_index_free(gj_index* index) {

@@ -130,6 +130,11 @@ const char* gj_index_type_name(int type);
  * (GJ_ERR_UNSORTED).  Synchronous: returns when the index is usable. */
 int gj_index_build(int type, const uint64_t* d_keys, const uint64_t* h_keys, uint64_t n,
                    const gj_index_params* params, void* stream, gj_index** out_index);
+/* Test hook of the builds' optional tables, with no counterpart in the
+ * reference: from now on, on the calling thread, a key start table of more than
+ * max_bytes finds no memory, as on a full device (SIZE_MAX: no limit).  Returns
+ * how many tables the thread's builds have allocated since the last call. */
+uint64_t gj_debug_start_tables(size_t max_bytes);
 int gj_index_free(gj_index* index);
 /* abstract_index::memory_consumption (src/indexes.cuh:38) in bytes */
 uint64_t gj_index_memory_consumption(const gj_index* index);
