@@ -136,6 +136,7 @@ _SIGNATURES = {
     "gj_index_device_view": (_i32, [_vp, _vp, _sz]),
     "gj_index_lookup": (_i32, [_vp, _vp, _u64, _vp, _vp]),
     "gj_inlj_pairs_workspace_size": (_i32, [_u64, ctypes.POINTER(_sz)]),
+    "gj_index_inlj_pairs_workspace_size": (_i32, [_vp, _u64, ctypes.POINTER(_sz)]),
     "gj_inlj_pairs": (_i32, [_vp, _vp, _u64, _vp, _vp, _vp, _sz, _vp]),
     "gj_inlj_pairs_unordered": (_i32, [_vp, _vp, _u64, _vp, _vp, _vp, _sz, _vp]),
     "gj_inlj_pairs_status": (_i32, [_vp, _sz, _u64, _vp]),
@@ -371,9 +372,18 @@ class abstract_index:
             out_count = _empty(1, torch.int64, dev)
         if workspace is None:
             need = _sz(0)
-            size = lib().gj_inlj_pairs_workspace_size if ordered else lib().gj_inlj_pairs_host_workspace_size
-            _check(size(m, ctypes.byref(need)))
-            workspace = _workspace(need.value, dev)
+            if ordered:
+                _check(lib().gj_index_inlj_pairs_workspace_size(self.handle, m, ctypes.byref(need)))
+            else:
+                _check(lib().gj_inlj_pairs_host_workspace_size(m, ctypes.byref(need)))
+            try:
+                workspace = _workspace(need.value, dev)
+            except torch.cuda.OutOfMemoryError:
+                offered = need.value
+                _check(lib().gj_inlj_pairs_host_workspace_size(m, ctypes.byref(need)))
+                if need.value >= offered:
+                    raise
+                workspace = _workspace(need.value, dev)  # no room to partition: slower, the same pairs
         fn = lib().gj_inlj_pairs if ordered else lib().gj_inlj_pairs_unordered
         _check(fn(self.handle, _ptr(d_probes), m, _ptr(out_pairs), _ptr(out_count), _ptr(workspace),
                   workspace.numel(), _stream(stream)))

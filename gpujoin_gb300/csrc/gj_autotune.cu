@@ -155,7 +155,7 @@ int gj_autotune_ordering(const gj_index* index, const uint64_t* d_probes, uint64
     GJ_CHECK_ARG(m > 0 && d_probes, "gj_autotune_ordering: no probes");
     cudaStream_t s = as_stream(stream);
     size_t ws_bytes = 0;
-    GJ_TRY(gj_inlj_pairs_workspace_size(m, &ws_bytes));
+    GJ_TRY(gj_index_inlj_pairs_workspace_size(index, m, &ws_bytes));
     device_buffer ws, pairs, count;
     GJ_TRY(ws.alloc(ws_bytes));
     GJ_TRY(pairs.alloc(2 * m * sizeof(uint32_t)));

@@ -1200,6 +1200,12 @@ int gj_inlj_pairs_workspace_size(uint64_t m, size_t* bytes) {
     return GJ_OK;
 }
 
+int gj_index_inlj_pairs_workspace_size(const gj_index* index, uint64_t m, size_t* bytes) {
+    GJ_CHECK_ARG(index && bytes, "gj_index_inlj_pairs_workspace_size: null argument");
+    *bytes = pairs_workspace_bytes(m) + (partitions_pairs(index) ? pairs_partition_bytes(m) : 0);
+    return GJ_OK;
+}
+
 int gj_inlj_pairs(const gj_index* index, const uint64_t* d_probes, uint64_t m, uint32_t* d_pairs, uint64_t* d_count,
                   void* d_workspace, size_t workspace_bytes, void* stream) {
     GJ_CHECK_ARG(index && d_count, "gj_inlj_pairs: null argument");

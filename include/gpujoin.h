@@ -184,8 +184,11 @@ int gj_index_lookup(const gj_index* index, const uint64_t* d_probes, uint64_t m,
  * d_pairs must hold 2*m uint32.  Workspace: gj_inlj_pairs_workspace_size,
  * which from 2^25 to 2^29 probes includes room (about 6.2 bytes a probe)
  * with which calls into columns far larger than L2 partition their probes
- * first; gj_inlj_pairs_host_workspace_size bytes serve every call without. */
+ * first; gj_index_inlj_pairs_workspace_size leaves that room out for an index
+ * whose calls never do, and gj_inlj_pairs_host_workspace_size bytes serve every
+ * call without. */
 int gj_inlj_pairs_workspace_size(uint64_t m, size_t* bytes);
+int gj_index_inlj_pairs_workspace_size(const gj_index* index, uint64_t m, size_t* bytes);
 int gj_inlj_pairs(const gj_index* index, const uint64_t* d_probes, uint64_t m, uint32_t* d_pairs,
                   uint64_t* d_count, void* d_workspace, size_t workspace_bytes, void* stream);
 /* gj_inlj_pairs in one pass with each tile's pairs placed by one atomicAdd

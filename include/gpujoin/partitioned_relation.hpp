@@ -297,7 +297,7 @@ void inlj_pairs_by_approach(const Index& index, const uint64_t* d_probes, size_t
             gj_partitioned_inlj(ix, d_probes, m, w, 0, nullptr, d_pairs, d_count, ws.data(), need, stream));
     } else {
         size_t need = 0;
-        gj::detail::check_rc(gj_inlj_pairs_workspace_size(m, &need));
+        gj::detail::check_rc(gj_index_inlj_pairs_workspace_size(ix, m, &need));
         device_array_wrapper<unsigned char> ws(need);
         gj::detail::check_rc(order == GJ_ORDER_SORTED_TILES
                                  ? gj_inlj_pairs_sorted(ix, d_probes, m, d_pairs, d_count, ws.data(), need, stream)

@@ -343,3 +343,47 @@ def test_pairs_by_partition_start_tables(gj, cuda, kind, column):
     got = pairs[: 2 * int(count)].view(-1, 2)
     assert torch.equal(got[:, 0].to(torch.int64), rows)
     assert torch.equal(got[:, 1], pos[rows])
+
+
+@pytest.mark.parametrize("kind,n", [("hash", 1 << 25), ("btree", 1 << 20), ("btree", 20_000_000)])
+def test_pairs_workspace_without_a_partition(gj, cuda, kind, n):
+    # an index whose pairs are never partitioned: large calls take no room for it
+    import torch
+
+    m = (1 << 25) + 3
+    keys = gj.generate_sorted_keys(n, gj.DIST_UNIFORM, 1 << 63, seed=5)
+    ix = gj.make_index(kind).construct(None, keys)
+    least, need = ctypes.c_size_t(0), ctypes.c_size_t(0)
+    gj.lib().gj_inlj_pairs_host_workspace_size(m, ctypes.byref(least))
+    assert gj.lib().gj_index_inlj_pairs_workspace_size(ix.handle, m, ctypes.byref(need)) == 0
+    assert need.value == least.value
+    probes = gj.generate_probes(keys, m, theta=0.5, seed=6)
+    out, count = torch.empty(2 * m, dtype=torch.int32, device="cuda"), torch.empty(1, dtype=torch.int64, device="cuda")
+    torch.cuda.reset_peak_memory_stats()
+    before = torch.cuda.memory_allocated()
+    ix.inlj_pairs(probes, out, count)
+    assert torch.cuda.max_memory_allocated() - before < least.value + (4 << 20)
+    assert int(count) == m
+
+
+def test_pairs_with_little_memory(gj, cuda, monkeypatch):
+    # no memory for the room to partition: the pairs come without it
+    import torch
+
+    n, m = (1 << 25) + 64, (1 << 25) + 3
+    keys = gj.generate_sorted_keys(n, gj.DIST_UNIFORM, 1 << 63, seed=5)
+    ix = gj.btree_index().construct(None, keys)
+    probes = gj.generate_probes(keys, m, theta=0.5, absent_fraction=0.1, seed=6)
+    pairs, count = ix.inlj_pairs(probes)
+    sizes, real = [], gj._workspace
+
+    def scarce(nbytes, device):
+        sizes.append(nbytes)
+        if nbytes > m:
+            raise torch.cuda.OutOfMemoryError("full")
+        return real(nbytes, device)
+
+    monkeypatch.setattr(gj, "_workspace", scarce)
+    again, recount = ix.inlj_pairs(probes)
+    assert len(sizes) == 2 and sizes[0] > 6 * m > sizes[1]
+    assert int(count) == int(recount) and torch.equal(pairs[: 2 * int(count)], again[: 2 * int(count)])
