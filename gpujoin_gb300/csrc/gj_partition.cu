@@ -566,6 +566,10 @@ struct pairs_scratch {
     void* inverse;
     size_t inverse_bytes;
 };
+// where it starts: behind the state, on the carver's boundary again (the state's
+// size is not a whole number of sectors, and every store of a warp would
+// straddle one more)
+size_t pairs_scratch_offset(uint64_t m) { return (pairs_workspace_bytes(m) + 255) & ~size_t(255); }
 size_t pairs_inverse_bytes(uint64_t m) {
     return workspace_carver::need({m * 2, (m / kTile + 1) * (2ull << kPairsRadixBits)});
 }
@@ -574,7 +578,8 @@ size_t pairs_inverse_bytes(uint64_t m) {
 size_t pairs_partition_bytes(uint64_t m) {
     if (m < kPartitionPairsMin || m > kPartitionPairsMax) return 0;
     // no device is asked: more SMs than there are only make the tables larger
-    return workspace_carver::need({partition_ws_bytes(m, kPairsRadixBits, 256) + (1u << 20), m * 4,
+    return pairs_scratch_offset(m) - pairs_workspace_bytes(m) +
+           workspace_carver::need({partition_ws_bytes(m, kPairsRadixBits, 256) + (1u << 20), m * 4,
                                    pairs_inverse_bytes(m)});
 }
 
@@ -614,7 +619,7 @@ int launch_pairs_by_partition(const gj_index* idx, const uint64_t* d_probes, uin
     const uint32_t bits = std::min(default_radix_bits(idx->n), kPairsRadixBits);
     device_info di;
     GJ_TRY(current_device_info(&di));
-    const size_t head = pairs_workspace_bytes(m);
+    const size_t head = pairs_scratch_offset(m);
     if (ws_bytes <= head) return GJ_OK;
     pairs_ws pw;
     size_t used = 0;

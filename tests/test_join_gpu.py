@@ -387,3 +387,22 @@ def test_pairs_with_little_memory(gj, cuda, monkeypatch):
     again, recount = ix.inlj_pairs(probes)
     assert len(sizes) == 2 and sizes[0] > 6 * m > sizes[1]
     assert int(count) == int(recount) and torch.equal(pairs[: 2 * int(count)], again[: 2 * int(count)])
+
+
+def test_partition_scratch_is_aligned(gj, cuda):
+    # the partition's arrays behind the state of an ordered call start on a
+    # 256-byte boundary of the workspace, as the state itself does
+    import torch
+
+    n, m = (1 << 25) + 64, (1 << 25) + 257
+    keys = gj.generate_sorted_keys(n, gj.DIST_UNIFORM, 1 << 63, seed=5)
+    ix = gj.btree_index().construct(None, keys)
+    probes = gj.generate_probes(keys, m, theta=0.5, seed=6)
+    least, need = ctypes.c_size_t(0), ctypes.c_size_t(0)
+    gj.lib().gj_inlj_pairs_host_workspace_size(m, ctypes.byref(least))
+    gj.lib().gj_index_inlj_pairs_workspace_size(ix.handle, m, ctypes.byref(need))
+    ws = torch.full((need.value,), 0xA5, dtype=torch.uint8, device="cuda")
+    _, count = ix.inlj_pairs(probes, workspace=ws)
+    assert int(count) == m and ws.data_ptr() % 256 == 0
+    first = int(torch.nonzero(ws[least.value: least.value + 4096] != 0xA5)[0])
+    assert (least.value + first) % 256 == 0
