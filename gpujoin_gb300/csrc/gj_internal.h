@@ -217,9 +217,11 @@ __host__ __device__ inline uint64_t value_index(uint32_t d) {
 // (ws: the partition pass's workspace, not written since)
 int gather_values(const uint32_t* d_values, uint64_t m, uint32_t radix_bits, void* ws, size_t ws_bytes,
                   const partition_inverse& iv, uint32_t* d_out, cudaStream_t s);
+// (stay: a device word; where it is not zero the pass does nothing)
 int range_partition_impl(const uint64_t* d_keys, uint64_t m, uint64_t min_key, uint32_t shift, uint32_t radix_bits,
                          uint64_t row_base, uint64_t* d_out_keys, uint32_t* d_out_rows, uint64_t* d_offsets, void* ws,
-                         size_t ws_bytes, cudaStream_t s, const partition_inverse* inverse = nullptr);
+                         size_t ws_bytes, cudaStream_t s, const partition_inverse* inverse = nullptr,
+                         const unsigned long long* stay = nullptr);
 // fanout for an index of n keys (about 2^21 keys a partition, 2^5..2^12)
 uint32_t default_radix_bits(uint64_t n);
 // smallest shift that maps [min_key, max_key] onto 2^radix_bits partitions

@@ -16,6 +16,7 @@
 //   3. k_part_scatter keys and row ids to their partition, in tile order
 // and, for callers that want values back in probe order, k_part_gather.
 // The windowed partitioned INLJ that drives it is in gj_partitioned.cu.
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -25,6 +26,8 @@
 
 namespace gj {
 namespace {
+
+namespace cg = cooperative_groups;
 
 constexpr uint32_t kMaxRadixBits = 12;
 
@@ -42,12 +45,21 @@ struct part_tables {
     uint32_t* chunk_start;  // chunks x fanout; the histogram leaves chunk counts, k_part_base their prefixes
     uint32_t* part_start;   // fanout
     uint32_t* done;         // blocks of k_part_base that are through
+    const unsigned long long* stay;  // null, or a word that is not zero where the caller turned out to need no partition
     uint32_t tiles, tiles_per_chunk, chunks, fanout;
 };
 struct part_func {
     uint64_t min_key;
     uint32_t shift;
 };
+
+// (the word is read by every block of a pass whose keys stream through L1)
+__device__ __forceinline__ bool stays(const unsigned long long* word) {
+    if (!word) return false;
+    unsigned long long v;
+    asm("ld.global.nc.L1::evict_last.u64 %0, [%1];" : "=l"(v) : "l"(word));
+    return v != 0;
+}
 
 // sub-histograms per block: warps spread their shared-memory atomics over
 // several copies when the fanout is small (fewer same-address conflicts)
@@ -63,6 +75,7 @@ template <int kB, int kTile>
 __global__ void __launch_bounds__(kB) k_part_hist(const uint64_t* __restrict__ keys, uint64_t m, part_func f,
                                                   part_tables t) {
     constexpr int kIt = kTile / kB;
+    if (stays(t.stay)) return;
     extern __shared__ uint32_t s_hist[];  // 2 x copies x fanout, then the chunk's counts so far
     const uint32_t fanout = t.fanout, copies = hist_copies(fanout);
     uint32_t* s_run = s_hist + 2 * copies * fanout;
@@ -153,6 +166,7 @@ __device__ __forceinline__ void block_exclusive_scan(const uint32_t* in, uint32_
 constexpr int kBaseBlock = 1024;
 __global__ void __launch_bounds__(kBaseBlock) k_part_base(part_tables t, uint64_t m, uint64_t* __restrict__ offsets) {
     constexpr uint32_t kWarps = kBaseBlock / 32;
+    if (stays(t.stay)) return;
     __shared__ uint32_t s_sum[kWarps][33];
     __shared__ bool s_last;
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, fanout = t.fanout;
@@ -223,6 +237,7 @@ __global__ void __launch_bounds__(kB, kPerSM) k_part_scatter(const uint64_t* __r
                                                              uint32_t* __restrict__ out_rows, partition_inverse iv) {
     constexpr uint32_t kTile = kB * kIt;
     static_assert(kTile <= (1u << 13) && (1u << kMaxRadixBits) <= (1u << 19), "slot packing");
+    if (stays(t.stay)) return;
     extern __shared__ unsigned long long s_mem[];
     uint64_t* s_keys = reinterpret_cast<uint64_t*>(s_mem);            // kTile
     uint32_t* s_start = reinterpret_cast<uint32_t*>(s_mem + kTile);   // fanout: counts, then starts in the tile
@@ -339,24 +354,79 @@ __global__ void __launch_bounds__(kB, kPerSM) k_part_gather(const uint32_t* __re
     }
 }
 
+// Whether a call's probes reuse the column as they come: skewed probes, whose
+// keys repeat, and probes in order or nearly so, whose neighbours lie side by
+// side.  Their plain search runs from L1 and L2, which is what a partition is
+// for, so it would only cost (2^25 probes into 2^26 uniform keys, partitioned /
+// plain: Zipf(1.25) 598 / 430 us, Zipf(1.1) 633 / 548, Zipf(1) 655 / 704,
+// Zipf(0.5) 698 / 1308; sorted 724 / 427).  Taken from kReuseSample probes, in
+// runs of a warp's width spread over the call: counted are the probes that fall
+// on a 128-byte line of the column that another one fell on (a bitmap of hashed
+// lines), and all of a run that lies within local_lines, a partition's share of
+// the column.  *word: 1 where they are more than kReuseMost: 4600 of 8192 lies
+// between Zipf(1.05) (3500 to 4000 on columns of 2*10^7 to 2^28 keys) and
+// Zipf(1.15) (5200 to 5500); the two ways break even at 1.0 to 1.1.
+// Bound by one chain of dependent loads, a search (8 us); a cluster shares the
+// bitmap, a slice a block.  The launch also clears the words 64-bit words of the
+// pairs' state, *word among them, in place of a memset.
+constexpr int kReuseBlock = 1024, kReuseBlocks = 8;
+constexpr uint32_t kReuseSample = kReuseBlocks * kReuseBlock, kReuseRuns = kReuseSample / 32;
+constexpr uint32_t kReuseSliceBits = 15, kReuseMost = 4600;
+__global__ void __cluster_dims__(kReuseBlocks, 1, 1) __launch_bounds__(kReuseBlock)
+    k_probe_reuse(const __grid_constant__ key_start t, const uint64_t* __restrict__ col, uint32_t n,
+                  const uint64_t* __restrict__ probes, uint64_t m, uint32_t local_lines, unsigned long long* state,
+                  uint32_t words, unsigned long long* word) {
+    __shared__ uint32_t s_seen[(1u << kReuseSliceBits) / 32];
+    __shared__ uint32_t s_again;
+    cg::cluster_group cluster = cg::this_cluster();
+    const uint32_t i = blockIdx.x * kReuseBlock + threadIdx.x;
+    const uint64_t run = i >> 5;
+    const uint64_t key = ld_ro(probes + run * (m - 32) / (kReuseRuns - 1) + (i & 31));
+    for (uint32_t w = i; w < words; w += kReuseSample) state[w] = 0;
+    for (uint32_t w = threadIdx.x; w < (1u << kReuseSliceBits) / 32; w += kReuseBlock) s_seen[w] = 0;
+    if (threadIdx.x == 0) s_again = 0;
+    bool eq;
+    const uint32_t line = start_lower_bound<false>(t, col, n, key, &eq) >> 4;
+    const uint32_t span = __reduce_max_sync(0xffffffffu, line) - __reduce_min_sync(0xffffffffu, line);
+    cluster.sync();
+    uint32_t again = 1;
+    if (span > local_lines) {
+        const uint32_t h = (line * 0x9E3779B1u) >> (32 - kReuseSliceBits - 3), bit = h & ((1u << kReuseSliceBits) - 1);
+        uint32_t* seen = cluster.map_shared_rank(s_seen, h >> kReuseSliceBits);
+        again = (atomicOr(seen + (bit >> 5), 1u << (bit & 31)) >> (bit & 31)) & 1u;
+    }
+    again = __reduce_add_sync(0xffffffffu, again);
+    if ((threadIdx.x & 31) == 0) atomicAdd(cluster.map_shared_rank(&s_again, 0), again);
+    cluster.sync();
+    if (i == 0) *word = s_again > kReuseMost ? 1u : 0u;
+}
+static_assert(kReuseBlocks == 1 << 3, "a slice of the bitmap a block");
+
 // values[i] = result of relation entry i through the index's key start table;
-// neighbouring probes share its and the column's lines in L2
+// neighbouring probes share its and the column's lines in L2.  Where the call
+// stays with its probes as they came (stay, k_probe_reuse), of probe i.
 template <bool kExact>
 __global__ void __launch_bounds__(kBlock, 8) k_relation_values(const __grid_constant__ key_start t,
                                                                const uint64_t* __restrict__ col, uint32_t n,
-                                                               const uint64_t* __restrict__ keys, uint64_t m,
+                                                               const uint64_t* __restrict__ relation,
+                                                               const uint64_t* __restrict__ probes, uint64_t m,
+                                                               const unsigned long long* __restrict__ stay,
                                                                uint32_t* __restrict__ values) {
     const uint64_t i = (uint64_t)blockIdx.x * kBlock + threadIdx.x;
     if (i >= m) return;
+    // the word is looked at while the relation's key is on its way: waiting for
+    // it first cost 150 us of 2^28 probes' 2.5 ms
+    uint64_t key = __ldcs(reinterpret_cast<const unsigned long long*>(relation) + i);
+    if (stays(stay)) key = __ldcs(reinterpret_cast<const unsigned long long*>(probes) + i);
     bool eq;
-    const uint32_t lb =
-        start_lower_bound<false>(t, col, n, __ldcs(reinterpret_cast<const unsigned long long*>(keys) + i), &eq);
+    const uint32_t lb = start_lower_bound<false>(t, col, n, key, &eq);
     __stcs(values + i, (kExact ? eq : lb < n) ? lb : kInvalid);
 }
 
 // k_part_gather into ordered pairs: a block claims tiles in order, gathers a
-// tile's values into probe order and places its pairs behind those of the
-// tiles before it.  6 bytes read and up to 8 written a probe.
+// tile's values into probe order (they are in it where the call stayed with its
+// probes) and places its pairs behind those of the tiles before it.  6 bytes
+// read and up to 8 written a probe.
 constexpr int kGatherItems = 16;
 constexpr uint32_t kGatherTile = kBlock * kGatherItems;
 __global__ void __launch_bounds__(kBlock, 6) k_gather_pairs(const uint32_t* __restrict__ values, uint64_t m,
@@ -368,9 +438,17 @@ __global__ void __launch_bounds__(kBlock, 6) k_gather_pairs(const uint32_t* __re
     uint32_t* s_delta = reinterpret_cast<uint32_t*>(s_mem);            // fanout
     uint16_t* s_start = reinterpret_cast<uint16_t*>(s_delta + fanout); // fanout + 2
     uint16_t* s_part = s_start + fanout + 2;                           // kGatherTile
+    const bool stay = stays(t.stay);
     auto gather = [&](uint64_t t0, uint32_t* pos) {
         const uint32_t tile = (uint32_t)(t0 / kGatherTile);
         const uint32_t tn = m - t0 < kGatherTile ? (uint32_t)(m - t0) : kGatherTile;
+        if (stay) {
+#pragma unroll 8
+            for (uint32_t j = threadIdx.x; j < kGatherTile; j += kBlock)
+                pos[j] = j < tn ? __ldcs(values + t0 + j) : kInvalid;
+            __syncthreads();
+            return;
+        }
         for (uint32_t p = threadIdx.x; p < fanout; p += kBlock) {
             const uint16_t at = __ldcs(iv.start + (uint64_t)tile * fanout + p);
             s_delta[p] = run_start(t, tile, p) - at;
@@ -472,6 +550,7 @@ bool carve_tables(void* ws, size_t ws_bytes, const partition_plan& pl, part_tabl
     t->tiles_per_chunk = pl.tiles_per_chunk;
     t->chunks = pl.chunks;
     t->fanout = pl.fanout;
+    t->stay = nullptr;
     return t->before && t->chunk_start && t->part_start && t->done;
 }
 
@@ -498,7 +577,8 @@ size_t partition_ws_bytes(uint64_t m, uint32_t radix_bits, int sm_count) {
 
 int range_partition_impl(const uint64_t* d_keys, uint64_t m, uint64_t min_key, uint32_t shift, uint32_t radix_bits,
                          uint64_t row_base, uint64_t* d_out_keys, uint32_t* d_out_rows, uint64_t* d_offsets, void* ws,
-                         size_t ws_bytes, cudaStream_t s, const partition_inverse* inverse) {
+                         size_t ws_bytes, cudaStream_t s, const partition_inverse* inverse,
+                         const unsigned long long* stay) {
     device_info di;
     GJ_TRY(current_device_info(&di));
     const partition_plan pl = plan_partition(m ? m : 1, radix_bits, di.sm_count);
@@ -508,6 +588,7 @@ int range_partition_impl(const uint64_t* d_keys, uint64_t m, uint64_t min_key, u
                   partition_ws_bytes(m, radix_bits, di.sm_count));
         return GJ_ERR_WORKSPACE;
     }
+    t.stay = stay;
     if (m == 0) {
         if (d_offsets) GJ_CUDA_TRY(cudaMemsetAsync(d_offsets, 0, ((size_t)pl.fanout + 1) * sizeof(uint64_t), s));
         return GJ_OK;
@@ -583,25 +664,23 @@ size_t pairs_partition_bytes(uint64_t m) {
                                    pairs_inverse_bytes(m)});
 }
 
-// Taken by large calls into columns far larger than L2: the partition, the
-// probes from L2 and the gather cost less than a random DRAM access a probe.
-// B+tree, plain / by partition: 2^28 probes into 2^26 uniform keys 6687 / 4998
-// us (histogram 349, scatter 911, probes 2956, gather 835; 4625 since the
-// probes' table is finer than the lookups'), 50 M 1284 / 1026; lognormal 6675
-// / 6083 (5219); 2^25 keys 5711 / 4679, 2^24 keys 4237 / 4567; 2^29 into 2^28
-// keys 21.5 / 12.4 ms (2^28 probes 6.27 ms, 5.09 with the finer table).  The relation's keys lie in the pairs buffer,
-// which has 8 bytes a probe and is not written before the gather.  Columns
-// whose table windows take long searches are left to the plain pairs: at once
-// below 2^26 keys (2^25 clustered keys 5505 / 5955), where those searches
-// dwarf the rest above (2^26 clustered keys 8628 / 5972).  Skewed probes, which L1
-// and L2 serve, gain little from the partition or lose: hash tables, whose plain
-// search is one load, are never partitioned (10^8 Zipf(1.25) probes into 2^26
-// keys 655 / 1561), the learned index, whose leaves know clustered keys, only
-// where the table's searches are short (2^25 clustered keys 1061 / 2148).  For
-// trees over uniform keys both are level (1596 / 1562); over lognormal keys the
-// partition costs a tenth there (1634 / 1806) and saves a quarter at even
-// probes (2692 / 2013).  34 M probes are about where lognormal columns break even (2^25 keys
-// 754 / 752; 2^26 865 / 839, 24 M 629 / 622).
+// Ordered pairs by way of a partition: large calls into columns far larger than
+// L2, where the partition, the probes from L2 and the gather cost less than a
+// random DRAM access a probe.  2^28 probes, plain / so: 2^26 uniform keys 6687 /
+// 4650 us (sample 11, histogram 350, scatter 925, probes 2550, gather 840),
+// lognormal 6675 / 5270, 2^28 uniform keys 10500 / 5230; 2^24 keys 4237 / 4567.
+// 2^25 probes are about where lognormal columns break even (754 / 752).  Never
+// hash tables, whose plain search is one load, and no columns whose table
+// windows take long searches: below 2^26 keys where those dwarf the rest (2^25
+// clustered keys, 2.4 loads a search, 5505 / 5955; 2^26 8628 / 5995), and for
+// the learned index, whose leaves know clustered keys.  Probes that reuse the
+// column as they come take the plain search through the same table, decided on
+// the device (k_probe_reuse): 2^25 probes into 2^26 keys 572 / 470 us at
+// Zipf(1.25), 703 / 466 sorted, for 1.5 % of an even call of 2^25 probes and
+// 0.5 % of 2^28.
+//
+// The relation's keys lie in the pairs buffer, which has 8 bytes a probe and is
+// not written before the gather.
 bool may_partition_pairs(const gj_index* idx) {
     return idx->type != GJ_INDEX_NO_OP && idx->type != GJ_INDEX_HASH && idx->in_hbm &&
            (reinterpret_cast<uintptr_t>(idx->d_col) & 31) == 0 && idx->n > partition_pairs_keys(idx->type);
@@ -641,13 +720,17 @@ int launch_pairs_by_partition(const gj_index* idx, const uint64_t* d_probes, uin
     static_assert(kGatherTile == kTile, "the gather's tiles are the scatter's");
     *taken = true;
     uint64_t* keys = reinterpret_cast<uint64_t*>(d_pairs);
-    GJ_CUDA_TRY(cudaMemsetAsync(ws, 0, used, s));
+    // (the totals are the unordered pairs' words of the state, which lies in
+    // whole 64-bit words at the head of the workspace)
+    t.stay = pw.totals;
+    GJ_TRY(launch(k_probe_reuse, kReuseBlocks, kReuseBlock, 0, s, idx->rel, idx->d_col, (uint32_t)idx->n, d_probes, m,
+                  (uint32_t)(idx->n >> 4 >> bits), pw.tile_state, (uint32_t)(used / 8), pw.totals));
     GJ_TRY(range_partition_impl(d_probes, m, idx->min_key, shift_for(idx->min_key, idx->max_key, bits), bits, 0, keys,
-                                nullptr, nullptr, sc.tables, sc.table_bytes, s, &iv));
+                                nullptr, nullptr, sc.tables, sc.table_bytes, s, &iv, t.stay));
     const uint32_t blocks = (uint32_t)((m + kBlock - 1) / kBlock);
     const bool exact = idx->type == GJ_INDEX_BTREE || idx->type == GJ_INDEX_HARMONIA;
     GJ_TRY(launch(exact ? k_relation_values<true> : k_relation_values<false>, blocks, kBlock, 0, s, idx->rel, idx->d_col,
-                  (uint32_t)idx->n, static_cast<const uint64_t*>(keys), m, sc.values));
+                  (uint32_t)idx->n, static_cast<const uint64_t*>(keys), d_probes, m, t.stay, sc.values));
     const size_t smem = (size_t)pl.fanout * 4 + ((size_t)pl.fanout + 2) * 2 + kGatherTile * 2;
     int grid = 0;
     GJ_TRY(grid_for(k_gather_pairs, smem, (uint64_t)pl.tiles * kBlock, &grid));

@@ -406,3 +406,119 @@ def test_partition_scratch_is_aligned(gj, cuda):
     assert int(count) == m and ws.data_ptr() % 256 == 0
     first = int(torch.nonzero(ws[least.value: least.value + 4096] != 0xA5)[0])
     assert (least.value + first) % 256 == 0
+
+
+def route_of(gj, ix, probes):
+    """(pairs, count, how) of an ordered call on the workspace its index asks
+    for: "plain" (no room to partition is asked for, or none is touched),
+    "stayed" (it was sampled, and its probes were searched as they came) or
+    "partitioned" (the partition's tables, first in that room, were written)"""
+    import torch
+
+    m = probes.numel()
+    least, need = ctypes.c_size_t(0), ctypes.c_size_t(0)
+    gj.lib().gj_inlj_pairs_host_workspace_size(m, ctypes.byref(least))
+    gj.lib().gj_index_inlj_pairs_workspace_size(ix.handle, m, ctypes.byref(need))
+    ws = torch.full((need.value,), 0xA5, dtype=torch.uint8, device="cuda")
+    pairs, count = ix.inlj_pairs(probes, workspace=ws)
+    ix.inlj_pairs_status(ws, m)
+    room = ws[least.value:]
+    if not bool((room != 0xA5).any()):
+        return pairs, count, "plain"
+    return pairs, count, "partitioned" if bool((room[256:4096] != 0xA5).any()) else "stayed"
+
+
+def skew(torch, gj, keys, m, form):
+    if form == "even":
+        return gj.generate_probes(keys, m, theta=0.5, absent_fraction=0.1, seed=6)
+    if form == "skewed":
+        return gj.generate_probes(keys, m, theta=1.5, absent_fraction=0.1, seed=6)
+    p = gj.generate_probes(keys, m, theta=0.0, seed=6)
+    p = torch.sort(p)[0] if int(keys[-1]) >= 0 else p
+    if form == "nearly sorted":  # shuffled inside windows of 4096
+        q = p[: m // 4096 * 4096].view(-1, 4096)
+        p[: m // 4096 * 4096] = q[:, torch.randperm(4096, device="cuda")].reshape(-1)
+    return p
+
+
+@pytest.mark.parametrize("column", ["uniform", "lognormal", "clusters", "whole range"])
+@pytest.mark.parametrize("form", ["even", "skewed", "sorted", "nearly sorted"])
+@pytest.mark.parametrize("kind", ["btree", "binary_search"])
+def test_ordered_pairs_look_at_their_probes(orc, gj, cuda, kind, form, column):
+    # even probes are partitioned; skewed ones and those in order or nearly so
+    # are searched as they come -- the same pairs in the same order, against the
+    # oracle, over a finer and a coarse table (clusters) and up to 2^64 - 1
+    import torch
+
+    m = (1 << 25) + 257
+    n = (1 << 26) if column == "clusters" else (1 << 25) + 64
+    if column == "whole range":
+        if form in ("sorted", "nearly sorted"):
+            pytest.skip("probes are sorted as signed numbers")
+        keys = gj.generate_sorted_keys(n, gj.DIST_UNIFORM, 1 << 63, seed=5) * 2  # above 2^63 too
+        keys[0], keys[-1] = 0, -1  # 2^64 - 1
+    else:
+        keys = gj.generate_sorted_keys(n, getattr(gj, "DIST_" + column.upper()), 1 << 63, seed=5)
+    probes = skew(torch, gj, keys, m, form)
+    probes[:4] = torch.tensor([0, 1, -1, -2], dtype=torch.int64, device="cuda")
+    ix = gj.make_index(kind).construct(None, keys)
+    pairs, count, how = route_of(gj, ix, probes)
+    assert how == ("partitioned" if form == "even" else "stayed")
+    col, pr = keys.cpu().numpy().view(np.uint64), probes.cpu().numpy().view(np.uint64)
+    exp = (orc.exact_lookup if kind == "btree" else orc.bs_lookup)(col, pr)
+    rows, pos = orc.pairs_from_positions(exp)
+    got = pairs[: 2 * int(count)].cpu().numpy().view(np.uint32).reshape(-1, 2)
+    assert int(count) == len(rows)
+    np.testing.assert_array_equal(got[:, 0], rows)
+    np.testing.assert_array_equal(got[:, 1], pos)
+
+
+@pytest.mark.parametrize("kind,n,m,how", [("hash", 1 << 25, (1 << 25) + 5, "plain"),
+                                          ("btree", 20_000_000, (1 << 25) + 5, "plain"),
+                                          ("btree", 3 << 23, (1 << 25) + 5, "plain"),
+                                          ("btree", (3 << 23) + 64, (1 << 25) + 5, "partitioned"),
+                                          ("btree", (3 << 23) + 64, 1 << 25, "partitioned"),
+                                          ("btree", (3 << 23) + 64, (1 << 25) - 1, "plain"),
+                                          ("radix_spline", (3 << 22) + 64, (1 << 25) + 5, "partitioned"),
+                                          ("learned", (3 << 22) + 64, (1 << 25) + 5, "partitioned")])
+def test_which_ordered_pairs_are_partitioned(gj, cuda, kind, n, m, how):
+    import torch
+
+    kw = {"learned_steps": 20} if kind == "learned" else {}
+    keys = gj.generate_sorted_keys(n, gj.DIST_UNIFORM, 1 << 63, seed=5)
+    ix = gj.make_index(kind, **kw).construct(None, keys)
+    probes = gj.generate_probes(keys, m, theta=0.5, absent_fraction=0.1, seed=6)
+    pairs, count, taken = route_of(gj, ix, probes)
+    assert taken == how
+    pos = ix.lookup(probes)
+    rows = torch.nonzero(pos != -1).flatten()
+    got = pairs[: 2 * int(count)].view(-1, 2)
+    assert torch.equal(got[:, 0].to(torch.int64), rows) and torch.equal(got[:, 1], pos[rows])
+
+
+def test_partitioned_pairs_under_capture(gj, cuda):
+    # one captured call, replayed on probes that are partitioned and on probes
+    # that are not: the choice is made on the device
+    import torch
+
+    n, m = (1 << 25) + 64, (1 << 25) + 257
+    keys = gj.generate_sorted_keys(n, gj.DIST_UNIFORM, 1 << 63, seed=5)
+    ix = gj.btree_index().construct(None, keys)
+    probes = skew(torch, gj, keys, m, "even")
+    need = ctypes.c_size_t(0)
+    gj.lib().gj_index_inlj_pairs_workspace_size(ix.handle, m, ctypes.byref(need))
+    ws = torch.empty(need.value, dtype=torch.uint8, device="cuda")
+    pairs, count = torch.empty(2 * m, dtype=torch.int32, device="cuda"), torch.empty(1, dtype=torch.int64, device="cuda")
+    ix.inlj_pairs(probes, pairs, count, ws)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        ix.inlj_pairs(probes, pairs, count, ws)
+    for form in ("skewed", "even", "sorted"):
+        probes.copy_(skew(torch, gj, keys, m, form))
+        graph.replay()
+        pos = ix.lookup(probes)
+        rows = torch.nonzero(pos != -1).flatten()
+        assert int(count) == rows.numel()
+        got = pairs[: 2 * int(count)].view(-1, 2)
+        assert torch.equal(got[:, 0].to(torch.int64), rows) and torch.equal(got[:, 1], pos[rows])
