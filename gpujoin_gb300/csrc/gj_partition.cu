@@ -668,7 +668,7 @@ size_t pairs_partition_bytes(uint64_t m) {
 // L2, where the partition, the probes from L2 and the gather cost less than a
 // random DRAM access a probe.  2^28 probes, plain / so: 2^26 uniform keys 6687 /
 // 4650 us (sample 11, histogram 350, scatter 925, probes 2550, gather 840),
-// lognormal 6675 / 5270, 2^28 uniform keys 10500 / 5230; 2^24 keys 4237 / 4567.
+// lognormal 6675 / 5270; 2^24 keys 4237 / 4567.
 // 2^25 probes are about where lognormal columns break even (754 / 752).  Never
 // hash tables, whose plain search is one load, and no columns whose table
 // windows take long searches: below 2^26 keys where those dwarf the rest (2^25
