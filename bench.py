@@ -177,6 +177,13 @@ def profile_traffic(kernel_tag: str):
 # ---------------------------------------------------------------------------
 # GPU arm
 # ---------------------------------------------------------------------------
+def pairs_bytes_per_probe(n: int, m: int) -> float:
+    """Bytes an ordered-pairs call of m probes into n keys cannot do without, per
+    probe: the probe read, its pair written, and the column read once or, where
+    there are fewer probes than sectors, a 32-byte sector each."""
+    return 8 + 8 + min(8.0 * n / m, 32.0)
+
+
 def count_launches(fn):
     """Kernels of the library that one call of fn launches, counted (not timed)
     by the profiler outside any timed region; None where it cannot trace."""
@@ -691,18 +698,20 @@ def inlj_workload(args, world, rank, device, stream):
                                                 "api": "gj_inlj_pairs_unordered (device buffers)",
                                                 "pairs": d_count, "parity": d_parity}}}
 
-    # Roofline of the step.  A pairs step of this size partitions its probes
-    # first: histogram (8 B read a probe), scatter (8 read, key and 16-bit tile
-    # offset written), probes (key read, u32 position written; the index and
-    # the column come from L2, each read from HBM about once), gather (position
-    # and offset read, pair written) -- or, where the call stays plain, one
-    # launch: probe in, one 32-byte column sector, pair out.  Beside it the
+    # Roofline of the step: the bytes it cannot do without over its time.  Its
+    # passes move more (pass_bytes_per_probe): a step of this size partitions its
+    # probes first -- histogram (8 B read a probe), scatter (8 read, key and
+    # 16-bit tile offset written), probes (key read, u32 position written; the
+    # index and the column come from L2, each read from HBM about once), gather
+    # (position and offset read, pair written) -- or, where the call stays plain,
+    # is one launch: probe in, one 32-byte column sector, pair out.  Beside it the
     # plain lookup of the same probes into positions, timed on its own: one
     # random column sector a probe.
     peak, peak_kind = measured_peak()
     lookup_bytes_per_probe = bytes_per_probe - 4
     per_step = count_launches(lambda: headline_ix.inlj_pairs(probes, pairs, count, ws))
-    step_bytes = bytes_per_probe if per_step is not None and per_step < 4 else 52 + 8.0 * n / m
+    step_bytes = pairs_bytes_per_probe(n, m)
+    pass_bytes = bytes_per_probe if per_step is not None and per_step < 4 else 52 + 8.0 * n / m
     lookup_ms = time_steps(lambda: headline_ix.lookup(probes, out=pairs[m:]), args.steps, args.warmup, stream, world,
                            device)
     lookup_ms = max_over_ranks(lookup_ms, world, device) / args.steps
@@ -711,7 +720,8 @@ def inlj_workload(args, world, rank, device, stream):
     roofline = {"bound": "hbm", "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
                 "frac": round(achieved / peak, 4), "traffic": None,
                 "peak_source": f"{peak_kind} hbm_gbs (copy, burst)",
-                "kernel": "the whole pairs step", "bytes_per_probe": step_bytes, "launches_per_step": per_step,
+                "kernel": "the whole pairs step", "bytes_per_probe": step_bytes,
+                "pass_bytes_per_probe": pass_bytes, "launches_per_step": per_step,
                 "plain_lookup": {
                     "kernel": f"k_lookup<{headline_index}> (positions of the same probes)",
                     "kernel_ms": round(lookup_ms, 4), "bytes_per_probe": lookup_bytes_per_probe,

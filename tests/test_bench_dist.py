@@ -98,3 +98,13 @@ def test_workload_sizes():
     assert sizes("--impl", "reference") == (26, 28)
     assert sizes("--workload", "partitioned", "--n-log2", "26", "--m-log2", "28") == (26, 28)
     assert sizes("--workload", "learned", "--n-log2", "20") == (20, 28)
+
+
+def test_roofline_counts_what_a_call_cannot_do_without():
+    # not the traffic of the passes it happens to be made of
+    import bench
+
+    n, m = 1 << 26, 1 << 28
+    assert bench.pairs_bytes_per_probe(n, m) == 18.0
+    assert bench.pairs_bytes_per_probe(n, n) == 24.0
+    assert bench.pairs_bytes_per_probe(n, 1 << 20) == 48.0  # a sector of the column each
