@@ -590,8 +590,15 @@ __device__ __forceinline__ void start_count(uint32_t tile, uint64_t* d_count) {
 // (33.3 M probes from host memory: 2109 us, 1808 with the write put off.)
 // Every look-back ends: it needs the counts of earlier tiles, which their
 // blocks publish before they wait for anything.
+//
+// The spline's search and the loop around it need 40 registers: at the 32 of
+// eight blocks they spill 56 bytes, which long calls feel (67 M unordered pairs
+// through a RadixSpline of 2^17 keys 1650 us, 1460 with six blocks) and calls
+// of few items a thread do not (2 M sorted probes into 2^25 keys 65 / 75).
+template <class Op, int kIt>
+constexpr int kPairsBlocks = std::is_same<Op, op_rs>::value && kIt == kItems ? GJ_BLOCKS(6) : Op::kMinBlocks;
 template <class Op, bool kOrdered, int kIt>
-__global__ void __launch_bounds__(kBlock, Op::kMinBlocks) k_pairs(const __grid_constant__ Op op, const stage_desc sd, const uint64_t* __restrict__ probes,
+__global__ void __launch_bounds__(kBlock, kPairsBlocks<Op, kIt>) k_pairs(const __grid_constant__ Op op, const stage_desc sd, const uint64_t* __restrict__ probes,
                                                   uint64_t m, uint2* __restrict__ pairs,
                                                   uint64_t* __restrict__ d_count, pairs_ws ws, uint32_t num_tiles) {
     extern __shared__ __align__(16) uint64_t cache[];

@@ -73,3 +73,21 @@ def test_launch_shapes(orc, gj, cuda, kind, m):
     out = torch.empty(m, dtype=torch.int32, device="cuda")
     ix.partitioned_lookup(d_pr, rows, out)
     np.testing.assert_array_equal(from_dev_u32(out)[rows.cpu().numpy()], exp)
+
+
+@pytest.mark.parametrize("n", [1 << 14, 300_007])
+@pytest.mark.parametrize("m", [(1 << 22) - 1, 1 << 22, (1 << 22) + 2049])
+def test_long_unordered_spline_pairs(orc, gj, cuda, n, m):
+    # the pairs kernel of eight probes a thread, at the size it starts from
+    import torch
+
+    rng = np.random.default_rng(n)
+    col = column(rng, n)
+    pr = probes_for(rng, col, m)[:m]
+    ix = gj.radix_spline_index().construct(None, to_dev(torch, col))
+    out, cnt = ix.inlj_pairs(to_dev(torch, pr), ordered=False)
+    got = out[: 2 * int(cnt)].cpu().numpy().view(np.uint32).reshape(-1, 2)
+    got = got[np.argsort(got[:, 0], kind="stable")]
+    rows, pos = orc.pairs_from_positions(orc.bs_lookup(col, pr))
+    np.testing.assert_array_equal(got[:, 0], rows)
+    np.testing.assert_array_equal(got[:, 1], pos)
