@@ -267,6 +267,21 @@ __device__ __forceinline__ void stage_cache(uint64_t* dst, const stage_desc& sd)
 constexpr uint64_t kL2Keys = 1ull << 23;  // columns of up to 64 MB stay in L2
 template <class Op>
 constexpr uint64_t kLookupLongKeys = std::is_same<Op, op_hash>::value ? UINT64_MAX : 1ull << 24;
+// The default B+tree's nodes are searched so a little further, in calls of 2^24
+// probes and more (67 M probes with 1 / 8: 20 M uniform keys 1186 / 1117 us,
+// lognormal 1250 / 1178; 2^25 keys, even probes, 1232 / 1268), and its ordered
+// pairs of that size take two passes, whose lookup can (1336 / 1262).  Scattered
+// results bind the partitioned lookups of 2^25 probes and more, whose stores
+// come from fewer warps at a time then (67 M into 20 M keys 2205 / 2090 us,
+// RadixSpline with 1 / 4 2240 / 2140; 17 M probes, whose results fit L2, into
+// 2^26 keys 240 / 320).
+constexpr uint64_t kNodeLongKeys = 3ull << 23, kNodeLongProbes = 1ull << 24, kScatterLongProbes = 1ull << 25;
+template <class Op>
+constexpr bool kNodeSearch = std::is_same<Op, op_btree<(int)kBtreeCompressed16>>::value;
+template <class Op>
+bool nodes_long(uint64_t n, uint64_t m) {
+    return kNodeSearch<Op> && n <= kNodeLongKeys && m >= kNodeLongProbes;
+}
 inline int long_blocks(uint64_t n, uint64_t m, bool* yes, uint64_t keys = kL2Keys) {
     device_info di;
     GJ_TRY(current_device_info(&di));
@@ -302,8 +317,11 @@ __global__ void __launch_bounds__(kBlock, Op::kMinBlocks) k_lookup(const __grid_
 }
 
 // scattered lookup over a partitioned relation: out[rows[i]] = lookup(keys[i])
+// (a spline's search in a loop needs 40 registers)
+template <class Op>
+constexpr int kScatterLong = std::is_same<Op, op_rs>::value ? 4 : Op::kLong;
 template <class Op, int kIt>
-__global__ void __launch_bounds__(kBlock, Op::kMinBlocks) k_scatter_lookup(const __grid_constant__ Op op, const stage_desc sd,
+__global__ void __launch_bounds__(kBlock, std::is_same<Op, op_rs>::value && kIt > 1 ? GJ_BLOCKS(6) : Op::kMinBlocks) k_scatter_lookup(const __grid_constant__ Op op, const stage_desc sd,
                                                            const uint64_t* __restrict__ keys,
                                                            const uint32_t* __restrict__ rows, uint64_t m,
                                                            uint32_t* __restrict__ out) {
@@ -921,6 +939,7 @@ int run_lookup(const Op& op, const stage_desc& sd, uint64_t n, const uint64_t* p
     if (clear) return launch(k_lookup<Op, 1, true>, 1);
     bool full = false;
     GJ_TRY(long_blocks(n, m, &full, kLookupLongKeys<Op>));
+    full |= nodes_long<Op>(n, m);
     return full ? launch(k_lookup<Op, Op::kLong>, Op::kLong) : launch(k_lookup<Op, 1>, 1);
 }
 
@@ -948,8 +967,10 @@ int run_scatter(const Op& op, const stage_desc& sd, uint64_t n, const uint64_t* 
         return (int)GJ_OK;
     };
     bool full = false;
-    GJ_TRY(long_blocks(n, m, &full));
-    return full ? launch(k_scatter_lookup<Op, Op::kLong>, Op::kLong) : launch(k_scatter_lookup<Op, 1>, 1);
+    if (std::is_same<Op, op_rs>::value) full = m >= kScatterLongProbes;
+    else GJ_TRY(long_blocks(n, m, &full));
+    full |= kNodeSearch<Op> && n <= (1ull << 25) && m >= kScatterLongProbes;
+    return full ? launch(k_scatter_lookup<Op, kScatterLong<Op>>, kScatterLong<Op>) : launch(k_scatter_lookup<Op, 1>, 1);
 }
 
 template <class Op>
@@ -968,12 +989,15 @@ int run_pairs(const Op& op, const stage_desc& sd, uint64_t n, const uint64_t* pr
         return GJ_OK;
     }
     if (spin_limit) pw.spin_limit = spin_limit;
-    const bool two_passes = stash && (m < kSinglePassMin || host_index);
+    const bool longs = nodes_long<Op>(n, m);
+    const bool two_passes = stash && (m < kSinglePassMin || host_index || longs);
     // the state lies in whole 64-bit words at the head of the workspace
-    if (two_passes)
+    if (two_passes && !longs) {
         GJ_TRY(run_lookup(op, sd, n, probes, m, stash, s, pw.tile_state, (uint32_t)(used / 8)));
-    else
+    } else {
         GJ_CUDA_TRY(cudaMemsetAsync(ws, 0, used, s));
+        if (two_passes) GJ_TRY(run_lookup(op, sd, n, probes, m, stash, s));
+    }
     // test hook: the tile counter starts at 1, so tile 0 is never claimed and
     // never publishes; every later tile's look-back runs out
     if (skip_first_tile) GJ_CUDA_TRY(cudaMemsetAsync(pw.tile_counter, 1, 1, s));

@@ -4,6 +4,8 @@ of a few keys, sizes around a sector and a table group, runs of consecutive
 keys, two scales of clusters (wide windows the guess misses), the extreme
 keys, unaligned columns, and probe counts around a block and a launch-shape
 threshold."""
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -91,3 +93,32 @@ def test_long_unordered_spline_pairs(orc, gj, cuda, n, m):
     rows, pos = orc.pairs_from_positions(orc.bs_lookup(col, pr))
     np.testing.assert_array_equal(got[:, 0], rows)
     np.testing.assert_array_equal(got[:, 1], pos)
+
+
+@pytest.mark.parametrize("kind,n", [("btree", (1 << 24) + 64), ("btree", 3 << 23), ("btree", (3 << 23) + 64),
+                                    ("radix_spline", 300_007)])
+@pytest.mark.parametrize("m", [(1 << 24) - 1, (1 << 25) + 2049])
+def test_long_calls_through_nodes_and_splines(orc, gj, cuda, kind, n, m):
+    # lookups, ordered pairs and partitioned lookups around the sizes from which
+    # a thread takes several probes (tree nodes above 2^24 keys, splines)
+    import torch
+
+    keys = gj.generate_sorted_keys(n, gj.DIST_UNIFORM, 1 << 63, seed=5)
+    probes = gj.generate_probes(keys, m, theta=0.5, absent_fraction=0.1, seed=6)
+    col, pr = keys.cpu().numpy().view(np.uint64), probes.cpu().numpy().view(np.uint64)
+    exp = (orc.exact_lookup if kind == "btree" else orc.bs_lookup)(col, pr)
+    ix = gj.make_index(kind).construct(None, keys)
+    np.testing.assert_array_equal(from_dev_u32(ix.lookup(probes)), exp)
+    least = ctypes.c_size_t(0)
+    gj.lib().gj_inlj_pairs_host_workspace_size(m, ctypes.byref(least))
+    ws = torch.full((least.value,), 0xA5, dtype=torch.uint8, device="cuda")
+    out, cnt = ix.inlj_pairs(probes, workspace=ws)
+    ix.inlj_pairs_status(ws, m)
+    rows, pos = orc.pairs_from_positions(exp)
+    got = out[: 2 * int(cnt)].cpu().numpy().view(np.uint32).reshape(-1, 2)
+    np.testing.assert_array_equal(got[:, 0], rows)
+    np.testing.assert_array_equal(got[:, 1], pos)
+    rel = gj.range_partition(probes, int(keys[0]), 63 - 8, 8)
+    scattered = torch.empty(m, dtype=torch.int32, device="cuda")
+    ix.partitioned_lookup(rel.keys, rel.rows, scattered)
+    np.testing.assert_array_equal(from_dev_u32(scattered), exp)
