@@ -38,9 +38,10 @@ constexpr int kBatchPerSM = 6;
 constexpr int kBatchBlock = 256;
 
 // What a tile's searches need to know of its index.  The common kinds have a
-// loop of their own in the kernel; the rest (trees that search their nodes,
-// MLP roots, indexes in host memory) share one behind a call, so that their
-// registers are not everyone's.
+// loop of their own in the kernel, wherever the index lives; the rest (trees
+// and binary searches without a key start table, as those of indexes in host
+// memory are, and MLP roots) share one behind a call, so that their registers
+// are not everyone's.
 enum view_kind : int32_t { kViewStartExact, kViewStartLower, kViewSpline, kViewLearned, kViewHash, kViewOther };
 struct start_view {
     key_start t;

@@ -268,13 +268,13 @@ constexpr uint64_t kL2Keys = 1ull << 23;  // columns of up to 64 MB stay in L2
 template <class Op>
 constexpr uint64_t kLookupLongKeys = std::is_same<Op, op_hash>::value ? UINT64_MAX : 1ull << 24;
 // The default B+tree's nodes are searched so a little further, in calls of 2^24
-// probes and more (67 M probes with 1 / 8: 20 M uniform keys 1186 / 1117 us,
-// lognormal 1250 / 1178; 2^25 keys, even probes, 1232 / 1268), and its ordered
-// pairs of that size take two passes, whose lookup can (1336 / 1262).  Scattered
+// probes and more (67 M probes with 1 / 8: 20 M uniform keys 1186 / 1116 us,
+// lognormal 1254 / 1185; 2^25 keys, Zipf(0.8), 1224 / 1256), and its ordered
+// pairs of that size take two passes, whose lookup can (1334 / 1261).  Scattered
 // results bind the partitioned lookups of 2^25 probes and more, whose stores
-// come from fewer warps at a time then (67 M into 20 M keys 2205 / 2090 us,
-// RadixSpline with 1 / 4 2240 / 2140; 17 M probes, whose results fit L2, into
-// 2^26 keys 240 / 320).
+// come from fewer warps at a time then (67 M into 20 M keys 2205 / 2089 us,
+// RadixSpline of 2^25 keys with 1 / 4 2272 / 2154; 17 M probes, whose results
+// fit L2, into 2^26 keys 385 / 513).
 constexpr uint64_t kNodeLongKeys = 3ull << 23, kNodeLongProbes = 1ull << 24, kScatterLongProbes = 1ull << 25;
 template <class Op>
 constexpr bool kNodeSearch = std::is_same<Op, op_btree<(int)kBtreeCompressed16>>::value;
@@ -610,9 +610,10 @@ __device__ __forceinline__ void start_count(uint32_t tile, uint64_t* d_count) {
 // blocks publish before they wait for anything.
 //
 // The spline's search and the loop around it need 40 registers: at the 32 of
-// eight blocks they spill 56 bytes, which long calls feel (67 M unordered pairs
-// through a RadixSpline of 2^17 keys 1650 us, 1460 with six blocks) and calls
-// of few items a thread do not (2 M sorted probes into 2^25 keys 65 / 75).
+// eight blocks they spill 56 bytes, which long calls feel (67 M probes through a
+// RadixSpline of 2^17 keys, unordered 1650 us, 1462 with six blocks, ordered 1673
+// / 1463) and calls of few items a thread do not (2 M sorted probes into 2^25
+// keys 61 / 69).
 template <class Op, int kIt>
 constexpr int kPairsBlocks = std::is_same<Op, op_rs>::value && kIt == kItems ? GJ_BLOCKS(6) : Op::kMinBlocks;
 template <class Op, bool kOrdered, int kIt>
