@@ -263,10 +263,12 @@ __device__ __forceinline__ void stage_cache(uint64_t* dst, const stage_desc& sd)
 // where most sectors still hit L2 (24 M probes with 1 / 4: B+tree, uniform
 // probes 358 / 352 us, Zipf(1.25) 212 / 189), and into a hash table, whose
 // search is one load, at any size (2^26 keys with 1 / 4 / 8: uniform 548 / 559
-// / 567, Zipf(1.25), which L1 and L2 serve, 160 / 133 / 132).
+// / 567, Zipf(1.25), which L1 and L2 serve, 160 / 133 / 132).  So do MLP roots,
+// which are bound by issue (34 M probes into 20 M keys, 16 wide, 1294 / 1040).
 constexpr uint64_t kL2Keys = 1ull << 23;  // columns of up to 64 MB stay in L2
 template <class Op>
-constexpr uint64_t kLookupLongKeys = std::is_same<Op, op_hash>::value ? UINT64_MAX : 1ull << 24;
+constexpr uint64_t kLookupLongKeys =
+    std::is_same<Op, op_hash>::value || std::is_same<Op, op_learned>::value ? UINT64_MAX : 1ull << 24;
 // The default B+tree's nodes are searched so a little further, in calls of 2^24
 // probes and more (67 M probes with 1 / 8: 20 M uniform keys 1186 / 1116 us,
 // lognormal 1254 / 1185; 2^25 keys, Zipf(0.8), 1224 / 1256), and its ordered
@@ -969,7 +971,7 @@ int run_scatter(const Op& op, const stage_desc& sd, uint64_t n, const uint64_t* 
     };
     bool full = false;
     if (std::is_same<Op, op_rs>::value) full = m >= kScatterLongProbes;
-    else GJ_TRY(long_blocks(n, m, &full));
+    else GJ_TRY(long_blocks(n, m, &full, std::is_same<Op, op_learned>::value ? UINT64_MAX : kL2Keys));
     full |= kNodeSearch<Op> && n <= (1ull << 25) && m >= kScatterLongProbes;
     return full ? launch(k_scatter_lookup<Op, kScatterLong<Op>>, kScatterLong<Op>) : launch(k_scatter_lookup<Op, 1>, 1);
 }

@@ -1113,8 +1113,10 @@ GJ_DEVICE_INLINE uint64_t window_lower_bound(const uint64_t* col, uint64_t n, ui
     // spline's window is 66 keys wide (2^26 probes: 2^16 clustered keys 1205
     // us halved, 1370 from the guess; 2^20 uniform keys 1292 / 1182, 2^26 keys
     // 3533 / 2921), a learned leaf's about 14 (2^20 keys 787 / 833, 2^26 keys
-    // 2191 / 2043).
-    if (aligned && b < e && n > (1ull << kLogKeys)) {
+    // 2191 / 2043).  Behind an MLP root, which leaves no issue slots or registers
+    // to spare, always halved (kLogKeys 32): 34 M probes into 2^24 keys 1690 us,
+    // 1864 from the guess, 32 wide; blocks of one probe a thread spilled too.
+    if (kLogKeys < 32 && aligned && b < e && n > (1ull << (kLogKeys & 31))) {
         const uint32_t sl = (uint32_t)(b >> 2), sr = (uint32_t)((e - 1) >> 2);
         const uint32_t s = (uint32_t)(guess >> 2);
         uint32_t edge;
@@ -1292,7 +1294,7 @@ GJ_DEVICE_INLINE uint32_t learned_lookup(const learned_view& v, const float* roo
     if (lo > hi) lo = hi;
     const int64_t at = pred < lo ? lo : pred > hi ? hi : pred;
     const uint64_t pos =
-        window_lower_bound<kScattered, 23>(v.col, v.n, (uint64_t)lo, (uint64_t)hi, (uint64_t)at, lf.slope * 0.25f, key,
+        window_lower_bound<kScattered, kMlp ? 32 : 23>(v.col, v.n, (uint64_t)lo, (uint64_t)hi, (uint64_t)at, lf.slope * 0.25f, key,
                                        v.col_aligned);
     return pos < v.n ? (uint32_t)pos : kInvalid;
 }

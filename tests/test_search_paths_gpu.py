@@ -122,3 +122,23 @@ def test_long_calls_through_nodes_and_splines(orc, gj, cuda, kind, n, m):
     scattered = torch.empty(m, dtype=torch.int32, device="cuda")
     ix.partitioned_lookup(rel.keys, rel.rows, scattered)
     np.testing.assert_array_equal(from_dev_u32(scattered), exp)
+
+
+@pytest.mark.parametrize("hidden", [16, 32])
+@pytest.mark.parametrize("n,m", [((1 << 23) + 32, (1 << 22) + 77), ((1 << 24) + 64, 5_000_011)])
+def test_long_calls_through_network_roots(orc, gj, cuda, hidden, n, m):
+    # learned indexes with an MLP root: several probes a thread from 16 waves of
+    # a full chip on, whatever the column, and windows halved on any column
+    import torch
+
+    keys = gj.generate_sorted_keys(n, gj.DIST_LOGNORMAL, 1 << 63, seed=5)
+    probes = gj.generate_probes(keys, m, theta=0.5, absent_fraction=0.1, seed=6)
+    exp = orc.bs_lookup(keys.cpu().numpy().view(np.uint64), probes.cpu().numpy().view(np.uint64))
+    ix = gj.make_index("learned", learned_root=gj.LEARNED_ROOT_MLP, learned_hidden=hidden,
+                       learned_steps=20).construct(None, keys)
+    np.testing.assert_array_equal(from_dev_u32(ix.lookup(probes)), exp)
+    np.testing.assert_array_equal(from_dev_u32(ix.lookup_sorted(probes)), exp)
+    rel = gj.range_partition(probes, int(keys[0]), 55, 8)
+    out = torch.empty(m, dtype=torch.int32, device="cuda")
+    ix.partitioned_lookup(rel.keys, rel.rows, out)
+    np.testing.assert_array_equal(from_dev_u32(out), exp)
