@@ -791,16 +791,14 @@ int build_radix_spline_index(gj_index* idx, const uint64_t* h_keys, cudaStream_t
     // points with the slope of their segment (the estimate's division, done once)
     std::vector<rs_point> pts(rs.sx.size());
     for (size_t i = 0; i < pts.size(); ++i) {
-        pts[i] = rs_point{rs.sx[i], rs.sy[i], 0, 0};
+        pts[i] = rs_point{rs.sx[i], (uint32_t)rs.sy[i], 0.f, 0, 0};
         if (i + 1 < pts.size()) {
             const uint64_t dx = rs.sx[i + 1] - rs.sx[i], dy = (uint64_t)(rs.sy[i + 1] - rs.sy[i]);
             // 1 <= dy <= dx, so the quotient is below 2^64
             const uint32_t sh = (uint32_t)__builtin_clzll(dx), up = (uint32_t)__builtin_clzll(dy) - 1;
-            const float rate = (float)((double)dy / (double)dx * 0.25);
-            uint32_t bits = 0;
-            std::memcpy(&bits, &rate, sizeof(bits));
+            pts[i].rate = (float)((double)dy / (double)dx * 0.25);
             pts[i].slope = (uint64_t)(((unsigned __int128)(dy << up) << 64) / (dx << sh));
-            pts[i].code = (uint64_t)bits << 32 | up << 6 | sh;
+            pts[i].code = up << 6 | sh;
         }
     }
     void *pt = nullptr, *pp = nullptr;

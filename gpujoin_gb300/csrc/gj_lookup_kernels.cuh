@@ -258,8 +258,7 @@ __device__ __forceinline__ void stage_cache(uint64_t* dst, const stage_desc& sd)
 // keeps most loads in flight when the column's sectors come from DRAM (2^26
 // probes into 2^26 keys 1568 against 1654 us); several save a block's start
 // where the searches run from L2 (hash table of 2^20 keys 406 against 485 us
-// with 8, key start table 534 against 569 with 4; RadixSpline, whose registers
-// then spill, is level or slower).  Plain lookups take several up to 2^24 keys,
+// with 8, key start table 534 against 569 with 4; RadixSpline is level).  Plain lookups take several up to 2^24 keys,
 // where most sectors still hit L2 (24 M probes with 1 / 4: B+tree, uniform
 // probes 358 / 352 us, Zipf(1.25) 212 / 189), and into a hash table, whose
 // search is one load, at any size (2^26 keys with 1 / 4 / 8: uniform 548 / 559
@@ -274,9 +273,9 @@ constexpr uint64_t kLookupLongKeys =
 // lognormal 1254 / 1185; 2^25 keys, Zipf(0.8), 1224 / 1256), and its ordered
 // pairs of that size take two passes, whose lookup can (1334 / 1261).  Scattered
 // results bind the partitioned lookups of 2^25 probes and more, whose stores
-// come from fewer warps at a time then (67 M into 20 M keys 2205 / 2089 us,
-// RadixSpline of 2^25 keys with 1 / 4 2272 / 2154; 17 M probes, whose results
-// fit L2, into 2^26 keys 385 / 513).
+// come from fewer warps at a time then (67 M into 20 M keys 2205 / 2089 us, 34 M
+// through a RadixSpline of 2^25 keys with 1 / 4 910 / 807; 17 M probes, whose
+// results fit L2, into 2^26 keys 385 / 513).
 constexpr uint64_t kNodeLongKeys = 3ull << 23, kNodeLongProbes = 1ull << 24, kScatterLongProbes = 1ull << 25;
 template <class Op>
 constexpr bool kNodeSearch = std::is_same<Op, op_btree<(int)kBtreeCompressed16>>::value;
@@ -319,11 +318,10 @@ __global__ void __launch_bounds__(kBlock, Op::kMinBlocks) k_lookup(const __grid_
 }
 
 // scattered lookup over a partitioned relation: out[rows[i]] = lookup(keys[i])
-// (a spline's search in a loop needs 40 registers)
 template <class Op>
 constexpr int kScatterLong = std::is_same<Op, op_rs>::value ? 4 : Op::kLong;
 template <class Op, int kIt>
-__global__ void __launch_bounds__(kBlock, std::is_same<Op, op_rs>::value && kIt > 1 ? GJ_BLOCKS(6) : Op::kMinBlocks) k_scatter_lookup(const __grid_constant__ Op op, const stage_desc sd,
+__global__ void __launch_bounds__(kBlock, Op::kMinBlocks) k_scatter_lookup(const __grid_constant__ Op op, const stage_desc sd,
                                                            const uint64_t* __restrict__ keys,
                                                            const uint32_t* __restrict__ rows, uint64_t m,
                                                            uint32_t* __restrict__ out) {
@@ -610,16 +608,8 @@ __device__ __forceinline__ void start_count(uint32_t tile, uint64_t* d_count) {
 // (33.3 M probes from host memory: 2109 us, 1808 with the write put off.)
 // Every look-back ends: it needs the counts of earlier tiles, which their
 // blocks publish before they wait for anything.
-//
-// The spline's search and the loop around it need 40 registers: at the 32 of
-// eight blocks they spill 56 bytes, which long calls feel (67 M probes through a
-// RadixSpline of 2^17 keys, unordered 1650 us, 1462 with six blocks, ordered 1673
-// / 1463) and calls of few items a thread do not (2 M sorted probes into 2^25
-// keys 61 / 69).
-template <class Op, int kIt>
-constexpr int kPairsBlocks = std::is_same<Op, op_rs>::value && kIt == kItems ? GJ_BLOCKS(6) : Op::kMinBlocks;
 template <class Op, bool kOrdered, int kIt>
-__global__ void __launch_bounds__(kBlock, kPairsBlocks<Op, kIt>) k_pairs(const __grid_constant__ Op op, const stage_desc sd, const uint64_t* __restrict__ probes,
+__global__ void __launch_bounds__(kBlock, Op::kMinBlocks) k_pairs(const __grid_constant__ Op op, const stage_desc sd, const uint64_t* __restrict__ probes,
                                                   uint64_t m, uint2* __restrict__ pairs,
                                                   uint64_t* __restrict__ d_count, pairs_ws ws, uint32_t num_tiles) {
     extern __shared__ __align__(16) uint64_t cache[];

@@ -1041,10 +1041,11 @@ GJ_DEVICE_INLINE uint32_t harmonia_lookup_cooperative(bool active, const harmoni
 // the double quotient of the reference's estimate has.
 struct rs_point {
     uint64_t x;
-    double y;        // a position: a whole number below 2^32
+    uint32_t y;      // a position
+    float rate;      // dy / dx / 4: sectors per unit of key
     uint64_t slope;  // floor(dy * 2^(64 + t) / (dx << s)); dx << s in [2^63, 2^64), dy << t in [2^62, 2^63);
                      // 0 for the last point
-    uint64_t code;   // s | t << 6 | the float dy / dx / 4 (sectors per unit of key) << 32
+    uint64_t code;   // s | t << 6
 };
 static_assert(sizeof(rs_point) == 32, "a spline point is one sector");
 
@@ -1060,13 +1061,6 @@ struct rs_view {
     uint32_t pad;
 };
 
-// a whole number below 2^53 held in a double, by its bits: GB300 runs double
-// arithmetic and conversions at a small fraction of its integer rate
-GJ_DEVICE_INLINE uint32_t whole_of_double(uint64_t bits) {
-    const uint32_t e = (uint32_t)(bits >> 52);
-    return e < 1023u ? 0u : (uint32_t)(((bits & ((1ull << 52) - 1)) | (1ull << 52)) >> (1075u - e));
-}
-
 // The spline's estimate of a key's position: y + (key - x) * slope rounded
 // down, in 64-bit fixed point (less than 2^-30 of a position is lost before the
 // rounding).  *rate: the segment's sectors per unit of key.
@@ -1077,15 +1071,14 @@ GJ_DEVICE_INLINE uint32_t rs_estimate(const rs_view& v, uint64_t key, float* rat
     const uint64_t prefix = (key - v.min_key) >> v.shift;
     const uint32_t b = ld_ro(v.table + prefix);
     const uint32_t e = ld_ro(v.table + prefix + 1);
-    // first spline point with x >= key in [b, e); w: the last point read, if
-    // it lies before the key (one point is the usual range)
-    uint32_t lo = b, cnt = e - b, have = 0xFFFFFFFFu;
-    uint64_t w[4];
+    // First spline point with x >= key in [b, e) (one point is the usual range),
+    // by its x alone: a sector kept from the loop in case it is the one saved a
+    // load from L1 and cost the kernels around it their registers (spills of 50
+    // to 60 bytes; 34 M unordered pairs into 2^17 keys 846 us, 721 so).
+    uint32_t lo = b, cnt = e - b;
     while (cnt > 0) {
         const uint32_t step = cnt >> 1, mid = lo + step;
-        ld_sector(reinterpret_cast<const uint64_t*>(v.pts + mid), w);
-        have = mid;
-        if (w[0] < key) {
+        if (ld_ro(&v.pts[mid].x) < key) {
             lo = mid + 1;
             cnt -= step + 1;
         } else {
@@ -1093,10 +1086,11 @@ GJ_DEVICE_INLINE uint32_t rs_estimate(const rs_view& v, uint64_t key, float* rat
         }
     }
     // segment [lo - 1, lo]: its left point and precomputed slope
-    if (have != lo - 1) ld_sector(reinterpret_cast<const uint64_t*>(v.pts + lo - 1), w);
-    *rate = __uint_as_float((uint32_t)(w[3] >> 32));
+    uint64_t w[4];
+    ld_sector(reinterpret_cast<const uint64_t*>(v.pts + lo - 1), w);
+    *rate = __uint_as_float((uint32_t)(w[1] >> 32));
     const uint32_t code = (uint32_t)w[3];
-    return whole_of_double(w[1]) + (uint32_t)(__umul64hi((key - w[0]) << (code & 63u), w[2]) >> ((code >> 6) & 63u));
+    return (uint32_t)w[1] + (uint32_t)(__umul64hi((key - w[0]) << (code & 63u), w[2]) >> (code >> 6));
 }
 
 // lower bound expected inside [b, e) and near `guess`, widened to the whole
