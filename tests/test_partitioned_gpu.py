@@ -193,3 +193,36 @@ def test_range_partition_with_a_larger_workspace(gj, cuda, bits):
         rel = gj.range_partition(keys, 0, max(0, m.bit_length() - bits), bits, workspace=ws)
         assert torch.equal(keys[rel.rows.to(torch.int64)], rel.keys)
         assert torch.equal(torch.sort(rel.rows.to(torch.int64))[0], torch.arange(m, device="cuda"))
+
+
+@pytest.mark.parametrize("prepared", [False, True])
+@pytest.mark.parametrize("aligned", [False, True])
+@pytest.mark.parametrize("kind,params", [("radix_spline", {}), ("btree", {"btree_node_keys": 8})])
+def test_large_windows_of_positions(orc, gj, cuda, kind, params, aligned, prepared):
+    # results in the relation's order (k_part_values): a column on and off the
+    # sector boundary, the directory kept with the index or built for the call,
+    # lower bounds and equal keys, a ragged last block
+    import torch
+
+    m = (1 << 22) + 4097
+    rng = np.random.default_rng(3)
+    col = column(rng, 300_006 if aligned else 300_007)
+    pr = probes_for(rng, col, m)[:m]
+    d_all = to_dev(torch, np.concatenate([np.zeros(4 if aligned else 1, dtype=np.uint64), col]))
+    d_col = d_all[4:] if aligned else d_all[1:]
+    assert (d_col.data_ptr() % 32 == 0) == aligned
+    ix = gj.make_index(kind, **params).construct(None, d_col)
+    if prepared:
+        ix.prepare_partitioned()
+    got, _, _ = ix.partitioned_inlj(to_dev(torch, pr))
+    np.testing.assert_array_equal(from_dev_u32(got), expected(orc, kind, col, pr))
+
+
+def test_large_windows_of_a_no_op_index(gj, cuda):
+    # a window and a column large enough not to take the plain lookup
+    import torch
+
+    keys = gj.generate_sorted_keys((1 << 25) + 64, 0, 1 << 63, seed=3)
+    probes = gj.generate_probes(keys, 3 << 24, theta=0.5, seed=4)
+    got, _, _ = gj.make_index("no_op").construct(None, keys).partitioned_inlj(probes)
+    assert bool((got == -1).all())
