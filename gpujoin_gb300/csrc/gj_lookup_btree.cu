@@ -5,12 +5,12 @@ namespace gj {
 
 template <>
 int lookup_call_btree<4>(const gj_index* idx, const lookup_call& c) {
-    return run_call(op_btree<4>{idx->bt}, idx, c);
+    return plain_nodes_call<4>(idx, c);
 }
 
 template <>
 int lookup_call_btree<8>(const gj_index* idx, const lookup_call& c) {
-    return run_call(op_btree<8>{idx->bt}, idx, c);
+    return plain_nodes_call<8>(idx, c);
 }
 
 }  // namespace gj

@@ -5,17 +5,17 @@ namespace gj {
 
 template <>
 int lookup_call_btree<16>(const gj_index* idx, const lookup_call& c) {
-    return run_call(op_btree<16>{idx->bt}, idx, c);
+    return plain_nodes_call<16>(idx, c);
 }
 
 template <>
 int lookup_call_btree<32>(const gj_index* idx, const lookup_call& c) {
-    return run_call(op_btree<32>{idx->bt}, idx, c);
+    return plain_nodes_call<32>(idx, c);
 }
 
 template <>
 int lookup_call_btree<64>(const gj_index* idx, const lookup_call& c) {
-    return run_call(op_btree<64>{idx->bt}, idx, c);
+    return plain_nodes_call<64>(idx, c);
 }
 
 }  // namespace gj

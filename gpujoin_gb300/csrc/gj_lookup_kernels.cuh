@@ -96,7 +96,7 @@ struct stage_desc {
 // and touch a slice of the tree, use the default class.
 struct op_bs {
     static constexpr int kMinBlocks = GJ_BLOCKS(8);
-    static constexpr int kLong = 4;
+    static constexpr int kLong = 8;
     static constexpr bool kStaged = true;
     bs_view v;
     template <bool kScattered = true>
@@ -125,23 +125,33 @@ struct op_start {
     __device__ __forceinline__ uint32_t operator()(const uint64_t* cache, uint64_t key) const { return lookup(cache, key); }
 };
 // Trees: a scattered lookup starts at its bucket's entry of the start table,
-// nearly always below the levels that fit shared memory, so only the sorted
-// tiles (whose common node is searched from the root) stage them; the kernels
-// without them keep the room for L1 and have nothing to load before the
-// first probe.
+// over large columns nearly always below the levels that fit shared memory, so
+// there only the sorted tiles (whose common node is searched from the root)
+// stage them; the kernels without them keep the room for L1 and have nothing to
+// load before the first probe.  kSm (plain nodes over up to kStageKeys keys):
+// blocks of several probes a thread stage them, as all or most levels of such a
+// tree lie there (6 M probes through nodes of 8 keys: 4096 keys 90 us, 118
+// unstaged, 2^16 keys 115 / 137; from 2^20 on the room is worth more to L1, 34 M
+// unordered pairs through nodes of 4 keys over 2^22 keys 1.47 times as long);
+// those of one probe a thread would pay for it at every block and do not.
 //
 // Sorted tiles: an op with a tile_hint searches once per tile for what all
 // keys of the tile's range share (for the B+tree: the deepest node on every
 // path) and starts each probe's search there.
-template <int W>
+template <int W, bool kSm = false>
 struct op_btree {
     static constexpr int kMinBlocks = GJ_BLOCKS(8);
     static constexpr int kLong = 8;
-    static constexpr bool kStaged = false;
+    static constexpr bool kStaged = kSm;
     btree_view v;
     template <bool kScattered = true>
     __device__ __forceinline__ uint32_t lookup(const uint64_t* cache, uint64_t key) const {
-        return btree_lookup<W, kScattered, false>(v, cache, key);
+        return btree_lookup<W, kScattered, kSm>(v, cache, key);
+    }
+    op_btree unstaged() const {
+        op_btree o = *this;
+        o.v.cached_levels = 0;
+        return o;
     }
     __device__ __forceinline__ uint32_t operator()(const uint64_t* cache, uint64_t key) const { return lookup(cache, key); }
     using tile_hint = btree_cursor;
@@ -152,6 +162,12 @@ struct op_btree {
         return btree_lookup_from<W, false>(v, cache, key, h);
     }
 };
+
+template <class Op>
+struct is_tree_nodes : std::false_type {};
+template <int W, bool kSm>
+struct is_tree_nodes<op_btree<W, kSm>> : std::true_type {};
+constexpr uint64_t kStageKeys = 1ull << 18;
 
 struct no_tile_hint {};
 template <class Op, class = void>
@@ -278,10 +294,18 @@ constexpr uint64_t kLookupLongKeys =
 // results fit L2, into 2^26 keys 385 / 513).
 constexpr uint64_t kNodeLongKeys = 3ull << 23, kNodeLongProbes = 1ull << 24, kScatterLongProbes = 1ull << 25;
 template <class Op>
-constexpr bool kNodeSearch = std::is_same<Op, op_btree<(int)kBtreeCompressed16>>::value;
+constexpr bool kNodeSearch = is_tree_nodes<Op>::value;
 template <class Op>
 bool nodes_long(uint64_t n, uint64_t m) {
     return kNodeSearch<Op> && n <= kNodeLongKeys && m >= kNodeLongProbes;
+}
+// their ordered pairs up to 2^24 keys take the two passes as soon as the lookup
+// does (6 M pairs, nodes of 15 keys over leaves of 8, 2^20 clustered keys: 894 us
+// in one pass, 714 in two; nodes of 8 over 4096 keys 160 / 110)
+template <class Op>
+bool nodes_two_passes(uint64_t n, uint64_t m, int sm_count) {
+    return nodes_long<Op>(n, m) ||
+           (kNodeSearch<Op> && n <= (1ull << 24) && m >= 16ull * sm_count * 8 * kBlock);
 }
 inline int long_blocks(uint64_t n, uint64_t m, bool* yes, uint64_t keys = kL2Keys) {
     device_info di;
@@ -918,17 +942,47 @@ int grid_for(Kernel kernel, size_t smem, uint64_t work_items, int* grid) {
     return GJ_OK;
 }
 
+// What a lookup launch of items probes a thread stages, and the op that goes
+// with it: a tree's levels where blocks are long, a fence always.
+template <class Op>
+struct staging_choice {
+    Op op;
+    stage_desc sd;
+    size_t bytes;
+};
+template <class Op, class = void>
+struct stages_always : std::true_type {};
+template <class Op>
+struct stages_always<Op, std::void_t<decltype(std::declval<Op>().unstaged())>> : std::false_type {};
+// A fence is 32 KB a block, from host memory where the index lies there, so its
+// blocks are long from kFenceLongProbes on (index of 2^20 keys in host memory,
+// 2048- / 256-probe blocks: 2 M probes 217 / 274 us, 120,000 42 / 40).
+template <class Op>
+constexpr bool fence_staged = Op::kStaged && stages_always<Op>::value;
+constexpr uint64_t kFenceLongProbes = 1ull << 18;
+template <class Op>
+staging_choice<Op> staging(const Op& op, const stage_desc& sd, int items) {
+    if constexpr (!stages_always<Op>::value) {
+        if (Op::kStaged && items == 1) return {op.unstaged(), stage_desc{}, 0};
+    }
+    return {op, sd, Op::kStaged ? stage_bytes(sd) : 0};
+}
+
 template <class Op>
 int run_lookup(const Op& op, const stage_desc& sd, uint64_t n, const uint64_t* probes, uint64_t m, uint32_t* out,
                cudaStream_t s, unsigned long long* clear = nullptr, uint32_t words = 0) {
-    const size_t smem = Op::kStaged ? stage_bytes(sd) : 0;
     auto launch = [&](auto kernel, int items) {
-        GJ_TRY(kernel_staged(kernel, smem));
+        const auto st = staging(op, sd, items);
+        GJ_TRY(kernel_staged(kernel, st.bytes));
         const uint64_t tile = (uint64_t)kBlock * items;
-        kernel<<<(unsigned)((m + tile - 1) / tile), kBlock, smem, s>>>(op, sd, probes, m, out, clear, words);
+        kernel<<<(unsigned)((m + tile - 1) / tile), kBlock, st.bytes, s>>>(st.op, st.sd, probes, m, out, clear, words);
         GJ_CUDA_TRY(cudaGetLastError());
         return (int)GJ_OK;
     };
+    if constexpr (fence_staged<Op>) {
+        if (m >= kFenceLongProbes)
+            return clear ? launch(k_lookup<Op, Op::kLong, true>, Op::kLong) : launch(k_lookup<Op, Op::kLong>, Op::kLong);
+    }
     if (clear) return launch(k_lookup<Op, 1, true>, 1);
     bool full = false;
     GJ_TRY(long_blocks(n, m, &full, kLookupLongKeys<Op>));
@@ -951,18 +1005,19 @@ int run_sorted_lookup(const Op& op, const stage_desc& sd, const uint64_t* probes
 template <class Op>
 int run_scatter(const Op& op, const stage_desc& sd, uint64_t n, const uint64_t* keys, const uint32_t* rows,
                 uint64_t m, uint32_t* out, cudaStream_t s) {
-    const size_t smem = Op::kStaged ? stage_bytes(sd) : 0;
     auto launch = [&](auto kernel, int items) {
-        GJ_TRY(kernel_staged(kernel, smem));
+        const auto st = staging(op, sd, items);
+        GJ_TRY(kernel_staged(kernel, st.bytes));
         const uint64_t tile = (uint64_t)kBlock * items;
-        kernel<<<(unsigned)((m + tile - 1) / tile), kBlock, smem, s>>>(op, sd, keys, rows, m, out);
+        kernel<<<(unsigned)((m + tile - 1) / tile), kBlock, st.bytes, s>>>(st.op, st.sd, keys, rows, m, out);
         GJ_CUDA_TRY(cudaGetLastError());
         return (int)GJ_OK;
     };
     bool full = false;
     if (std::is_same<Op, op_rs>::value) full = m >= kScatterLongProbes;
     else GJ_TRY(long_blocks(n, m, &full, std::is_same<Op, op_learned>::value ? UINT64_MAX : kL2Keys));
-    full |= kNodeSearch<Op> && n <= (1ull << 25) && m >= kScatterLongProbes;
+    full |= (kNodeSearch<Op> && n <= (1ull << 25) && m >= kScatterLongProbes) ||
+            (fence_staged<Op> && m >= kFenceLongProbes);
     return full ? launch(k_scatter_lookup<Op, kScatterLong<Op>>, kScatterLong<Op>) : launch(k_scatter_lookup<Op, 1>, 1);
 }
 
@@ -982,7 +1037,9 @@ int run_pairs(const Op& op, const stage_desc& sd, uint64_t n, const uint64_t* pr
         return GJ_OK;
     }
     if (spin_limit) pw.spin_limit = spin_limit;
-    const bool longs = nodes_long<Op>(n, m);
+    device_info di;
+    GJ_TRY(current_device_info(&di));
+    const bool longs = nodes_two_passes<Op>(n, m, di.sm_count);
     const bool two_passes = stash && (m < kSinglePassMin || host_index || longs);
     // the state lies in whole 64-bit words at the head of the workspace
     if (two_passes && !longs) {
@@ -1002,12 +1059,14 @@ int run_pairs(const Op& op, const stage_desc& sd, uint64_t n, const uint64_t* pr
         GJ_CUDA_TRY(cudaGetLastError());
         return GJ_OK;
     }
-    const size_t smem = Op::kStaged ? stage_bytes(sd) : 0;
+    // (the tiles of ordered pairs leave no room for a tree's levels beside L1)
+    const auto st = staging(op, sd, unordered ? kItems : 1);
     auto single = [&](auto kernel, uint32_t items) {
         const uint32_t num_tiles = (uint32_t)((m + kBlock * items - 1) / (kBlock * items));
         int grid = 0;
-        GJ_TRY(grid_for(kernel, smem, (uint64_t)num_tiles * kBlock, &grid));
-        kernel<<<grid, kBlock, smem, s>>>(op, sd, probes, m, reinterpret_cast<uint2*>(pairs), d_count, pw, num_tiles);
+        GJ_TRY(grid_for(kernel, st.bytes, (uint64_t)num_tiles * kBlock, &grid));
+        kernel<<<grid, kBlock, st.bytes, s>>>(st.op, st.sd, probes, m, reinterpret_cast<uint2*>(pairs), d_count, pw,
+                                              num_tiles);
         GJ_CUDA_TRY(cudaGetLastError());
         return (int)GJ_OK;
     };
@@ -1063,6 +1122,14 @@ int run_call(const Op& op, const gj_index* idx, const lookup_call& c) {
     }
     set_error("probe kernels: unknown action");
     return GJ_ERR_INVALID_ARGUMENT;
+}
+
+// trees of plain nodes: sorted tiles stage their levels by themselves
+template <int W>
+int plain_nodes_call(const gj_index* idx, const lookup_call& c) {
+    const bool sorted = c.action == lookup_action::sorted_pairs || c.action == lookup_action::sorted_positions;
+    if (idx->n <= kStageKeys && !sorted) return run_call(op_btree<W, true>{idx->bt}, idx, c);
+    return run_call(op_btree<W>{idx->bt}, idx, c);
 }
 
 }  // namespace

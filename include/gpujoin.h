@@ -88,8 +88,8 @@ typedef struct gj_index_params {
     uint32_t rs_max_error;      /* RadixSpline spline error (default 32) */
     uint32_t bs_cache_keys;     /* binary search: sampled keys staged in shared memory where no key start table
                                    serves the lookup (index in host memory) (default 4096, 0 = off) */
-    uint32_t smem_cache_bytes;  /* B+tree: upper levels staged in shared memory by the sorted-tile kernels
-                                   (default 16384) */
+    uint32_t smem_cache_bytes;  /* B+tree: upper levels staged in shared memory by the sorted-tile kernels and,
+                                   where no key start table serves the lookup, by long calls (default 16384) */
     uint32_t learned_leaves;    /* learned index: linear leaf models (default 0: about 128 keys per leaf, a
                                    power of two in [2^10, 2^20]) */
     uint32_t learned_root;      /* GJ_LEARNED_ROOT_LINEAR, _MLP, _SEGMENTS or _AUTO (default AUTO) */

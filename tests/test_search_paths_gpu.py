@@ -142,3 +142,56 @@ def test_long_calls_through_network_roots(orc, gj, cuda, hidden, n, m):
     out = torch.empty(m, dtype=torch.int32, device="cuda")
     ix.partitioned_lookup(rel.keys, rel.rows, out)
     np.testing.assert_array_equal(from_dev_u32(out), exp)
+
+
+@pytest.mark.parametrize("W,L", [(4, 4), (7, 4), (8, 8), (15, 8), (16, 16), (32, 8), (64, 32)])
+@pytest.mark.parametrize("n", [4096, 300_007, (1 << 24) + 64])
+def test_long_calls_stage_tree_levels(orc, gj, cuda, W, L, n):
+    # node formats without a key start table: blocks of several probes a thread
+    # stage the upper levels, those of one search without them -- whole trees in
+    # shared memory, and the top of larger ones
+    import torch
+
+    m = 5_000_011
+    keys = gj.generate_sorted_keys(n, gj.DIST_UNIFORM, 1 << 63, seed=5)
+    probes = gj.generate_probes(keys, m, theta=0.5, absent_fraction=0.1, seed=6)
+    exp = orc.exact_lookup(keys.cpu().numpy().view(np.uint64), probes.cpu().numpy().view(np.uint64))
+    ix = gj.btree_index(btree_node_keys=W, btree_leaf_keys=L).construct(None, keys)
+    np.testing.assert_array_equal(from_dev_u32(ix.lookup(probes)), exp)
+    np.testing.assert_array_equal(from_dev_u32(ix.lookup(probes[:1001])), exp[:1001])
+    rel = gj.range_partition(probes, int(keys[0]), 55, 8)
+    out = torch.empty(m, dtype=torch.int32, device="cuda")
+    ix.partitioned_lookup(rel.keys, rel.rows, out)
+    np.testing.assert_array_equal(from_dev_u32(out), exp)
+    rows, pos = orc.pairs_from_positions(exp)
+    for ordered in (True, False):
+        prs, cnt = ix.inlj_pairs(probes, ordered=ordered)
+        got = prs[: 2 * int(cnt)].cpu().numpy().view(np.uint32).reshape(-1, 2)
+        if not ordered:
+            got = got[np.argsort(got[:, 0], kind="stable")]
+        np.testing.assert_array_equal(got[:, 0], rows)
+        np.testing.assert_array_equal(got[:, 1], pos)
+
+
+@pytest.mark.parametrize("m", [1, (1 << 18) - 1, 1 << 18, (1 << 18) + 2049])
+def test_fence_in_host_memory(orc, gj, cuda, m):
+    # a binary search whose sampled keys lie in host memory: lookups, ordered
+    # pairs (two passes) and partitioned lookups around the size of long blocks
+    import torch
+
+    rng = np.random.default_rng(m)
+    col = column(rng, 70_001)
+    pr = probes_for(rng, col, m)[:m]
+    exp = orc.bs_lookup(col, pr)
+    ix = gj.binary_search_index(index_memory=gj.INDEX_MEMORY_HOST).construct(None, to_dev(torch, col))
+    d_pr = to_dev(torch, pr)
+    np.testing.assert_array_equal(from_dev_u32(ix.lookup(d_pr)), exp)
+    prs, cnt = ix.inlj_pairs(d_pr)
+    got = prs[: 2 * int(cnt)].cpu().numpy().view(np.uint32).reshape(-1, 2)
+    rows, pos = orc.pairs_from_positions(exp)
+    np.testing.assert_array_equal(got[:, 0], rows)
+    np.testing.assert_array_equal(got[:, 1], pos)
+    rel = gj.range_partition(d_pr, int(col[0]), 55, 8)
+    out = torch.empty(m, dtype=torch.int32, device="cuda")
+    ix.partitioned_lookup(rel.keys, rel.rows, out)
+    np.testing.assert_array_equal(from_dev_u32(out), exp)
