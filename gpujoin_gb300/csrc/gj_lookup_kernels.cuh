@@ -131,8 +131,9 @@ struct op_start {
 // load before the first probe.  kSm (plain nodes over up to kStageKeys keys):
 // blocks of several probes a thread stage them, as all or most levels of such a
 // tree lie there (6 M probes through nodes of 8 keys: 4096 keys 90 us, 118
-// unstaged, 2^16 keys 115 / 137; from 2^20 on the room is worth more to L1, 34 M
-// unordered pairs through nodes of 4 keys over 2^22 keys 1.47 times as long);
+// unstaged, 2^16 keys of Zipf(1.25) 116 / 137, uniform 131 / 133; from 2^20 on the
+// room is worth more to L1, 34 M unordered pairs through nodes of 4 keys over 2^22
+// keys 984 / 676);
 // those of one probe a thread would pay for it at every block and do not.
 //
 // Sorted tiles: an op with a tile_hint searches once per tile for what all
@@ -300,8 +301,8 @@ bool nodes_long(uint64_t n, uint64_t m) {
     return kNodeSearch<Op> && n <= kNodeLongKeys && m >= kNodeLongProbes;
 }
 // their ordered pairs up to 2^24 keys take the two passes as soon as the lookup
-// does (6 M pairs, nodes of 15 keys over leaves of 8, 2^20 clustered keys: 894 us
-// in one pass, 714 in two; nodes of 8 over 4096 keys 160 / 110)
+// does (6 M pairs, nodes of 15 keys over leaves of 8, 2^20 clustered keys, Zipf(1.25):
+// 878 us in one pass, 702 in two; nodes of 8 over 4096 keys 163 / 110)
 template <class Op>
 bool nodes_two_passes(uint64_t n, uint64_t m, int sm_count) {
     return nodes_long<Op>(n, m) ||
